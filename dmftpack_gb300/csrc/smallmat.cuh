@@ -315,6 +315,31 @@ __device__ inline void block_matmul(int n, const double2 *A, const double2 *B, d
     __syncthreads();
 }
 
+// Is the Hermitian matrix whose lower triangle is in A (n x n, column-major, shared or global, this warp's) positive
+// definite?  Cholesky by one warp, L left in the lower triangle; all 32 lanes call it, the answer is warp-uniform.
+__device__ inline bool warp_cholesky(int n, double2 *A) {
+    const int lane = threadIdx.x & 31;
+    for (int j = 0; j < n; j++) {
+        const double p = DG_AT(A, n, j, j).x;
+        if (!(p > 0.0)) return false;
+        const double r = 1.0 / sqrt(p);
+        __syncwarp();
+        if (lane == 0) DG_AT(A, n, j, j) = cmk(p * r, 0.0);
+        for (int i = j + 1 + lane; i < n; i += 32) DG_AT(A, n, i, j) = cscale(DG_AT(A, n, i, j), r);
+        __syncwarp();
+        const int c = n - j - 1;
+        for (int e = lane; e < c * c; e += 32) {
+            const int i = j + 1 + e % c, k = j + 1 + e / c;
+            if (i < k) continue;
+            double2 v = csub(DG_AT(A, n, i, k), cmul(DG_AT(A, n, i, j), cconj(DG_AT(A, n, k, j))));
+            if (i == k) v.y = 0.0;
+            DG_AT(A, n, i, k) = v;
+        }
+        __syncwarp();
+    }
+    return true;
+}
+
 // Cholesky test of one n x n Hermitian matrix held as its lower triangle in t[idx(i, j)] (i >= j), with
 // t[idx] = tri[(idx) * stride] (stride = threads sharing the interleaved shared array).  Destroys t.
 // strict: positive definite; else positive semidefinite (an exactly zero pivot with an exactly zero

@@ -59,6 +59,30 @@ CASES = {
 }
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("D,nf,green", [(1, 20, False), (2, 33, False), (7, 64, False), (20, 65, False), (33, 40, False),
+                                        (46, 24, False), (2, 8600, False), (1, 20, True), (11, 97, True),
+                                        (46, 24, True), (2, 8600, True)])
+def test_moments_edges(ctx, orc, D, nf, green):
+    """Smallest and ragged N_freq, N_freq beyond the staged sums, matrices beyond the gates' shared memory.  The moments
+    describe the tail beyond the data: it is compared there, relative to its size.  Bound: the fits' 2 x 2 normal
+    matrices over a window of a tenth of the axis amplify the rounding of sums of nf terms by ~1e3: 2e-16 1e3 sqrt(nf)
+    < 2e-11, with a factor 5 for the extrapolation."""
+    rng = np.random.default_rng([D, nf])
+    w = np.pi * (2 * np.arange(nf) + 1) / 30.0
+    if green:
+        A = rng.normal(size=(D, D)) + 1j * rng.normal(size=(D, D))
+        F = np.linalg.inv(1j * w[:, None, None] * np.eye(D) - (A + A.conj().T) / (2 * np.sqrt(D)))
+    else:
+        F = np.zeros((nf, D, D), complex)
+        F[:, np.arange(D), np.arange(D)] = -1j * rng.uniform(0.4, 0.6, D) / (w[:, None] + rng.uniform(0.8, 1.2, D))
+    x = 1j * np.pi * (2 * np.array([nf, 2 * nf, 4 * nf]) + 1) / 30.0
+    tail = lambda m: sum(m[i][None] / x[:, None, None] ** i for i in range(4))
+    a, b = tail(ctx.getAsymto_moments(F, 30.0, greenFtnAsym=green)), tail(orc.moments(F, 30.0, green_asym=green))
+    for p, q in zip(a, b):
+        assert np.abs(p - q).max() <= 1e-10 * np.abs(q).max()
+
+
 @pytest.mark.parametrize("explicit", [False, True])
 @pytest.mark.parametrize("case", list(CASES))
 def test_greenftn_w_matches_oracle(ctx, orc, case, explicit):
