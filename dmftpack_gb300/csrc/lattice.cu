@@ -312,32 +312,52 @@ int launch_schur_prep(dmftgpu_ctx *ctx, cudaStream_t s, int nk, int n, int D, co
 }
 
 // Fermi parts: occ_k = P U f U^H P (with the +-100 cut-offs of src/GreenFtn.cpp:314-316) for NumMatrix,
-// and sum_l f, beta f (1-f) for N(mu) (src/GreenFtn.cpp:616-620, no cut-off there)
-__global__ void k_fermi(int nk, int n, int D, double beta, double mu, const double *__restrict__ eps,
-                        const double2 *__restrict__ UP, double2 *occ, double *fs) {
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= nk) return;
-    double fsum = 0, dfsum = 0;
-    for (int l = 0; l < n; l++) {
-        double e = eps[(size_t)k * n + l];
-        double f = 1. / (1 + exp(beta * (e - mu)));
-        fsum += f;
-        dfsum += beta * f * (1 - f);
+// and sum_l f, beta f (1-f) for N(mu) (src/GreenFtn.cpp:616-620, no cut-off there).  A CTA takes kb k points, forms
+// their Fermi factors once in shared memory and spreads the elements a <= b of occ_k over its threads; it is bound by
+// the FP64 products (n D^2 complex ones per k).  One thread per k with an exponential per element and level took
+// 2.2 ms at n = 28, D = 10, 1000 k; this takes 33 us.
+constexpr int FERMI_THREADS = 128;
+inline int fermi_kb(int n, int D) { return std::max(1, FERMI_THREADS / std::max(n, D * (D + 1) / 2)); }
+__global__ void __launch_bounds__(FERMI_THREADS) k_fermi(int nk, int n, int D, int kb, double beta, double mu,
+                                                         const double *__restrict__ eps,
+                                                         const double2 *__restrict__ UP, double2 *occ, double *fs) {
+    extern __shared__ double fsh[];  // [kb][n] f without and then with the cut-offs
+    const int k0 = blockIdx.x * kb, nkb = min(kb, nk - k0);
+    double *fc = fsh + kb * n;
+    for (int t = threadIdx.x; t < nkb * n; t += FERMI_THREADS) {
+        const double x = beta * (eps[(size_t)k0 * n + t] - mu), f = 1. / (1 + exp(x));
+        fsh[t] = f;
+        fc[t] = x > 100.0 ? 0.0 : (x < -100.0 ? 1.0 : f);
     }
-    fs[2 * k] = fsum;
-    fs[2 * k + 1] = dfsum;
-    if (!occ) return;
-    for (int b = 0; b < D; b++)
-        for (int a = 0; a < D; a++) {
-            double2 s = cmk(0, 0);
-            for (int l = 0; l < n; l++) {
-                double x = beta * (eps[(size_t)k * n + l] - mu);
-                double f = x > 100.0 ? 0.0 : (x < -100.0 ? 1.0 : 1. / (1. + exp(x)));
-                const double2 *u = UP + ((size_t)k * n + l) * D;
-                s = cadd(s, cscale(cmulc(u[a], u[b]), f));
-            }
-            occ[(size_t)k * D * D + a + b * D] = s;
+    __syncthreads();
+    for (int k = threadIdx.x; k < nkb; k += FERMI_THREADS) {
+        double fsum = 0, dfsum = 0;
+        for (int l = 0; l < n; l++) {
+            const double f = fsh[k * n + l];
+            fsum += f;
+            dfsum += beta * f * (1 - f);
         }
+        fs[2 * (k0 + k)] = fsum;
+        fs[2 * (k0 + k) + 1] = dfsum;
+    }
+    if (!occ) return;
+    const int P = D * (D + 1) / 2;
+    for (int t = threadIdx.x; t < nkb * P; t += FERMI_THREADS) {
+        const int k = t / P;
+        int a = 0, b = t % P;  // pair of the row-major upper triangle
+        while (b >= D - a) {
+            b -= D - a;
+            a++;
+        }
+        b += a;
+        const double2 *u = UP + (size_t)(k0 + k) * n * D;
+        double2 s = cmk(0, 0);
+#pragma unroll 4
+        for (int l = 0; l < n; l++) s = cadd(s, cscale(cmulc(u[(size_t)l * D + a], u[(size_t)l * D + b]), fc[k * n + l]));
+        double2 *o = occ + (size_t)(k0 + k) * D * D;
+        o[a + b * D] = s;
+        if (a != b) o[b + a * D] = cconj(s);
+    }
 }
 
 // G_loc, GwHF (src/GreenFtn.cpp:298-305, 371-383): scale the per-frequency k sums, keep within-cluster blocks
@@ -354,18 +374,22 @@ __global__ void k_gloc_scale(int Nf, int nk, int D, int nh, const double2 *blk, 
 }
 
 // NumMatrix (src/GreenFtn.cpp:283-290, 322-354): one CTA per element, fixed-order tree reductions over the
-// 2 N_freq frequency sums and the N_k Fermi terms
-__global__ void k_nummat(int Nf, int nk, int D, double beta, const double2 *blk, const double2 *blk0,
+// 2 N_freq frequency sums and the N_k Fermi terms.  Latency-bound (D^2 CTAs of short strided sums): 1024 threads and
+// unrolled loads take 38 us at D = 3, N_freq = 4096, 13824 k (256 threads: 75 us)
+constexpr int NUM_THREADS = 1024;
+__global__ void __launch_bounds__(NUM_THREADS) k_nummat(int Nf, int nk, int D, double beta, const double2 *blk, const double2 *blk0,
                          const double2 *occ, double2 *nummat) {
-    __shared__ double2 r0[256], r1[256], r2[256];
+    __shared__ double2 r0[NUM_THREADS], r1[NUM_THREADS], r2[NUM_THREADS];
     const int DD = D * D, e = blockIdx.x;
     const int a = e % D, b = e / D, et = b + a * D;
     double2 s = cmk(0, 0), s0 = cmk(0, 0), o = cmk(0, 0);
-    for (int f = threadIdx.x; f < 2 * Nf; f += blockDim.x) {
+#pragma unroll 4
+    for (int f = threadIdx.x; f < 2 * Nf; f += NUM_THREADS) {
         s = cadd(s, cadd(blk[(size_t)f * DD + e], cconj(blk[(size_t)f * DD + et])));
         s0 = cadd(s0, cadd(blk0[(size_t)f * DD + e], cconj(blk0[(size_t)f * DD + et])));
     }
-    for (int k = threadIdx.x; k < nk; k += blockDim.x) o = cadd(o, occ[(size_t)k * DD + e]);
+#pragma unroll 8
+    for (int k = threadIdx.x; k < nk; k += NUM_THREADS) o = cadd(o, occ[(size_t)k * DD + e]);
     r0[threadIdx.x] = s;
     r1[threadIdx.x] = s0;
     r2[threadIdx.x] = o;
@@ -392,16 +416,19 @@ __global__ void k_nummat(int Nf, int nk, int D, double beta, const double2 *blk,
     }
 }
 
-// single CTA: N(mu) = (2/beta sum tr + sum f)/nk and dN/dmu
-__global__ void k_nele_finalize(int nf2, int nk, double beta, const double *tr, const double *dtr, const double *fs,
+// single CTA: N(mu) = (2/beta sum tr + sum f)/nk and dN/dmu; latency-bound like k_nummat (8192 points and 4096 k:
+// 22 us with 256 threads, 11.6 us now)
+__global__ void __launch_bounds__(NUM_THREADS) k_nele_finalize(int nf2, int nk, double beta, const double *tr, const double *dtr, const double *fs,
                                 int deriv, double *out) {
-    __shared__ double red[4][256];
+    __shared__ double red[4][NUM_THREADS];
     double a = 0, b = 0, c = 0, d = 0;
-    for (int f = threadIdx.x; f < nf2; f += blockDim.x) {
+#pragma unroll 4
+    for (int f = threadIdx.x; f < nf2; f += NUM_THREADS) {
         a += tr[f];
         if (deriv) b += dtr[f];
     }
-    for (int k = threadIdx.x; k < nk; k += blockDim.x) {
+#pragma unroll 4
+    for (int k = threadIdx.x; k < nk; k += NUM_THREADS) {
         c += fs[2 * k];
         d += fs[2 * k + 1];
     }
@@ -786,6 +813,15 @@ int run_schur(dmftgpu_ctx *ctx, const Prepared &P, int mode, double mu, int wgri
     return DMFTGPU_OK;
 }
 
+// the Fermi parts of a prepared lattice at mu (occ may be nullptr)
+int launch_fermi(dmftgpu_ctx *ctx, const Prepared &P, double mu, double2 *occ, double *fs) {
+    const int kb = fermi_kb(P.n, P.D);
+    k_fermi<<<dg_ceil_div(P.nk, kb), FERMI_THREADS, 2 * (size_t)kb * P.n * sizeof(double), ctx->stream>>>(
+        P.nk, P.n, P.D, kb, P.beta, mu, P.eps, P.UP, occ, fs);
+    DG_LAUNCH(ctx, "k_fermi");
+    return DMFTGPU_OK;
+}
+
 // one N(mu) evaluation on a prepared lattice; result (N, dN/dmu) in device out[2]
 int nele_pass(dmftgpu_ctx *ctx, const Prepared &P, double mu, bool deriv, double *dout, bool explicit_inv,
               bool mixed) {
@@ -819,9 +855,8 @@ int nele_pass(dmftgpu_ctx *ctx, const Prepared &P, double mu, bool deriv, double
                          mixed));
     }
     DG_CUDA(cudaStreamWaitEvent(ctx->stream, P.static_ready, 0));
-    k_fermi<<<dg_ceil_div(P.nk, 128), 128, 0, ctx->stream>>>(P.nk, P.n, P.D, P.beta, mu, P.eps, P.UP, nullptr, fs);
-    DG_LAUNCH(ctx, "k_fermi");
-    k_nele_finalize<<<1, 256, 0, ctx->stream>>>(nf2, P.nk, P.beta, tr, dtr, fs, deriv ? 1 : 0, dout);
+    DG_TRY(launch_fermi(ctx, P, mu, nullptr, fs));
+    k_nele_finalize<<<1, NUM_THREADS, 0, ctx->stream>>>(nf2, P.nk, P.beta, tr, dtr, fs, deriv ? 1 : 0, dout);
     DG_LAUNCH(ctx, "k_nele_finalize");
     return DMFTGPU_OK;
 }
@@ -952,11 +987,10 @@ int greenftn_w_dev(dmftgpu_ctx *ctx, const dmftgpu_lattice *L, const double2 *dH
         DG_TRY(run_gloc(ctx, P, M_BLOCK, mu, 0, blk, blk0, nullptr, nullptr, (flags & DMFTGPU_MIXED) != 0));
     else DG_TRY(run_schur(ctx, P, dg::S_BLOCK, mu, 0, blk, blk0, nullptr, nullptr, (flags & DMFTGPU_MIXED) != 0));
     DG_CUDA(cudaStreamWaitEvent(ctx->stream, P.static_ready, 0));
-    k_fermi<<<dg_ceil_div(L->nk, 128), 128, 0, ctx->stream>>>(L->nk, L->n, D, L->beta, mu, P.eps, P.UP, occ, fs);
-    DG_LAUNCH(ctx, "k_fermi");
+    DG_TRY(launch_fermi(ctx, P, mu, occ, fs));
     k_gloc_scale<<<dg_ceil_div((long long)Nf * DD, 256), 256, 0, ctx->stream>>>(Nf, L->nk, D, L->nh, blk, blk0, dG, dG0);
     DG_LAUNCH(ctx, "k_gloc_scale");
-    k_nummat<<<(int)DD, 256, 0, ctx->stream>>>(Nf, L->nk, D, L->beta, blk, blk0, occ, dN);
+    k_nummat<<<(int)DD, NUM_THREADS, 0, ctx->stream>>>(Nf, L->nk, D, L->beta, blk, blk0, occ, dN);
     DG_LAUNCH(ctx, "k_nummat");
     return DMFTGPU_OK;
 }
