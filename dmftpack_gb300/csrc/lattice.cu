@@ -536,9 +536,12 @@ int prepare_real(dmftgpu_ctx *ctx, const dmftgpu_lattice *L, const double2 *dH, 
 
 // df (the DMFTGPU_MIXED passes): the per-k eigendecompositions (n <= 32) in double-float on the FP32 pipe, and the
 // static one on the main stream after the Schur data instead of on the side stream (the mixed lattice kernels fill
-// the SMs; an eigendecomposition beside them slows them by more than it takes alone)
+// the SMs; an eigendecomposition beside them slows them by more than it takes alone).
+// derivs (dmftgpu_gloc_vjp / _jvp): only the Schur data and Sigma(iw_n), n < N_freq, enter the derivatives of G_loc;
+// the tail moments, the 2 N_freq table and the static spectrum (10.5 ms of a 5^3 k call of the 56-orbital model, in
+// front of a 60-70 ms derivative kernel) are left out.
 int prepare(dmftgpu_ctx *ctx, const dmftgpu_lattice *L, const double2 *dH, const double2 *dS, int mask, Prepared &P,
-            bool vectors = false, bool df = false) {
+            bool vectors = false, bool df = false, bool derivs = false) {
     P.n = L->n;
     P.nk = L->nk;
     P.Nf = L->nfreq;
@@ -593,6 +596,13 @@ int prepare(dmftgpu_ctx *ctx, const dmftgpu_lattice *L, const double2 *dH, const
         P.Vq = (double2 *)dg_buf(ctx, "lat.Vq", (size_t)nk * (m * m + 1) * sizeof(double2));
         P.Uf = (double2 *)dg_buf(ctx, "lat.Uf", (size_t)nk * n * n * sizeof(double2));
         if (!P.Vq || !P.Uf) return DMFTGPU_NOMEM;
+    }
+    if (derivs) {
+        // the sizes the moment fit of the other passes accepts (its windows need N_freq - 3 > 2 max(1, N_freq/20))
+        if (Nf - 3 - 2 * std::max(1, Nf / 20) < 1) return dg_fail(ctx, DMFTGPU_BADARG, "moments: N_freq too small");
+        P.sig = const_cast<double2 *>(dS);
+        if (m > 0) DG_TRY(launch_schur_prep(ctx, s, nk, n, D, P.H, P.epsQ, P.B, P.Vq, df));
+        return DMFTGPU_OK;
     }
     DG_TRY(dg_moments_dev(ctx, D, Nf, P.beta, dS, 0, P.mom));
     long long tot = 2LL * Nf * D * D;
@@ -1401,11 +1411,10 @@ int dmftgpu_gloc_vjp(dmftgpu_ctx *ctx, const dmftgpu_lattice *L, const double *h
     if (!dmu) return DMFTGPU_NOMEM;
     DG_TRY(dg_status_reset(ctx));
     Prepared P;
-    DG_TRY(prepare(ctx, L, dH, dS, 0, P));
+    DG_TRY(prepare(ctx, L, dH, dS, 0, P, false, false, true));
     DG_TRY(run_ad(ctx, P, dg::AD_VJP, mu, dGb, 0.0, dSb, dmu));
     DG_TRY(dg_out_done(ctx, sigma_bar, dSb, Nf * DD * sizeof(double2), flags));
     DG_CUDA(cudaMemcpyAsync(mu_bar, dmu, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-    DG_CUDA(cudaStreamWaitEvent(ctx->stream, P.static_ready, 0));
     int code = 0;
     DG_TRY(dg_status_read(ctx, &code));
     return code;
@@ -1454,10 +1463,9 @@ int dmftgpu_gloc_jvp(dmftgpu_ctx *ctx, const dmftgpu_lattice *L, const double *h
     if (st) return st;
     DG_TRY(dg_status_reset(ctx));
     Prepared P;
-    DG_TRY(prepare(ctx, L, dH, dS, 0, P));
+    DG_TRY(prepare(ctx, L, dH, dS, 0, P, false, false, true));
     DG_TRY(run_ad(ctx, P, dg::AD_JVP, mu, dSd, mu_dot, dGd, nullptr));
     DG_TRY(dg_out_done(ctx, gloc_dot, dGd, Nf * DD * sizeof(double2), flags));
-    DG_CUDA(cudaStreamWaitEvent(ctx->stream, P.static_ready, 0));
     int code = 0;
     DG_TRY(dg_status_read(ctx, &code));
     return code;
