@@ -10,11 +10,14 @@
 //
 // What bounds it: the work is ~1e7 FP64 operations, so on this chip (two FP64 lanes per SM and clock) it is the
 // spread over SMs and the length of the dependent chains that count, not memory.  Hence one CTA per series with the
-// terms formed by all its threads and only the ordered sums left to one warp, Hermitian pairs (a <= b) computed
+// terms formed by all its threads and only the ordered sums left to two warps, Hermitian pairs (a <= b) computed
 // once, windows along the lanes so that every load is coalesced, and the gates by Cholesky, one warp per window
 // (the eigenvalue signs asked for are those of m1 and of its Schur complement).  One call, measured with the host's
-// wait: D = 1, N_freq = 400: 255 -> 234 us; D = 10, N_freq = 4096: 3.5 -> 0.48 ms (green 1.04 -> 0.33 ms); D = 20,
-// N_freq = 400, dense F: 148 -> 0.28 ms (one thread per window ran Jacobi eigensolvers in global scratch before).
+// wait: D = 1, N_freq = 400: 255 -> 111 us; D = 10, N_freq = 4096: 3.55 -> 0.30 ms, with a dense F 15.8 -> 0.42 ms
+// (green fit 1.04 -> 0.24 ms); D = 20, N_freq = 400, dense F: 148 ms before (one thread per window ran Jacobi
+// eigensolvers in global scratch).
+#include <algorithm>
+
 #include "smallmat.cuh"
 
 namespace {
@@ -29,7 +32,7 @@ struct MomArgs {
     double *KS;         // [6][R]         suffix sums for K^T K
     double2 *mt;        // [P][ncol][R]   fitted moments per window ("momentstest")
     double *tr;         // [ncol][R]
-    double2 *avg;       // [ncol][C][D*D]
+    double2 *avg;       // [ncol][C][P]   window sums (not yet divided by 2 Nv + 1)
     double *var;        // [ncol][C]
     int *ok;            // [C]
     double2 *work;      // [C][3][D*D], gates of matrices too large for shared memory
@@ -59,8 +62,7 @@ __global__ void k_mom_weights(MomArgs g) {
     g.wt[2 * g.Nf + wn] = 1. / z3;
 }
 
-// Term wn of a series as (value, weight): the sum adds value * weight.  Series q < P ncol: column c of K^T G for a
-// pair; the last six: K^T K.
+// element (a, b) of the data in the form column c of K^T G weighs
 __device__ __forceinline__ double2 mom_value(const MomArgs &g, int a, int b, int c, int wn) {
     const int DD = g.D * g.D;
     const double2 fab = g.fw[(size_t)wn * DD + a + b * g.D], fba = g.fw[(size_t)wn * DD + b + a * g.D];
@@ -71,78 +73,72 @@ __device__ __forceinline__ double2 mom_value(const MomArgs &g, int a, int b, int
     return im;
 }
 
-// One CTA per series: suffix sums S(w) = sum_{wn >= w} term(wn).  All threads form the terms in shared memory; one
-// warp sums them, lane l owning the l-th of 32 contiguous ranges (first the range totals, a suffix scan of them over
-// the lanes, then the running sums), and all threads write the sums out.  STAGED = false (N_freq beyond the shared
-// memory): the same sums with the terms formed where they are added.
+// One CTA per series: suffix sums S(w) = sum_{wn >= w} term(wn).  All threads form the terms in shared memory; two
+// warps sum them, one the real and one the imaginary parts (an FP64 instruction holds its quarter of the SM for 64
+// cycles whatever lanes are active), lane l owning the l-th of 32 contiguous ranges (first the range totals, a suffix
+// scan of them over the lanes, then the running sums), and all threads write the sums out.  Terms are rounded before they are added (the
+// window choice compares variances down to their rounding, so it must not depend on which sums are fused).
+// STAGED = false (N_freq beyond the shared memory): the same sums with the terms formed where they are added.
 constexpr int SUF_THREADS = 256;
-inline size_t suffix_smem(int Nf) { return (size_t)(Nf + 32) * (sizeof(double2) + sizeof(double)); }
+inline size_t suffix_smem(int Nf) { return (size_t)(Nf + 32) * sizeof(double2); }
 template <bool STAGED>
 __global__ void __launch_bounds__(SUF_THREADS) k_mom_suffix(MomArgs g) {
     extern __shared__ double2 ssm[];
     const int series = blockIdx.x, nG = g.P * g.ncol;
     const int chunk = (g.Nf + 31) / 32;
-    double2 *sv = ssm;                                         // value of term wn at wn + wn / chunk (bank spread)
-    double *sw = reinterpret_cast<double *>(ssm + g.Nf + 32);  // its weight
+    double2 *sv = ssm;  // term wn at wn + wn / chunk (bank spread)
     int a = 0, b = 0;
     const int c = series < nG ? series % g.ncol : series - nG;
     if (series < nG) pair_of(series / g.ncol, g.D, a, b);
-    auto term = [&](int wn, double2 &v, double &w) {
+    auto term = [&](int wn) {
+        const double *wt = g.wt + wn;
+        const int Nf = g.Nf;
         if (series < nG) {
-            v = mom_value(g, a, b, c, wn);
-            const int p = g.green ? 1 + c : c - 1;             // weight series; c = 0 of the general fit has none
-            w = p < 0 ? 1.0 : g.wt[(size_t)p * g.Nf + wn];
-        } else {
-            const double i1 = g.wt[wn], i2 = g.wt[g.Nf + wn], i3 = g.wt[2 * g.Nf + wn];
-            if (c == 0) v = cmk(1.0, 0.0), w = 1.0;
-            else if (c == 1) v = cmk(1.0, 0.0), w = i2;        // K(.,0) K(.,2) on Re rows
-            else if (c == 2) v = cmk(i2, 0.0), w = i2;
-            else if (c == 3) v = cmk(i1, 0.0), w = i1;
-            else if (c == 4) v = cmk(i1, 0.0), w = i3;
-            else v = cmk(i3, 0.0), w = i3;
+            const double2 v = mom_value(g, a, b, c, wn);
+            const int p = g.green ? 1 + c : c - 1;  // the weight series; column 0 of the general fit has none
+            if (p < 0) return v;
+            const double w = wt[(size_t)p * Nf];
+            return cmk(__dmul_rn(v.x, w), __dmul_rn(v.y, w));
         }
+        if (c == 0) return cmk(1.0, 0.0);
+        if (c == 1) return cmk(wt[Nf], 0.0);  // K(.,0) K(.,2) on Re rows
+        const double x = c == 2 ? wt[Nf] : (c == 5 ? wt[2 * Nf] : wt[0]);
+        const double y = c == 2 ? wt[Nf] : (c == 3 ? wt[0] : wt[2 * Nf]);
+        return cmk(__dmul_rn(x, y), 0.0);
     };
     if (STAGED) {
-        for (int wn = threadIdx.x; wn < g.Nf; wn += blockDim.x) {
-            const int o = wn + wn / chunk;
-            term(wn, sv[o], sw[o]);
-        }
+        for (int wn = threadIdx.x; wn < g.Nf; wn += blockDim.x) sv[wn + wn / chunk] = term(wn);
         __syncthreads();
     }
     double2 *So = g.S + (size_t)series * g.R;
     double *Ko = g.KS + (size_t)(series - nG) * g.R;
-    if (threadIdx.x < 32) {
-        const int lane = threadIdx.x;
+    if (threadIdx.x < 64) {
+        const int lane = threadIdx.x & 31, im = threadIdx.x >> 5;
         const int lo = min(g.Nf, lane * chunk), hi = min(g.Nf, lo + chunk);
-        double2 part = cmk(0, 0);
-        auto add = [&](double2 s, int wn) {
-            double2 v;
-            double w;
-            if (STAGED) {
-                v = sv[wn + lane];
-                w = sw[wn + lane];
-            } else {
-                term(wn, v, w);
-            }
-            return cmk(fma(v.x, w, s.x), fma(v.y, w, s.y));
+        double *sc = reinterpret_cast<double *>(sv) + im;  // this warp's component
+        auto at = [&](int wn) {
+            if (STAGED) return sc[2 * (wn + lane)];
+            const double2 v = term(wn);
+            return im ? v.y : v.x;
         };
+        double part = 0;
 #pragma unroll 4
-        for (int wn = hi - 1; wn >= lo; wn--) part = add(part, wn);
+        for (int wn = hi - 1; wn >= lo; wn--) part += at(wn);
         // carry = sum of the ranges of all higher lanes (inclusive suffix scan, then shift)
-        double2 incl = part;
+        double incl = part;
 #pragma unroll
         for (int off = 1; off < 32; off <<= 1) {
-            const double2 v = shfl2(incl, min(31, lane + off), 32);
-            if (lane + off < 32) incl = cadd(incl, v);
+            const double v = __shfl_sync(0xffffffffu, incl, min(31, lane + off), 32);
+            if (lane + off < 32) incl += v;
         }
-        double2 run = csub(incl, part);
+        double run = incl - part;
 #pragma unroll 4
         for (int wn = hi - 1; wn >= lo; wn--) {
-            run = add(run, wn);
-            if (STAGED) sv[wn + lane] = run;
+            run += at(wn);
+            if (STAGED) sc[2 * (wn + lane)] = run;
             else if (wn < g.R) {
-                if (series < nG) So[wn] = run;
-                else Ko[wn] = run.x;
+                if (series < nG) (im ? So[wn].y : So[wn].x) = run;
+                else if (!im) Ko[wn] = run;
             }
         }
     }
@@ -232,18 +228,23 @@ __global__ void __launch_bounds__(SOLVE_THREADS) k_mom_solve(MomArgs g) {
 }
 
 // Over 2 Nv + 1 consecutive windows: variances of the traces (the first nvar CTAs, one centre per thread, the traces
-// staged in shared memory) and averages of the moments for the gates (one thread per run of AVG_RUN centres of one
-// series: the first range summed directly, the next ones by sliding)
+// staged in shared memory) and sums of the moments for the gates (the other CTAs, one series and a tile of centres
+// each: staged, then one thread per component and run of AVG_RUN centres, the first range summed directly and the next
+// ones by sliding).  Bound by the FP64 adds, (2 Nv + 1)/AVG_RUN + 2 per centre and component: longer runs mean fewer
+// adds but a longer chain; with 64 the green fit takes 68 us at D = 10, N_freq = 4096 (one thread per run of 32 centres
+// reading the fits at a stride: 148 us).
 constexpr int AVG_RUN = 64;
 constexpr int AVG_THREADS = 128;
-__global__ void __launch_bounds__(AVG_THREADS) k_mom_avg(MomArgs g, int nvar, int staged) {
+constexpr int AVG_TILE = AVG_RUN * AVG_THREADS / 2;  // centres per tile
+__host__ __device__ constexpr int avg_pad(int i) { return i + i / AVG_RUN; }
+__global__ void __launch_bounds__(AVG_THREADS) k_mom_avg(MomArgs g, int nvar, int vstaged, int astaged) {
     extern __shared__ double2 ssm[];
     const int L = 2 * g.Nv + 1;
     if ((int)blockIdx.x < nvar) {
         const int ncb = (g.C + AVG_THREADS - 1) / AVG_THREADS;
         const int i = blockIdx.x / ncb, c0 = (blockIdx.x % ncb) * AVG_THREADS, ci = c0 + threadIdx.x;
         const double *tr = g.tr + (size_t)i * g.R + c0;
-        if (staged) {
+        if (vstaged) {
             double *st = reinterpret_cast<double *>(ssm);
             const int len = min(g.C - c0, AVG_THREADS) + L - 1;
             for (int t = threadIdx.x; t < len; t += AVG_THREADS) st[t] = tr[t];
@@ -262,25 +263,25 @@ __global__ void __launch_bounds__(AVG_THREADS) k_mom_avg(MomArgs g, int nvar, in
         g.var[(size_t)i * g.C + ci] = sqrt(ss / L);
         return;
     }
-    const int DD = g.D * g.D, nrun = (g.C + AVG_RUN - 1) / AVG_RUN;
-    const long long t = (long long)(blockIdx.x - nvar) * AVG_THREADS + threadIdx.x;
-    if (t >= (long long)nrun * g.P * g.ncol) return;
-    const int run = (int)(t % nrun);
-    const long long r = t / nrun;
-    const int i = (int)(r % g.ncol), pr = (int)(r / g.ncol);
-    int a, b;
-    pair_of(pr, g.D, a, b);
-    const double2 *x = g.mt + ((size_t)pr * g.ncol + i) * g.R;
-    const int c0 = run * AVG_RUN, c1 = min(g.C, c0 + AVG_RUN);
-    double2 s = cmk(0, 0);
+    const int ntile = (g.C + AVG_TILE - 1) / AVG_TILE, q = blockIdx.x - nvar;
+    const int series = q / ntile, tile0 = (q % ntile) * AVG_TILE;
+    const int pr = series / g.ncol, i = series % g.ncol, nc = min(AVG_TILE, g.C - tile0);
+    const double2 *x = g.mt + (size_t)series * g.R + tile0;
+    if (astaged) {
+        for (int t = threadIdx.x; t < nc + L - 1; t += AVG_THREADS) ssm[avg_pad(t)] = x[t];
+        __syncthreads();
+    }
+    const int im = threadIdx.x & 1, c0 = (threadIdx.x >> 1) * AVG_RUN, c1 = min(nc, c0 + AVG_RUN);
+    const double *xs = reinterpret_cast<const double *>(astaged ? ssm : x) + im;
+    auto at = [&](int t) { return xs[2 * (astaged ? avg_pad(t) : t)]; };
+    double *o = reinterpret_cast<double *>(g.avg + ((size_t)i * g.C + tile0) * g.P + pr) + im;
+    if (c0 >= nc) return;
+    double s = 0;
 #pragma unroll 8
-    for (int iw = c0; iw < c0 + L; iw++) s = cadd(s, x[iw]);
+    for (int t = c0; t < c0 + L; t++) s += at(t);
     for (int ci = c0; ci < c1; ci++) {
-        if (ci > c0) s = csub(cadd(s, x[ci + L - 1]), x[ci - 1]);
-        double2 *o = g.avg + ((size_t)i * g.C + ci) * DD;
-        const double2 v = cmk(s.x / L, s.y / L);
-        o[a + b * g.D] = v;
-        if (a != b) o[b + a * g.D] = cconj(v);
+        if (ci > c0) s = (s + at(ci + L - 1)) - at(ci - 1);
+        o[2 * (size_t)ci * g.P] = s;
     }
 }
 
@@ -305,14 +306,23 @@ __global__ void __launch_bounds__(128) k_mom_gate(MomArgs g) {
     double2 *A = SHM ? ssm + (size_t)warp * 3 * DD : g.work + (size_t)ci * 3 * DD;
     double2 *W = A + DD, *X = W + DD;
     bool ok = true;
-    if (!g.green) {
-        const double2 *m1 = g.avg + ((size_t)1 * g.C + ci) * DD, *m2 = g.avg + ((size_t)2 * g.C + ci) * DD;
-        const double2 *m3 = g.avg + ((size_t)3 * g.C + ci) * DD;
-        for (int e = lane; e < DD; e += 32) {
-            A[e] = m1[e];
-            W[e] = m2[e];
-            X[e] = m3[e];
+    const int P = g.P;
+    const double L = 2 * g.Nv + 1;
+    // the averaged moment `col` into M
+    auto load = [&](int col, double2 *M) {
+        const double2 *sum = g.avg + ((size_t)col * g.C + ci) * P;
+        for (int q = lane; q < P; q += 32) {
+            int a, b;
+            pair_of(q, D, a, b);
+            const double2 v = cmk(sum[q].x / L, sum[q].y / L);
+            M[a + b * D] = v;
+            if (a != b) M[b + a * D] = cconj(v);
         }
+    };
+    if (!g.green) {
+        load(1, A);
+        load(2, W);
+        load(3, X);
         __syncwarp();
         ok = warp_cholesky(D, A);
         if (ok) {
@@ -335,13 +345,13 @@ __global__ void __launch_bounds__(128) k_mom_gate(MomArgs g) {
             ok = warp_cholesky(D, X);
         }
     } else {
-        const double2 *m0 = g.avg + (size_t)ci * DD, *m1 = g.avg + ((size_t)g.C + ci) * DD;
-        for (int e = lane; e < DD; e += 32) W[e] = m0[e];
+        load(0, W);
+        load(1, X);
         __syncwarp();
         for (int e = lane; e < DD; e += 32) {
             const int i = e % D, j = e / D;
             if (i < j) continue;
-            double2 s = m1[e];
+            double2 s = X[e];
             for (int k = 0; k < D; k++) s = csub(s, cmul(DG_AT(W, D, i, k), DG_AT(W, D, k, j)));
             if (i == j) s = cmk(s.x - 1.0, 0.0);
             X[e] = s;
@@ -406,13 +416,15 @@ __global__ void __launch_bounds__(FIN_THREADS) k_mom_final(MomArgs g, int staged
         __syncthreads();
         x = ssm;
     }
-    if (tid != 0) return;
-    double2 s = cmk(0, 0);
+    if (tid > 1) return;
+    const double *xs = reinterpret_cast<const double *>(x) + tid;  // thread 0: real parts, thread 1: imaginary parts
+    double s = 0;
 #pragma unroll 8
-    for (int w = 0; w < L; w++) s = cadd(s, x[w]);
-    const double2 v = a == b ? cmk(s.x / L, 0.0) : cmk(s.x / L, s.y / L);
-    o[a + b * D] = v;
-    if (a != b) o[b + a * D] = cconj(v);
+    for (int w = 0; w < L; w++) s += xs[2 * w];
+    s /= L;
+    if (a == b && tid == 1) s = 0.0;
+    reinterpret_cast<double *>(o + a + b * D)[tid] = s;
+    if (a != b) reinterpret_cast<double *>(o + b + a * D)[tid] = tid ? -s : s;
 }
 
 }  // namespace
@@ -445,7 +457,7 @@ int dg_moments_dev(dmftgpu_ctx *ctx, int dim, int nfreq, double beta, const doub
     };
     size_t oWt = carve(3 * (size_t)nfreq * sizeof(double)), oS = carve(P * g.ncol * g.R * sizeof(double2)),
            oKS = carve(6 * (size_t)g.R * sizeof(double)), oMt = carve(P * g.R * g.ncol * sizeof(double2)),
-           oTr = carve((size_t)g.ncol * g.R * sizeof(double)), oAvg = carve((size_t)g.ncol * g.C * DD * sizeof(double2)),
+           oTr = carve((size_t)g.ncol * g.R * sizeof(double)), oAvg = carve((size_t)g.ncol * g.C * P * sizeof(double2)),
            oVar = carve((size_t)g.ncol * g.C * sizeof(double)), oOk = carve((size_t)g.C * sizeof(int)),
            oW = carve(gate_shm ? 0 : (size_t)g.C * gate_warp);
     char *base = (char *)dg_buf(ctx, "moments.work", off);
@@ -471,16 +483,19 @@ int dg_moments_dev(dmftgpu_ctx *ctx, int dim, int nfreq, double beta, const doub
         DG_CUDA(cudaFuncSetAttribute(k_mom_suffix<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sms));
         k_mom_suffix<true><<<nseries, SUF_THREADS, sms, s>>>(g);
     } else {
-        k_mom_suffix<false><<<nseries, 32, 0, s>>>(g);
+        k_mom_suffix<false><<<nseries, 64, 0, s>>>(g);
     }
     DG_LAUNCH(ctx, "k_mom_suffix");
     k_mom_solve<<<dg_ceil_div(g.R, 32), SOLVE_THREADS, 0, s>>>(g);
     DG_LAUNCH(ctx, "k_mom_solve");
     const int nvar = g.ncol * dg_ceil_div(g.C, AVG_THREADS);
-    const long long navg = (long long)dg_ceil_div(g.C, AVG_RUN) * g.P * g.ncol;
-    const size_t sma = (AVG_THREADS + L) * sizeof(double), smf = L * sizeof(double2);
-    const int sta = sma <= 48 * 1024, stf = smf <= 40 * 1024;
-    k_mom_avg<<<nvar + dg_ceil_div(navg, AVG_THREADS), AVG_THREADS, sta ? sma : 0, s>>>(g, nvar, sta);
+    const int navg = g.P * g.ncol * dg_ceil_div(g.C, AVG_TILE);
+    const size_t smv = (AVG_THREADS + L) * sizeof(double), smf = L * sizeof(double2);
+    const size_t sma = (size_t)(avg_pad(std::min(g.C, AVG_TILE) + (int)L) + 1) * sizeof(double2);
+    const int stv = smv <= 48 * 1024, sta = sma <= 160 * 1024, stf = smf <= 40 * 1024;
+    const size_t smavg = std::max(stv ? smv : 0, sta ? sma : 0);
+    DG_CUDA(cudaFuncSetAttribute(k_mom_avg, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smavg));
+    k_mom_avg<<<nvar + navg, AVG_THREADS, smavg, s>>>(g, nvar, stv, sta);
     DG_LAUNCH(ctx, "k_mom_avg");
     if (gate_shm) {
         const size_t smg = gw * gate_warp;

@@ -61,8 +61,8 @@ CASES = {
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("D,nf,green", [(1, 20, False), (2, 33, False), (7, 64, False), (20, 65, False), (33, 40, False),
-                                        (46, 24, False), (2, 8600, False), (1, 20, True), (11, 97, True),
-                                        (46, 24, True), (2, 8600, True)])
+                                        (46, 24, False), (2, 12900, False), (1, 20, True), (11, 97, True),
+                                        (46, 24, True), (1, 12900, True)])
 def test_moments_edges(ctx, orc, D, nf, green):
     """Smallest and ragged N_freq, N_freq beyond the staged sums, matrices beyond the gates' shared memory.  The moments
     describe the tail beyond the data: it is compared there, relative to its size.  Bound: the fits' 2 x 2 normal
