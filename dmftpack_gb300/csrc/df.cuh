@@ -8,7 +8,14 @@
 // hi + lo in FP64.
 //
 // Ops policies used by the templated lattice kernels:
-//   OpsD: complex FP64 (double2)       OpsF: complex double-float (cdf)
+//   OpsD: complex FP64 (double2)       OpsF: complex double-float (cdf)       OpsP: the same on packed pairs (pdf)
+//
+// OpsP works on the real and imaginary parts at once with the packed FP32 instructions (add / sub / mul / fma .f32x2):
+// the same roundings in the same order as OpsF, hence the same bits.  A packed instruction holds the FP32 pipe as long
+// as the two scalar ones it replaces (measured: 125 of 128 lane operations per SM and clock, where 8-16 warps of
+// scalar FMAs reach 85-105) but takes one issue slot, which leaves slots for pivot selects, shuffles and loads.
+// Broadcast operands and negations cost nothing (they fold into the instruction, measured); putting two unrelated
+// registers side by side costs two moves, so a pdf is kept as (re.h, im.h, re.l, im.l) in registers and in memory.
 #pragma once
 #include <cmath>
 
@@ -47,9 +54,13 @@ DG_HD float f_fma(float a, float b, float c) {
     return std::fma(a, b, c);
 #endif
 }
+// 1/a to within an ulp: on the device the approximate reciprocal and one Newton step (the correctly rounded division
+// takes ~20 issue slots, this three)
 DG_HD float f_rcp(float a) {
 #ifdef __CUDA_ARCH__
-    return __frcp_rn(a);
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
+    return __fmaf_rn(r, __fmaf_rn(-a, r, 1.0f), r);
 #else
     return 1.0f / a;
 #endif
@@ -144,14 +155,13 @@ DG_HD dfl df_fma_lazy(dfl a, dfl b, dfl acc) {
     return {s.h, f_add(f_add(acc.l, e), s.l)};
 }
 DG_HD dfl df_renorm(dfl a) { return fast_two_sum(a.h, a.l); }
-// 1/a: FP32 reciprocal refined by one Newton step in double-float (24 -> ~48 bits)
+// 1/a = r / (1 - e) with the FP32 reciprocal r and the residual e = 1 - a r, which an FMA gives exactly up to its own
+// rounding: r + r (e + e^2), the neglected e^3 below 2^-66 (without e^2 every reciprocal would come out low by up to
+// 2^-46, and the sums over k would keep that bias)
 DG_HD dfl df_rcp(dfl a) {
     const float r = f_rcp(a.h);
-    // e = 1 - a*r in double-float
-    dfl ar = df_mul(a, {r, 0.0f});
-    dfl e = df_sub({1.0f, 0.0f}, ar);
-    // r + r*e
-    return df_fma({r, 0.0f}, e, {r, 0.0f});
+    const float e = f_fma(-a.l, r, f_fma(-a.h, r, 1.0f));
+    return fast_two_sum(r, f_mul(r, f_fma(e, e, e)));
 }
 
 DG_HD cdf cdf_make(double2 z) { return {df_make(z.x), df_make(z.y)}; }
@@ -187,12 +197,14 @@ struct OpsD {
     static DG_HD R rsub(R a, R b) { return a - b; }
     static DG_HD R rneg(R a) { return -a; }
     static DG_HD R rrcp(R a) { return 1.0 / a; }
-    // lazy running sums of a few terms (double-float: unnormalised low parts, read through rnorm)
-    static DG_HD R racc(R a, R b, R acc) { return ::fma(a, b, acc); }
-    static DG_HD R rnorm(R a) { return a; }
     static DG_HD C mk(R re, R im) { return cmk(re, im); }
     static DG_HD R cre(C a) { return a.x; }
     static DG_HD R cim(C a) { return a.y; }
+    // two running sums of a few products with a common second factor, acc + (w.re, w.im) p (double-float: lazy sums,
+    // unnormalised low parts, read through pnorm)
+    static DG_HD C pacc(C w, R p, C acc) { return cmk(::fma(w.x, p, acc.x), ::fma(w.y, p, acc.y)); }
+    static DG_HD C pnorm(C a) { return a; }
+    static DG_HD C pscale(C a, R r) { return cmk(a.x * r, a.y * r); }
 };
 
 struct OpsF {
@@ -238,8 +250,6 @@ struct OpsF {
     static DG_HD R rsub(R a, R b) { return df_sub(a, b); }
     static DG_HD R rneg(R a) { return df_neg(a); }
     static DG_HD R rrcp(R a) { return df_rcp(a); }
-    static DG_HD R racc(R a, R b, R acc) { return df_fma_lazy(a, b, acc); }
-    static DG_HD R rnorm(R a) { return df_renorm(a); }
     static DG_HD C mk(R re, R im) { return {re, im}; }
     static DG_HD R cre(C a) { return a.re; }
     static DG_HD R cim(C a) { return a.im; }
@@ -249,6 +259,142 @@ struct OpsF {
         o.re.l = __shfl_sync(0xffffffffu, v.re.l, src, w);
         o.im.h = __shfl_sync(0xffffffffu, v.im.h, src, w);
         o.im.l = __shfl_sync(0xffffffffu, v.im.l, src, w);
+        return o;
+    }
+};
+
+// ---- packed pairs (device only) ----
+__device__ __forceinline__ float2 p2(float x, float y) { return make_float2(x, y); }
+__device__ __forceinline__ float2 p2(float x) { return make_float2(x, x); }
+#define DG_P2_OP(NAME, INSN)                                                                               \
+    __device__ __forceinline__ float2 NAME(float2 a, float2 b) {                                           \
+        float2 d;                                                                                          \
+        asm("{\n\t.reg .b64 a, b, d;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\t" INSN              \
+            " d, a, b;\n\tmov.b64 {%0, %1}, d;\n\t}"                                                       \
+            : "=f"(d.x), "=f"(d.y)                                                                         \
+            : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));                                                     \
+        return d;                                                                                          \
+    }
+DG_P2_OP(p2_add, "add.rn.f32x2")
+DG_P2_OP(p2_sub, "sub.rn.f32x2")
+DG_P2_OP(p2_mul, "mul.rn.f32x2")
+#undef DG_P2_OP
+__device__ __forceinline__ float2 p2_fma(float2 a, float2 b, float2 c) {
+    float2 d;
+    asm("{\n\t.reg .b64 a, b, c, d;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tmov.b64 c, {%6, %7};\n\t"
+        "fma.rn.f32x2 d, a, b, c;\n\tmov.b64 {%0, %1}, d;\n\t}"
+        : "=f"(d.x), "=f"(d.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return d;
+}
+__device__ __forceinline__ float2 p2_neg(float2 a) { return p2(-a.x, -a.y); }
+
+// two double-float numbers side by side: the parts of a complex number, or two real sums
+struct __align__(16) pdf {
+    float2 h, l;
+};
+__device__ __forceinline__ pdf pdf_fast_two_sum(float2 a, float2 b) {
+    const float2 s = p2_add(a, b);
+    return {s, p2_sub(b, p2_sub(s, a))};
+}
+__device__ __forceinline__ pdf pdf_two_sum(float2 a, float2 b) {
+    const float2 s = p2_add(a, b), bb = p2_sub(s, a);
+    return {s, p2_add(p2_sub(a, p2_sub(s, bb)), p2_sub(b, bb))};
+}
+__device__ __forceinline__ pdf pdf_neg(pdf a) { return {p2_neg(a.h), p2_neg(a.l)}; }
+__device__ __forceinline__ pdf pdf_add(pdf a, pdf b) {
+    const pdf s = pdf_two_sum(a.h, b.h);
+    return pdf_fast_two_sum(s.h, p2_add(s.l, p2_add(a.l, b.l)));
+}
+// df_prod on both halves
+__device__ __forceinline__ float2 pdf_prod(pdf a, pdf b, float2 &e) {
+    const float2 p = p2_mul(a.h, b.h);
+    e = p2_fma(a.h, b.h, p2_neg(p));
+    e = p2_fma(a.h, b.l, e);
+    e = p2_fma(a.l, b.h, e);
+    return p;
+}
+// df_mul, df_dot2 (a1 b1 + a2 b2), df_fma2 (acc + a1 b1 + a2 b2) and df_fma_lazy on both halves
+__device__ __forceinline__ pdf pdf_mul(pdf a, pdf b) {
+    float2 e;
+    const float2 p = pdf_prod(a, b, e);
+    return pdf_fast_two_sum(p, e);
+}
+__device__ __forceinline__ pdf pdf_dot2(pdf a1, pdf b1, pdf a2, pdf b2) {
+    float2 e1, e2;
+    const float2 x1 = pdf_prod(a1, b1, e1), x2 = pdf_prod(a2, b2, e2);
+    const pdf s = pdf_two_sum(x1, x2);
+    return pdf_fast_two_sum(s.h, p2_add(s.l, p2_add(e1, e2)));
+}
+__device__ __forceinline__ pdf pdf_fma2(pdf a1, pdf b1, pdf a2, pdf b2, pdf acc) {
+    float2 e1, e2;
+    const float2 x1 = pdf_prod(a1, b1, e1), x2 = pdf_prod(a2, b2, e2);
+    const pdf s1 = pdf_two_sum(acc.h, x1);
+    const pdf s2 = pdf_two_sum(s1.h, x2);
+    return pdf_fast_two_sum(s2.h, p2_add(p2_add(s1.l, s2.l), p2_add(acc.l, p2_add(e1, e2))));
+}
+__device__ __forceinline__ pdf pdf_fma_lazy(pdf a, pdf b, pdf acc) {
+    float2 e;
+    const float2 x = pdf_prod(a, b, e);
+    const pdf s = pdf_two_sum(acc.h, x);
+    return {s.h, p2_add(p2_add(acc.l, e), s.l)};
+}
+__device__ __forceinline__ pdf pdf_both(dfl a) { return {p2(a.h), p2(a.l)}; }
+// real part twice, imaginary part twice, and i z = (-im, re)
+__device__ __forceinline__ pdf pdf_re(pdf z) { return {p2(z.h.x), p2(z.l.x)}; }
+__device__ __forceinline__ pdf pdf_im(pdf z) { return {p2(z.h.y), p2(z.l.y)}; }
+__device__ __forceinline__ pdf pdf_i(pdf z) { return {p2(-z.h.y, z.h.x), p2(-z.l.y, z.l.x)}; }
+
+struct OpsP {
+    typedef pdf C;
+    typedef float M;
+    static __device__ __forceinline__ C zero() { return {p2(0.f), p2(0.f)}; }
+    static __device__ __forceinline__ C one() { return {p2(1.f, 0.f), p2(0.f)}; }
+    static __device__ __forceinline__ C from(double2 z) { return mk(df_make(z.x), df_make(z.y)); }
+    static __device__ __forceinline__ double2 to(C z) { return make_double2(df_val(cre(z)), df_val(cim(z))); }
+    static __device__ __forceinline__ C add(C a, C b) { return pdf_add(a, b); }
+    static __device__ __forceinline__ C sub(C a, C b) { return pdf_add(a, pdf_neg(b)); }
+    static __device__ __forceinline__ C neg(C a) { return pdf_neg(a); }
+    static __device__ __forceinline__ C conj(C a) { return {p2(a.h.x, -a.h.y), p2(a.l.x, -a.l.y)}; }
+    static __device__ __forceinline__ C mul(C a, C b) { return pdf_dot2(pdf_re(a), b, pdf_im(a), pdf_i(b)); }
+    static __device__ __forceinline__ C mulc(C a, C b) {  // a conj(b) = b.re a + b.im (-i a)
+        return pdf_dot2(a, pdf_re(b), pdf_neg(pdf_i(a)), pdf_im(b));
+    }
+    static __device__ __forceinline__ C fma(C a, C b, C acc) { return pdf_fma2(pdf_re(a), b, pdf_im(a), pdf_i(b), acc); }
+    static __device__ __forceinline__ C fms(C a, C b, C acc) {
+        return pdf_fma2(pdf_re(a), pdf_neg(b), pdf_im(a), pdf_neg(pdf_i(b)), acc);
+    }
+    static __device__ __forceinline__ C rcp(C a) {  // conj(a)/|a|^2
+        float2 e;
+        const float2 p = pdf_prod(a, a, e);
+        const dfl s = two_sum(p.x, p.y);
+        const dfl r = df_rcp(fast_two_sum(s.h, f_add(s.l, f_add(e.x, e.y))));
+        return pdf_mul(conj(a), pdf_both(r));
+    }
+    static __device__ __forceinline__ double re(C a) { return df_val(cre(a)); }
+    static __device__ __forceinline__ double im(C a) { return df_val(cim(a)); }
+    static __device__ __forceinline__ float mag2(C a) { return f_fma(a.h.x, a.h.x, f_mul(a.h.y, a.h.y)); }
+    typedef dfl R;
+    static __device__ __forceinline__ R rfrom(double x) { return df_make(x); }
+    static __device__ __forceinline__ R rfma(R a, R b, R acc) { return df_fma(a, b, acc); }
+    static __device__ __forceinline__ R rmul(R a, R b) { return df_mul(a, b); }
+    static __device__ __forceinline__ R radd(R a, R b) { return df_add(a, b); }
+    static __device__ __forceinline__ R rsub(R a, R b) { return df_sub(a, b); }
+    static __device__ __forceinline__ R rneg(R a) { return df_neg(a); }
+    static __device__ __forceinline__ R rrcp(R a) { return df_rcp(a); }
+    static __device__ __forceinline__ C mk(R re, R im) { return {p2(re.h, im.h), p2(re.l, im.l)}; }
+    static __device__ __forceinline__ R cre(C a) { return {a.h.x, a.l.x}; }
+    static __device__ __forceinline__ R cim(C a) { return {a.h.y, a.l.y}; }
+    // two lazy real sums with a common second factor: acc + (wx, wy) p
+    static __device__ __forceinline__ C pacc(C w, R p, C acc) { return pdf_fma_lazy(w, pdf_both(p), acc); }
+    static __device__ __forceinline__ C pnorm(C a) { return pdf_fast_two_sum(a.h, a.l); }
+    static __device__ __forceinline__ C pscale(C a, R r) { return pdf_mul(a, pdf_both(r)); }
+    static __device__ __forceinline__ C shfl(C v, int src, int w) {
+        C o;
+        o.h.x = __shfl_sync(0xffffffffu, v.h.x, src, w);
+        o.h.y = __shfl_sync(0xffffffffu, v.h.y, src, w);
+        o.l.x = __shfl_sync(0xffffffffu, v.l.x, src, w);
+        o.l.y = __shfl_sync(0xffffffffu, v.l.y, src, w);
         return o;
     }
 };

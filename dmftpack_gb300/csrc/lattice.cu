@@ -706,16 +706,18 @@ int run_schur(dmftgpu_ctx *ctx, const Prepared &P, int mode, double mu, int wgri
     const SInst *in = pick_schur(P.D);
     // BLOCK passes of correlated blocks up to 3 x 3: one thread per frequency (k_schur_tpi).  It stages the
     // Hermitian pole products of each staged k; prepare() caps n at 64 (the static eigensolver), so one k needs
-    // at most 63 * (3 * 16 + 3 * 8 + 8) + 9 * 16 B = 5.2 KB and the 200 KB check below never rejects a tpi pass.
+    // at most 63 * (3 * 16 + 3 * 8 + 8) + 9 * 16 B = 5.2 KB (beside 55 KB of per-thread sums) and the 200 KB check below never rejects a tpi pass.
     const bool tpi = mode == dg::S_BLOCK && P.D <= 3;
     SchurKernel kern = tpi ? dg::schur_tpi_kernel(P.D, mixed) : in->get(mode, mixed);
     const int m = P.n - P.D, NG = tpi ? 128 : dg::schur_groups(in->SW), DD = P.D * P.D;
     const int nf2 = (mode & dg::S_REAL) ? P.Nf : 2 * P.Nf;  // the real axis has exactly the caller's points
     auto smem_of = [&](int kc_) {
-        return tpi ? dg::schur_tpi_smem(kc_, P.D, m) : dg::schur_smem(in->DP, in->SW, mode, kc_, P.D, m, P.n);
+        return tpi ? dg::schur_tpi_smem(kc_, P.D, m, mixed) : dg::schur_smem(in->DP, in->SW, mode, kc_, P.D, m, P.n);
     };
     int kc = 16;
-    while (kc > 1 && smem_of(kc) > 96 * 1024) kc /= 2;
+    // three CTAs per SM where the thread-per-frequency kernel keeps its sums in shared memory, else two
+    const size_t cap = (tpi && mixed && P.D == 3 ? 74 : 96) * 1024;
+    while (kc > 1 && smem_of(kc) > cap) kc /= 2;
     const size_t smem = smem_of(kc);
     if (smem > 200 * 1024) return dg_fail(ctx, DMFTGPU_BADARG, "lattice: correlated block too large");
     DG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));

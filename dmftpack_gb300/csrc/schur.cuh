@@ -22,7 +22,7 @@
 // accumulates column c of the k sum in registers.  A CTA = 128/W frequencies x one k chunk; the per-k data
 // (b_l, mu - e_l, -H_PP) of kc k points at a time is staged once in shared memory in the kernel's
 // arithmetic type.  Per-chunk sums are reduced over chunks in a fixed order by a second kernel.
-// Ops = OpsD (FP64) or OpsF (double-float on the FP32 pipe; FP64 appears only when staging and storing).
+// Ops = OpsD (FP64) or OpsP (double-float on the FP32 pipe, packed; FP64 appears only when staging and storing).
 #pragma once
 #include <type_traits>
 #include "df.cuh"
@@ -54,7 +54,7 @@ struct SchurArgs {
 // kernels are instruction-fetch bound, FP64 ones FP64-pipe bound), the unrolled one otherwise
 template <class Ops, int DP, int W>
 __device__ __forceinline__ bool gj_inverse(typename Ops::C (&a)[DP], int c) {
-    if constexpr (DP >= 8 || (std::is_same<Ops, OpsF>::value && DP >= 2))
+    if constexpr (DP >= 8 || (!std::is_same<Ops, OpsD>::value && DP >= 2))
         return warp_gj_inverse_rolled<Ops, DP, W>(a, c);
     else
         return warp_gj_inverse_t<Ops, DP, W>(a, c);
@@ -387,6 +387,17 @@ DG_HD bool thread_inverse(typename Ops::C (&a)[N][N]) {
     return sing;
 }
 
+// staged per k: P_l off-diagonal pairs [m][D(D-1)/2] and -H_PP - m0 [D][D] (16 B complex), P_l diagonal [m][D] and
+// mu - e_l [m] (8 B real; double and double-float alike)
+__host__ __device__ inline size_t schur_tpi_stage(int kc, int D, int m) {
+    return ((((size_t)kc * m * (D * (D - 1) / 2) + (size_t)kc * D * D) * 16 + ((size_t)kc * m * D + (size_t)kc * m) * 8) +
+            15) / 16 * 16;
+}
+// the whole launch (per-thread sums in shared memory: tpi_shared)
+inline size_t schur_tpi_smem(int kc, int D, int m, bool mixed) {
+    return schur_tpi_stage(kc, D, m) + (mixed && D == 3 ? 3 * (size_t)D * D * 16 * 128 : 0);
+}
+
 // BLOCK mode (G_loc and GwHF) for correlated blocks of D <= 3: one thread per Matsubara frequency, the whole
 // D x D S(z) and S0(z) of that thread's (k, iw) in its registers, inverted by thread_inverse.  A lane-group
 // k_schur at these widths leaves lanes idle (D < W) and spends its issue slots on the group's pivot broadcasts;
@@ -399,18 +410,29 @@ DG_HD bool thread_inverse(typename Ops::C (&a)[N][N]) {
 // sum_l w_l P_l = A + i B with A = sum_l Re(w_l) P_l and B = sum_l Im(w_l) P_l both Hermitian, so only the
 // diagonal (real) and the upper triangle of A and B are accumulated: 2 D + 4 D(D-1)/2 real multiply-adds per pole
 // instead of 4 D^2, and the lower triangle follows as A_ba + i B_ba = conj(A_ab) + i conj(B_ab).
+//
+// Bound by the packed double-float arithmetic and its latency: at D = 3 the k sums of G and G0 and Sigma - m0 (27
+// complex numbers) would take the kernel to 250 registers and two CTAs per SM, so they live in shared memory
+// (`tpi_shared`), one column per thread, and three CTAs fit:
+// the headline pass (24^3 k, 8192 points) takes 25.5 ms against 26.2 ms with all of it in registers and 31.2 ms with
+// scalar double-float instructions.
 template <class Ops, int D>
-__global__ void __launch_bounds__(128) k_schur_tpi(SchurArgs g) {
+constexpr bool tpi_shared = std::is_same<Ops, OpsP>::value && D == 3;
+template <class Ops, int D>
+__global__ void __launch_bounds__(128, tpi_shared<Ops, D> ? 3 : 1) k_schur_tpi(SchurArgs g) {
     typedef typename Ops::C C;
     typedef typename Ops::R R;
     extern __shared__ double2 sm[];
     constexpr int DD = D * D, NP = D * (D - 1) / 2;
+    constexpr bool SH = tpi_shared<Ops, D>;
     const int m = g.m;
     // staged per k: P_l off-diagonal pairs [m][NP] (C), -H_PP - m0 [DD] (C), P_l diagonal [m][D] (R), mu - e_l [m] (R)
     C *sPo = reinterpret_cast<C *>(sm);
     C *sH = sPo + (size_t)g.kc * m * NP;
     R *sPd = reinterpret_cast<R *>(sH + (size_t)g.kc * DD);
     R *sE = sPd + (size_t)g.kc * m * D;
+    // SH: G sums, G0 sums and Sigma - m0 of this thread, element e at [e * 128]
+    C *mine = sPo + schur_tpi_stage(g.kc, D, m) / sizeof(C) + threadIdx.x;
     const int f_raw = blockIdx.x * blockDim.x + threadIdx.x;
     const bool fvalid = f_raw < g.nf2;
     const int f = fvalid ? f_raw : g.nf2 - 1;
@@ -419,14 +441,14 @@ __global__ void __launch_bounds__(128) k_schur_tpi(SchurArgs g) {
     const double w = g.wgrid ? (DG_PI / g.beta + f * ((2 * DG_PI) / g.beta)) : (DG_PI * (2. * f + 1.) / g.beta);
     const C zc = Ops::from(cmk(g.mu, w));
     const R wr = Ops::rfrom(w), w2 = Ops::rmul(wr, wr);
-    C sd[D][D], aG[D][D], aG0[D][D];  // sd = Sigma(iw) - m0
+    C reg[SH ? 1 : 3 * DD];
+    // element e (row + D * column) of the k sum of G (w = 0), of G0 (w = 1), and of Sigma(iw) - m0 (w = 2)
+    auto at = [&](int w, int e) -> C & { return SH ? mine[(w * DD + e) * 128] : reg[SH ? 0 : w * DD + e]; };
 #pragma unroll
-    for (int a = 0; a < D; a++)
-#pragma unroll
-        for (int b = 0; b < D; b++) {
-            sd[a][b] = Ops::from(csub(g.sig[(size_t)f * DD + a + b * D], g.m0[a + b * D]));
-            aG[a][b] = aG0[a][b] = Ops::zero();
-        }
+    for (int e = 0; e < DD; e++) {
+        at(2, e) = Ops::from(csub(g.sig[(size_t)f * DD + e], g.m0[e]));
+        at(0, e) = at(1, e) = Ops::zero();
+    }
     bool sing = false;
     for (int k0 = kbeg; k0 < kend; k0 += g.kc) {
         const int nkc = min(g.kc, kend - k0);
@@ -454,44 +476,34 @@ __global__ void __launch_bounds__(128) k_schur_tpi(SchurArgs g) {
         for (int kk = 0; kk < nkc; kk++) {
             const C *po = sPo + (size_t)kk * m * NP, *hp = sH + (size_t)kk * DD;
             const R *pd = sPd + (size_t)kk * m * D, *es = sE + (size_t)kk * m;
-            R Ad[D], Bd[D], Ar[NP ? NP : 1], Ai[NP ? NP : 1], Br[NP ? NP : 1], Bi[NP ? NP : 1];
+            // (A, B) side by side: diagonal, real and imaginary parts of the upper triangle
+            C Pd[D], Pr[NP ? NP : 1], Pi[NP ? NP : 1];
 #pragma unroll
-            for (int a = 0; a < D; a++) Ad[a] = Bd[a] = Ops::rzero();
+            for (int a = 0; a < D; a++) Pd[a] = Ops::zero();
 #pragma unroll
-            for (int q = 0; q < NP; q++) Ar[q] = Ai[q] = Br[q] = Bi[q] = Ops::rzero();
+            for (int q = 0; q < NP; q++) Pr[q] = Pi[q] = Ops::zero();
             // the pole sums are lazy double-float sums, renormalised after every 16 poles and at the end
             auto renorm = [&]() {
 #pragma unroll
-                for (int a = 0; a < D; a++) {
-                    Ad[a] = Ops::rnorm(Ad[a]);
-                    Bd[a] = Ops::rnorm(Bd[a]);
-                }
+                for (int a = 0; a < D; a++) Pd[a] = Ops::pnorm(Pd[a]);
 #pragma unroll
                 for (int q = 0; q < NP; q++) {
-                    Ar[q] = Ops::rnorm(Ar[q]);
-                    Ai[q] = Ops::rnorm(Ai[q]);
-                    Br[q] = Ops::rnorm(Br[q]);
-                    Bi[q] = Ops::rnorm(Bi[q]);
+                    Pr[q] = Ops::pnorm(Pr[q]);
+                    Pi[q] = Ops::pnorm(Pi[q]);
                 }
             };
             for (int l = 0; l < m; l++) {
                 if (l > 0 && (l & 15) == 0) renorm();
                 const R x = es[l];
                 const R r = Ops::rrcp(Ops::rfma(x, x, w2));
-                const R re = Ops::rmul(x, r), im = Ops::rneg(Ops::rmul(wr, r));  // w_l
+                const C wl = Ops::pscale(Ops::mk(x, Ops::rneg(wr)), r);
 #pragma unroll
-                for (int a = 0; a < D; a++) {
-                    const R p = pd[(size_t)l * D + a];
-                    Ad[a] = Ops::racc(re, p, Ad[a]);
-                    Bd[a] = Ops::racc(im, p, Bd[a]);
-                }
+                for (int a = 0; a < D; a++) Pd[a] = Ops::pacc(wl, pd[(size_t)l * D + a], Pd[a]);
 #pragma unroll
                 for (int q = 0; q < NP; q++) {
                     const C p = po[(size_t)l * NP + q];
-                    Ar[q] = Ops::racc(re, Ops::cre(p), Ar[q]);
-                    Ai[q] = Ops::racc(re, Ops::cim(p), Ai[q]);
-                    Br[q] = Ops::racc(im, Ops::cre(p), Br[q]);
-                    Bi[q] = Ops::racc(im, Ops::cim(p), Bi[q]);
+                    Pr[q] = Ops::pacc(wl, Ops::cre(p), Pr[q]);
+                    Pi[q] = Ops::pacc(wl, Ops::cim(p), Pi[q]);
                 }
             }
             renorm();
@@ -499,7 +511,7 @@ __global__ void __launch_bounds__(128) k_schur_tpi(SchurArgs g) {
 #pragma unroll
             for (int a = 0; a < D; a++) {
                 const C h = Ops::add(hp[a + a * D], zc);
-                s0[a][a] = Ops::sub(h, Ops::mk(Ad[a], Bd[a]));
+                s0[a][a] = Ops::sub(h, Pd[a]);
             }
             {
                 int q = 0;
@@ -508,42 +520,36 @@ __global__ void __launch_bounds__(128) k_schur_tpi(SchurArgs g) {
 #pragma unroll
                     for (int b = a + 1; b < D; b++, q++) {
                         // S_ab = (Ar - Bi) + i (Ai + Br), S_ba = (Ar + Bi) + i (Br - Ai)
-                        s0[a][b] = Ops::sub(hp[a + b * D], Ops::mk(Ops::rsub(Ar[q], Bi[q]), Ops::radd(Ai[q], Br[q])));
-                        s0[b][a] = Ops::sub(hp[b + a * D], Ops::mk(Ops::radd(Ar[q], Bi[q]), Ops::rsub(Br[q], Ai[q])));
+                        const R Ar = Ops::cre(Pr[q]), Br = Ops::cim(Pr[q]), Ai = Ops::cre(Pi[q]), Bi = Ops::cim(Pi[q]);
+                        s0[a][b] = Ops::sub(hp[a + b * D], Ops::mk(Ops::rsub(Ar, Bi), Ops::radd(Ai, Br)));
+                        s0[b][a] = Ops::sub(hp[b + a * D], Ops::mk(Ops::radd(Ar, Bi), Ops::rsub(Br, Ai)));
                     }
             }
             C s[D][D];
 #pragma unroll
             for (int a = 0; a < D; a++)
 #pragma unroll
-                for (int b = 0; b < D; b++) s[a][b] = Ops::sub(s0[a][b], sd[a][b]);
+                for (int b = 0; b < D; b++) s[a][b] = Ops::sub(s0[a][b], at(2, a + b * D));
+            auto sum = [&](int w, const C (&x)[D][D]) {
+#pragma unroll
+                for (int a = 0; a < D; a++)
+#pragma unroll
+                    for (int b = 0; b < D; b++) at(w, a + b * D) = Ops::add(at(w, a + b * D), x[a][b]);
+            };
             sing |= thread_inverse<Ops, D>(s);
+            sum(0, s);
             sing |= thread_inverse<Ops, D>(s0);
-#pragma unroll
-            for (int a = 0; a < D; a++)
-#pragma unroll
-                for (int b = 0; b < D; b++) {
-                    aG[a][b] = Ops::add(aG[a][b], s[a][b]);
-                    aG0[a][b] = Ops::add(aG0[a][b], s0[a][b]);
-                }
+            sum(1, s0);
         }
     }
     if (sing && fvalid) dg_flag(g.status, DG_SINGULAR);
     if (!fvalid) return;
     const size_t o = ((size_t)chunk * g.nf2 + f) * DD;
 #pragma unroll
-    for (int a = 0; a < D; a++)
-#pragma unroll
-        for (int b = 0; b < D; b++) {
-            g.pblk[o + a + b * D] = Ops::to(aG[a][b]);
-            g.pblk0[o + a + b * D] = Ops::to(aG0[a][b]);
-        }
-}
-
-// staged per k: P_l off-diagonal pairs [m][D(D-1)/2] and -H_PP - m0 [D][D] (16 B complex), P_l diagonal [m][D] and
-// mu - e_l [m] (8 B real; double and double-float alike)
-inline size_t schur_tpi_smem(int kc, int D, int m) {
-    return ((size_t)kc * m * (D * (D - 1) / 2) + (size_t)kc * D * D) * 16 + ((size_t)kc * m * D + (size_t)kc * m) * 8;
+    for (int e = 0; e < DD; e++) {
+        g.pblk[o + e] = Ops::to(at(0, e));
+        g.pblk0[o + e] = Ops::to(at(1, e));
+    }
 }
 
 // shared-memory bytes of one k_schur launch
@@ -572,7 +578,7 @@ SchurKernel schur_pick_ops(int mode) {
 // mixed = true selects the double-float arithmetic
 template <int DP, int W>
 SchurKernel schur_pick(int mode, bool mixed) {
-    return mixed ? schur_pick_ops<OpsF, DP, W>(mode) : schur_pick_ops<OpsD, DP, W>(mode);
+    return mixed ? schur_pick_ops<OpsP, DP, W>(mode) : schur_pick_ops<OpsD, DP, W>(mode);
 }
 
 // the thread-per-frequency BLOCK kernels, D = 1 .. 3 (schur_tpi.cu)

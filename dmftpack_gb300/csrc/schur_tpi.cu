@@ -4,9 +4,9 @@
 namespace dg {
 SchurKernel schur_tpi_kernel(int D, bool mixed) {
     switch (D) {
-        case 1: return mixed ? k_schur_tpi<OpsF, 1> : k_schur_tpi<OpsD, 1>;
-        case 2: return mixed ? k_schur_tpi<OpsF, 2> : k_schur_tpi<OpsD, 2>;
-        case 3: return mixed ? k_schur_tpi<OpsF, 3> : k_schur_tpi<OpsD, 3>;
+        case 1: return mixed ? k_schur_tpi<OpsP, 1> : k_schur_tpi<OpsD, 1>;
+        case 2: return mixed ? k_schur_tpi<OpsP, 2> : k_schur_tpi<OpsD, 2>;
+        case 3: return mixed ? k_schur_tpi<OpsP, 3> : k_schur_tpi<OpsD, 3>;
     }
     return nullptr;
 }
