@@ -458,13 +458,15 @@ __device__ __forceinline__ bool warp_gj_inverse_t(typename Ops::C (&a)[N], const
 // the rows of each lane's column are rotated by one after every step, so the current pivot row is always
 // register a[0] and the loop body is the same for every step (no dynamic register indexing).  The code is N
 // times shorter than the unrolled form, which matters for large N, where the kernels are bound by instruction
-// fetch.  Row r of step j sits in register (r - j) mod N; after N steps every row is back in place.
+// fetch.  Row r of step j sits in register (r - j) mod N; after N steps every row is back in place.  The interchange
+// of a step (8 selects per row) and its undoing at the end (N^2 exchanges) are skipped when no group of the warp pivots
+// off the diagonal, which is the rule: above the first hundred or so Matsubara frequencies iw dominates the matrix.
 template <class Ops, int N, int W>
 __device__ __forceinline__ bool warp_gj_inverse_rolled(typename Ops::C (&a)[N], const int c) {
     typedef typename Ops::C C;
     typedef typename Ops::M M;
     static_assert(N <= W && W <= 32 && (W & (W - 1)) == 0, "bad lane group");
-    bool singular = false;
+    bool singular = false, moved = false;
     int perm[N];
 #pragma unroll 1
     for (int j = 0; j < N; j++) {
@@ -483,13 +485,16 @@ __device__ __forceinline__ bool warp_gj_inverse_rolled(typename Ops::C (&a)[N], 
         best = __shfl_sync(0xffffffffu, best, j, W);
         singular |= !(best > M(0));
         perm[j] = pp + j;  // the row index of the pivot
+        if (__any_sync(0xffffffffu, pp != 0)) {
+            moved = true;
 #pragma unroll
-        for (int i = 1; i < N; i++)
-            if (i == pp) {
-                const C t = a[0];
-                a[0] = a[i];
-                a[i] = t;
-            }
+            for (int i = 1; i < N; i++)
+                if (i == pp) {
+                    const C t = a[0];
+                    a[0] = a[i];
+                    a[i] = t;
+                }
+        }
         const C piv = Ops::shfl(a[0], j, W);
         const C ipiv = Ops::rcp(piv);
         const C t = Ops::mul(a[0], ipiv);
@@ -507,6 +512,7 @@ __device__ __forceinline__ bool warp_gj_inverse_rolled(typename Ops::C (&a)[N], 
         for (int i = 0; i < N - 1; i++) a[i] = a[i + 1];
         a[N - 1] = r0;
     }
+    if (!moved) return singular;
 #pragma unroll 1
     for (int j = N - 1; j >= 0; j--) {
         const int p = perm[j];
@@ -526,7 +532,7 @@ template <class Ops, int N>
 __device__ __forceinline__ bool group_gj_inverse(typename Ops::C (&a)[N], const int c, const int base) {
     typedef typename Ops::C C;
     typedef typename Ops::M M;
-    bool singular = false;
+    bool singular = false, moved = false;
     int perm[N];
 #pragma unroll 1
     for (int j = 0; j < N; j++) {
@@ -544,13 +550,16 @@ __device__ __forceinline__ bool group_gj_inverse(typename Ops::C (&a)[N], const 
         best = __shfl_sync(0xffffffffu, best, base + j, 32);
         singular |= !(best > M(0));
         perm[j] = pp + j;
+        if (__any_sync(0xffffffffu, pp != 0 && base <= 32 - N)) {
+            moved = true;
 #pragma unroll
-        for (int i = 1; i < N; i++)
-            if (i == pp) {
-                const C t = a[0];
-                a[0] = a[i];
-                a[i] = t;
-            }
+            for (int i = 1; i < N; i++)
+                if (i == pp) {
+                    const C t = a[0];
+                    a[0] = a[i];
+                    a[i] = t;
+                }
+        }
         const C piv = Ops::shfl(a[0], base + j, 32);
         const C ipiv = Ops::rcp(piv);
         const C t = Ops::mul(a[0], ipiv);
@@ -567,6 +576,7 @@ __device__ __forceinline__ bool group_gj_inverse(typename Ops::C (&a)[N], const 
         for (int i = 0; i < N - 1; i++) a[i] = a[i + 1];
         a[N - 1] = r0;
     }
+    if (!moved) return singular;
 #pragma unroll 1
     for (int j = N - 1; j >= 0; j--) {
         const int p = perm[j];
