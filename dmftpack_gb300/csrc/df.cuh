@@ -205,6 +205,8 @@ struct OpsD {
     static DG_HD C pacc(C w, R p, C acc) { return cmk(::fma(w.x, p, acc.x), ::fma(w.y, p, acc.y)); }
     static DG_HD C pnorm(C a) { return a; }
     static DG_HD C pscale(C a, R r) { return cmk(a.x * r, a.y * r); }
+    static DG_HD R rdotc(C a, C b) { return ::fma(a.x, b.x, a.y * b.y); }  // Re(a conj b)
+    static DG_HD void balance(C &, C &) {}
 };
 
 struct OpsF {
@@ -365,11 +367,7 @@ struct OpsP {
         return pdf_fma2(pdf_re(a), pdf_neg(b), pdf_im(a), pdf_neg(pdf_i(b)), acc);
     }
     static __device__ __forceinline__ C rcp(C a) {  // conj(a)/|a|^2
-        float2 e;
-        const float2 p = pdf_prod(a, a, e);
-        const dfl s = two_sum(p.x, p.y);
-        const dfl r = df_rcp(fast_two_sum(s.h, f_add(s.l, f_add(e.x, e.y))));
-        return pdf_mul(conj(a), pdf_both(r));
+        return pdf_mul(conj(a), pdf_both(df_rcp(rdotc(a, a))));
     }
     static __device__ __forceinline__ double re(C a) { return df_val(cre(a)); }
     static __device__ __forceinline__ double im(C a) { return df_val(cim(a)); }
@@ -389,6 +387,19 @@ struct OpsP {
     static __device__ __forceinline__ C pacc(C w, R p, C acc) { return pdf_fma_lazy(w, pdf_both(p), acc); }
     static __device__ __forceinline__ C pnorm(C a) { return pdf_fast_two_sum(a.h, a.l); }
     static __device__ __forceinline__ C pscale(C a, R r) { return pdf_mul(a, pdf_both(r)); }
+    // num and den by the power of two that takes |den| to about 1, so that |den|^2 stays in the FP32 range
+    static __device__ __forceinline__ void balance(C &num, C &den) {
+        const float mx = fmaxf(fabsf(den.h.x), fabsf(den.h.y));
+        const float2 sc = p2(__int_as_float((254 << 23) - (__float_as_int(mx) & 0x7f800000)));
+        num = {p2_mul(num.h, sc), p2_mul(num.l, sc)};
+        den = {p2_mul(den.h, sc), p2_mul(den.l, sc)};
+    }
+    static __device__ __forceinline__ R rdotc(C a, C b) {  // Re(a conj b)
+        float2 e;
+        const float2 p = pdf_prod(a, b, e);
+        const dfl s = two_sum(p.x, p.y);
+        return fast_two_sum(s.h, f_add(s.l, f_add(e.x, e.y)));
+    }
     static __device__ __forceinline__ C shfl(C v, int src, int w) {
         C o;
         o.h.x = __shfl_sync(0xffffffffu, v.h.x, src, w);

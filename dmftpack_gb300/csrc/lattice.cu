@@ -704,29 +704,33 @@ __global__ void k_schur_reduce(int nchunk, int nf2, int DD, int mode, const doub
 int run_schur(dmftgpu_ctx *ctx, const Prepared &P, int mode, double mu, int wgrid, double2 *blk, double2 *blk0,
               double *tr, double *dtr, bool mixed) {
     const SInst *in = pick_schur(P.D);
-    // BLOCK passes of correlated blocks up to 3 x 3: one thread per frequency (k_schur_tpi).  It stages the
-    // Hermitian pole products of each staged k; prepare() caps n at 64 (the static eigensolver), so one k needs
+    // Matsubara passes of correlated blocks up to 3 x 3: one thread per frequency (k_schur_tpi, k_trace_tpi), which beats
+    // the lane groups at every width they cover (their groups idle at D = 3 and spend their issue slots on exchanges).
+    // They stage the Hermitian pole products of each staged k; prepare() caps n at 64 (the static eigensolver), so one k needs
     // at most 63 * (3 * 16 + 3 * 8 + 8) + 9 * 16 B = 5.2 KB (beside 55 KB of per-thread sums) and the 200 KB check below never rejects a tpi pass.
-    const bool tpi = mode == dg::S_BLOCK && P.D <= 3;
-    SchurKernel kern = tpi ? dg::schur_tpi_kernel(P.D, mixed) : in->get(mode, mixed);
+    const bool tpi = !(mode & dg::S_REAL) && P.D <= 3, trace = (mode & dg::S_TRACE) != 0;
+    SchurKernel kern = tpi ? dg::schur_tpi_kernel(P.D, mode, mixed) : in->get(mode, mixed);
     const int m = P.n - P.D, NG = tpi ? 128 : dg::schur_groups(in->SW), DD = P.D * P.D;
     const int nf2 = (mode & dg::S_REAL) ? P.Nf : 2 * P.Nf;  // the real axis has exactly the caller's points
     auto smem_of = [&](int kc_) {
-        return tpi ? dg::schur_tpi_smem(kc_, P.D, m, mixed) : dg::schur_smem(in->DP, in->SW, mode, kc_, P.D, m, P.n);
+        return tpi && trace ? dg::trace_tpi_stage(kc_, P.D, m, P.n)
+               : tpi          ? dg::schur_tpi_smem(kc_, P.D, m, mixed)
+                              : dg::schur_smem(in->DP, in->SW, mode, kc_, P.D, m, P.n);
     };
     int kc = 16;
     // three CTAs per SM where the thread-per-frequency kernel keeps its sums in shared memory, else two
-    const size_t cap = (tpi && mixed && P.D == 3 ? 74 : 96) * 1024;
+    const size_t cap = (tpi && !trace && mixed && P.D == 3 ? 74 : 96) * 1024;
     while (kc > 1 && smem_of(kc) > cap) kc /= 2;
     const size_t smem = smem_of(kc);
     if (smem > 200 * 1024) return dg_fail(ctx, DMFTGPU_BADARG, "lattice: correlated block too large");
     DG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    // k chunks: enough CTAs for `cps` per SM (8 unless tuned), at least 64 k points per chunk
+    // k chunks: enough CTAs for `cps` per SM (8 unless tuned), at least 8 k points per chunk (below that a CTA's setup
+    // and the partial sums cost more than the idle SMs; with 64 a 484-k, 800-point pass ran 56 CTAs on 152 SMs)
     const int fblocks = dg_ceil_div(nf2, NG);
     int nsm = 152;
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, ctx->device);
     auto chunks = [&](int cps, int *kchunk_out) {
-        int nc = std::max(1, std::min(dg_ceil_div(P.nk, 64), dg_ceil_div(cps * nsm, fblocks)));
+        int nc = std::max(1, std::min(dg_ceil_div(P.nk, 8), dg_ceil_div(cps * nsm, fblocks)));
         const int kch = dg_ceil_div(P.nk, nc);
         *kchunk_out = kch;
         return dg_ceil_div(P.nk, kch);
@@ -773,7 +777,7 @@ int run_schur(dmftgpu_ctx *ctx, const Prepared &P, int mode, double mu, int wgri
     g.ptr = ptr;
     g.status = ctx->d_status;
     // the TRACE passes read the static eigenvalues (Tr G0), computed on the side stream
-    if (!(mode & dg::S_REAL) && ((mode & dg::S_TRACE) || ((mode & dg::S_BLOCK) && in->DP >= 8)))
+    if (!(mode & dg::S_REAL) && (trace || ((mode & dg::S_BLOCK) && in->DP >= 8)))
         DG_CUDA(cudaStreamWaitEvent(ctx->stream, P.static_ready, 0));
     // autotuning: time 4, 8 and 16 CTAs per SM once per (width, mode, precision, N_k, points) and keep the fastest
     auto tuned = ctx->tuned.find(key);

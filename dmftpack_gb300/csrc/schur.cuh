@@ -398,6 +398,35 @@ inline size_t schur_tpi_smem(int kc, int D, int m, bool mixed) {
     return schur_tpi_stage(kc, D, m) + (mixed && D == 3 ? 3 * (size_t)D * D * 16 * 128 : 0);
 }
 
+// the staged data of the thread-per-frequency kernels for nkc k points from k0: P_l off-diagonal pairs, P_l diagonal,
+// mu - e_l and -H_PP (minus m0 with `static_part`)
+template <class Ops, int D>
+__device__ __forceinline__ void tpi_stage(const SchurArgs &g, int k0, int nkc, typename Ops::C *sPo, typename Ops::R *sPd,
+                                          typename Ops::R *sE, typename Ops::C *sH, bool static_part) {
+    constexpr int DD = D * D, NP = D * (D - 1) / 2;
+    const int m = g.m;
+    for (int t = threadIdx.x; t < nkc * m * D; t += blockDim.x) {
+        const double2 b = g.B[((size_t)k0 * m + t / D) * D + t % D];
+        sPd[t] = Ops::rfrom(b.x * b.x + b.y * b.y);
+    }
+    if constexpr (NP > 0)
+        for (int t = threadIdx.x; t < nkc * m * NP; t += blockDim.x) {
+            int q = t % NP, a = 0;  // pair q in row-major order over the strict upper triangle
+            while (q >= D - 1 - a) {
+                q -= D - 1 - a;
+                a++;
+            }
+            const double2 *bl = g.B + ((size_t)k0 * m + t / NP) * D;
+            sPo[t] = Ops::from(cmulc(bl[a], bl[a + 1 + q]));
+        }
+    for (int t = threadIdx.x; t < nkc * m; t += blockDim.x) sE[t] = Ops::rfrom(g.mu - g.epsQ[(size_t)k0 * m + t]);
+    for (int t = threadIdx.x; t < nkc * DD; t += blockDim.x) {
+        const int kk = t / DD, e = t % DD, a = e % D, b = e / D;
+        const double2 h = cneg(g.H[(size_t)(k0 + kk) * g.n * g.n + a + (size_t)b * g.n]);
+        sH[t] = Ops::from(static_part ? csub(h, g.m0[e]) : h);
+    }
+}
+
 // BLOCK mode (G_loc and GwHF) for correlated blocks of D <= 3: one thread per Matsubara frequency, the whole
 // D x D S(z) and S0(z) of that thread's (k, iw) in its registers, inverted by thread_inverse.  A lane-group
 // k_schur at these widths leaves lanes idle (D < W) and spends its issue slots on the group's pivot broadcasts;
@@ -453,25 +482,7 @@ __global__ void __launch_bounds__(128, tpi_shared<Ops, D> ? 3 : 1) k_schur_tpi(S
     for (int k0 = kbeg; k0 < kend; k0 += g.kc) {
         const int nkc = min(g.kc, kend - k0);
         __syncthreads();
-        for (int t = threadIdx.x; t < nkc * m * D; t += blockDim.x) {
-            const double2 b = g.B[((size_t)k0 * m + t / D) * D + t % D];
-            sPd[t] = Ops::rfrom(b.x * b.x + b.y * b.y);
-        }
-        if (NP > 0)
-            for (int t = threadIdx.x; t < nkc * m * NP; t += blockDim.x) {
-                int q = t % NP, a = 0;  // pair q in row-major order over the strict upper triangle
-                while (q >= D - 1 - a) {
-                    q -= D - 1 - a;
-                    a++;
-                }
-                const double2 *bl = g.B + ((size_t)k0 * m + t / NP) * D;
-                sPo[t] = Ops::from(cmulc(bl[a], bl[a + 1 + q]));
-            }
-        for (int t = threadIdx.x; t < nkc * m; t += blockDim.x) sE[t] = Ops::rfrom(g.mu - g.epsQ[(size_t)k0 * m + t]);
-        for (int t = threadIdx.x; t < nkc * DD; t += blockDim.x) {
-            const int kk = t / DD, e = t % DD, a = e % D, b = e / D;
-            sH[t] = Ops::from(csub(cneg(g.H[(size_t)(k0 + kk) * g.n * g.n + a + (size_t)b * g.n]), g.m0[e]));
-        }
+        tpi_stage<Ops, D>(g, k0, nkc, sPo, sPd, sE, sH, true);
         __syncthreads();
         for (int kk = 0; kk < nkc; kk++) {
             const C *po = sPo + (size_t)kk * m * NP, *hp = sH + (size_t)kk * DD;
@@ -552,6 +563,219 @@ __global__ void __launch_bounds__(128, tpi_shared<Ops, D> ? 3 : 1) k_schur_tpi(S
     }
 }
 
+// TRACE modes (N(mu), dN/dmu) for D <= 3: one thread per Matsubara frequency, like k_schur_tpi and on the same staged
+// Hermitian pole products.  With M = z - H_PP - Sigma - sum_l w_l P_l, R = sum_l w_l^2 P_l = M' - I, T = sum_l w_l^3 P_l:
+//   Tr G = Tr[M^-1 (I + R)] + sum_l w_l,   d/dz Tr G = -(Tr X^2 + 2 Tr[M^-1 T] + sum_l w_l^2),   X = M^-1 (I + R),
+// and only real parts are summed.  2 x 2 blocks take the closed form Tr[adj(M) (I + R)] / det M, so the whole point of
+// a ligand-free two-orbital model is one complex determinant.  In FP64 the kernel is bound by the FP64 pipe (0.63e12
+// FMA/s), where a division costs as much as ten products: the real fractions of a point (the block's trace and the
+// x_j / (x_j^2 + w^2) of Tr G0) are therefore added over a common denominator, four at a time.  A pass over 64 x 64 k
+// and 4096 points of the two-orbital model takes 1.3 ms (lane groups: 4.1 ms), in double-float 0.37 ms (0.89 ms).
+__host__ __device__ inline size_t trace_tpi_stage(int kc, int D, int m, int n) {
+    return schur_tpi_stage(kc, D, m) + ((size_t)kc * n * 8 + 15) / 16 * 16;
+}
+// running sum of real fractions: FP64 keeps one numerator and denominator for four terms, double-float (whose
+// reciprocal costs less than the products) divides each
+template <class Ops>
+struct FracSum;
+template <>
+struct FracSum<OpsD> {
+    double sum = 0.0, num = 0.0, den = 1.0;
+    int cnt = 0;
+    __device__ __forceinline__ void add(double n, double d) {
+        if (cnt == 0) {
+            num = n;
+            den = d;
+        } else {
+            num = ::fma(num, d, n * den);
+            den *= d;
+        }
+        if (++cnt == 4) flush();
+    }
+    __device__ __forceinline__ void flush() {
+        if (cnt) sum += num / den;
+        cnt = 0;
+    }
+    __device__ __forceinline__ double value() {
+        flush();
+        return sum;
+    }
+};
+template <>
+struct FracSum<OpsP> {
+    dfl sum = {0.f, 0.f};
+    __device__ __forceinline__ void add(dfl n, dfl d) { sum = df_fma(n, df_rcp(d), sum); }
+    __device__ __forceinline__ double value() { return df_val(sum); }
+};
+
+template <class Ops, int D, bool DERIV>
+__global__ void __launch_bounds__(128) k_trace_tpi(SchurArgs g) {
+    typedef typename Ops::C C;
+    typedef typename Ops::R R;
+    extern __shared__ double2 sm[];
+    constexpr int DD = D * D, NP = D * (D - 1) / 2, NS = DERIV ? 3 : 2;
+    const int m = g.m, n = g.n;
+    C *sPo = reinterpret_cast<C *>(sm);
+    C *sH = sPo + (size_t)g.kc * m * NP;
+    R *sPd = reinterpret_cast<R *>(sH + (size_t)g.kc * DD);
+    R *sE = sPd + (size_t)g.kc * m * D;
+    R *sE0 = reinterpret_cast<R *>(reinterpret_cast<char *>(sm) + schur_tpi_stage(g.kc, D, m));
+    const int f_raw = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool fvalid = f_raw < g.nf2;
+    const int f = fvalid ? f_raw : g.nf2 - 1;
+    const int chunk = blockIdx.y;
+    const int kbeg = chunk * g.kchunk, kend = min(g.nk, kbeg + g.kchunk);
+    const double w = g.wgrid ? (DG_PI / g.beta + f * ((2 * DG_PI) / g.beta)) : (DG_PI * (2. * f + 1.) / g.beta);
+    const R wr = Ops::rfrom(w), w2 = Ops::rmul(wr, wr);
+    C zs[D][D];  // z - Sigma(iw)
+#pragma unroll
+    for (int a = 0; a < D; a++)
+#pragma unroll
+        for (int b = 0; b < D; b++) {
+            const C sg = Ops::from(g.sig[(size_t)f * DD + a + b * D]);
+            zs[a][b] = a == b ? Ops::sub(Ops::from(cmk(g.mu, w)), sg) : Ops::neg(sg);
+        }
+    double acc1 = 0.0, acc2 = 0.0;
+    bool sing = false;
+    for (int k0 = kbeg; k0 < kend; k0 += g.kc) {
+        const int nkc = min(g.kc, kend - k0);
+        __syncthreads();
+        tpi_stage<Ops, D>(g, k0, nkc, sPo, sPd, sE, sH, false);
+        for (int t = threadIdx.x; t < nkc * n; t += blockDim.x) sE0[t] = Ops::rfrom(g.mu - g.eps0[(size_t)k0 * n + t]);
+        __syncthreads();
+        for (int kk = 0; kk < nkc; kk++) {
+            const C *po = sPo + (size_t)kk * m * NP, *hp = sH + (size_t)kk * DD;
+            const R *pd = sPd + (size_t)kk * m * D, *es = sE + (size_t)kk * m, *e0 = sE0 + (size_t)kk * n;
+            // pole sums of w, w^2 (and w^3): [diagonal, (A, B)], [upper triangle: real parts], [imaginary parts]
+            C Q[NS][D], Qr[NS][NP ? NP : 1], Qi[NS][NP ? NP : 1];
+            C sw = Ops::zero(), sw2 = Ops::zero();  // sum_l w_l, sum_l w_l^2
+#pragma unroll
+            for (int t = 0; t < NS; t++) {
+#pragma unroll
+                for (int a = 0; a < D; a++) Q[t][a] = Ops::zero();
+#pragma unroll
+                for (int q = 0; q < NP; q++) Qr[t][q] = Qi[t][q] = Ops::zero();
+            }
+            auto renorm = [&]() {
+#pragma unroll
+                for (int t = 0; t < NS; t++) {
+#pragma unroll
+                    for (int a = 0; a < D; a++) Q[t][a] = Ops::pnorm(Q[t][a]);
+#pragma unroll
+                    for (int q = 0; q < NP; q++) {
+                        Qr[t][q] = Ops::pnorm(Qr[t][q]);
+                        Qi[t][q] = Ops::pnorm(Qi[t][q]);
+                    }
+                }
+            };
+            for (int l = 0; l < m; l++) {
+                if (l > 0 && (l & 15) == 0) renorm();
+                const R x = es[l];
+                C wt[NS];
+                wt[0] = Ops::pscale(Ops::mk(x, Ops::rneg(wr)), Ops::rrcp(Ops::rfma(x, x, w2)));
+                wt[1] = Ops::mul(wt[0], wt[0]);
+                if (DERIV) wt[2] = Ops::mul(wt[1], wt[0]);
+                sw = Ops::add(sw, wt[0]);
+                if (DERIV) sw2 = Ops::add(sw2, wt[1]);
+#pragma unroll
+                for (int t = 0; t < NS; t++) {
+#pragma unroll
+                    for (int a = 0; a < D; a++) Q[t][a] = Ops::pacc(wt[t], pd[(size_t)l * D + a], Q[t][a]);
+#pragma unroll
+                    for (int q = 0; q < NP; q++) {
+                        const C p = po[(size_t)l * NP + q];
+                        Qr[t][q] = Ops::pacc(wt[t], Ops::cre(p), Qr[t][q]);
+                        Qi[t][q] = Ops::pacc(wt[t], Ops::cim(p), Qi[t][q]);
+                    }
+                }
+            }
+            // entry (a, b) of sum t
+            auto entry = [&](int t, int a, int b) {
+                if (a == b) return Q[t][a];
+                const int i = a < b ? a : b, j = a < b ? b : a, q = i * D - i * (i + 1) / 2 + (j - i - 1);
+                const R Ar = Ops::cre(Qr[t][q]), Br = Ops::cim(Qr[t][q]), Ai = Ops::cre(Qi[t][q]), Bi = Ops::cim(Qi[t][q]);
+                return a < b ? Ops::mk(Ops::rsub(Ar, Bi), Ops::radd(Ai, Br)) : Ops::mk(Ops::radd(Ar, Bi), Ops::rsub(Br, Ai));
+            };
+            C M[D][D];
+#pragma unroll
+            for (int a = 0; a < D; a++)
+#pragma unroll
+                for (int b = 0; b < D; b++) M[a][b] = Ops::add(hp[a + b * D], zs[a][b]);
+            if (m > 0) {
+                renorm();
+#pragma unroll
+                for (int a = 0; a < D; a++)
+#pragma unroll
+                    for (int b = 0; b < D; b++) M[a][b] = Ops::sub(M[a][b], entry(0, a, b));
+            }
+            // (I + R)(a, b)
+            auto IR = [&](int a, int b) {
+                C v = m > 0 ? entry(1, a, b) : Ops::zero();
+                return a == b ? Ops::add(v, Ops::one()) : v;
+            };
+            FracSum<Ops> fr;
+            if constexpr (D == 2 && !DERIV) {
+                C det = Ops::fms(M[0][1], M[1][0], Ops::mul(M[0][0], M[1][1]));
+                C num;
+                if (m > 0) {
+                    num = Ops::fma(M[0][0], IR(1, 1), Ops::mul(M[1][1], IR(0, 0)));
+                    num = Ops::fms(M[0][1], IR(1, 0), num);
+                    num = Ops::fms(M[1][0], IR(0, 1), num);
+                } else {
+                    num = Ops::add(M[0][0], M[1][1]);
+                }
+                Ops::balance(num, det);
+                sing |= !(Ops::mag2(det) > 0);
+                fr.add(Ops::rdotc(num, det), Ops::rdotc(det, det));  // Re(num / det) = Re(num conj det) / |det|^2
+            } else if constexpr (D == 1 && !DERIV) {
+                C num = m > 0 ? IR(0, 0) : Ops::one(), det = M[0][0];
+                Ops::balance(num, det);
+                sing |= !(Ops::mag2(det) > 0);
+                fr.add(Ops::rdotc(num, det), Ops::rdotc(det, det));
+            } else {
+                sing |= thread_inverse<Ops, D>(M);
+                C t = Ops::zero(), t2 = Ops::zero(), X[D][D];
+#pragma unroll
+                for (int a = 0; a < D; a++)
+#pragma unroll
+                    for (int b = 0; b < D; b++) {
+                        if (!DERIV && a != b) continue;
+                        if (m > 0) {
+                            X[a][b] = Ops::zero();
+#pragma unroll
+                            for (int c = 0; c < D; c++) X[a][b] = Ops::fma(M[a][c], IR(c, b), X[a][b]);
+                        } else {
+                            X[a][b] = M[a][b];
+                        }
+                        if (a == b) t = Ops::add(t, X[a][b]);
+                        if (DERIV && m > 0) t2 = Ops::fma(Ops::add(M[a][b], M[a][b]), entry(2, b, a), t2);
+                    }
+                acc1 += Ops::re(t);
+                if (DERIV) {
+#pragma unroll
+                    for (int a = 0; a < D; a++)
+#pragma unroll
+                        for (int b = 0; b < D; b++) t2 = Ops::fma(X[a][b], X[b][a], t2);
+                    acc2 -= Ops::re(Ops::add(t2, sw2));
+                }
+            }
+            if (m > 0) acc1 += Ops::re(sw);
+            // - Tr G0 = - sum_j Re 1/(z - e0_j) (and + sum_j Re 1/(z - e0_j)^2)
+            for (int j = 0; j < n; j++) {
+                const R x = e0[j], d = Ops::rfma(x, x, w2);
+                fr.add(Ops::rneg(x), d);
+                if (DERIV) {
+                    const C r = Ops::pscale(Ops::mk(x, Ops::rneg(wr)), Ops::rrcp(d));
+                    acc2 += Ops::re(Ops::mul(r, r));
+                }
+            }
+            acc1 += fr.value();
+        }
+    }
+    if (sing && fvalid) dg_flag(g.status, DG_SINGULAR);
+    if (fvalid) g.ptr[(size_t)chunk * g.nf2 + f] = cmk(acc1, acc2);
+}
+
 // shared-memory bytes of one k_schur launch
 inline size_t schur_smem(int DP, int W, int mode, int kc, int D, int m, int n) {
     const int NG = schur_groups(W);
@@ -581,8 +805,8 @@ SchurKernel schur_pick(int mode, bool mixed) {
     return mixed ? schur_pick_ops<OpsP, DP, W>(mode) : schur_pick_ops<OpsD, DP, W>(mode);
 }
 
-// the thread-per-frequency BLOCK kernels, D = 1 .. 3 (schur_tpi.cu)
-SchurKernel schur_tpi_kernel(int D, bool mixed);
+// the thread-per-frequency kernels, D = 1 .. 3: BLOCK, TRACE or TRACE | DERIV (schur_tpi.cu)
+SchurKernel schur_tpi_kernel(int D, int mode, bool mixed);
 
 #define DG_SCHUR_INST(DP, W) \
     SchurKernel schur_kernel_##DP(int mode, bool mixed) { return schur_pick<DP, W>(mode, mixed); }
