@@ -145,6 +145,7 @@ int dmftgpu_destroy(dmftgpu_ctx *ctx) {
     delete ctx->pulay;
     for (auto &kv : ctx->bufs)
         if (kv.second.p) cudaFree(kv.second.p);
+    if (ctx->pinned) cudaFreeHost(ctx->pinned);
     if (ctx->d_status) cudaFree(ctx->d_status);
     if (ctx->side) {
         cudaStreamSynchronize(ctx->side);

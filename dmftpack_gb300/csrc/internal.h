@@ -52,6 +52,8 @@ struct dmftgpu_ctx {
     cudaGraphExec_t graph = nullptr;  // the last captured batched pass
     std::string graph_key;
     std::map<std::string, std::vector<std::pair<cudaEvent_t, cudaEvent_t>>> events;
+    void *pinned = nullptr;           // pinned staging of dmftgpu_hk's hopping table (grow-only)
+    size_t pinned_bytes = 0;
     std::string hk_phase_key;         // (k mesh, R list) of the phase-slice image in workspace "hk.tc.A"
     bool tensor = true;               // tensor-core contractions allowed in the mixed form (!DMFTGPU_NO_TENSOR)
     int nk_krylov = 0;                // Jacobian-vector products of the last Newton-Krylov mixer step (0: none)
