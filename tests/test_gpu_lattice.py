@@ -29,6 +29,18 @@ def test_hk_matches_oracle(ctx, orc):
     assert rel_err(Hd.cpu().numpy(), H) < 1e-13
 
 
+@pytest.mark.parametrize("mixed", [False, True])
+def test_hk_rows_in_any_order(ctx, orc, mixed):
+    """Rows of one lattice vector that do not follow each other, repeated rows, a table larger than the previous one."""
+    rng = np.random.default_rng(5)
+    for n, nvec in ((2, 3), (5, 27)):
+        R = rng.integers(-3, 4, size=(nvec, 3))
+        rows = np.concatenate([R[rng.integers(0, nvec, 40 * nvec)], rng.integers(0, n, size=(40 * nvec, 2))], 1).astype(np.int32)
+        hr = rng.normal(size=len(rows)) + 1j * rng.normal(size=len(rows))
+        H = orc.hk(n, rows, hr, orc.kmesh(3, 4, 5))
+        assert rel_err(ctx.Construct_Hk(n, rows, hr, (3, 4, 5), mixed=mixed), H) < (1e-10 if mixed else 1e-13)
+
+
 @pytest.mark.parametrize("case", ["t2g_p", "dp28", "soc56", "hubbard"])
 def test_hk_tensor_cores_match_oracle(ctx, orc, case):
     """H(k) as a tcgen05 GEMM (bf16 slices, exact level sums): k counts and 2 n^2 that are not multiples of the
@@ -213,6 +225,33 @@ def test_adjust_mu_bisection_matches_oracle_and_newton_converges(ctx, orc):
     assert abs(mu_n - mu_o) < 2e-5
     assert abs(orc.nele(H, wl.sigma, mu_n, wl.beta, wl.ncl, wl.nh) - target) < 1e-9
     assert ne_n < ne_o
+
+
+def _random_lattice(n, D, kgrid, nf, seed):
+    rng = np.random.default_rng(seed)
+    nk = kgrid[0] * kgrid[1] * kgrid[2]
+    A = rng.normal(size=(nk, n, n)) + 1j * rng.normal(size=(nk, n, n))
+    H = (A + A.conj().transpose(0, 2, 1)) / 2
+    w = np.pi * (2 * np.arange(nf) + 1) / 15.0
+    S = np.zeros((nf, D, D), complex)
+    S[:, np.arange(D), np.arange(D)] = -1j * rng.uniform(0.4, 0.6, D) / (w[:, None] + rng.uniform(0.8, 1.2, D))
+    return H, S, lib.Lattice(n, nk, nf, 15.0, 1, D)
+
+
+@pytest.mark.parametrize("n,D,kgrid,nf", [(1, 1, (3, 1, 1), 24), (2, 1, (5, 3, 1), 64), (2, 2, (7, 1, 1), 65),
+                                          (3, 2, (3, 3, 1), 24), (3, 3, (9, 1, 1), 24), (9, 3, (17, 1, 1), 70),
+                                          (40, 3, (2, 2, 2), 24), (33, 2, (3, 1, 1), 129)])
+def test_nele_small_blocks(ctx, orc, n, D, kgrid, nf):
+    """N(mu) and dN/dmu of correlated blocks up to 3 x 3 (one thread per frequency): without ligands, with one and with
+    more poles than a renormalisation run, k counts around the staging and chunk sizes, ragged frequency tiles; bounds
+    of the other N(mu) tests (FP64 1e-11, double-float 1e-9)."""
+    H, S, lat = _random_lattice(n, D, kgrid, nf, [n, D, nf])
+    for mu in (-0.4, 0.3):
+        N, dN = orc.nele(H, S, mu, 15.0, 1, D, deriv=True)
+        for mixed, tol in ((False, 1e-11), (True, 1e-9)):
+            g, dg = ctx.GiwToNele(lat, H, S, mu, deriv=True, mixed=mixed)
+            assert abs(g - N) <= tol * max(1, abs(N)) and abs(dg - dN) <= 10 * tol * max(1, abs(dN))
+            assert abs(ctx.GiwToNele(lat, H, S, mu, mixed=mixed) - N) <= tol * max(1, abs(N))
 
 
 @pytest.mark.parametrize("newton", [False, True])
