@@ -5,7 +5,7 @@
 //  * block_heig: Hermitian eigen-decomposition by one thread block.  Like thread_heig (and
 //    Eigen::SelfAdjointEigenSolver) it reads only the lower triangle, takes the diagonal real and returns
 //    ascending eigenvalues, with the same complex Jacobi rotation and the same stopping rule
-//    (off-diagonal mass <= 1e-28 of the total); the rotations of one sweep are applied in round-robin
+//    (off-diagonal mass <= 1e-28 of the total); the rotations (jacobi_rotation) of one sweep are applied in round-robin
 //    ("tournament") order, n/2 disjoint (p, q) pairs at a time, so a sweep takes n - 1 parallel steps.
 //  * block_matmul: C = A B, one thread per element.
 //  * posdef_lower: is the Hermitian matrix s * (lower triangle of M) - shift * I positive definite (strict)
@@ -21,6 +21,45 @@ struct DgRot {
     double c, s;
     double2 ph;
 };
+
+// The rotation of the (p, q) plane.  What must hold to rounding is that it is unitary: c^2 + s^2 = 1 and |ph| = 1; the
+// angle only has to be close (each rotation then leaves 1e-6 of a_pq, and the sweeps still end quadratically), so it
+// comes from FP32, and c = (1 + t^2)^-1/2 and ph = a_pq / |a_pq| from one reciprocal-square-root refinement each.  A lone
+// warp's FP64 instruction takes 64 cycles, so the square roots and divisions of the exact angle (seven, ~10 dependent
+// instructions each) were two thirds of a round; this is 24 instructions.
+__device__ __forceinline__ double fast_rsqrt(double x) {  // x in [0.25, 1e30]
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-x * y, y, 1.0);                  // y (1 - e)^-1/2 = y (1 + e/2 + 3/8 e^2 + O(e^3))
+    return fma(y * e, fma(0.375, e, 0.5), y);
+}
+__device__ __forceinline__ DgRot jacobi_rotation(int p, int q, double2 apq, double app, double aqq) {
+    DgRot R;
+    R.p = p;
+    R.q = q;
+    R.on = 0;
+    R.c = 1.0;
+    R.s = 0.0;
+    R.ph = cmk(1, 0);
+    // a_pq scaled by a power of two to modulus [1, 2) or a little above; zero and denormal entries are left alone
+    const int ex = max(__double2hiint(fabs(apq.x)), __double2hiint(fabs(apq.y))) & 0x7ff00000;
+    if (ex == 0) return R;
+    const double sc = __hiloint2double(0x7fe00000 - ex, 0);
+    const double2 z = cscale(apq, sc);
+    const double r2 = cabs2(z), inv = fast_rsqrt(r2);
+    const double rr = r2 * inv, d = (aqq - app) * sc;
+    const float x = (float)d, r = (float)rr, ax = fabsf(x);
+    float t;
+    if (ax > 1e9f) t = __fdividef(r, ax);
+    else t = __fdividef(2.f * r, ax + sqrtf(fmaf(x, x, 4.f * r * r)));
+    if (ax > 1e30f) t = 0.f;
+    const double td = x < 0.f ? -(double)t : (double)t;
+    R.c = fast_rsqrt(fma(td, td, 1.0));
+    R.s = td * R.c;
+    R.ph = cscale(z, inv);
+    R.on = 1;
+    return R;
+}
 
 // all threads of the block call it; a, u: n*n shared, w: n shared doubles, order: n shared ints,
 // rot: n/2+1 shared DgRot, red: blockDim.x shared doubles.  Returns DG_OK or DG_NONCONV (block-uniform).
@@ -85,42 +124,21 @@ __device__ inline int block_heig(int n, const double2 *A0, double2 *a, double2 *
                     q = t;
                 }
                 DgRot R;
-                R.p = p;
-                R.q = q;
-                R.on = 0;
-                R.c = 1.0;
-                R.s = 0.0;
-                R.ph = cmk(1, 0);
-                if (q < n) {
-                    const double2 apq = DG_AT(a, n, p, q);
-                    const double rr = sqrt(cabs2(apq));
-                    if (rr != 0.0) {
-                        const double app = DG_AT(a, n, p, p).x, aqq = DG_AT(a, n, q, q).x;
-                        const double theta = (aqq - app) / (2.0 * rr);
-                        const double t = (theta >= 0 ? 1.0 : -1.0) / (fabs(theta) + sqrt(theta * theta + 1.0));
-                        R.c = 1.0 / sqrt(t * t + 1.0);
-                        R.s = t * R.c;
-                        R.ph = cmk(apq.x / rr, apq.y / rr);
-                        R.on = 1;
-                    }
-                }
+                if (q < n) R = jacobi_rotation(p, q, DG_AT(a, n, p, q), DG_AT(a, n, p, p).x, DG_AT(a, n, q, q).x);
+                else R.on = 0;
                 rot[tid] = R;
             }
             __syncthreads();
             // columns p, q of a (and u): a(:,p) = c a(:,p) - s conj(ph) a(:,q); a(:,q) = s a(:,p) + c conj(ph) a(:,q)
-            for (int x = tid; x < half * n; x += nt) {
-                const DgRot R = rot[x / n];
+            for (int x = tid; x < (u ? 2 : 1) * half * n; x += nt) {
+                double2 *M = x < half * n ? a : u;  // different threads take a's and u's columns
+                const int y = x < half * n ? x : x - half * n;
+                const DgRot R = rot[y / n];
                 if (!R.on) continue;
-                const int k = x % n;
-                const double2 phc = cconj(R.ph);
-                const double2 akp = DG_AT(a, n, k, R.p), akq = DG_AT(a, n, k, R.q);
-                DG_AT(a, n, k, R.p) = csub(cscale(akp, R.c), cscale(cmul(phc, akq), R.s));
-                DG_AT(a, n, k, R.q) = cadd(cscale(akp, R.s), cscale(cmul(phc, akq), R.c));
-                if (u) {
-                    const double2 ukp = DG_AT(u, n, k, R.p), ukq = DG_AT(u, n, k, R.q);
-                    DG_AT(u, n, k, R.p) = csub(cscale(ukp, R.c), cscale(cmul(phc, ukq), R.s));
-                    DG_AT(u, n, k, R.q) = cadd(cscale(ukp, R.s), cscale(cmul(phc, ukq), R.c));
-                }
+                const int k = y % n;
+                const double2 akp = DG_AT(M, n, k, R.p), z = cmul(cconj(R.ph), DG_AT(M, n, k, R.q));
+                DG_AT(M, n, k, R.p) = csub(cscale(akp, R.c), cscale(z, R.s));
+                DG_AT(M, n, k, R.q) = cadd(cscale(akp, R.s), cscale(z, R.c));
             }
             __syncthreads();
             // rows p, q: a(p,:) = c a(p,:) - s ph a(q,:); a(q,:) = s a(p,:) + c ph a(q,:)
@@ -133,14 +151,9 @@ __device__ inline int block_heig(int n, const double2 *A0, double2 *a, double2 *
                 DG_AT(a, n, R.q, k) = cadd(cscale(apk, R.s), cscale(cmul(R.ph, aqk), R.c));
             }
             __syncthreads();
-            if (tid < half) {
-                const DgRot R = rot[tid];
-                if (R.on) {
-                    DG_AT(a, n, R.p, R.q) = cmk(0, 0);
-                    DG_AT(a, n, R.q, R.p) = cmk(0, 0);
-                    DG_AT(a, n, R.p, R.p).y = 0.0;
-                    DG_AT(a, n, R.q, R.q).y = 0.0;
-                }
+            if (tid < half && rot[tid].on) {
+                DG_AT(a, n, rot[tid].p, rot[tid].p).y = 0.0;
+                DG_AT(a, n, rot[tid].q, rot[tid].q).y = 0.0;
             }
             __syncthreads();
         }
@@ -223,25 +236,8 @@ __device__ inline int warp_heig(int n, const double2 *A0, double2 *a, double2 *u
                     q = t;
                 }
                 DgRot R;
-                R.p = p;
-                R.q = q;
-                R.on = 0;
-                R.c = 1.0;
-                R.s = 0.0;
-                R.ph = cmk(1, 0);
-                if (q < n) {
-                    const double2 apq = DG_AT(a, n, p, q);
-                    const double rr = sqrt(cabs2(apq));
-                    if (rr != 0.0) {
-                        const double app = DG_AT(a, n, p, p).x, aqq = DG_AT(a, n, q, q).x;
-                        const double theta = (aqq - app) / (2.0 * rr);
-                        const double t = (theta >= 0 ? 1.0 : -1.0) / (fabs(theta) + sqrt(theta * theta + 1.0));
-                        R.c = 1.0 / sqrt(t * t + 1.0);
-                        R.s = t * R.c;
-                        R.ph = cmk(apq.x / rr, apq.y / rr);
-                        R.on = 1;
-                    }
-                }
+                if (q < n) R = jacobi_rotation(p, q, DG_AT(a, n, p, q), DG_AT(a, n, p, p).x, DG_AT(a, n, q, q).x);
+                else R.on = 0;
                 rot[lane] = R;
             }
             __syncwarp();
@@ -267,14 +263,9 @@ __device__ inline int warp_heig(int n, const double2 *A0, double2 *a, double2 *u
                 DG_AT(a, n, R.q, k) = cadd(cscale(apk, R.s), cscale(cmul(R.ph, aqk), R.c));
             }
             __syncwarp();
-            if (lane < half) {
-                const DgRot R = rot[lane];
-                if (R.on) {
-                    DG_AT(a, n, R.p, R.q) = cmk(0, 0);
-                    DG_AT(a, n, R.q, R.p) = cmk(0, 0);
-                    DG_AT(a, n, R.p, R.p).y = 0.0;
-                    DG_AT(a, n, R.q, R.q).y = 0.0;
-                }
+            if (lane < half && rot[lane].on) {
+                DG_AT(a, n, rot[lane].p, rot[lane].p).y = 0.0;
+                DG_AT(a, n, rot[lane].q, rot[lane].q).y = 0.0;
             }
             __syncwarp();
         }

@@ -27,6 +27,16 @@ DG_HD dfl df_div(dfl a, dfl b) {
     return fast_two_sum(q1, q2);
 }
 
+// a^-1/2, a > 0: the approximate root refined in FP32, then one double-float step on its residual e = 1 - a y^2,
+// y (1 + e/2 + 3/8 e^2)
+__device__ __forceinline__ dfl df_rsqrt(dfl a) {
+    float y = rsqrtf(a.h);
+    y = fmaf(0.5f * y, fmaf(-a.h * y, y, 1.f), y);
+    const dfl y2 = df_mul({y, 0.f}, {y, 0.f});
+    const dfl e = df_sub({1.f, 0.f}, df_mul(a, y2));
+    return fast_two_sum(y, y * e.h * fmaf(0.375f, e.h, 0.5f) + 0.5f * y * e.l);
+}
+
 // one Jacobi rotation of the (p, q) plane in double-float
 struct DfRot {
     int p, q, on;
@@ -101,27 +111,23 @@ __device__ inline int warp_heig_df(int n, const cdf *A0, cdf *a, cdf *u, double 
                     if (mx > 1e-37f) {
                         // |a_pq| and its phase from the entry scaled by a power of two to [0.5, 1): the squares of a
                         // small entry would otherwise lose their low parts to FP32 underflow (|a_pq|^2 < 1e-31), and
-                        // a phase that is not unit to double-float precision breaks the rotation's unitarity
+                        // a phase that is not unit to double-float precision breaks the rotation's unitarity.  The angle
+                        // only has to be close and is plain FP32 (jacobi_rotation, smallmat.cuh)
                         int ex = 0;
                         frexpf(mx, &ex);
                         const float sc = ldexpf(1.f, -ex);
                         const dfl ar = {apq.re.h * sc, apq.re.l * sc}, ai = {apq.im.h * sc, apq.im.l * sc};
-                        const dfl rrs = df_sqrt(df_fma(ai, ai, df_mul(ar, ar)));  // |a_pq| sc
-                        const dfl rr = {rrs.h / sc, rrs.l / sc};                  // exact: a power of two
-                        const dfl app = DG_AT(a, n, p, p).re, aqq = DG_AT(a, n, q, q).re;
-                        const dfl d = df_sub(aqq, app);
-                        dfl t;
-                        if (fabsf(d.h) > 2e15f * rr.h) {
-                            t = df_div(rr, d);  // t ~ 1/(2 theta) = |a_pq| / (a_qq - a_pp): theta^2 would overflow
-                        } else {
-                            const dfl theta = df_div(d, {2.f * rr.h, 2.f * rr.l});
-                            const dfl den = df_add({fabsf(theta.h), theta.h < 0.f ? -theta.l : theta.l},
-                                                   df_sqrt(df_fma(theta, theta, {1.f, 0.f})));
-                            t = df_div({theta.h < 0.f ? -1.f : 1.f, 0.f}, den);
-                        }
-                        R.c = df_div({1.f, 0.f}, df_sqrt(df_fma(t, t, {1.f, 0.f})));
-                        R.s = df_mul(t, R.c);
-                        const dfl ir = df_div({1.f, 0.f}, rrs);
+                        const dfl r2 = df_fma(ai, ai, df_mul(ar, ar));
+                        const dfl ir = df_rsqrt(r2);
+                        const float r = r2.h * ir.h;                            // |a_pq| sc
+                        const float x = df_sub(DG_AT(a, n, q, q).re, DG_AT(a, n, p, p).re).h * sc, ax = fabsf(x);
+                        float t;
+                        if (ax > 1e9f) t = __fdividef(r, ax);
+                        else t = __fdividef(2.f * r, ax + sqrtf(fmaf(x, x, 4.f * r * r)));
+                        if (!(ax < 1e30f)) t = 0.f;
+                        if (x < 0.f) t = -t;
+                        R.c = df_rsqrt(df_fma({t, 0.f}, {t, 0.f}, {1.f, 0.f}));
+                        R.s = df_mul({t, 0.f}, R.c);
                         R.ph = {df_mul(ar, ir), df_mul(ai, ir)};
                         R.on = 1;
                     }
@@ -157,14 +163,9 @@ __device__ inline int warp_heig_df(int n, const cdf *A0, cdf *a, cdf *u, double 
                 DG_AT(a, n, R.q, k) = OpsF::fma(cph, aqk, {df_mul(apk.re, R.s), df_mul(apk.im, R.s)});
             }
             __syncwarp();
-            if (lane < half) {
-                const DfRot R = rot[lane];
-                if (R.on) {
-                    DG_AT(a, n, R.p, R.q) = zero;
-                    DG_AT(a, n, R.q, R.p) = zero;
-                    DG_AT(a, n, R.p, R.p).im = {0.f, 0.f};
-                    DG_AT(a, n, R.q, R.q).im = {0.f, 0.f};
-                }
+            if (lane < half && rot[lane].on) {
+                DG_AT(a, n, rot[lane].p, rot[lane].p).im = {0.f, 0.f};
+                DG_AT(a, n, rot[lane].q, rot[lane].q).im = {0.f, 0.f};
             }
             __syncwarp();
         }
