@@ -207,6 +207,7 @@ struct OpsD {
     static DG_HD C pscale(C a, R r) { return cmk(a.x * r, a.y * r); }
     static DG_HD R rdotc(C a, C b) { return ::fma(a.x, b.x, a.y * b.y); }  // Re(a conj b)
     static DG_HD void balance(C &, C &) {}
+    static DG_HD C times_i(C a) { return cmk(-a.y, a.x); }
 };
 
 struct OpsF {
@@ -387,6 +388,7 @@ struct OpsP {
     static __device__ __forceinline__ C pacc(C w, R p, C acc) { return pdf_fma_lazy(w, pdf_both(p), acc); }
     static __device__ __forceinline__ C pnorm(C a) { return pdf_fast_two_sum(a.h, a.l); }
     static __device__ __forceinline__ C pscale(C a, R r) { return pdf_mul(a, pdf_both(r)); }
+    static __device__ __forceinline__ C times_i(C a) { return pdf_i(a); }
     // num and den by the power of two that takes |den| to about 1, so that |den|^2 stays in the FP32 range
     static __device__ __forceinline__ void balance(C &num, C &den) {
         const float mx = fmaxf(fabsf(den.h.x), fabsf(den.h.y));

@@ -56,32 +56,29 @@ __global__ void k_hyb_delta(int dim, int nfreq, int D, double beta, double mu, c
 // ---------------------------------------------------------------------------------------------------
 // FourierTransform_tau: the tau-independent tail data (src/FourierTransform.cpp:22-44, 66-83)
 // ---------------------------------------------------------------------------------------------------
-// T layout (complex slots, d x d each): V, H, H2, UH, UH2, then eH, eH2 (d doubles each, in a slot), then
-// W1 = UH^H V, W2 = UH2^H V (the tail term V^H G0_H(tau) V = W1^H diag(g(tau)) W1)
-constexpr int TAIL_SLOTS = 9;
+// T layout: the 2 d pole energies e = (eH, eH2) as doubles (in d complex slots), then per pole l and pair a <= b the
+// product conj(W(l, a)) W(l, b), W1 = UH^H V and W2 = UH2^H V stacked: every tail term is V^H f(H) V =
+// sum_l f(e_l) conj(W(l, a)) W(l, b), and its (b, a) element is the conjugate product
 struct TailPtrs {
-    double2 *V, *H, *H2, *UH, *UH2, *W1, *W2;
-    double *eH, *eH2;
+    const double *e;
+    const double2 *P;  // [2 d][d (d + 1) / 2]
 };
-__device__ TailPtrs tail_ptrs(double2 *T, int d) {
-    const size_t dd = (size_t)d * d;
-    TailPtrs p;
-    p.V = T;
-    p.H = T + dd;
-    p.H2 = T + 2 * dd;
-    p.UH = T + 3 * dd;
-    p.UH2 = T + 4 * dd;
-    p.eH = (double *)(T + 5 * dd);
-    p.eH2 = (double *)(T + 6 * dd);
-    p.W1 = T + 7 * dd;
-    p.W2 = T + 8 * dd;
-    return p;
+__device__ TailPtrs tail_ptrs(const double2 *T, int d) { return {(const double *)T, T + d}; }
+// pair q of the row-major upper triangle (a <= b)
+__device__ __forceinline__ void pair_of(int q, int d, int &a, int &b) {
+    a = 0;
+    while (q >= d - a) {
+        q -= d - a;
+        a++;
+    }
+    b = a + q;
 }
 
-// FourierTransform_tau's tail data (src/FourierTransform.cpp:22-44, 66-83) by one block, the smallmat.cuh
-// routines in shared memory: V = sqrt(m1); M2' = V^-H (2 m2) V^-1, M3' likewise; H = M2'/2 + sqrt(M3'/2 -
-// M2'^2/4) (or M2'/2 if that is not positive), H2 = M2' - H; eigen-decompositions of H and H2.  V^-1 =
-// U diag(ev^-1/2) U^H comes from the same eigen-decomposition as V = U diag(ev^1/2) U^H.
+// FourierTransform_tau's tail data (src/FourierTransform.cpp:22-44, 66-83), the smallmat.cuh routines in shared memory:
+// V = sqrt(m1); M2' = V^-H (2 m2) V^-1, M3' likewise; H = M2'/2 + sqrt(M3'/2 - M2'^2/4) (or M2'/2 if that is not
+// positive), H2 = M2' - H; eigen-decompositions of H and H2.  V^-1 = U diag(ev^-1/2) U^H comes from the same
+// eigen-decomposition as V = U diag(ev^1/2) U^H.  Two blocks: both go through to H and H2, block 0 then decomposes H and
+// block 1 H2 (the chain of Jacobi rounds is what takes the time, not the work).
 constexpr int TAIL_THREADS = 128;
 __host__ __device__ inline size_t tail_smem_bytes(int d) {
     return (size_t)8 * d * d * sizeof(double2) + 32 * sizeof(double) + 32 * sizeof(int) + 17 * sizeof(DgRot) +
@@ -89,13 +86,12 @@ __host__ __device__ inline size_t tail_smem_bytes(int d) {
 }
 __global__ void __launch_bounds__(TAIL_THREADS) k_tail_setup_blk(int d, const double2 *mom, double2 *T, int *status) {
     extern __shared__ double2 sm[];
-    const int dd = d * d, tid = threadIdx.x, nt = blockDim.x;
+    const int dd = d * d, tid = threadIdx.x, nt = blockDim.x, second = blockIdx.x;
     double2 *A = sm, *U = A + dd, *X = U + dd, *M2 = X + dd, *M3 = M2 + dd, *t1 = M3 + dd, *V = t1 + dd, *Vi = V + dd;
     double *ev = (double *)(Vi + dd);
     int *ord = (int *)(ev + 32);
     DgRot *rot = (DgRot *)(ord + 32);
     double *red = (double *)(rot + 17);
-    TailPtrs p = tail_ptrs(T, d);
     const double2 *m1 = mom + dd, *m2 = mom + 2 * dd, *m3 = mom + 3 * dd;
     int st = block_heig(d, m1, A, U, ev, ord, rot, red);
     const bool pos = ev[0] > 0;
@@ -131,37 +127,30 @@ __global__ void __launch_bounds__(TAIL_THREADS) k_tail_setup_blk(int d, const do
             if (pos2)
                 for (int l = 0; l < d; l++)
                     h = cadd(h, cscale(cmul(DG_AT(U, d, i, l), cconj(DG_AT(U, d, j, l))), sqrt(ev[l])));
-            p.H[e] = h;
-            p.H2[e] = csub(M2[e], h);
-            p.V[e] = V[e];
+            X[e] = second ? csub(M2[e], h) : h;
         }
     } else {
-        for (int e = tid; e < dd; e += nt) {
-            V[e] = cmk(0, 0);
-            p.V[e] = p.H[e] = p.H2[e] = cmk(0, 0);
-        }
+        for (int e = tid; e < dd; e += nt) V[e] = X[e] = cmk(0, 0);
     }
     __syncthreads();
-    st |= block_heig(d, p.H, A, U, ev, ord, rot, red);
+    st |= block_heig(d, X, A, U, ev, ord, rot, red);
     for (int e = tid; e < dd; e += nt) {
-        p.UH[e] = U[e];
-        M3[e] = U[e];
-    }
-    for (int l = tid; l < d; l += nt) p.eH[l] = ev[l];
-    __syncthreads();
-    st |= block_heig(d, p.H2, A, U, ev, ord, rot, red);
-    for (int e = tid; e < dd; e += nt) {
-        p.UH2[e] = U[e];
         const int i = e % d, j = e / d;
-        double2 w1 = cmk(0, 0), w2 = cmk(0, 0);
-        for (int l = 0; l < d; l++) {
-            w1 = cfma(cconj(DG_AT(M3, d, l, i)), DG_AT(V, d, l, j), w1);
-            w2 = cfma(cconj(DG_AT(U, d, l, i)), DG_AT(V, d, l, j), w2);
-        }
-        p.W1[e] = w1;
-        p.W2[e] = w2;
+        double2 w = cmk(0, 0);
+        for (int l = 0; l < d; l++) w = cfma(cconj(DG_AT(U, d, l, i)), DG_AT(V, d, l, j), w);
+        t1[e] = w;  // W(i, j)
     }
-    for (int l = tid; l < d; l += nt) p.eH2[l] = ev[l];
+    __syncthreads();
+    const int P = d * (d + 1) / 2;
+    double2 *Po = T + d + (size_t)(second ? d : 0) * P;
+    for (int x = tid; x < d * P; x += nt) {
+        int a, b;
+        const int l = x / P;
+        pair_of(x % P, d, a, b);
+        Po[x] = cmul(cconj(DG_AT(t1, d, l, a)), DG_AT(t1, d, l, b));
+    }
+    double *eo = (double *)T + (second ? d : 0);
+    for (int l = tid; l < d; l += nt) eo[l] = ev[l];
     if (st && tid == 0) dg_flag(status, DG_NONCONV);
 }
 
@@ -170,34 +159,37 @@ __global__ void k_tail_g(int d, int ntau, double beta, const double2 *T, double 
     long long x = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (x >= (long long)(ntau + 1) * 2 * d) return;
     const int t = (int)(x / (2 * d)), l = (int)(x % (2 * d));
-    TailPtrs p = tail_ptrs(const_cast<double2 *>(T), d);
-    const double e = l < d ? p.eH[l] : p.eH2[l - d];
+    const double e = tail_ptrs(T, d).e[l];
     const double tau = t * beta / ntau;
     G[x] = -1.0 / (exp(e * tau) + exp(e * (tau - beta)));
 }
 
-// one thread per (tau, element): (S + S^H)/beta + V^H G0_H V/2 + V^H G0_H2 V/2, symmetrised
+// one thread per (tau, pair a <= b): (S + S^H)/beta + V^H G0_H V/2 + V^H G0_H2 V/2, Hermitian by construction.  Bound by
+// the 2 FP64 multiply-adds per pole and pair (from W1, W2 themselves, for both elements of a pair: 14): 0.37 -> 0.09 ms
+// at d = 10, 8193 tau
 __global__ void k_ft_finish_el(int d, int ntau, double beta, const double2 *T, const double *G, const double2 *S,
                                double2 *out) {
-    const int dd = d * d;
+    const int dd = d * d, P = d * (d + 1) / 2;
     long long x = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (x >= (long long)(ntau + 1) * dd) return;
-    const int t = (int)(x / dd), e = (int)(x % dd), a = e % d, b = e / d;
-    TailPtrs p = tail_ptrs(const_cast<double2 *>(T), d);
+    if (x >= (long long)(ntau + 1) * P) return;
+    const int t = (int)(x / P), q = (int)(x % P);
+    int a, b;
+    pair_of(q, d, a, b);
+    const double2 *pp = tail_ptrs(T, d).P + q;
     const double2 *Sj = S + (size_t)t * dd;
     const double *g = G + (size_t)t * 2 * d;
-    double2 tab = cmk(0, 0), tba = cmk(0, 0);
-    for (int l = 0; l < d; l++) {
-        const double2 w1a = DG_AT(p.W1, d, l, a), w1b = DG_AT(p.W1, d, l, b);
-        const double2 w2a = DG_AT(p.W2, d, l, a), w2b = DG_AT(p.W2, d, l, b);
-        tab = cadd(tab, cadd(cscale(cmul(cconj(w1a), w1b), g[l]), cscale(cmul(cconj(w2a), w2b), g[d + l])));
-        tba = cadd(tba, cadd(cscale(cmul(cconj(w1b), w1a), g[l]), cscale(cmul(cconj(w2b), w2a), g[d + l])));
+    double2 tab = cmk(0, 0);
+#pragma unroll 4
+    for (int l = 0; l < 2 * d; l++) {
+        const double2 p = pp[(size_t)l * P];
+        tab = cmk(fma(p.x, g[l], tab.x), fma(p.y, g[l], tab.y));
     }
     const double2 sab = cadd(DG_AT(Sj, d, a, b), cconj(DG_AT(Sj, d, b, a)));
-    const double2 sba = cadd(DG_AT(Sj, d, b, a), cconj(DG_AT(Sj, d, a, b)));
-    const double2 Aab = cadd(cscale(sab, 1.0 / beta), cscale(tab, 0.5));
-    const double2 Aba = cadd(cscale(sba, 1.0 / beta), cscale(tba, 0.5));
-    out[x] = cscale(cadd(Aab, cconj(Aba)), 0.5);
+    double2 v = cadd(cscale(sab, 1.0 / beta), cscale(tab, 0.5));
+    if (a == b) v.y = 0.0;
+    double2 *o = out + (size_t)t * dd;
+    DG_AT(o, d, a, b) = v;
+    if (a != b) DG_AT(o, d, b, a) = cconj(v);
 }
 
 // Definiteness of nmat Hermitian d x d matrices, one thread each, lower triangles interleaved in shared memory.
@@ -231,21 +223,43 @@ __global__ void k_posdef(int d, int nmat, const double2 *M, int mode, double sig
 }
 
 
-// one thread per (frequency, element): Dw_i = F_i - V^H [(iw - H)^-1 + (iw - H2)^-1] V / 2 (:55-60), the
-// inverses through the eigen-decompositions of H and H2: V^H (iw - H)^-1 V = W1^H diag(1/(iw - eH)) W1
-__global__ void k_ft_subtract_el(int d, int nfreq, double beta, const double2 *F, const double2 *T, double2 *Dw) {
-    const int dd = d * d;
-    long long x = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (x >= (long long)nfreq * dd) return;
-    const int i = (int)(x / dd), e = (int)(x % dd), a = e % d, b = e / d;
-    TailPtrs p = tail_ptrs(const_cast<double2 *>(T), d);
-    const double w = (DG_PI / beta) + i * ((2 * DG_PI) / beta);
-    double2 tl = cmk(0, 0);
-    for (int l = 0; l < d; l++) {
-        tl = cadd(tl, cmul(cmul(cconj(DG_AT(p.W1, d, l, a)), DG_AT(p.W1, d, l, b)), crcp(cmk(-p.eH[l], w))));
-        tl = cadd(tl, cmul(cmul(cconj(DG_AT(p.W2, d, l, a)), DG_AT(p.W2, d, l, b)), crcp(cmk(-p.eH2[l], w))));
+// Dw_i = F_i - V^H [(iw - H)^-1 + (iw - H2)^-1] V / 2 (:55-60): with the pole products, sum_l P_l(a, b)/(iw - e_l) =
+// A - i w B, A = -sum_l P_l e_l r_l, B = sum_l P_l r_l, r_l = 1/(e_l^2 + w^2), and the (b, a) element is A^* - i w B^*.  A block
+// takes SUB_F frequencies: their reciprocals once in shared memory (a division per pole and element before), then
+// (frequency, pair) items of 4 FP64 multiply-adds per pole.  0.29 -> 0.05 ms at d = 10, 4096 frequencies
+constexpr int SUB_F = 8, SUB_THREADS = 128;
+__global__ void __launch_bounds__(SUB_THREADS) k_ft_subtract_el(int d, int nfreq, double beta, const double2 *F,
+                                                                const double2 *T, double2 *Dw) {
+    extern __shared__ double rsm[];  // [SUB_F][2 d] (r, -e r)
+    const int dd = d * d, P = d * (d + 1) / 2, i0 = blockIdx.x * SUB_F, nf = min(SUB_F, nfreq - i0);
+    const TailPtrs p = tail_ptrs(T, d);
+    auto freq = [&](int i) { return (DG_PI / beta) + i * ((2 * DG_PI) / beta); };
+    for (int x = threadIdx.x; x < nf * 2 * d; x += SUB_THREADS) {
+        const double w = freq(i0 + x / (2 * d)), e = p.e[x % (2 * d)], r = 1.0 / fma(e, e, w * w);
+        rsm[2 * x] = r;
+        rsm[2 * x + 1] = -e * r;
     }
-    Dw[x] = csub(F[x], cscale(tl, 0.5));
+    __syncthreads();
+    for (int x = threadIdx.x; x < nf * P; x += SUB_THREADS) {
+        const int i = x / P, q = x % P;
+        int a, b;
+        pair_of(q, d, a, b);
+        const double2 *pp = p.P + q;
+        const double *r = rsm + (size_t)i * 4 * d;
+        double2 A = cmk(0, 0), B = cmk(0, 0);
+#pragma unroll 4
+        for (int l = 0; l < 2 * d; l++) {
+            const double2 v = pp[(size_t)l * P];
+            B = cmk(fma(v.x, r[2 * l], B.x), fma(v.y, r[2 * l], B.y));
+            A = cmk(fma(v.x, r[2 * l + 1], A.x), fma(v.y, r[2 * l + 1], A.y));
+        }
+        const double w = 0.5 * freq(i0 + i);
+        const double2 *Fi = F + (size_t)(i0 + i) * dd;
+        double2 *o = Dw + (size_t)(i0 + i) * dd;
+        DG_AT(o, d, a, b) = csub(DG_AT(Fi, d, a, b), cmk(fma(w, B.y, 0.5 * A.x), fma(-w, B.x, 0.5 * A.y)));
+        if (a != b)
+            DG_AT(o, d, b, a) = csub(DG_AT(Fi, d, b, a), cmk(fma(-w, B.y, 0.5 * A.x), fma(-w, B.x, -0.5 * A.y)));
+    }
 }
 
 // exact phase table: ph[q] = exp(-i pi q / ntau), q in [0, 2 ntau)
@@ -334,10 +348,36 @@ __global__ void __launch_bounds__(FFT_THREADS) k_fft_w2tau(int dd, int nfreq, in
     for (int j = threadIdx.x; j <= N; j += blockDim.x) S[(size_t)j * dd + e] = cmul(ph[j], x[j & (N - 1)]);
 }
 
+// (K(t_n), Im E(t_n)) of the hat functions, once per frequency (an element's transform then only multiplies by them: the
+// sines and divisions took half of a 10 x 10 transform)
+__global__ void k_tau2w_weights(int nfreq, int N, double2 *KE) {
+    const int n = blockIdx.x * blockDim.x + threadIdx.x;
+    if (n >= nfreq) return;
+    const double q = (2.0 * n + 1.0) / N;  // t_n / pi
+    const double t = DG_PI * q;
+    const double sh = sinpi(0.5 * q);
+    const double K = (sh / (0.5 * t)) * (sh / (0.5 * t));
+    double eim;  // (t - sin t) / t^2
+    if (t < 1.0) {
+        // sum_{k>=1} (-1)^{k+1} t^{2k-1} / (2k+1)!, nine terms (truncation < 1e-17 relative for t < 1)
+        const double t2 = t * t;
+        double term = t / 6.0, acc = 0.0;
+        for (int k = 1; k <= 9; k++) {
+            acc += term;
+            term *= -t2 / ((2.0 * k + 2.0) * (2.0 * k + 3.0));
+        }
+        eim = acc;
+    } else {
+        eim = (t - sinpi(q)) / (t * t);
+    }
+    KE[n] = cmk(K, eim);
+}
+
 // FT_t_to_w by hat functions: W_n = dt K (Y_n - F_0) + dt (F_0 E - F_N conj E)
 __global__ void __launch_bounds__(FFT_THREADS) k_fft_tau2w(int dd, int nfreq, int logn, double beta,
                                                            const double2 *__restrict__ Ft,
-                                                           const double2 *__restrict__ ph, double2 *__restrict__ W) {
+                                                           const double2 *__restrict__ ph,
+                                                           const double2 *__restrict__ KE, double2 *__restrict__ W) {
     extern __shared__ double2 x[];
     const int e = blockIdx.x, N = 1 << logn;
     // conj(F_s e^{i pi s/N}) = conj(F_s) ph[s]: a forward FFT of it, conjugated, gives Y
@@ -347,26 +387,9 @@ __global__ void __launch_bounds__(FFT_THREADS) k_fft_tau2w(int dd, int nfreq, in
     const double dt = beta / N;
     const double2 f0 = Ft[e], fN = Ft[(size_t)N * dd + e];
     for (int n = threadIdx.x; n < nfreq; n += blockDim.x) {
-        const double2 Y = cconj(x[n & (N - 1)]);
-        const double q = (2.0 * n + 1.0) / N;  // t_n / pi
-        const double t = DG_PI * q;
-        const double sh = sinpi(0.5 * q);
-        const double K = (sh / (0.5 * t)) * (sh / (0.5 * t));
-        double eim;  // (t - sin t) / t^2
-        if (t < 1.0) {
-            // sum_{k>=1} (-1)^{k+1} t^{2k-1} / (2k+1)!, nine terms (truncation < 1e-17 relative for t < 1)
-            const double t2 = t * t;
-            double term = t / 6.0, acc = 0.0;
-            for (int k = 1; k <= 9; k++) {
-                acc += term;
-                term *= -t2 / ((2.0 * k + 2.0) * (2.0 * k + 3.0));
-            }
-            eim = acc;
-        } else {
-            eim = (t - sinpi(q)) / (t * t);
-        }
-        const double2 E = cmk(0.5 * K, eim);
-        double2 w = cscale(csub(Y, f0), dt * K);
+        const double2 Y = cconj(x[n & (N - 1)]), ke = KE[n];
+        const double2 E = cmk(0.5 * ke.x, ke.y);
+        double2 w = cscale(csub(Y, f0), dt * ke.x);
         w = cadd(w, cscale(csub(cmul(f0, E), cmul(fN, cconj(E))), dt));
         W[(size_t)n * dd + e] = w;
     }
@@ -480,11 +503,109 @@ __global__ void k_tau2w(int dd, int nfreq, int ntau, double beta, const double2 
 
 // ---------------------------------------------------------------------------------------------------
 // getStimp (src/SCGF2_fullLoop.cpp:603-653): Sigma_ij(tau) = sum over U entries x1 = (i,q,m,k), x2 = (l,n,p,j)
-// of U1 U2 (-G_pq(beta - tau)) (G_kn G_ml - G_kl G_mn).  One block per S2_TB tau points, one thread per output
-// (i, j) for all of them; the U list is pre-sorted on the host by its first index (x1 role) and by its last
-// index (x2 role).  Per (x1, x2) pair the thread forms the 2x2 minor G_kn G_ml - G_kl G_mn once per tau and
-// accumulates U2 G'_pq times it; U1 multiplies the inner sum.
+// of U1 U2 (-G_pq(beta - tau)) (G_kn G_ml - G_kl G_mn).
+//
+// The bracket is a 2 x 2 minor of G(tau), antisymmetric in (m, k) and in (l, n): of the (entries)^2 / d pairs a matrix
+// element sums over, only np1 x np2 minors are distinct (45 x 45 of 32,400 pairs for ten Kanamori orbitals).  Per tau:
+//   Mn[P1][P2]  the minors of the index pairs P1 = (m < k) and P2 = (l < n) that occur,
+//   B[q][s]     for every slot s = (j, P2): the sum over its entries of -+U2 G_pq(beta - tau),
+//   Sigma_ij = sum over e1 in L1(i) of +-U1 sum over slots s of j of B[q(e1)][s] Mn[P1(e1)][P2(s)],
+// one multiply-add per pair in place of four complex products.  The host prepares the lists (dg_ulist).  In double-float
+// (OpsP) the inner sums are lazy sums of the two real halves, acc1 += Re B (Re M, Im M), acc2 += Im B (Re M, Im M).
+// Bound by the FP32 (FP64) multiply-adds.  Twelve loops of the ten-orbital solver (8193 tau, double-float), with the
+// other impurity kernels: 85.7 -> 39.0 ms
 // ---------------------------------------------------------------------------------------------------
+constexpr int S2_THREADS = 128;
+__host__ __device__ inline int s2_ldm(int np2) { return np2 | 1; }       // odd strides: lanes on different rows hit
+__host__ __device__ inline int s2_ldb(int nslot) { return nslot | 1; }  // different banks
+// shared memory per tau: G(tau), G(beta - tau), minors, B (16-byte elements)
+__host__ __device__ inline size_t s2_tau_elems(int d, int np1, int np2, int nslot) {
+    return 2 * (size_t)d * d + (size_t)np1 * s2_ldm(np2) + (size_t)d * s2_ldb(nslot);
+}
+// tau points per block: as many as outputs fit in its threads and 96 KB
+inline int s2_taus(int d, int np1, int np2, int nslot) {
+    const size_t per = s2_tau_elems(d, np1, np2, nslot) * 16;
+    return std::max(1, std::min(S2_THREADS / (d * d), (int)(96 * 1024 / per)));
+}
+
+template <class Ops>
+__global__ void __launch_bounds__(S2_THREADS) k_sigma2_min(S2Lists L, int ntau, int tb, const double2 *__restrict__ G,
+                                                           double2 *__restrict__ S, int *status) {
+    typedef typename Ops::C C;
+    extern __shared__ double2 s2sm[];
+    const int d = L.d, dd = d * d, t0 = blockIdx.x * tb, nb = min(tb, ntau + 1 - t0), tid = threadIdx.x;
+    const int ldm = s2_ldm(L.np2), ldb = s2_ldb(L.nslot);
+    const size_t per = s2_tau_elems(d, L.np1, L.np2, L.nslot);
+    const int *off1 = L.i, *offs = off1 + d + 1, *offb = offs + d + 1, *pr1 = offb + L.nslot + 1, *pr2 = pr1 + 2 * L.np1;
+    const int *e1 = pr2 + 2 * L.np2, *sp2 = e1 + 2 * L.ne1, *bp = sp2 + L.nslot;
+    const double2 *c1 = L.c, *cb = c1 + L.ne1;
+    auto tau = [&](int b) { return reinterpret_cast<C *>(s2sm) + (size_t)b * per; };
+    for (int x = tid; x < nb * dd; x += S2_THREADS) {
+        const int b = x / dd, q = x % dd;
+        tau(b)[q] = Ops::from(G[(size_t)(t0 + b) * dd + q]);
+        tau(b)[dd + q] = Ops::from(G[(size_t)(ntau - t0 - b) * dd + q]);
+    }
+    __syncthreads();
+    const int nm = L.np1 * L.np2, nB = d * L.nslot;
+    for (int x = tid; x < nb * nm; x += S2_THREADS) {
+        const int b = x / nm, P1 = (x % nm) / L.np2, P2 = x % L.np2;
+        const C *g = tau(b);
+        const int m = pr1[2 * P1], k = pr1[2 * P1 + 1], l = pr2[2 * P2], n = pr2[2 * P2 + 1];
+        // G_kn G_ml - G_kl G_mn
+        tau(b)[2 * dd + P1 * ldm + P2] = Ops::fms(g[k + l * d], g[m + n * d], Ops::mul(g[k + n * d], g[m + l * d]));
+    }
+    for (int x = tid; x < nb * nB; x += S2_THREADS) {
+        const int b = x / nB, q = (x % nB) / L.nslot, sl = x % L.nslot;
+        const C *gm = tau(b) + dd;
+        C v = Ops::zero();
+        for (int y = offb[sl]; y < offb[sl + 1]; y++) v = Ops::fma(Ops::from(cb[y]), gm[bp[y] + q * d], v);
+        tau(b)[2 * dd + (size_t)L.np1 * ldm + q * ldb + sl] = v;
+    }
+    __syncthreads();
+    double ns = 0, ng = 0;  // norms of the anti-Hermitian parts, below
+    for (int x = tid; x < nb * dd; x += S2_THREADS) {
+        const int b = x / dd, o = x % dd, i = o % d, j = o / d, s0 = offs[j], s1 = offs[j + 1];
+        const C *Mn = tau(b) + 2 * dd, *B = Mn + (size_t)L.np1 * ldm;
+        C acc = Ops::zero();
+        for (int a1 = off1[i]; a1 < off1[i + 1]; a1++) {
+            const C *row = Mn + e1[2 * a1] * ldm, *bq = B + e1[2 * a1 + 1] * ldb;
+            C x1 = Ops::zero(), x2 = Ops::zero();
+            for (int sl = s0; sl < s1; sl++) {
+                const C m = row[sp2[sl]], v = bq[sl];
+                x1 = Ops::pacc(m, Ops::cre(v), x1);
+                x2 = Ops::pacc(m, Ops::cim(v), x2);
+                if (((sl - s0) & 15) == 15) {
+                    x1 = Ops::pnorm(x1);
+                    x2 = Ops::pnorm(x2);
+                }
+            }
+            acc = Ops::fma(Ops::from(c1[a1]), Ops::add(Ops::pnorm(x1), Ops::times_i(Ops::pnorm(x2))), acc);
+        }
+        S[(size_t)(t0 + b) * dd + o] = Ops::to(acc);
+    }
+    __syncthreads();
+    // Hermiticity asserts of the reference (:641-651): ||(G - G^H)/2i|| > 1e-10, ||(S - S^H)/2i|| > 1e-5; a warp per tau
+    const int lane = tid & 31;
+    for (int b = tid >> 5; b < nb; b += S2_THREADS / 32) {
+        const double2 *Gt = G + (size_t)(t0 + b) * dd, *St = S + (size_t)(t0 + b) * dd;
+        ng = ns = 0;
+        for (int e = lane; e < dd; e += 32) {
+            const int a = e % d, c = e / d;
+            ng += cabs2(csub(Gt[e], cconj(DG_AT(Gt, d, c, a)))) / 4;
+            ns += cabs2(csub(St[e], cconj(DG_AT(St, d, c, a)))) / 4;
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            ng += __shfl_xor_sync(0xffffffffu, ng, o);
+            ns += __shfl_xor_sync(0xffffffffu, ns, o);
+        }
+        if (lane == 0 && (sqrt(ng) > 1e-10 || sqrt(ns) > 1e-5)) dg_flag(status, DG_HERMIT);
+    }
+}
+
+// The same sum entry by entry, for interaction lists whose minors do not fit in shared memory: one block per S2_TB tau
+// points, one thread per output (i, j) for all of them; the U list is pre-sorted by its first index (x1 role) and by its
+// last index (x2 role).  Per (x1, x2) pair the thread forms the minor once per tau; U1 multiplies the inner sum.
 constexpr int S2_TB = 4;
 __global__ void k_sigma2(int d, int ntau, const int *__restrict__ byI, const int *__restrict__ byIoff,
                          const int *__restrict__ byJ, const int *__restrict__ byJoff, const int *__restrict__ uidx,
@@ -624,15 +745,21 @@ __global__ void __launch_bounds__(128) k_sigma2_df(int d, int ntau, int nu, cons
     }
 }
 
-// getFockOperator (:583-597), single thread
-__global__ void k_fock(int d, int nu, const int *uidx, const double2 *ut, const double2 *occ, double2 *fock) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    for (int q = 0; q < d * d; q++) fock[q] = cmk(0, 0);
+// getFockOperator (:583-597): one thread per element, the list's entries in order (a single thread took 124 us for 180
+// entries of ten orbitals)
+__global__ void k_fock(int d, int nu, const int *__restrict__ uidx, const double2 *__restrict__ ut,
+                       const double2 *__restrict__ occ, double2 *fock) {
+    const int o = blockIdx.x * blockDim.x + threadIdx.x;
+    if (o >= d * d) return;
+    const int row = o % d, col = o / d;
+    double2 f = cmk(0, 0);
     for (int x = 0; x < nu; x++) {
-        const int a = uidx[4 * x], b = uidx[4 * x + 1], c = uidx[4 * x + 2], dd_ = uidx[4 * x + 3];
-        DG_AT(fock, d, b, dd_) = cadd(DG_AT(fock, d, b, dd_), cmul(ut[x], DG_AT(occ, d, c, a)));
-        DG_AT(fock, d, b, c) = csub(DG_AT(fock, d, b, c), cmul(ut[x], DG_AT(occ, d, dd_, a)));
+        if (uidx[4 * x + 1] != row) continue;
+        const int a = uidx[4 * x], c = uidx[4 * x + 2], e = uidx[4 * x + 3];
+        if (e == col) f = cadd(f, cmul(ut[x], DG_AT(occ, d, c, a)));
+        if (c == col) f = csub(f, cmul(ut[x], DG_AT(occ, d, e, a)));
     }
+    fock[o] = f;
 }
 
 // getGwimp (:551-570): one thread per frequency
@@ -655,10 +782,43 @@ __global__ void k_dyson(int d, int nfreq, double beta, double mu, const double2 
     if (thread_gj_inverse(d, G, iwork + (size_t)n * d)) dg_flag(status, DG_SINGULAR);
 }
 
-// estimate_asymto (:736-787), single thread; F holds nfreq+3 matrices
-__global__ void k_estimate_asymto(int d, int Nf, double beta, double2 *F, int order) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+// getGwimp for d <= 20: a lane group of W lanes per frequency, lane c holds column c (df.cuh's Gauss-Jordan).  The
+// one-thread form above walks its matrix in global memory: 0.31 ms at d = 10, 4096 frequencies, against 0.07
+template <int DP, int W>
+__global__ void __launch_bounds__(128) k_dyson_grp(int d, int nfreq, double beta, double mu, const double2 *himp,
+                                                   const double2 *delta, const double2 *fock, const double2 *s2, double2 *gw,
+                                                   int *status) {
+    const int c = threadIdx.x & (W - 1), n_raw = blockIdx.x * (128 / W) + threadIdx.x / W;
+    const bool valid = n_raw < nfreq && c < d;
+    const int n = min(n_raw, nfreq - 1);
     const size_t dd = (size_t)d * d;
+    const double wn = (DG_PI * (2. * n + 1.)) / beta;
+    double2 a[DP];
+#pragma unroll
+    for (int r = 0; r < DP; r++) {
+        if (r < d && c < d) {
+            const int e = r + c * d;
+            double2 v = (r == c) ? cmk(mu, wn) : cmk(0, 0);
+            v = csub(csub(v, himp[e]), delta[n * dd + e]);
+            a[r] = csub(csub(v, fock[e]), s2[n * dd + e]);
+        } else {
+            a[r] = cmk(r == c ? 1.0 : 0.0, 0.0);
+        }
+    }
+    const bool sing = warp_gj_inverse_rolled<OpsD, DP, W>(a, c);
+    if (!valid) return;
+#pragma unroll
+    for (int r = 0; r < DP; r++)
+        if (r < d) gw[n * dd + r + c * d] = a[r];
+    if (sing) dg_flag(status, DG_SINGULAR);
+}
+
+// estimate_asymto (:736-787), one thread per element; F holds nfreq+3 matrices
+__global__ void k_estimate_asymto(int d, int Nf, double beta, double2 *F, int order) {
+    const int el = blockIdx.x * blockDim.x + threadIdx.x;
+    if (el >= d * d) return;
+    const size_t dd = (size_t)d * d;
+    const int a = el % d, b = el / d;
     auto wn = [&](int i) { return (2 * (Nf - 3 + i) + 1) * DG_PI / beta; };
     double w0, w1, w2;
     int p = (order == 1) ? 2 : (order == 2 ? 4 : 6);
@@ -667,31 +827,28 @@ __global__ void k_estimate_asymto(int d, int Nf, double beta, double2 *F, int or
     w2 = 1. / pow(wn(2), p);
     const double wsum = w0 + w1 + w2;
     double2 *dst = F + (size_t)(Nf + order - 1) * dd;
-    for (int b = 0; b < d; b++)
-        for (int a = 0; a < d; a++) {
-            double2 acc = cmk(0, 0);
-            for (int w = 0; w < 3; w++) {
-                const double2 *T = F + (size_t)(Nf - 3 + w) * dd;
-                double2 tab = DG_AT(T, d, a, b), tba = DG_AT(T, d, b, a);
-                double2 v;
-                if (order == 1) {
-                    v = cscale(csub(cconj(tba), tab), 0.5);   // (t^H - t)/2
-                    v = cmul(v, crcp(cmk(0, wn(w))));          // / (i w)
-                } else if (order == 2) {
-                    v = cscale(cadd(tab, cconj(tba)), 0.5);
-                    v = cscale(v, -1.0 / pow(wn(w), 2));
-                } else {
-                    const double2 *F0 = F + (size_t)Nf * dd;
-                    const double2 ir = crcp(cmk(0, wn(w)));
-                    double2 xab = csub(tab, cmul(DG_AT(F0, d, a, b), ir));
-                    double2 xba = csub(tba, cmul(DG_AT(F0, d, b, a), ir));
-                    v = cscale(csub(cconj(xba), xab), 0.5);
-                    v = cscale(cmul(cmk(0, 1), v), 1.0 / pow(wn(w), 3));
-                }
-                acc = cadd(acc, v);
-            }
-            DG_AT(dst, d, a, b) = cscale(acc, 1.0 / wsum);
+    double2 acc = cmk(0, 0);
+    for (int w = 0; w < 3; w++) {
+        const double2 *T = F + (size_t)(Nf - 3 + w) * dd;
+        double2 tab = DG_AT(T, d, a, b), tba = DG_AT(T, d, b, a);
+        double2 v;
+        if (order == 1) {
+            v = cscale(csub(cconj(tba), tab), 0.5);   // (t^H - t)/2
+            v = cmul(v, crcp(cmk(0, wn(w))));          // / (i w)
+        } else if (order == 2) {
+            v = cscale(cadd(tab, cconj(tba)), 0.5);
+            v = cscale(v, -1.0 / pow(wn(w), 2));
+        } else {
+            const double2 *F0 = F + (size_t)Nf * dd;
+            const double2 ir = crcp(cmk(0, wn(w)));
+            double2 xab = csub(tab, cmul(DG_AT(F0, d, a, b), ir));
+            double2 xba = csub(tba, cmul(DG_AT(F0, d, b, a), ir));
+            v = cscale(csub(cconj(xba), xab), 0.5);
+            v = cscale(cmul(cmk(0, 1), v), 1.0 / pow(wn(w), 3));
         }
+        acc = cadd(acc, v);
+    }
+    DG_AT(dst, d, a, b) = cscale(acc, 1.0 / wsum);
 }
 
 // Kajueter-Kotliar interpolation of the IPT self-energy on (0,0), (1,1) (:1033-1046)
@@ -720,7 +877,7 @@ int dg_phase_table(dmftgpu_ctx *ctx, int ntau, double2 **ph) {
 int dg_tail_setup_dev(dmftgpu_ctx *ctx, int d, const double2 *mom, double2 *T) {
     const size_t sm = tail_smem_bytes(d);
     DG_CUDA(cudaFuncSetAttribute(k_tail_setup_blk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    k_tail_setup_blk<<<1, TAIL_THREADS, sm, ctx->stream>>>(d, mom, T, ctx->d_status);
+    k_tail_setup_blk<<<2, TAIL_THREADS, sm, ctx->stream>>>(d, mom, T, ctx->d_status);
     DG_LAUNCH(ctx, "k_tail_setup_blk");
     return DMFTGPU_OK;
 }
@@ -754,7 +911,8 @@ int dg_tail_prepare_dev(dmftgpu_ctx *ctx, int d, int nfreq, double beta, const d
                         double2 *T, double2 *Dw) {
     const size_t dd = (size_t)d * d;
     DG_TRY(dg_tail_setup_dev(ctx, d, mom, T));
-    k_ft_subtract_el<<<dg_ceil_div((long long)nfreq * dd, 256), 256, 0, ctx->stream>>>(d, nfreq, beta, fw, T, Dw);
+    k_ft_subtract_el<<<dg_ceil_div(nfreq, SUB_F), SUB_THREADS, (size_t)SUB_F * 4 * d * sizeof(double), ctx->stream>>>(
+        d, nfreq, beta, fw, T, Dw);
     DG_LAUNCH(ctx, "k_ft_subtract_el");
     return DMFTGPU_OK;
 }
@@ -788,7 +946,7 @@ int dg_w2tau_tail_dev(dmftgpu_ctx *ctx, int d, int nfreq, int ntau, double beta,
     }
     k_tail_g<<<dg_ceil_div((long long)(ntau + 1) * 2 * d, 256), 256, 0, s>>>(d, ntau, beta, T, gtail);
     DG_LAUNCH(ctx, "k_tail_g");
-    k_ft_finish_el<<<dg_ceil_div((long long)(ntau + 1) * dd, 256), 256, 0, s>>>(d, ntau, beta, T, gtail, S, ft);
+    k_ft_finish_el<<<dg_ceil_div((long long)(ntau + 1) * (d * (d + 1) / 2), 256), 256, 0, s>>>(d, ntau, beta, T, gtail, S, ft);
     DG_LAUNCH(ctx, "k_ft_finish_el");
     DG_TRY(dg_posdef_dev(ctx, d, ntau + 1, ft, 0, 1.0, 0.0, false, mineig, 0, 0));
     return dg_fixup_dev(ctx, d, ntau, beta, ft, mineig);
@@ -797,7 +955,7 @@ int dg_w2tau_tail_dev(dmftgpu_ctx *ctx, int d, int nfreq, int ntau, double beta,
 int dg_w2tau_dev(dmftgpu_ctx *ctx, int d, int nfreq, int ntau, double beta, const double2 *fw, const double2 *mom,
                  double2 *ft) {
     const size_t dd = (size_t)d * d;
-    double2 *T = (double2 *)dg_buf(ctx, "imp.tail", TAIL_SLOTS * dd * sizeof(double2));
+    double2 *T = (double2 *)dg_buf(ctx, "imp.tail", dg_tail_elems(d) * sizeof(double2));
     double2 *Dw = (double2 *)dg_buf(ctx, "imp.Dw", (size_t)nfreq * dd * sizeof(double2));
     if (!T || !Dw) return DMFTGPU_NOMEM;
     DG_TRY(dg_tail_prepare_dev(ctx, d, nfreq, beta, fw, mom, T, Dw));
@@ -824,10 +982,14 @@ int dg_tau2w_dev(dmftgpu_ctx *ctx, int d, int nfreq, int ntau, double beta, cons
     DG_TRY(dg_phase_table(ctx, ntau, &ph));
     if (fft_ok(ctx, ntau)) {
         const size_t sm = (size_t)ntau * sizeof(double2);
+        double2 *ke = (double2 *)dg_buf(ctx, "imp.t2w", (size_t)nfreq * sizeof(double2));
+        if (!ke) return DMFTGPU_NOMEM;
+        k_tau2w_weights<<<dg_ceil_div(nfreq, 64), 64, 0, ctx->stream>>>(nfreq, ntau, ke);
+        DG_LAUNCH(ctx, "k_tau2w_weights");
         DG_CUDA(cudaFuncSetAttribute(k_fft_tau2w, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
         {
             DgTimer tm(ctx, "k_fft_tau2w");
-            k_fft_tau2w<<<(int)dd, FFT_THREADS, sm, ctx->stream>>>((int)dd, nfreq, ilog2(ntau), beta, ft, ph, fw);
+            k_fft_tau2w<<<(int)dd, FFT_THREADS, sm, ctx->stream>>>((int)dd, nfreq, ilog2(ntau), beta, ft, ph, ke, fw);
         }
         DG_LAUNCH(ctx, "k_fft_tau2w");
     } else {
@@ -849,8 +1011,15 @@ int dg_sigma2_dev(dmftgpu_ctx *ctx, int d, int ntau, double beta, const DgUList 
     const size_t dd = (size_t)d * d;
     {
         DgTimer tm(ctx, "k_sigma2");
+        const S2Lists &L = U.s2;
         const size_t sm = S2_TB * 2 * dd * sizeof(double2);
-        if (ctx->imp_mixed) {
+        if (!U.byI) {
+            const int tb = s2_taus(d, L.np1, L.np2, L.nslot);
+            const size_t smm = tb * s2_tau_elems(d, L.np1, L.np2, L.nslot) * sizeof(double2);
+            auto kern = ctx->imp_mixed ? k_sigma2_min<OpsP> : k_sigma2_min<OpsD>;
+            DG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smm));
+            kern<<<dg_ceil_div(ntau + 1, tb), S2_THREADS, smm, ctx->stream>>>(L, ntau, tb, gt, st, ctx->d_status);
+        } else if (ctx->imp_mixed) {
             const size_t smf = sm + (size_t)U.nu * sizeof(double2);
             DG_CUDA(cudaFuncSetAttribute(k_sigma2_df, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smf));
             k_sigma2_df<<<dg_ceil_div(ntau + 1, S2_TB), 128, smf, ctx->stream>>>(
@@ -871,18 +1040,31 @@ int dg_sigma2_dev(dmftgpu_ctx *ctx, int d, int ntau, double beta, const DgUList 
 }
 
 int dg_fock_dev(dmftgpu_ctx *ctx, int d, const DgUList &U, const double2 *occ, double2 *fock) {
-    k_fock<<<1, 1, 0, ctx->stream>>>(d, U.nu, U.uidx, U.ut, occ, fock);
+    k_fock<<<dg_ceil_div(d * d, 32), 32, 0, ctx->stream>>>(d, U.nu, U.uidx, U.ut, occ, fock);
     DG_LAUNCH(ctx, "k_fock");
     return DMFTGPU_OK;
 }
 
 int dg_dyson_dev(dmftgpu_ctx *ctx, int d, int nfreq, double beta, double mu, const double2 *himp,
                  const double2 *delta, const double2 *fock, const double2 *s2, double2 *gw, bool check) {
-    const size_t dd = (size_t)d * d;
+    // lane groups for the widths their kernel is instantiated at, one thread per matrix beyond
+#define DG_DYSON(DP, W)                                                                                                \
+    k_dyson_grp<DP, W><<<dg_ceil_div(nfreq, 128 / W), 128, 0, ctx->stream>>>(d, nfreq, beta, mu, himp, delta, fock, s2, \
+                                                                             gw, ctx->d_status)
+    if (d <= 2) DG_DYSON(2, 2);
+    else if (d <= 4) DG_DYSON(4, 4);
+    else if (d <= 6) DG_DYSON(6, 8);
+    else if (d <= 8) DG_DYSON(8, 8);
+    else if (d <= 10) DG_DYSON(10, 16);
+    else if (d <= 14) DG_DYSON(14, 16);
+    else if (d <= 20) DG_DYSON(20, 32);
+    else {
+#undef DG_DYSON
     int *iw = (int *)dg_buf(ctx, "imp.dysiwork", (size_t)nfreq * d * sizeof(int));
     if (!iw) return DMFTGPU_NOMEM;
     k_dyson<<<dg_ceil_div(nfreq, 64), 64, 0, ctx->stream>>>(d, nfreq, beta, mu, himp, delta, fock, s2, gw, iw,
                                                             ctx->d_status);
+    }
     DG_LAUNCH(ctx, "k_dyson");
     if (check) {
         // getGwimp asserts max eig of (G - G^H)/2i < 0: -(G - G^H)/2i positive definite
@@ -892,50 +1074,57 @@ int dg_dyson_dev(dmftgpu_ctx *ctx, int d, int nfreq, double beta, double mu, con
 }
 
 int dg_estimate_asymto_dev(dmftgpu_ctx *ctx, int d, int nfreq, double beta, double2 *f, int order) {
-    k_estimate_asymto<<<1, 1, 0, ctx->stream>>>(d, nfreq, beta, f, order);
+    k_estimate_asymto<<<dg_ceil_div(d * d, 32), 32, 0, ctx->stream>>>(d, nfreq, beta, f, order);
     DG_LAUNCH(ctx, "k_estimate_asymto");
     return DMFTGPU_OK;
 }
 
 // getoccMat: n = -G(tau = beta) with the m0 = 0, m1 = I green tail (src/SCGF2_fullLoop.cpp:539-549).
-// S(beta) = sum_i Dw_i exp(-i w_i beta) = -sum_i Dw_i (exp(-i pi (2i+1)) = -1); one block: per element, P
-// threads sum fixed frequency ranges and the ranges are combined in order; then the tail term per element
-constexpr int OCC_THREADS = 1024;
-__global__ void __launch_bounds__(OCC_THREADS) k_occ_finish_blk(int d, int nfreq, double beta, const double2 *T,
-                                                                const double2 *Dw, double2 *occ) {
-    extern __shared__ double2 sw[];  // dd sums, then dd * P partials
-    const int dd = d * d, P = max(1, OCC_THREADS / dd), chunk = (nfreq + P - 1) / P;
-    double2 *part = sw + dd;
-    for (int x = threadIdx.x; x < dd * P; x += blockDim.x) {
-        const int e = x % dd, pp = x / dd;
-        double2 s = cmk(0, 0);
-        const int i1 = min(nfreq, (pp + 1) * chunk);
-        for (int i = pp * chunk; i < i1; i++) s = csub(s, Dw[(size_t)i * dd + e]);
-        part[x] = s;
+// S(beta) = sum_i Dw_i exp(-i w_i beta) = -sum_i Dw_i (exp(-i pi (2i+1)) = -1): sums over ranges of OCC_RANGE frequencies by
+// a block each, then one block adds the ranges in order and the tail term, a thread per real part (one block for all of
+// it was 0.29 ms of FP64 adds on one SM at d = 10, 4096 frequencies; the two take 0.02)
+constexpr int OCC_RANGE = 64, OCC_THREADS = 256;
+__global__ void __launch_bounds__(OCC_THREADS) k_occ_part(int dd, int nfreq, const double2 *__restrict__ Dw, double2 *part) {
+    const int i0 = blockIdx.x * OCC_RANGE, i1 = min(nfreq, i0 + OCC_RANGE);
+    const double *x = reinterpret_cast<const double *>(Dw);
+    double *o = reinterpret_cast<double *>(part) + (size_t)blockIdx.x * 2 * dd;
+    for (int e = threadIdx.x; e < 2 * dd; e += OCC_THREADS) {
+        double s = 0;
+#pragma unroll 8
+        for (int i = i0; i < i1; i++) s -= x[(size_t)i * 2 * dd + e];
+        o[e] = s;
     }
-    __syncthreads();
-    for (int e = threadIdx.x; e < dd; e += blockDim.x) {
-        double2 s = cmk(0, 0);
-        for (int pp = 0; pp < P; pp++) s = cadd(s, part[pp * dd + e]);
+}
+__global__ void __launch_bounds__(OCC_THREADS) k_occ_finish_blk(int d, int nrange, double beta, const double2 *T,
+                                                                const double2 *part, double2 *occ) {
+    extern __shared__ double osm[];  // 2 dd sums, 2 d values g
+    const int dd = d * d;
+    double *sw = osm, *g = osm + 2 * dd;
+    const TailPtrs p = tail_ptrs(T, d);
+    const double *x = reinterpret_cast<const double *>(part);
+    for (int e = threadIdx.x; e < 2 * dd; e += OCC_THREADS) {
+        double s = 0;
+#pragma unroll 8
+        for (int r = 0; r < nrange; r++) s += x[(size_t)r * 2 * dd + e];
         sw[e] = s;
     }
+    for (int l = threadIdx.x; l < 2 * d; l += OCC_THREADS) g[l] = -1.0 / (exp(p.e[l] * beta) + 1.0);
     __syncthreads();
-    TailPtrs p = tail_ptrs(const_cast<double2 *>(T), d);
-    for (int e = threadIdx.x; e < dd; e += blockDim.x) {
-        const int a = e % d, b = e / d;
-        double2 tab = cmk(0, 0), tba = cmk(0, 0);
-        for (int l = 0; l < d; l++) {
-            const double e1 = p.eH[l], e2 = p.eH2[l];
-            const double g1 = -1.0 / (exp(e1 * beta) + exp(e1 * (beta - beta)));
-            const double g2 = -1.0 / (exp(e2 * beta) + exp(e2 * (beta - beta)));
-            const double2 w1a = DG_AT(p.W1, d, l, a), w1b = DG_AT(p.W1, d, l, b);
-            const double2 w2a = DG_AT(p.W2, d, l, a), w2b = DG_AT(p.W2, d, l, b);
-            tab = cadd(tab, cadd(cscale(cmul(cconj(w1a), w1b), g1), cscale(cmul(cconj(w2a), w2b), g2)));
-            tba = cadd(tba, cadd(cscale(cmul(cconj(w1b), w1a), g1), cscale(cmul(cconj(w2b), w2a), g2)));
+    const int P = d * (d + 1) / 2;
+    for (int q = threadIdx.x; q < P; q += OCC_THREADS) {
+        int a, b;
+        pair_of(q, d, a, b);
+        double2 tab = cmk(0, 0);
+        for (int l = 0; l < 2 * d; l++) {
+            const double2 v = p.P[(size_t)l * P + q];
+            tab = cmk(fma(v.x, g[l], tab.x), fma(v.y, g[l], tab.y));
         }
-        const double2 Aab = cadd(cscale(cadd(sw[a + b * d], cconj(sw[b + a * d])), 1.0 / beta), cscale(tab, 0.5));
-        const double2 Aba = cadd(cscale(cadd(sw[b + a * d], cconj(sw[a + b * d])), 1.0 / beta), cscale(tba, 0.5));
-        occ[e] = cscale(cadd(Aab, cconj(Aba)), -0.5);
+        const int ab = a + b * d, ba = b + a * d;
+        double2 v = cmk(sw[2 * ab] + sw[2 * ba], sw[2 * ab + 1] - sw[2 * ba + 1]);
+        v = cscale(cadd(cscale(v, 1.0 / beta), cscale(tab, 0.5)), -1.0);
+        if (a == b) v.y = 0.0;
+        occ[ab] = v;
+        if (a != b) occ[ba] = cconj(v);
     }
 }
 
@@ -948,8 +1137,12 @@ __global__ void k_set_identity_slot(int d, double2 *m1) {
 int dg_occ_tail_dev(dmftgpu_ctx *ctx, int d, int nfreq, double beta, const double2 *T, const double2 *Dw,
                     double2 *occ) {
     const size_t dd = (size_t)d * d;
-    const int P = std::max(1, OCC_THREADS / (int)dd);
-    k_occ_finish_blk<<<1, OCC_THREADS, dd * (1 + P) * sizeof(double2), ctx->stream>>>(d, nfreq, beta, T, Dw, occ);
+    const int nrange = dg_ceil_div(nfreq, OCC_RANGE);
+    double2 *part = (double2 *)dg_buf(ctx, "occ.part", (size_t)nrange * dd * sizeof(double2));
+    if (!part) return DMFTGPU_NOMEM;
+    k_occ_part<<<nrange, OCC_THREADS, 0, ctx->stream>>>((int)dd, nfreq, Dw, part);
+    DG_LAUNCH(ctx, "k_occ_part");
+    k_occ_finish_blk<<<1, OCC_THREADS, (2 * dd + 2 * d) * sizeof(double), ctx->stream>>>(d, nrange, beta, T, part, occ);
     DG_LAUNCH(ctx, "k_occ_finish_blk");
     return DMFTGPU_OK;
 }
@@ -968,7 +1161,7 @@ int dg_green_tail_dev(dmftgpu_ctx *ctx, int d, int nfreq, double beta, const dou
 
 int dg_occ_dev(dmftgpu_ctx *ctx, int d, int nfreq, double beta, const double2 *gw, double2 *occ) {
     const size_t dd = (size_t)d * d;
-    double2 *T = (double2 *)dg_buf(ctx, "occ.tail", TAIL_SLOTS * dd * sizeof(double2));
+    double2 *T = (double2 *)dg_buf(ctx, "occ.tail", dg_tail_elems(d) * sizeof(double2));
     double2 *Dw = (double2 *)dg_buf(ctx, "occ.Dw", (size_t)nfreq * dd * sizeof(double2));
     if (!T || !Dw) return DMFTGPU_NOMEM;
     DG_TRY(dg_green_tail_dev(ctx, d, nfreq, beta, gw, T, Dw));
@@ -981,47 +1174,111 @@ int dg_ipt_kk_dev(dmftgpu_ctx *ctx, int nfreq, const double *a, const double *b,
     return DMFTGPU_OK;
 }
 
-// U list on the device with the two index orders getStimp's output-stationary kernel needs
+// U list on the device with getStimp's lists (k_sigma2_min, or the entry orders of k_sigma2 / k_sigma2_df where the
+// minors of one tau do not fit in shared memory), in two uploads
 int dg_ulist(dmftgpu_ctx *ctx, int d, int nu, const int *uidx, const double *ut, DgUList &U) {
     for (int x = 0; x < nu; x++)
         for (int q = 0; q < 4; q++)
             if (uidx[4 * x + q] < 0 || uidx[4 * x + q] >= d) return dg_fail(ctx, DMFTGPU_BADARG, "U list index");
-    std::vector<int> byI, byJ, offI(d + 1, 0), offJ(d + 1, 0);
-    for (int i = 0; i < d; i++) {
-        offI[i] = (int)byI.size();
-        for (int x = 0; x < nu; x++)
-            if (uidx[4 * x] == i) byI.push_back(x);
+    std::vector<int> ints(uidx, uidx + 4 * (size_t)nu);
+    std::vector<double2> vals(nu);
+    for (int x = 0; x < nu; x++) vals[x] = cmk(ut[2 * x], ut[2 * x + 1]);
+    // distinct ordered pairs and the entries in terms of them; entries whose two indices are equal have no minor
+    std::vector<int> id1((size_t)d * d, -1), id2((size_t)d * d, -1), pairs1, pairs2;
+    auto pair_id = [&](std::vector<int> &id, std::vector<int> &pairs, int a, int b) {
+        int &v = id[std::min(a, b) + (size_t)std::max(a, b) * d];
+        if (v < 0) {
+            v = (int)pairs.size() / 2;
+            pairs.push_back(std::min(a, b));
+            pairs.push_back(std::max(a, b));
+        }
+        return v;
+    };
+    std::vector<int> off1(1, 0), offs(1, 0), offb(1, 0), e1, sp2, bp;
+    std::vector<double2> c1, cb;
+    for (int i = 0; i < d; i++) {  // x1 = (i, q, m, k)
+        for (int x = 0; x < nu; x++) {
+            const int *u = uidx + 4 * x;
+            if (u[0] != i || u[2] == u[3]) continue;
+            e1.push_back(pair_id(id1, pairs1, u[2], u[3]));
+            e1.push_back(u[1]);
+            c1.push_back(cscale(vals[x], u[2] < u[3] ? 1.0 : -1.0));
+        }
+        off1.push_back((int)c1.size());
     }
-    offI[d] = (int)byI.size();
-    for (int j = 0; j < d; j++) {
-        offJ[j] = (int)byJ.size();
-        for (int x = 0; x < nu; x++)
-            if (uidx[4 * x + 3] == j) byJ.push_back(x);
+    for (int j = 0; j < d; j++) {  // x2 = (l, n, p, j), grouped by the pair (l, n)
+        const size_t first = sp2.size();
+        std::vector<std::vector<int>> members;
+        for (int x = 0; x < nu; x++) {
+            const int *u = uidx + 4 * x;
+            if (u[3] != j || u[0] == u[1]) continue;
+            const int P2 = pair_id(id2, pairs2, u[0], u[1]);
+            size_t s = first;
+            while (s < sp2.size() && sp2[s] != P2) s++;
+            if (s == sp2.size()) {
+                sp2.push_back(P2);
+                members.emplace_back();
+            }
+            members[s - first].push_back(x);
+        }
+        for (const auto &m : members) {
+            for (int x : m) {
+                const int *u = uidx + 4 * x;
+                bp.push_back(u[2]);
+                cb.push_back(cscale(vals[x], u[0] < u[1] ? -1.0 : 1.0));  // - U2 G_pq(beta - tau)
+            }
+            offb.push_back((int)bp.size());
+        }
+        offs.push_back((int)sp2.size());
     }
-    offJ[d] = (int)byJ.size();
-    const size_t nb = (size_t)std::max(nu, 1);
-    int *dI = (int *)dg_buf(ctx, "u.byI", nb * sizeof(int)), *dJ = (int *)dg_buf(ctx, "u.byJ", nb * sizeof(int));
-    int *dOI = (int *)dg_buf(ctx, "u.offI", (d + 1) * sizeof(int)), *dOJ = (int *)dg_buf(ctx, "u.offJ", (d + 1) * sizeof(int));
-    int *dU = (int *)dg_buf(ctx, "u.idx", nb * 4 * sizeof(int));
-    double2 *dT = (double2 *)dg_buf(ctx, "u.val", nb * sizeof(double2));
-    if (!dI || !dJ || !dOI || !dOJ || !dU || !dT) return DMFTGPU_NOMEM;
+    S2Lists L;
+    L.d = d;
+    L.np1 = (int)pairs1.size() / 2;
+    L.np2 = (int)pairs2.size() / 2;
+    L.nslot = (int)sp2.size();
+    L.ne1 = (int)c1.size();
+    const size_t o_lists = ints.size(), o_c = vals.size();
+    const bool fits = s2_tau_elems(d, L.np1, L.np2, L.nslot) * sizeof(double2) <= 200 * 1024;
+    size_t o_by = 0;
+    if (fits) {
+        for (const auto *v : {&off1, &offs, &offb, &pairs1, &pairs2, &e1, &sp2, &bp}) ints.insert(ints.end(), v->begin(), v->end());
+        vals.insert(vals.end(), c1.begin(), c1.end());
+        vals.insert(vals.end(), cb.begin(), cb.end());
+    } else {
+        // byIoff, byJoff, byI, byJ
+        o_by = ints.size();
+        std::vector<int> byI, byJ, offI(1, 0), offJ(1, 0);
+        for (int i = 0; i < d; i++) {
+            for (int x = 0; x < nu; x++) {
+                if (uidx[4 * x] == i) byI.push_back(x);
+                if (uidx[4 * x + 3] == i) byJ.push_back(x);
+            }
+            offI.push_back((int)byI.size());
+            offJ.push_back((int)byJ.size());
+        }
+        for (const auto *v : {&offI, &offJ, &byI, &byJ}) ints.insert(ints.end(), v->begin(), v->end());
+    }
+    int *dI = (int *)dg_buf(ctx, "u.int", std::max<size_t>(ints.size(), 1) * sizeof(int));
+    double2 *dV = (double2 *)dg_buf(ctx, "u.val", std::max<size_t>(vals.size(), 1) * sizeof(double2));
+    if (!dI || !dV) return DMFTGPU_NOMEM;
     cudaStream_t s = ctx->stream;
-    if (nu > 0) {
-        DG_CUDA(cudaMemcpyAsync(dI, byI.data(), nu * sizeof(int), cudaMemcpyHostToDevice, s));
-        DG_CUDA(cudaMemcpyAsync(dJ, byJ.data(), nu * sizeof(int), cudaMemcpyHostToDevice, s));
-        DG_CUDA(cudaMemcpyAsync(dU, uidx, (size_t)nu * 4 * sizeof(int), cudaMemcpyHostToDevice, s));
-        DG_CUDA(cudaMemcpyAsync(dT, ut, (size_t)nu * sizeof(double2), cudaMemcpyHostToDevice, s));
-    }
-    DG_CUDA(cudaMemcpyAsync(dOI, offI.data(), (d + 1) * sizeof(int), cudaMemcpyHostToDevice, s));
-    DG_CUDA(cudaMemcpyAsync(dOJ, offJ.data(), (d + 1) * sizeof(int), cudaMemcpyHostToDevice, s));
+    if (!ints.empty()) DG_CUDA(cudaMemcpyAsync(dI, ints.data(), ints.size() * sizeof(int), cudaMemcpyHostToDevice, s));
+    if (!vals.empty()) DG_CUDA(cudaMemcpyAsync(dV, vals.data(), vals.size() * sizeof(double2), cudaMemcpyHostToDevice, s));
     DG_CUDA(cudaStreamSynchronize(s));  // host vectors go out of scope
     U.nu = nu;
-    U.byI = dI;
-    U.byJ = dJ;
-    U.byIoff = dOI;
-    U.byJoff = dOJ;
-    U.uidx = dU;
-    U.ut = dT;
+    U.uidx = dI;
+    U.ut = dV;
+    U.byI = U.byJ = U.byIoff = U.byJoff = nullptr;
+    if (fits) {
+        L.i = dI + o_lists;
+        L.c = dV + o_c;
+    } else {
+        U.byIoff = dI + o_by;
+        U.byJoff = U.byIoff + d + 1;
+        U.byI = U.byJoff + d + 1;
+        U.byJ = U.byI + nu;
+    }
+    U.s2 = L;
     return DMFTGPU_OK;
 }
 

@@ -44,39 +44,42 @@ __global__ void k_write_results(int d, int nfreq, const double2 *s2, const doubl
     if (gimp_out) gimp_out[t] = g;
 }
 
-// MatsubaraFtnnorm (src/SCGF2_fullLoop.cpp:791-805) of g - gin (gin == nullptr: of g) squared, per frequency
-__global__ void k_scgf_norm_terms(int d, int nfreq, double beta, const double2 *gin, const double2 *g, double *terms) {
-    const int n = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= nfreq) return;
+// MatsubaraFtnnorm (src/SCGF2_fullLoop.cpp:791-805) of g - gin (gin == nullptr: of g) squared, per frequency: a warp each,
+// lanes along the elements
+__global__ void __launch_bounds__(128) k_scgf_norm_terms(int d, int nfreq, double beta, const double2 *gin, const double2 *g,
+                                                         double *terms) {
+    const int n = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (n >= nfreq) return;  // whole warps
     const size_t dd = (size_t)d * d;
-    const double wn = (2 * n + 1) * DG_PI / beta;
     double a = 0;
-    for (size_t e = 0; e < dd; e++) {
-        const double2 x = gin ? csub(gin[(size_t)n * dd + e], g[(size_t)n * dd + e]) : g[(size_t)n * dd + e];
+    for (size_t e = lane; e < dd; e += 32) {
+        const double2 x = gin ? csub(gin[n * dd + e], g[n * dd + e]) : g[n * dd + e];
         a += cabs2(x);
     }
-    terms[n] = a / wn;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+    if (lane == 0) terms[n] = a / ((2 * n + 1) * DG_PI / beta);
 }
 
-// fixed-order sum of the per-frequency terms, and ||occ - occ_in||_F^2; one block
-__global__ void k_scgf_norms(int d, int nfreq, const double *terms, const double2 *occ_in, const double2 *occ,
-                             double *out) {
-    __shared__ double red[256];
+// fixed-order sums of the per-frequency terms (half the block) and of ||occ - occ_in||_F^2 (the other half); one block
+__global__ void __launch_bounds__(1024) k_scgf_norms(int d, int nfreq, const double *terms, const double2 *occ_in,
+                                                     const double2 *occ, double *out) {
+    __shared__ double red[1024];
+    const int half = threadIdx.x >> 9, t = threadIdx.x & 511;
     double s = 0;
-    for (int n = threadIdx.x; n < nfreq; n += blockDim.x) s += terms[n];
+    if (half == 0) {
+#pragma unroll 4
+        for (int n = t; n < nfreq; n += 512) s += terms[n];
+    } else if (occ_in) {
+        for (int e = t; e < d * d; e += 512) s += cabs2(csub(occ[e], occ_in[e]));
+    }
     red[threadIdx.x] = s;
     __syncthreads();
-    for (int h = blockDim.x / 2; h > 0; h >>= 1) {
-        if (threadIdx.x < h) red[threadIdx.x] += red[threadIdx.x + h];
+    for (int h = 256; h > 0; h >>= 1) {
+        if (t < h) red[threadIdx.x] += red[threadIdx.x + h];
         __syncthreads();
     }
-    if (threadIdx.x == 0) {
-        double o = 0;
-        if (occ_in)
-            for (int e = 0; e < d * d; e++) o += cabs2(csub(occ[e], occ_in[e]));
-        out[0] = red[0];
-        out[1] = o;
-    }
+    if (t == 0) out[half] = red[threadIdx.x];
 }
 
 // (1 - a) x + a y over n elements (the linear mixing branch of SCGF2, :481-485)
@@ -158,7 +161,7 @@ int dg_scgf2_dev(dmftgpu_ctx *ctx, int d, int nfreq, int ntau, double beta, doub
     double2 *fock = (double2 *)dg_buf(ctx, "scgf.fock", dd * sizeof(double2));
     double *nrm = (double *)dg_buf(ctx, "scgf.norms", 2 * sizeof(double));
     double *nterm = (double *)dg_buf(ctx, "scgf.nterms", (size_t)nfreq * sizeof(double));
-    double2 *gT = (double2 *)dg_buf(ctx, "scgf.tail", 9 * dd * sizeof(double2));
+    double2 *gT = (double2 *)dg_buf(ctx, "scgf.tail", dg_tail_elems(d) * sizeof(double2));
     double2 *gDw = (double2 *)dg_buf(ctx, "scgf.Dw", (size_t)nfreq * dd * sizeof(double2));
     if (!G || !Gin || !s2 || !gt || !st || !occ || !fock || !nrm || !nterm || !gT || !gDw) return DMFTGPU_NOMEM;
     double2 *occ_in = occ + dd;
@@ -170,9 +173,9 @@ int dg_scgf2_dev(dmftgpu_ctx *ctx, int d, int nfreq, int ntau, double beta, doub
     k_set_identity<<<1, 32 * (int)((dd + 31) / 32), 0, s>>>(d, Gtail);
     DG_LAUNCH(ctx, "k_set_identity");
     DG_TRY(dg_occ_dev(ctx, d, nfreq, beta, G, occ));
-    k_scgf_norm_terms<<<dg_ceil_div(nfreq, 128), 128, 0, s>>>(d, nfreq, beta, nullptr, G, nterm);
+    k_scgf_norm_terms<<<dg_ceil_div(nfreq, 4), 128, 0, s>>>(d, nfreq, beta, nullptr, G, nterm);
     DG_LAUNCH(ctx, "k_scgf_norm_terms");
-    k_scgf_norms<<<1, 256, 0, s>>>(d, nfreq, nterm, nullptr, occ, nrm);
+    k_scgf_norms<<<1, 1024, 0, s>>>(d, nfreq, nterm, nullptr, occ, nrm);
     DG_LAUNCH(ctx, "k_scgf_norms");
     double hn[2];
     DG_CUDA(cudaMemcpyAsync(hn, nrm, sizeof(hn), cudaMemcpyDeviceToHost, s));
@@ -198,9 +201,9 @@ int dg_scgf2_dev(dmftgpu_ctx *ctx, int d, int nfreq, int ntau, double beta, doub
         // G = [(iw + mu) - H_imp - Delta - F - Sigma^(2)]^-1
         DG_TRY(dg_dyson_dev(ctx, d, nfreq, beta, mu, himp, weiss, fock, s2, G, true));
         DG_TRY(dg_occ_dev(ctx, d, nfreq, beta, G, occ));
-        k_scgf_norm_terms<<<dg_ceil_div(nfreq, 128), 128, 0, s>>>(d, nfreq, beta, Gin, G, nterm);
+        k_scgf_norm_terms<<<dg_ceil_div(nfreq, 4), 128, 0, s>>>(d, nfreq, beta, Gin, G, nterm);
         DG_LAUNCH(ctx, "k_scgf_norm_terms");
-        k_scgf_norms<<<1, 256, 0, s>>>(d, nfreq, nterm, occ_in, occ, nrm);
+        k_scgf_norms<<<1, 1024, 0, s>>>(d, nfreq, nterm, occ_in, occ, nrm);
         DG_LAUNCH(ctx, "k_scgf_norms");
         DG_CUDA(cudaMemcpyAsync(hn, nrm, sizeof(hn), cudaMemcpyDeviceToHost, s));
         int code = 0;
@@ -325,7 +328,7 @@ int dg_weak_solver_dev(dmftgpu_ctx *ctx, int solver, int d, int nfreq, int ntau,
     if (solver != DMFTGPU_WEAK_HF) {
         double2 *gt = (double2 *)dg_buf(ctx, "weak.gt", (size_t)(ntau + 1) * dd * sizeof(double2));
         double2 *st = (double2 *)dg_buf(ctx, "weak.st", (size_t)(ntau + 1) * dd * sizeof(double2));
-        double2 *T = (double2 *)dg_buf(ctx, "weak.tail", 9 * dd * sizeof(double2));
+        double2 *T = (double2 *)dg_buf(ctx, "weak.tail", dg_tail_elems(d) * sizeof(double2));
         double2 *Dw = (double2 *)dg_buf(ctx, "weak.Dw", (size_t)nfreq * dd * sizeof(double2));
         if (!gt || !st || !T || !Dw) return DMFTGPU_NOMEM;
         // FourierTransform(G0, Gt0, G0[N_freq] = I, true): the green-tail fit of G0
