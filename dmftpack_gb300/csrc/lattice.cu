@@ -26,7 +26,7 @@
 #include "smallmat_df.cuh"
 #include "adjoint.cuh"
 #include "density.cuh"
-#include "trace_tc.h"
+#include "lat_tc.h"
 
 namespace {
 
@@ -506,7 +506,7 @@ struct Prepared {
     double e0 = 0, de = 0, eta = 0;      // real-axis grid (S_REAL passes)
     const int *perm = nullptr;           // device orbital permutation (nullptr: identity)
     double2 *Vq = nullptr, *Uf = nullptr;  // with `vectors`: V of H_QQ [nk][m][m], U of H + m0 [nk][n][n]
-    mutable bool tc_ready = false;         // the tensor-core N(mu) pass's per-k operand images are built
+    mutable bool tc_ready = false;         // the tensor-core N(mu) passes' per-k operand images are built
 };
 
 // the per-k Schur data for a real-axis pass (no self-energy tail, no static spectrum): sig = Sigma(E) as given
@@ -829,6 +829,27 @@ int run_schur(dmftgpu_ctx *ctx, const Prepared &P, int mode, double mu, int wgri
     return DMFTGPU_OK;
 }
 
+LatTcArgs lat_tc_args(const Prepared &P, double mu, int wgrid) {
+    LatTcArgs a;
+    a.H = P.H;
+    a.B = P.B;
+    a.epsQ = P.epsQ;
+    a.sig = P.sig;
+    a.eps0 = P.eps;
+    a.UP = P.UP;
+    a.m0 = P.m0;
+    a.static_ready = P.static_ready;
+    a.n = P.n;
+    a.m = P.n - P.D;
+    a.nk = P.nk;
+    a.nf2 = 2 * P.Nf;
+    a.D = P.D;
+    a.wgrid = wgrid;
+    a.beta = P.beta;
+    a.mu = mu;
+    return a;
+}
+
 // the Fermi parts of a prepared lattice at mu (occ may be nullptr)
 int launch_fermi(dmftgpu_ctx *ctx, const Prepared &P, double mu, double2 *occ, double *fs) {
     const int kb = fermi_kb(P.n, P.D);
@@ -848,24 +869,11 @@ int nele_pass(dmftgpu_ctx *ctx, const Prepared &P, double mu, bool deriv, double
     if (!tr || !dtr || !fs) return DMFTGPU_NOMEM;
     if (explicit_inv) {
         DG_TRY(run_gloc(ctx, P, deriv ? (M_TRACE | M_DERIV) : M_TRACE, mu, 1, nullptr, nullptr, tr, dtr, mixed));
-    } else if (mixed && !deriv && ctx->tensor && !ctx->capturing && dg_trace_tc_supported(P.n, P.D)) {
-        // the pole sums on the tensor cores (trace_tc.cu)
+    } else if (mixed && ctx->tensor && !ctx->capturing &&
+               (deriv ? dg_lat_tc_deriv_supported(P.n, P.D) : dg_lat_tc_supported(P.n, P.D))) {
+        // the pole sums on the tensor cores (lat_tc.cu)
         DG_CUDA(cudaStreamWaitEvent(ctx->stream, P.static_ready, 0));
-        TraceTcArgs a;
-        a.H = P.H;
-        a.B = P.B;
-        a.epsQ = P.epsQ;
-        a.sig = P.sig;
-        a.eps0 = P.eps;
-        a.n = P.n;
-        a.m = P.n - P.D;
-        a.nk = P.nk;
-        a.nf2 = nf2;
-        a.D = P.D;
-        a.wgrid = 1;
-        a.beta = P.beta;
-        a.mu = mu;
-        DG_TRY(dg_trace_tc(ctx, a, &P.tc_ready, tr));
+        DG_TRY(dg_lat_tc_trace(ctx, lat_tc_args(P, mu, 1), &P.tc_ready, tr, deriv ? dtr : nullptr));
     } else {
         DG_TRY(run_schur(ctx, P, deriv ? (dg::S_TRACE | dg::S_DERIV) : dg::S_TRACE, mu, 1, nullptr, nullptr, tr, dtr,
                          mixed));
@@ -1001,7 +1009,10 @@ int greenftn_w_dev(dmftgpu_ctx *ctx, const dmftgpu_lattice *L, const double2 *dH
     if (!blk || !blk0 || !occ || !fs) return DMFTGPU_NOMEM;
     if (flags & DMFTGPU_EXPLICIT)
         DG_TRY(run_gloc(ctx, P, M_BLOCK, mu, 0, blk, blk0, nullptr, nullptr, (flags & DMFTGPU_MIXED) != 0));
-    else DG_TRY(run_schur(ctx, P, dg::S_BLOCK, mu, 0, blk, blk0, nullptr, nullptr, (flags & DMFTGPU_MIXED) != 0));
+    else if ((flags & DMFTGPU_MIXED) && !(flags & DMFTGPU_NO_TENSOR) && ctx->tensor && dg_lat_tc_block_supported(P.n, D)) {
+        // pole sums and GwHF on the tensor cores (lat_tc.cu)
+        DG_TRY(dg_lat_tc_block(ctx, lat_tc_args(P, mu, 0), blk, blk0));
+    } else DG_TRY(run_schur(ctx, P, dg::S_BLOCK, mu, 0, blk, blk0, nullptr, nullptr, (flags & DMFTGPU_MIXED) != 0));
     DG_CUDA(cudaStreamWaitEvent(ctx->stream, P.static_ready, 0));
     DG_TRY(launch_fermi(ctx, P, mu, occ, fs));
     k_gloc_scale<<<dg_ceil_div((long long)Nf * DD, 256), 256, 0, ctx->stream>>>(Nf, L->nk, D, L->nh, blk, blk0, dG, dG0);

@@ -303,6 +303,26 @@ def test_nele_tensor_cores_match_oracle(ctx, orc, n, D, nf):
         assert abs(gC - gF) < 1e-11 * max(1.0, abs(gF)), (gC, gF)
 
 
+@pytest.mark.parametrize("n,D,nk,nf", [(4, 4, 1, 24), (5, 5, 2, 33), (9, 6, 3, 40), (7, 7, 5, 31), (22, 8, 6, 32),
+                                       (32, 9, 9, 24), (10, 10, 4, 65), (28, 10, 17, 47), (32, 10, 26, 24), (9, 5, 3, 33),
+                                       (13, 5, 2, 40), (14, 6, 18, 24), (38, 6, 9, 31), (12, 8, 3, 24), (15, 7, 3, 33)])
+def test_tensor_core_block_and_derivative_passes(ctx, orc, n, D, nk, nf):
+    """G_loc, GwHF and NumMatrix, and dN/dmu, of the mixed form at 4 <= D <= 10: no ligands up to the 32 poles a k point
+    may have, the counts from which each pass is on the tensor cores (4, 6, 8), k counts around the points GwHF's sums
+    share and the chunks, frequency counts that leave partial tiles of 32.  Against the FP64 oracle (the mixed tolerance)
+    and the GPU's FP64 pass (1e-11: the slices leave less than 2^-41, inversions of matrices of condition < 1e2)."""
+    H, S, lat = _random_lattice(n, D, (nk, 1, 1), nf, [n, D, nk])
+    for mu in (-0.4, 0.3):
+        want = orc.greenftn_w(H, S, mu, 15.0, 1, D)
+        f64 = ctx.GreenFtn_w(lat, H, S, mu)
+        got = ctx.GreenFtn_w(lat, H, S, mu, mixed=True)
+        for g, w, f in zip(got, want, f64):
+            assert rel_err(g, w) < TOL_MIXED and rel_err(g, f) < 1e-11
+        N, dN = ctx.GiwToNele(lat, H, S, mu, deriv=True)
+        g, dg = ctx.GiwToNele(lat, H, S, mu, deriv=True, mixed=True)
+        assert abs(g - N) <= 1e-11 * max(1, abs(N)) and abs(dg - dN) <= 1e-10 * max(1, abs(dN))
+
+
 def test_newton_mu_through_tensor_core_passes(ctx, orc):
     """The mixed Newton mu search on the 28-orbital d+p model (D = 10): its secant passes run on the tensor cores;
     the mu it returns gives the target occupation in the FP64 oracle."""
