@@ -11,198 +11,326 @@
 // is recomputed for every (k, iw) from the per-k Schur data, as the forward pass does, and never stored: the
 // memory is O(N_freq D^2) whatever N_k, N_freq and n are.
 //
-// Mapping as in k_schur (schur.cuh): a lane group of W lanes per frequency, lane c = column c, a CTA = 128/W
-// frequencies x one chunk of k points staged in shared memory, FP64, per-chunk sums reduced in fixed order.
+// What bounds the pass is FP64 instructions: a warp's FP64 instruction holds its SM sub-partition's pipe for 64 cycles
+// whatever its lanes do, so lanes have to be full and everything else (shared memory, index arithmetic) is free beside it.
+//   - One matrix per group of LW lanes, its D^2 elements dealt over the lanes (at most 13 each): 12.5 of 13 slots carry an
+//     element at D = 20 with 32 lanes, 12.5 of 13 at D = 10 with 8.  One column per lane left 12 of 32 lanes idle at D = 20.
+//   - S and S' as sums of real weights times the Hermitian products b_l b_l^H: a thread takes a pair (a <= c) and four or
+//     eight frequencies and forms the product once for them: 4 FMA per pole, pair and sum where rank-one updates of both
+//     triangles take 8 (and a complex product each for their weights).
+//   - VJP: Re Tr[(G S' G)^H Gbar] = Re Tr[S'^H Z] with the Z = G^H Gbar G^H that Sigma_bar sums, which leaves two D^3
+//     products of four.  S' is formed after Z, so two tiles per matrix serve and two CTAs fit an SM.
+// 56 orbitals, D = 20, 125 k x 512 frequencies: 61.8 -> 23.9 ms (JVP) and 72.6 -> 23.9 (VJP),
+// the eigensolvers of the preparation (3.5 ms) included; 10 + 18 orbitals 9.4 -> 4.6 and 10.8 -> 4.7, 4 + 12 2.4 -> 0.9 and 2.7 -> 1.0.
+// CTA = F frequencies x one chunk of k points; per-chunk sums are reduced in fixed order.
 #pragma once
-#include "schur.cuh"
+#include "internal.h"
+#include "linalg.cuh"
 
 namespace dg {
 
 enum { AD_VJP = 1, AD_JVP = 2 };
+constexpr int AD_EL = 13;        // matrix elements per lane at most
+constexpr int AD_THREADS = 256;  // at most; two CTAs per SM
 
 struct AdArgs {
-    const double2 *H, *B;  // as SchurArgs
-    const double *epsQ;
+    const double2 *H, *B;  // [nk][n][n]; [nk][m][D] b_l(a)
+    const double *epsQ;    // [nk][m]
     const double2 *sig;    // [nf][D][D] Sigma(iw_n), n < nf
     const double2 *gin;    // VJP: Gbar [nf][D][D]; JVP: Sigma_dot [nf][D][D]
     double mu_dot;         // JVP
-    int n, m, nk, nf, D, kc, kchunk;
+    int n, m, nk, nf, D, kchunk, F;
     double beta, mu;
     double2 *pout;         // [nchunk][nf][D][D] per-chunk sums (Sigma_bar or G_loc_dot, before the 1/N_k)
     double *pmu;           // [nchunk][nf] VJP: per-chunk Re Tr[(G S' G)^H Gbar]
     int *status;
 };
 
-template <int DP, int W, int MODE>
-__global__ void __launch_bounds__(128) k_gloc_ad(AdArgs g) {
-    typedef OpsD Ops;
-    typedef double2 C;
-    constexpr int NG = 128 / W;
-    extern __shared__ double2 sm[];
-    const int D = g.D, DD = D * D, m = g.m;
-    C *sB = sm, *sE = sB + (size_t)g.kc * m * D, *sH = sE + (size_t)g.kc * m;
-    C *wla = sH + (size_t)g.kc * DD;                  // [NG][m]
-    C *tla = wla + (size_t)NG * m;                    // [NG][4][DP][DP]: S', G, input (Gbar or Sigma_dot), work
-    const int c = threadIdx.x & (W - 1), grp = threadIdx.x / W;
-    const int f_raw = blockIdx.x * NG + grp;
-    const bool fvalid = f_raw < g.nf;
-    const int f = fvalid ? f_raw : g.nf - 1;
-    const int chunk = blockIdx.y;
-    const int kbeg = chunk * g.kchunk, kend = min(g.nk, kbeg + g.kchunk);
-    C *tS = tla + (size_t)grp * 4 * DP * DP, *tG = tS + DP * DP, *tX = tG + DP * DP, *tV = tX + DP * DP;
-    C *wl = wla + (size_t)grp * m;
-    const bool col = c < D;
-    const double w = DG_PI * (2. * f + 1.) / g.beta;
-    const C zc = cmk(g.mu, w), iwc = cmk(0.0, w);
-    // the group's frequency data: Sigma(:, c) in registers, Gbar / Sigma_dot as a tile
-    C sgc[DP];
-#pragma unroll
-    for (int a = 0; a < DP; a++) sgc[a] = (col && a < D) ? g.sig[(size_t)f * DD + a + (size_t)c * D] : cmk(0, 0);
-    if (c < DP)
-        for (int a = 0; a < DP; a++)
-            tX[a + c * DP] = (col && a < D) ? g.gin[(size_t)f * DD + a + (size_t)c * D] : cmk(0, 0);
-    C acc[DP];
-#pragma unroll
-    for (int a = 0; a < DP; a++) acc[a] = cmk(0, 0);
-    double accmu = 0.0;
-    bool sing = false;
-    for (int k0 = kbeg; k0 < kend; k0 += g.kc) {
-        const int nkc = min(g.kc, kend - k0);
-        __syncthreads();
-        for (int t = threadIdx.x; t < nkc * m * D; t += blockDim.x) sB[t] = g.B[(size_t)k0 * m * D + t];
-        for (int t = threadIdx.x; t < nkc * m; t += blockDim.x) sE[t] = cmk(g.mu - g.epsQ[(size_t)k0 * m + t], 0.0);
-        for (int t = threadIdx.x; t < nkc * DD; t += blockDim.x) {
-            const int kk = t / DD, e = t % DD, a = e % D, b = e / D;
-            sH[t] = cneg(g.H[(size_t)(k0 + kk) * g.n * g.n + a + (size_t)b * g.n]);
-        }
-        __syncthreads();
-        for (int kk = 0; kk < nkc; kk++) {
-            const C *bs = sB + (size_t)kk * m * D, *es = sE + (size_t)kk * m, *hp = sH + (size_t)kk * DD;
-            __syncwarp();
-            for (int l = c; l < m; l += W) wl[l] = crcp(cadd(es[l], iwc));
-            __syncwarp();
-            // column c of S(z) = z - H_PP - Sigma - sum_l w_l b_l b_l^H, and of S' = I + sum_l w_l^2 b_l b_l^H
-            C s[DP], sp[DP];
-#pragma unroll
-            for (int a = 0; a < DP; a++) {
-                if (col && a < D) s[a] = csub(hp[a + c * D], sgc[a]);
-                else s[a] = (a == c) ? cmk(1, 0) : cmk(0, 0);
-                if (a == c && col) s[a] = cadd(s[a], zc);
-                sp[a] = (a == c && col) ? cmk(1, 0) : cmk(0, 0);
-            }
-            if (col)
-                for (int l = 0; l < m; l++) {
-                    const C q = cmulc(wl[l], bs[l * D + c]);
-                    const C q2 = cmul(wl[l], q);
-#pragma unroll
-                    for (int a = 0; a < DP; a++)
-                        if (a < D) {
-                            s[a] = cfms(bs[l * D + a], q, s[a]);
-                            sp[a] = cfma(bs[l * D + a], q2, sp[a]);
-                        }
-                }
-            sing |= gj_inverse<Ops, DP, W>(s, c);  // s = G(:, c)
-            __syncwarp();
-            if (c < DP) {
-#pragma unroll
-                for (int a = 0; a < DP; a++) {
-                    tG[a + c * DP] = s[a];
-                    tS[a + c * DP] = sp[a];
-                }
-            }
-            __syncwarp();
-            // the intermediate column v goes through the group's work tile, so only G(:, c), S'(:, c), Sigma(:, c)
-            // and the accumulator live in registers; the inner sums are rolled loops over shared memory
-            if (MODE == AD_JVP) {
-                // column c of G (Sigma_dot - mu_dot S') G: v = (Sigma_dot - mu_dot S') G(:, c), then G v
-                if (c < DP)
-                    for (int a = 0; a < DP; a++) {
-                        C x = cmk(0, 0);
-#pragma unroll 4
-                        for (int b = 0; b < DP; b++)
-                            x = cfma(csub(tX[a + b * DP], cscale(tS[a + b * DP], g.mu_dot)), tG[b + c * DP], x);
-                        tV[a + c * DP] = x;
-                    }
-                __syncwarp();
-#pragma unroll
-                for (int a = 0; a < DP; a++) {
-                    C x = cmk(0, 0);
-                    if (c < DP)
-#pragma unroll 4
-                        for (int b = 0; b < DP; b++) x = cfma(tG[a + b * DP], tV[b + c * DP], x);
-                    acc[a] = cadd(acc[a], x);
-                }
-                __syncwarp();
-            } else {
-                // column c of G^H Gbar G^H: v = Gbar conj(G(c, :))^T, then G^H v
-                if (c < DP)
-                    for (int a = 0; a < DP; a++) {
-                        C x = cmk(0, 0);
-#pragma unroll 4
-                        for (int b = 0; b < DP; b++) x = cfma(tX[a + b * DP], cconj(tG[c + b * DP]), x);
-                        tV[a + c * DP] = x;
-                    }
-                __syncwarp();
-#pragma unroll
-                for (int a = 0; a < DP; a++) {
-                    C x = cmk(0, 0);
-                    if (c < DP)
-#pragma unroll 4
-                        for (int b = 0; b < DP; b++) x = cfma(cconj(tG[b + a * DP]), tV[b + c * DP], x);
-                    acc[a] = cadd(acc[a], x);
-                }
-                __syncwarp();
-                // Re Tr[(G S' G)^H Gbar], column c: u = S' G(:, c) in the work tile, y = G u, sum_a Re(Gbar(a,c) conj(y_a))
-                if (c < DP)
-                    for (int a = 0; a < DP; a++) {
-                        C x = cmk(0, 0);
-#pragma unroll 4
-                        for (int b = 0; b < DP; b++) x = cfma(tS[a + b * DP], tG[b + c * DP], x);
-                        tV[a + c * DP] = x;
-                    }
-                __syncwarp();
-                double t = 0.0;
-                if (col)
-                    for (int a = 0; a < D; a++) {
-                        C y = cmk(0, 0);
-#pragma unroll 4
-                        for (int b = 0; b < DP; b++) y = cfma(tG[a + b * DP], tV[b + c * DP], y);
-                        t += cmulc(tX[a + c * DP], y).x;
-                    }
-                accmu += group_sum<DP, W>(t, 0);
-                __syncwarp();
-            }
-        }
-    }
-    if (sing && fvalid) dg_flag(g.status, DG_SINGULAR);
-    if (!fvalid) return;
-    if (col) {
-        const size_t o = ((size_t)chunk * g.nf + f) * DD + (size_t)c * D;
-#pragma unroll
-        for (int a = 0; a < DP; a++)
-            if (a < D) g.pout[o + a] = acc[a];
-    }
-    if (MODE == AD_VJP && c == 0) g.pmu[(size_t)chunk * g.nf + f] = accmu;
+// shared memory of one frequency, in double2: two tiles, the weights (w_l, w_l^2), and the inversion's row, column and
+// pivot buffers, which lie over the second tile (VJP) or over the weights (JVP), both free then
+__host__ __device__ inline int ad_bufs(int D) { return 2 * D + (D + 3) / 4; }
+__host__ __device__ inline int ad_tile1(int D, int mode) {
+    return mode == AD_VJP && ad_bufs(D) > D * D ? ad_bufs(D) : D * D;
+}
+__host__ __device__ inline int ad_weights(int D, int m, int mode) {
+    return mode == AD_JVP && ad_bufs(D) > 2 * m ? ad_bufs(D) : 2 * m;
+}
+inline size_t ad_smem(int F, int D, int m, int mode) {
+    return (size_t)F * (D * D + ad_tile1(D, mode) + ad_weights(D, m, mode)) * 16 + (size_t)(D * (D + 1) / 2) * 4;
 }
 
-inline size_t ad_smem(int DP, int W, int kc, int D, int m) {
-    const int NG = 128 / W;
-    return ((size_t)kc * m * D + (size_t)kc * m + (size_t)kc * D * D + (size_t)NG * m + (size_t)NG * 4 * DP * DP) * 16;
+// In-place inverse of the D x D tile A (column-major) by LW lanes; every group of the warp calls it together.  Gauss-Jordan
+// with partial pivoting by max(|re|, |im|) compared on the high words (no FP64 work): every element is updated alike as
+// A - col(r) row(c), with row k and column k read as zero, row = the scaled pivot row with 1/pivot at k and col(k) = -1.
+template <int LW>
+__device__ __forceinline__ bool tile_inverse(double2 *A, int D, double2 *rowb, double2 *colb, int *perm, int g) {
+    bool sing = false, moved = false;
+    const int DD = D * D;
+#pragma unroll 1
+    for (int k = 0; k < D; k++) {
+        unsigned best = 0;
+        int p = k;
+        for (int r = k + g; r < D; r += LW) {
+            const double2 v = A[r + k * D];
+            const unsigned key = max((unsigned)__double2hiint(v.x) & 0x7fffffffu, (unsigned)__double2hiint(v.y) & 0x7fffffffu);
+            if (key > best) {
+                best = key;
+                p = r;
+            }
+        }
+#pragma unroll
+        for (int o = LW / 2; o > 0; o >>= 1) {
+            const unsigned ob = __shfl_xor_sync(0xffffffffu, best, o, LW);
+            const int op = __shfl_xor_sync(0xffffffffu, p, o, LW);
+            if (ob > best || (ob == best && op < p)) {
+                best = ob;
+                p = op;
+            }
+        }
+        if (g == 0) perm[k] = p;
+        if (__any_sync(0xffffffffu, p != k)) {
+            moved = true;
+            for (int c = g; c < D; c += LW) {
+                const double2 t = A[k + c * D];
+                A[k + c * D] = A[p + c * D];
+                A[p + c * D] = t;
+            }
+            __syncwarp();
+        }
+        const double2 piv = A[k + k * D];
+        const double den = fma(piv.x, piv.x, piv.y * piv.y);
+        sing |= !(den > 0.0);
+        const double q = 1.0 / den;
+        const double2 ip = cmk(piv.x * q, -piv.y * q);
+        for (int c = g; c < D; c += LW) {
+            rowb[c] = c == k ? ip : cmul(A[k + c * D], ip);
+            colb[c] = c == k ? cmk(-1.0, 0.0) : A[c + k * D];
+        }
+        __syncwarp();
+        int r = g % D, c = g / D;
+#pragma unroll 4
+        for (int e = g; e < DD; e += LW) {
+            const bool z = r == k || c == k;
+            A[e] = cfms(colb[r], rowb[c], z ? cmk(0.0, 0.0) : A[e]);
+            r += LW;
+            while (r >= D) {
+                r -= D;
+                c++;
+            }
+        }
+        __syncwarp();
+    }
+    if (!moved) return sing;
+#pragma unroll 1
+    for (int k = D - 1; k >= 0; k--) {  // undo the row interchanges as column interchanges, last first
+        const int p = perm[k];
+        for (int r = g; r < D; r += LW) {
+            const double2 t = A[r + k * D];
+            A[r + k * D] = A[r + p * D];
+            A[r + p * D] = t;
+        }
+        __syncwarp();
+    }
+    return sing;
+}
+
+// sums over the poles of one pair (a, c) and SUB frequencies: s[i] = sum_l (Re, Im of the weight) x (p, q), with
+// b_a conj(b_c) = p + iq; slot: the weights' slot (0: w, 1: w^2)
+struct PairSum {
+    double up, uq, vp, vq;
+    __device__ __forceinline__ void add(double2 w, double p, double q) {
+        up = fma(w.x, p, up);
+        uq = fma(w.x, q, uq);
+        vp = fma(w.y, p, vp);
+        vq = fma(w.y, q, vq);
+    }
+    // sum_l w_l b_a conj(b_c) and sum_l w_l b_c conj(b_a)
+    __device__ __forceinline__ double2 ac() const { return cmk(up - vq, uq + vp); }
+    __device__ __forceinline__ double2 ca() const { return cmk(up + vq, vp - uq); }
+};
+
+template <int LW, int MODE>
+__global__ void __launch_bounds__(AD_THREADS, 2) k_gloc_ad(AdArgs g) {
+    typedef double2 C;
+    constexpr int SUB = MODE == AD_JVP ? 4 : 8;
+    extern __shared__ double2 sm[];
+    const int D = g.D, DD = D * D, m = g.m, F = g.F, npair = D * (D + 1) / 2;
+    const int t1 = ad_tile1(D, MODE), ws = ad_weights(D, m, MODE);
+    C *T0 = sm, *T1 = T0 + (size_t)F * DD, *sW = T1 + (size_t)F * t1;
+    ushort2 *sPair = reinterpret_cast<ushort2 *>(sW + (size_t)F * ws);
+    const int lane = threadIdx.x % LW, grp = threadIdx.x / LW, f0 = blockIdx.x * F;
+    const bool fvalid = f0 + grp < g.nf;
+    const int f = min(f0 + grp, g.nf - 1);
+    const int chunk = blockIdx.y, kbeg = chunk * g.kchunk, kend = min(g.nk, kbeg + g.kchunk);
+    C *A = T0 + (size_t)grp * DD, *V = T1 + (size_t)grp * t1;
+    C *buf = MODE == AD_VJP ? V : sW + (size_t)grp * ws;
+    for (int t = threadIdx.x; t < npair; t += blockDim.x) {  // t = a + c (c + 1) / 2, a <= c
+        int c = 0;
+        while ((c + 1) * (c + 2) / 2 <= t) c++;
+        sPair[t] = make_ushort2((unsigned short)(t - c * (c + 1) / 2), (unsigned short)c);
+    }
+    C acc[AD_EL];
+#pragma unroll
+    for (int i = 0; i < AD_EL; i++) acc[i] = cmk(0, 0);
+    double accmu = 0.0;
+    bool sing = false;
+    const int nsub = (F + SUB - 1) / SUB;
+    for (int k = kbeg; k < kend; k++) {
+        const C *__restrict__ Bk = g.B + (size_t)k * m * D, *__restrict__ Hk = g.H + (size_t)k * g.n * g.n;
+        __syncthreads();
+        for (int t = threadIdx.x; t < F * m; t += blockDim.x) {
+            const int fl = t / m, l = t - fl * m;
+            const double w = DG_PI * (2. * min(f0 + fl, g.nf - 1) + 1.) / g.beta;
+            const C wl = crcp(cmk(g.mu - g.epsQ[(size_t)k * m + l], w));
+            sW[(size_t)fl * ws + 2 * l] = wl;
+            sW[(size_t)fl * ws + 2 * l + 1] = cmul(wl, wl);
+        }
+        __syncthreads();
+        // M = z - H_PP - Sigma - S into the first tile; JVP: Sigma_dot - mu_dot S' into the second
+        for (int t = threadIdx.x; t < npair * nsub; t += blockDim.x) {
+            const int s = t / npair;
+            const ushort2 pr = sPair[t - s * npair];
+            const int a = pr.x, c = pr.y;
+            PairSum x[SUB], y[MODE == AD_JVP ? SUB : 1];
+#pragma unroll
+            for (int i = 0; i < SUB; i++) {
+                x[i] = {0, 0, 0, 0};
+                if (MODE == AD_JVP) y[i] = {0, 0, 0, 0};
+            }
+            for (int l = 0; l < m; l++) {
+                const C pq = cmulc(Bk[l * D + a], Bk[l * D + c]);
+#pragma unroll
+                for (int i = 0; i < SUB; i++) {
+                    const C *w = sW + (size_t)min(s * SUB + i, F - 1) * ws + 2 * l;
+                    x[i].add(w[0], pq.x, pq.y);
+                    if (MODE == AD_JVP) y[i].add(w[1], pq.x, pq.y);
+                }
+            }
+            const C h = Hk[a + c * g.n], ht = Hk[c + a * g.n];
+#pragma unroll
+            for (int i = 0; i < SUB; i++) {
+                const int fl = s * SUB + i;
+                if (fl >= F) break;
+                const int ff = min(f0 + fl, g.nf - 1);
+                const C *sg = g.sig + (size_t)ff * DD;
+                C d = cneg(cadd(cadd(h, sg[a + c * D]), x[i].ac())), e = cneg(cadd(cadd(ht, sg[c + a * D]), x[i].ca()));
+                if (a == c) d = e = cadd(d, cmk(g.mu, DG_PI * (2. * ff + 1.) / g.beta));
+                T0[(size_t)fl * DD + a + c * D] = d;
+                T0[(size_t)fl * DD + c + a * D] = e;
+                if (MODE == AD_JVP) {
+                    const C *sd = g.gin + (size_t)ff * DD;
+                    const double one = a == c ? 1.0 : 0.0;
+                    const C u = y[i].ac(), v = y[i].ca();
+                    T1[(size_t)fl * DD + a + c * D] = csub(sd[a + c * D], cscale(cmk(one + u.x, u.y), g.mu_dot));
+                    T1[(size_t)fl * DD + c + a * D] = csub(sd[c + a * D], cscale(cmk(one + v.x, v.y), g.mu_dot));
+                }
+            }
+        }
+        __syncthreads();
+        sing |= tile_inverse<LW>(A, D, buf, buf + D, reinterpret_cast<int *>(buf + 2 * D), lane) && fvalid;
+        if (MODE == AD_JVP) {
+            // elements e = r + D c: X G, then G (X G)
+            C v[AD_EL];
+#pragma unroll
+            for (int i = 0; i < AD_EL; i++) {
+                const int e = lane + i * LW;
+                v[i] = cmk(0, 0);
+                if (e < DD) {
+                    const int c = e / D, r = e - c * D;
+#pragma unroll 4
+                    for (int b = 0; b < D; b++) v[i] = cfma(V[r + b * D], A[b + c * D], v[i]);
+                }
+            }
+            __syncwarp();
+#pragma unroll
+            for (int i = 0; i < AD_EL; i++)
+                if (lane + i * LW < DD) V[lane + i * LW] = v[i];
+            __syncwarp();
+#pragma unroll
+            for (int i = 0; i < AD_EL; i++) {
+                const int e = lane + i * LW;
+                if (e < DD) {
+                    const int c = e / D, r = e - c * D;
+                    C x = cmk(0, 0);
+#pragma unroll 4
+                    for (int b = 0; b < D; b++) x = cfma(A[r + b * D], V[b + c * D], x);
+                    acc[i] = cadd(acc[i], x);
+                }
+            }
+        } else {
+            // elements e = c + D r, so that lanes read along columns of G: Gbar G^H, then Z = G^H (Gbar G^H), transposed
+            const C *gb = g.gin + (size_t)f * DD;
+#pragma unroll 1
+            for (int e = lane; e < DD; e += LW) {
+                const int r = e / D, c = e - r * D;
+                C x = cmk(0, 0);
+#pragma unroll 4
+                for (int b = 0; b < D; b++) x = cfma(gb[r + b * D], cconj(A[c + b * D]), x);
+                V[e] = x;
+            }
+            __syncwarp();
+            C z[AD_EL];
+#pragma unroll
+            for (int i = 0; i < AD_EL; i++) {
+                const int e = lane + i * LW;
+                z[i] = cmk(0, 0);
+                if (e < DD) {
+                    const int r = e / D, c = e - r * D;
+#pragma unroll 4
+                    for (int b = 0; b < D; b++) z[i] = cfma(cconj(A[b + r * D]), V[c + b * D], z[i]);
+                    acc[i] = cadd(acc[i], z[i]);
+                }
+            }
+            __syncwarp();
+#pragma unroll
+            for (int i = 0; i < AD_EL; i++)
+                if (lane + i * LW < DD) V[lane + i * LW] = z[i];
+            __syncthreads();
+            // S' over G, transposed as Z is
+            for (int t = threadIdx.x; t < npair * nsub; t += blockDim.x) {
+                const int s = t / npair;
+                const ushort2 pr = sPair[t - s * npair];
+                const int a = pr.x, c = pr.y;
+                PairSum y[SUB];
+#pragma unroll
+                for (int i = 0; i < SUB; i++) y[i] = {0, 0, 0, 0};
+                for (int l = 0; l < m; l++) {
+                    const C pq = cmulc(Bk[l * D + a], Bk[l * D + c]);
+#pragma unroll
+                    for (int i = 0; i < SUB; i++)
+                        y[i].add(sW[(size_t)min(s * SUB + i, F - 1) * ws + 2 * l + 1], pq.x, pq.y);
+                }
+#pragma unroll
+                for (int i = 0; i < SUB; i++) {
+                    const int fl = s * SUB + i;
+                    if (fl >= F) break;
+                    const double one = a == c ? 1.0 : 0.0;
+                    const C u = y[i].ac(), v = y[i].ca();
+                    T0[(size_t)fl * DD + c + a * D] = cmk(one + u.x, u.y);
+                    T0[(size_t)fl * DD + a + c * D] = cmk(one + v.x, v.y);
+                }
+            }
+            __syncthreads();
+            for (int e = lane; e < DD; e += LW) accmu = fma(A[e].x, V[e].x, fma(A[e].y, V[e].y, accmu));
+        }
+    }
+    if (sing) dg_flag(g.status, DG_SINGULAR);
+    if (MODE == AD_VJP) {
+#pragma unroll
+        for (int o = LW / 2; o > 0; o >>= 1) accmu += __shfl_xor_sync(0xffffffffu, accmu, o, LW);
+    }
+    if (!fvalid) return;
+    C *o = g.pout + ((size_t)chunk * g.nf + f) * DD;
+#pragma unroll
+    for (int i = 0; i < AD_EL; i++) {
+        const int e = lane + i * LW;
+        if (e < DD) o[MODE == AD_JVP ? e : e / D + (e % D) * D] = acc[i];
+    }
+    if (MODE == AD_VJP && lane == 0) g.pmu[(size_t)chunk * g.nf + f] = accmu;
 }
 
 typedef void (*AdKernel)(AdArgs);
-#define DG_AD_DECL(DP) AdKernel ad_kernel_##DP(int mode);
-DG_AD_DECL(1)
-DG_AD_DECL(2)
-DG_AD_DECL(3)
-DG_AD_DECL(4)
-DG_AD_DECL(6)
-DG_AD_DECL(8)
-DG_AD_DECL(10)
-DG_AD_DECL(12)
-DG_AD_DECL(16)
-DG_AD_DECL(20)
-#define DG_AD_INST(DP, W) \
-    AdKernel ad_kernel_##DP(int mode) { return mode == AD_VJP ? k_gloc_ad<DP, W, AD_VJP> : k_gloc_ad<DP, W, AD_JVP>; }
+// the kernel and its lanes per matrix: the fewest that hold D^2 elements at 13 a lane
+AdKernel ad_kernel(int D, int mode, int *lanes);
 
 }  // namespace dg

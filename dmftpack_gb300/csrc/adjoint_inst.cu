@@ -1,15 +1,14 @@
-// adjoint_inst.cu -- explicit instantiations of k_gloc_ad (adjoint.cuh), one translation unit for all widths.
+// adjoint_inst.cu -- explicit instantiations of k_gloc_ad (adjoint.cuh), one translation unit for all lane groups.
 #include "adjoint.cuh"
 
 namespace dg {
-DG_AD_INST(1, 1)
-DG_AD_INST(2, 2)
-DG_AD_INST(3, 4)
-DG_AD_INST(4, 4)
-DG_AD_INST(6, 8)
-DG_AD_INST(8, 8)
-DG_AD_INST(10, 16)
-DG_AD_INST(12, 16)
-DG_AD_INST(16, 16)
-DG_AD_INST(20, 32)
+AdKernel ad_kernel(int D, int mode, int *lanes) {
+    const int lw = D <= 7 ? 4 : (D <= 10 ? 8 : (D <= 14 ? 16 : 32));
+    *lanes = lw;
+    if (D > 20) return nullptr;
+    if (lw == 4) return mode == AD_VJP ? k_gloc_ad<4, AD_VJP> : k_gloc_ad<4, AD_JVP>;
+    if (lw == 8) return mode == AD_VJP ? k_gloc_ad<8, AD_VJP> : k_gloc_ad<8, AD_JVP>;
+    if (lw == 16) return mode == AD_VJP ? k_gloc_ad<16, AD_VJP> : k_gloc_ad<16, AD_JVP>;
+    return mode == AD_VJP ? k_gloc_ad<32, AD_VJP> : k_gloc_ad<32, AD_JVP>;
+}
 }  // namespace dg

@@ -926,37 +926,35 @@ __global__ void k_ad_mu(int n, double scale, const double *p, double *out) {
     if (threadIdx.x == 0) *out = red[0] * scale;
 }
 
-struct AdInst {
-    int DP, W;
-    dg::AdKernel (*get)(int);
-};
-const AdInst kAdInst[] = {
-    {1, 1, dg::ad_kernel_1},    {2, 2, dg::ad_kernel_2},    {3, 4, dg::ad_kernel_3},   {4, 4, dg::ad_kernel_4},
-    {6, 8, dg::ad_kernel_6},    {8, 8, dg::ad_kernel_8},    {10, 16, dg::ad_kernel_10}, {12, 16, dg::ad_kernel_12},
-    {16, 16, dg::ad_kernel_16}, {20, 32, dg::ad_kernel_20},
-};
-
 // one derivative pass: VJP (gin = Gbar; out = Sigma_bar; *dmu_out = mu_bar on the device) or JVP (gin =
 // Sigma_dot, mu_dot; out = G_loc_dot)
 int run_ad(dmftgpu_ctx *ctx, const Prepared &P, int mode, double mu, const double2 *gin, double mu_dot, double2 *out,
            double *dmu_out) {
-    const AdInst *in = nullptr;
-    for (const auto &x : kAdInst)
-        if (x.DP >= P.D) {
-            in = &x;
-            break;
-        }
-    if (!in) return dg_fail(ctx, DMFTGPU_BADARG, "derivatives: correlated block larger than 20");
-    dg::AdKernel kern = in->get(mode);
-    const int m = P.n - P.D, NG = 128 / in->W, nf = P.Nf, DD = P.D * P.D;
-    int kc = 16;
-    while (kc > 1 && dg::ad_smem(in->DP, in->W, kc, P.D, m) > 96 * 1024) kc /= 2;
-    const size_t smem = dg::ad_smem(in->DP, in->W, kc, P.D, m);
+    int lanes = 0;
+    dg::AdKernel kern = dg::ad_kernel(P.D, mode, &lanes);
+    if (!kern) return dg_fail(ctx, DMFTGPU_BADARG, "derivatives: correlated block larger than 20");
+    const int m = P.n - P.D, nf = P.Nf, DD = P.D * P.D, step = std::max(1, 32 / lanes);
+    // frequencies per CTA: whole warps, no more than there are, two CTAs per SM (228 KB, 1 KB of it taken per CTA)
+    int F = std::min(dg::AD_THREADS / lanes, dg_ceil_div(nf, step) * step);
+    while (F > step && dg::ad_smem(F, P.D, m, mode) > 113 * 1024) F -= step;
+    const size_t smem = dg::ad_smem(F, P.D, m, mode);
     DG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const int fblocks = dg_ceil_div(nf, NG);
-    int nchunk = std::max(1, std::min(dg_ceil_div(P.nk, 64), dg_ceil_div(8 * 152, fblocks)));
-    const int kchunk = dg_ceil_div(P.nk, nchunk);
-    nchunk = dg_ceil_div(P.nk, kchunk);
+    // k points per CTA: the fewest rounds of CTAs x (their k points and a little for their start), at most eight rounds
+    int nsm = 152;
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, ctx->device);
+    const int fblocks = dg_ceil_div(nf, F), slots = 2 * nsm;
+    int kchunk = P.nk;
+    double best = 1e300;
+    for (int kch = P.nk; kch >= 1; kch--) {
+        const long long ctas = (long long)fblocks * dg_ceil_div(P.nk, kch), rounds = (ctas + slots - 1) / slots;
+        if (rounds > 8 && kch < P.nk) break;
+        const double cost = rounds * (kch + 0.3);
+        if (cost < best) {
+            best = cost;
+            kchunk = kch;
+        }
+    }
+    const int nchunk = dg_ceil_div(P.nk, kchunk);
     double2 *pout = (double2 *)dg_buf(ctx, "ad.pout", (size_t)nchunk * nf * DD * sizeof(double2));
     double *pmu = (double *)dg_buf(ctx, "ad.pmu", (size_t)nchunk * nf * sizeof(double));
     if (!pout || !pmu) return DMFTGPU_NOMEM;
@@ -972,8 +970,8 @@ int run_ad(dmftgpu_ctx *ctx, const Prepared &P, int mode, double mu, const doubl
     g.nk = P.nk;
     g.nf = nf;
     g.D = P.D;
-    g.kc = kc;
     g.kchunk = kchunk;
+    g.F = F;
     g.beta = P.beta;
     g.mu = mu;
     g.pout = pout;
@@ -981,7 +979,7 @@ int run_ad(dmftgpu_ctx *ctx, const Prepared &P, int mode, double mu, const doubl
     g.status = ctx->d_status;
     {
         DgTimer tm(ctx, "k_gloc_ad");
-        kern<<<dim3(fblocks, nchunk), 128, smem, ctx->stream>>>(g);
+        kern<<<dim3(fblocks, nchunk), F * lanes, smem, ctx->stream>>>(g);
     }
     DG_LAUNCH(ctx, "k_gloc_ad");
     const long long len = (long long)nf * DD;

@@ -110,3 +110,39 @@ def test_autograd_gradient_matches_finite_differences(ctx):
             e[i] = h
             fd[i] = (float(loss(theta + e)) - float(loss(theta - e))) / (2 * h)
     assert np.allclose(grad, fd, rtol=1e-6, atol=1e-9 * abs(L.item())), (grad, fd)
+
+
+@pytest.mark.parametrize("n,D,nk,nf", [(1, 1, 3, 24), (4, 2, 2, 65), (9, 7, 3, 33), (8, 8, 1, 31), (13, 10, 5, 25),
+                                       (14, 11, 2, 34), (20, 14, 3, 31), (17, 15, 2, 25), (64, 20, 2, 25), (20, 20, 4, 24)])
+def test_derivatives_against_the_full_inverse(ctx, n, D, nk, nf):
+    """J v and J^H Gbar at the edges of the lane groups (7, 10, 14, 20 orbitals), without poles and with the most, frequency
+    counts around the CTAs' against numpy inverses of the full n x n matrices.  1e-11: 64-bit products of some 20 terms
+    behind inversions of condition < 1e2 and eigenvectors good to 1e-14."""
+    import torch
+    rng = np.random.default_rng([n, D, nk, nf])
+    beta, mu, mud = 12.0, 0.15, 0.6
+    c = lambda *s: rng.normal(size=s) + 1j * rng.normal(size=s)
+    H = c(nk, n, n) / np.sqrt(n)
+    H = 0.5 * (H + H.conj().transpose(0, 2, 1))
+    w = np.pi * (2 * np.arange(nf) + 1) / beta
+    X = c(D, D)
+    S = 0.05 * np.eye(D) + 0.2 * (X @ X.conj().T / D)[None] / (1j * w[:, None, None] + 1.0)
+    Sd, Gb = c(nf, D, D), c(nf, D, D)
+    full = np.zeros((nf, n, n), complex)
+    full[:, :D, :D] = S
+    dX = np.zeros((nf, n, n), complex)
+    dX[:, :D, :D] = Sd
+    dX -= mud * np.eye(n)
+    G = np.linalg.inv((1j * w + mu)[None, :, None, None] * np.eye(n) - H[:, None] - full[None])
+    want = (G @ dX @ G)[:, :, :D, :D].mean(0)
+    GP = G[:, :, :D, :D].conj().transpose(0, 1, 3, 2)
+    wsb = (GP @ Gb @ GP).mean(0)
+    wmb = -np.einsum("kfab,fab->", (G @ G)[:, :, :D, :D].conj(), Gb).real / nk
+    dev = torch.device("cuda:0")
+    t = lambda x: torch.from_numpy(np.ascontiguousarray(x)).to(dev)
+    lat = lib.Lattice(n, nk, nf, beta, 1, D)
+    got = ctx.GreenFtn_w_jvp(lat, t(H), t(S), mu, t(Sd), mud)
+    sb, mb = ctx.GreenFtn_w_vjp(lat, t(H), t(S), mu, t(Gb))
+    assert rel_err(got.cpu().numpy(), want) < 1e-11
+    assert rel_err(sb.cpu().numpy(), wsb) < 1e-11
+    assert abs(mb - wmb) <= 1e-11 * max(abs(wmb), np.abs(Gb).sum() / nk)
