@@ -25,21 +25,26 @@
 //     512, and all 128 lanes carry rows.
 //   dN/dmu: 6 slices, levels 0 .. 3 exact, 4 and 5 shared (rounding ~2^-52).  Five accumulators of 112 columns (D > 8) do
 //     not fit: the columns are then multiplied and drained in two parts, 64 and NP - 64.
-//   G_loc / GwHF: 6 slices likewise, but only 64 rows are needed (32 frequencies x Re w, Im w): the shared levels
-//     accumulate in the other 64 lanes of the first accumulator.  In the A image every block of 64 rows stands between
-//     64 rows of zeros, and an MMA that starts at the block fills lanes 0 .. 63, one that starts at the zeros before it
-//     lanes 64 .. 127.
+//   G_loc / GwHF: 6 slices likewise, but only 64 rows are needed (32 frequencies x Re w, Im w): the lower columns
+//     accumulate in lanes 0 .. 63 and the upper ones in lanes 64 .. 127 of the same accumulators, so that five fit and all
+//     four lane quarters drain alike.  In the A image every block of 64 rows stands between 64 rows of zeros; an MMA that
+//     starts at the block fills lanes 0 .. 63, one that starts at the zeros before it lanes 64 .. 127.
 // (5 slices of 8 bits left 2^-41: five to ten times the error of double-float sums in G_loc, and
 // 5 of 9 twenty times in dN/dmu.)
 //
 // Work split: what bounds the passes is the double-float D x D inversions on the FP32 pipe, so they run on warps of their
 // own, one frequency per group of DP lanes (32/DP groups per warp, group_gj_inverse in packed arithmetic), and four
 // producer warps prepare the next k beside them: pole weights and slices (A image), MMAs, and the drain of TMEM, which
-// combines A and B into the complex entries of S (with H_PP added) and R and leaves them in shared memory.  The
-// hand-over is by named barriers: FULL (the tiles of k are there), EMPTY (every inversion warp has its columns in
-// registers).  On the d + p model (n = 28, D = 10, 1,000 k x 2,048 frequencies, 512 k for the search) the G_loc pass
-// takes 30.2 ms end to end where k_schur's took 66.8, the Newton search for mu 69.6 where its derivative passes by k_schur
-// and its traces with an inversion per producer step took 119.8.
+// leaves the dofs of A and B in shared memory as they are; the inversion warps form S = A + iB and I + R from them and add
+// H_PP.  The hand-over is by named barriers: FULL (the tiles of k are there), EMPTY (every inversion warp has its columns
+// in registers).
+// On the d + p model (n = 28, D = 10, 1,000 k x 2,048 frequencies; 512 k for the search for mu) G_loc took 66.8 ms end to
+// end by k_schur, 30.2 with the complex entries formed and H_PP added in the drain and the shared levels of G_loc in a
+// fifth sum passed through shared memory, and takes 25.7; the search 119.8 (derivatives by k_schur), 69.6, and 60.8.
+// The producers were the longer chain then (38,000 cycles per k of which 19,000 the drain, 7,000 the MMAs issued by a
+// rolled loop); now it is the inversions: 36,000 cycles per k and CTA, of which the FP32 pipe is busy 24,000.  Without the
+// producers' work the pass takes as long; searching the next pivot and forming its reciprocal beside the update, or
+// hand-overs by mbarriers (no rendezvous of the inversion warps), gain nothing for G_loc and lose 5 - 8 % for N(mu).
 #include <algorithm>
 
 #include <cuda_bf16.h>
@@ -90,23 +95,25 @@ struct TT {
     static constexpr int A_EL = (NS * KSTEPS * ROWS + (TWO ? BLK : 0)) * 16;
     static constexpr int B_EL = NSB * KSTEPS * NP * 16;  // stored per k
     static constexpr int B_USED = NS * KSTEPS * NP * 16; // copied to shared memory
-    static constexpr int NACC = MODE == TC_DERIV ? 5 : 4;  // TMEM accumulators: the last (TWO: the upper lanes) shared
-    static constexpr int NA = NACC * NP > 512 ? 64 : NP;   // columns multiplied at a time
+    static constexpr int NACC = NS - 1;                    // TMEM accumulators, the last of the shared levels
+    static constexpr int LO = NP / 32 * 16;                // TWO: columns in lanes 0 .. 63
+    static constexpr int NA = TWO ? NP - LO : (NACC * NP > 512 ? 64 : NP);  // columns of an accumulator
+    static constexpr bool PARTS = !TWO && NA < NP;         // the columns in two parts, one after the other
     static constexpr int TMEM = pow2_at_least(NACC * NA);
     // shared memory layout (bytes)
     static constexpr int O_A = 0;
     static constexpr int O_B = O_A + A_EL * 2;
-    static constexpr int O_S = O_B + B_USED * 2;                 // [FT][r][c] pdf: S + H_PP (DERIV: then T, transposed)
-    static constexpr int O_R = O_S + FT * DD * 16;               // [FT]: I + R (TRACE: transposed); TWO: see LDH
-    static constexpr int LDH = NP + 1;                           // TWO: [BLK][LDH] floats, the shared levels' sums
-    static constexpr int O_H = O_R + (TWO ? (BLK * LDH * 4 + 15) / 16 * 16 : FT * DD * 16);  // [r][c] pdf: H_PP
-    static constexpr int O_COL = O_H + DD * 16;                  // NP floats: dof column scales of k
+    // drained sums: [FT][TILE] pdf, per frequency the D^2 dofs of A, then (RS on, an odd row: no bank conflicts) of B
+    static constexpr int RS = DD / 2 + 1 - (DD / 2) % 2, TILE = 2 * RS > DD ? 2 * RS : DD;
+    static constexpr int O_S = O_B + B_USED * 2;                 // S (DERIV: then T)
+    static constexpr int O_R = O_S + FT * TILE * 16;             // R, not TWO (DERIV: then G and X as [r][c])
+    static constexpr int O_H = O_R + (TWO ? 0 : FT * TILE * 16); // [3][r][c] pdf: H_PP (slot k mod 3)
+    static constexpr int O_COL = O_H + 3 * DD * 16;                  // NP floats: dof column scales of k
     static constexpr int O_ROW = O_COL + NP * 4;                 // ROWS floats: row scales
     static constexpr int O_E0 = O_ROW + ROWS * 4;                // [3][NE0] dfl: mu - e0_j (slot k mod 3)
     static constexpr int O_SW = O_E0 + 3 * NE0 * 8;              // [3][FT] two dfl: Re sum_l w_l, Re sum_l w_l^2
     static constexpr int O_EQ = O_SW + 3 * FT * 16;              // KP dfl: mu - e_l
-    static constexpr int O_PAIR = O_EQ + KP * 8;                 // (a, c) of every pair
-    static constexpr int O_BAR = (O_PAIR + (DP * (DP - 1) / 2) * 4 + 15) / 16 * 16;  // 2 mbarriers, TMEM slot, error flag
+    static constexpr int O_BAR = (O_EQ + KP * 8 + 15) / 16 * 16;  // 2 mbarriers, TMEM slot, error flag
     static constexpr int SMEM = O_BAR + 32;
     static_assert(NACC * NA <= 512 && NP <= 2 * NA, "accumulators exceed TMEM");
     static_assert(NP <= 256 && NP % 16 == 0, "MMA N");
@@ -114,14 +121,11 @@ struct TT {
     static_assert(O_B % 128 == 0 && O_COL % 16 == 0 && O_E0 % 16 == 0 && O_SW % 16 == 0, "alignment");
 };
 
-// pair (a < c) number idx of the strict upper triangle, row-major
-__host__ __device__ __forceinline__ void pair_of(int idx, int D, int &a, int &c) {
-    a = 0;
-    while (idx >= D - 1 - a) {
-        idx -= D - 1 - a;
-        a++;
-    }
-    c = a + 1 + idx;
+// pair (a < c) number idx = c (c - 1) / 2 + a
+__host__ __device__ __forceinline__ void pair_of(int idx, int &a, int &c) {
+    c = 1;
+    while (idx >= c) idx -= c++;
+    a = idx;
 }
 
 // x = h + l in [-1, 1] -> NS weighted slices, both halves of a pair at once: slice s is x rounded to a multiple of
@@ -162,7 +166,7 @@ __global__ void k_tc_prep(int nk, int m, int D, int unit, const double2 *__restr
         const int k = (int)(t / T::NP), p = (int)(t % T::NP);
         int a = 0, c = 0;
         const bool pair = p < 2 * npair, live = p < D * D;
-        if (pair) pair_of(p >> 1, D, a, c);
+        if (pair) pair_of(p >> 1, a, c);
         else if (live) a = c = p - 2 * npair;
         const double2 *b = B + (size_t)k * m * D;
         double v[KP], mx = 0.0;
@@ -256,15 +260,17 @@ __device__ __forceinline__ void tmem_ld16x4(uint32_t addr, uint32_t stride, uint
 #pragma unroll
         for (int j = 0; j < 16; j++) asm volatile("" : "+r"(v[i][j]));
 }
-// columns 2j, 2j+1 of the drained sums; SIX: `top` has the shared levels'
+// columns 2j, 2j+1 of the drained sums; SIX: `top` has the shared levels'.  Level L is an integer multiple of 2^{-(16 + 9 L)}
+// and level L + 1 below 2^{-2 - 9 L}, so every partial sum is a multiple of the next level's last place, for which the
+// three-operation sum is exact whatever the order of magnitudes
 template <bool SIX>
 __device__ __forceinline__ pdf drained(const uint32_t (&v)[4][16], int j, const float *top) {
     float2 x[4];
 #pragma unroll
     for (int i = 0; i < 4; i++) x[i] = p2(__uint_as_float(v[i][2 * j]), __uint_as_float(v[i][2 * j + 1]));
-    const pdf s = pdf_two_sum(x[0], x[1]), t = pdf_two_sum(s.h, x[2]);
+    const pdf s = pdf_fast_two_sum(x[0], x[1]), t = pdf_fast_two_sum(s.h, x[2]);
     if (SIX) {
-        const pdf u = pdf_two_sum(t.h, x[3]);
+        const pdf u = pdf_fast_two_sum(t.h, x[3]);
         return pdf_fast_two_sum(u.h, p2_add(p2_add(u.l, p2_add(t.l, s.l)), p2(top[2 * j], top[2 * j + 1])));
     }
     return pdf_fast_two_sum(t.h, p2_add(p2_add(t.l, s.l), x[3]));
@@ -287,26 +293,28 @@ __device__ __forceinline__ pdf combine(pdf own, pdf oth, bool odd) {
     return pdf_add({p2(A.h.x, s * A.h.y), p2(A.l.x, s * A.l.y)}, {p2(-s * B.h.y, B.h.x), p2(-s * B.l.y, B.l.x)});
 }
 
-// The MMAs of N columns of one K = 32 image pair into accumulators NA columns apart (b0: the first column's image row);
-// `started` bit L: accumulator L holds a sum already.  Four channels: slice level i + j in accumulator min(i + j, NACC - 1).
-// Two channels: levels 0 .. 3 in lanes 0 .. 63 of accumulators 0 .. 3, levels 4 and 5 in lanes 64 .. 127 of accumulator 0
-// (the zero rows leave the other lanes as they are)
-template <class T, int N>
-__device__ __forceinline__ void issue_mmas(uint32_t tbase, uint32_t a0, uint32_t b0, int &started) {
-    constexpr uint32_t IDESC = tc::idesc_bf16_f32(ROWS, N);
-#pragma unroll 1
+// The MMAs of N columns of one K = 32 image pair, slice level i + j in accumulator min(i + j, NACC - 1), accumulators NA
+// columns apart (b0: the first column's image row); FRESH: the accumulators start from zero.  Two channels: the
+// upper columns, which are no fewer, go first, to lanes 64 .. 127, and their zero rows clear the other lanes; the lower
+// columns then add to lanes 0 .. 63.
+template <class T, int N, bool FRESH>
+__device__ __forceinline__ void issue_mmas(uint32_t tbase, uint32_t a0, uint32_t b0) {
+    constexpr uint32_t IDESC = tc::idesc_bf16_f32(ROWS, N), IDLO = tc::idesc_bf16_f32(ROWS, T::TWO ? T::LO : N);
+    constexpr int UP = T::TWO ? T::LO * 16 * 2 : 0;
+    // unrolled: one thread issues them all while four warps wait, and the descriptors are a base and constants
+    const uint64_t ad = tc::smem_desc(a0, 128, 256), bd = tc::smem_desc(b0, 128, 256);
+#pragma unroll
     for (int q = 0; q < KSTEPS; q++)
-#pragma unroll 1
+#pragma unroll
         for (int i = 0; i < T::NS; i++)
-#pragma unroll 1
+#pragma unroll
             for (int j = 0; j < T::NS - i; j++) {
-                const bool upper = T::TWO && i + j > 3;
-                const int L = upper ? 0 : min(i + j, T::NACC - 1);
-                const uint32_t aoff = (uint32_t)(((i * KSTEPS + q) * ROWS + (T::TWO && !upper ? BLK : 0)) * 16 * 2);
-                const uint64_t ad = tc::smem_desc(a0 + aoff, 128, 256);
-                const uint64_t bd = tc::smem_desc(b0 + (uint32_t)((j * KSTEPS + q) * T::NP * 16 * 2), 128, 256);
-                tc::mma_bf16(tbase + (uint32_t)(L * T::NA), ad, bd, IDESC, (started >> L) & 1);
-                started |= 1 << L;
+                const int L = i + j < T::NACC - 1 ? i + j : T::NACC - 1;
+                const uint32_t d = tbase + (uint32_t)(L * T::NA);
+                const uint64_t ab = ad + (uint64_t)((i * KSTEPS + q) * ROWS * 16 * 2 / 16),
+                               bb = bd + (uint64_t)((j * KSTEPS + q) * T::NP * 16 * 2 / 16);
+                tc::mma_bf16(d, ab, bb + UP / 16, IDESC, !(FRESH && q == 0 && i == 0 && j <= T::NACC - 1));
+                if (T::TWO) tc::mma_bf16(d, ab + BLK * 16 * 2 / 16, bb, IDLO, 1);
             }
 }
 
@@ -358,12 +366,10 @@ __global__ void __launch_bounds__(TT<DP, MODE>::NT, 1) k_lat_tc(TcKArgs g) {
     __nv_bfloat16 *sA = reinterpret_cast<__nv_bfloat16 *>(sm + T::O_A);
     __nv_bfloat16 *sB = reinterpret_cast<__nv_bfloat16 *>(sm + T::O_B);
     pdf *sS = reinterpret_cast<pdf *>(sm + T::O_S), *sR = reinterpret_cast<pdf *>(sm + T::O_R);
-    float *sTop = reinterpret_cast<float *>(sm + T::O_R);  // two channels only
     pdf *sH = reinterpret_cast<pdf *>(sm + T::O_H);
     float *sCol = reinterpret_cast<float *>(sm + T::O_COL), *rowsc = reinterpret_cast<float *>(sm + T::O_ROW);
     dfl *sE0 = reinterpret_cast<dfl *>(sm + T::O_E0), *sSw = reinterpret_cast<dfl *>(sm + T::O_SW);
     dfl *sEq = reinterpret_cast<dfl *>(sm + T::O_EQ);
-    ushort2 *sPair = reinterpret_cast<ushort2 *>(sm + T::O_PAIR);
     uint64_t *barB = reinterpret_cast<uint64_t *>(sm + T::O_BAR), *barM = barB + 1;
     uint32_t *tslot = reinterpret_cast<uint32_t *>(barB + 2);
     volatile int *err = reinterpret_cast<volatile int *>(tslot + 1);
@@ -383,15 +389,10 @@ __global__ void __launch_bounds__(TT<DP, MODE>::NT, 1) k_lat_tc(TcKArgs g) {
         tc::mbar_init(barM, 1);
         *err = 0;
     }
-    for (int t = tid; t < (TWO ? 1 : 2) * FT * DD; t += NT) sS[t] = Ops::zero();  // the padding stays zero (S, R adjacent)
+    for (int t = tid; t < (TWO ? 1 : 2) * FT * T::TILE; t += NT) sS[t] = Ops::zero();  // S and R are adjacent
     if (TWO)  // the zero rows of the A image stay
         for (int t = tid; t < T::A_EL / 8; t += NT) reinterpret_cast<uint4 *>(sA)[t] = make_uint4(0, 0, 0, 0);
-    for (int t = tid; t < DD; t += NT) sH[t] = Ops::zero();
-    for (int t = tid; t < npair; t += NT) {
-        int x, y;
-        pair_of(t, D, x, y);
-        sPair[t] = make_ushort2((unsigned short)x, (unsigned short)y);
-    }
+    for (int t = tid; t < 3 * DD; t += NT) sH[t] = Ops::zero();
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
@@ -432,10 +433,9 @@ __global__ void __launch_bounds__(TT<DP, MODE>::NT, 1) k_lat_tc(TcKArgs g) {
             if (tid == 0) {
                 tc::fence_after_sync();
                 if (!first || tc::mbar_wait(barB, bphase, WAIT_LIMIT)) {
-                    int started = 0;
-                    if (part == 0) issue_mmas<T, T::NA>(tbase, tc::smem_u32(sA), tc::smem_u32(sB), started);
-                    if constexpr (T::NA < T::NP) {
-                        if (part) issue_mmas<T, T::NP - T::NA>(tbase, tc::smem_u32(sA), tc::smem_u32(sB + T::NA * 16), started);
+                    if (part == 0) issue_mmas<T, T::NA, true>(tbase, tc::smem_u32(sA), tc::smem_u32(sB));
+                    if constexpr (T::PARTS) {
+                        if (part) issue_mmas<T, T::NP - T::NA, true>(tbase, tc::smem_u32(sA), tc::smem_u32(sB + T::NA * 16));
                     }
                     tc::mma_commit(barM);
                 } else {
@@ -450,66 +450,30 @@ __global__ void __launch_bounds__(TT<DP, MODE>::NT, 1) k_lat_tc(TcKArgs g) {
             tc::fence_after_sync();
             return *err == 0;
         };
-        // TMEM -> complex entries in shared memory.  third: the T round of DERIV (rows Re w^3, Im w^3).  Two channels: warps 2
-        // and 3 hand the shared levels' sums to warps 0 and 1, whose lanes have the frequencies
+        // TMEM -> shared memory, the dofs of A or B of this lane's frequency and sum as they are: the inversion warps put the
+        // complex entries together, for these four warps were the longer chain.  third: the T round of DERIV (rows Re w^3,
+        // Im w^3); part: of the columns.  Two channels: warps 0 and 1 have the lower columns, 2 and 3 the upper
         auto drain = [&](bool third, int part) {
-            if (TWO) {
-                if (warp >= 2) {
-                    float *o = sTop + (size_t)((warp - 2) * 32 + lane) * T::LDH;
-                    for (int qg = 0; qg * 16 < D * D; qg++) {
-                        float v[16];
-                        __syncwarp();
-                        tmem_ld16_tied(tbase + ((uint32_t)(warp * 32) << 16) + (uint32_t)(qg * 16), v);
-#pragma unroll
-                        for (int j = 0; j < 16; j++) o[qg * 16 + j] = v[j];
-                    }
-                }
-                bar_sync(BAR_PROD, PT);
-                if (warp >= 2) {
-                    tc::fence_before_sync();
-                    return;
-                }
-            }
-            const int f = TWO ? warp * 16 + (lane >> 1) : warp * 8 + (lane >> 2);
-            const float rs = rowsc[warp * 32 + lane];
-            const float *const stop = sTop + (size_t)(warp * 32 + lane) * T::LDH;
-            const bool odd = lane & 1, second = !TWO && ch >= 2, store = third ? !second : true;
-            const bool transposed = third || (MODE == TC_TRACE && second);
-            pdf *tile = (second ? sR : sS) + (size_t)f * DD;
+            const int f = TWO ? (warp & 1) * 16 + (lane >> 1) : warp * 8 + (lane >> 2);
+            const float rs = rowsc[(TWO ? warp & 1 : warp) * 32 + lane];
+            const bool second = !TWO && ch >= 2;
+            pdf *row = (second ? sR : sS) + (size_t)f * T::TILE + (lane & 1) * T::RS;
             const uint32_t la = tbase + ((uint32_t)(warp * 32) << 16);
+            const int first = TWO ? (warp < 2 ? 0 : T::LO) : part * T::NA;  // columns first .. last - 1
+            const int last = min(D * D, TWO && warp < 2 ? T::LO : first + T::NA);
 #pragma unroll 1
-            for (int qg = part * (T::NA / 16); qg * 16 < min(D * D, (part + 1) * T::NA); qg++) {
+            for (int c0 = first; c0 < last; c0 += 16) {
                 uint32_t v[4][16];
-                float last[16];
-                const float *top = TWO ? stop + qg * 16 : last;
-                const uint32_t at = la + (uint32_t)(qg * 16 - part * T::NA);
+                float top[16];
+                const uint32_t at = la + (uint32_t)(c0 - first);
                 __syncwarp();
-                if (T::NACC == 5) tmem_ld16_tied(at + 4 * T::NA, last);
+                if (T::NACC == 5) tmem_ld16_tied(at + 4 * T::NA, top);
                 tmem_ld16x4(at, (uint32_t)T::NA, v);
 #pragma unroll
                 for (int j = 0; j < 8; j++) {
-                    const int p = qg * 16 + 2 * j;
-                    if (p >= D * D) break;
-                    pdf own = drained<T::NS == 6>(v, j, top);
-                    const float2 sc = p2_mul(*reinterpret_cast<const float2 *>(sCol + p), p2(rs));
-                    own = {p2_mul(own.h, sc), p2_mul(own.l, sc)};
-                    const pdf oth = shfl_xor1(own);
-                    if (p < 2 * npair) {
-                        const ushort2 ac = sPair[p >> 1];
-                        const int r = odd ? ac.y : ac.x, c = odd ? ac.x : ac.y;
-                        pdf x = combine(own, oth, odd);
-                        if (!third && !second) x = Ops::add(x, sH[r * DP + c]);
-                        if (store) tile[transposed ? c * DP + r : r * DP + c] = x;
-                    } else {
-                        // two diagonal entries, (A, B) from the lane pair; the even lane has the first, the odd the second
-                        const int di = p - 2 * npair + (odd ? 1 : 0), e = min(di, D - 1);
-                        const bool live = di < D;
-                        const pdf x0 = odd ? pdf{p2(oth.h.y, own.h.y), p2(oth.l.y, own.l.y)}
-                                           : pdf{p2(own.h.x, oth.h.x), p2(own.l.x, oth.l.x)};
-                        pdf x = x0;
-                        if (!third) x = Ops::add(x, second ? Ops::one() : sH[e * DP + e]);
-                        if (store && live) tile[e * DP + e] = x;
-                    }
+                    const pdf own = drained<T::NS == 6>(v, j, top);
+                    const float2 sc = p2_mul(*reinterpret_cast<const float2 *>(sCol + c0 + 2 * j), p2(rs));
+                    if (c0 + 2 * j < DD && !(third && second)) row[c0 / 2 + j] = {p2_mul(own.h, sc), p2_mul(own.l, sc)};
                 }
             }
             tc::fence_before_sync();
@@ -519,7 +483,7 @@ __global__ void __launch_bounds__(TT<DP, MODE>::NT, 1) k_lat_tc(TcKArgs g) {
         prefetch(kbeg);
         for (int k = kbeg, it = 0; k < kend; k++, it++) {
             const int slot = it % 3;  // inversion warps may still read the slot of k - 1 while k + 1 is staged
-            if (tid < D * D) sH[(tid % D) * DP + tid / D] = Ops::from(hpre);
+            if (tid < D * D) sH[slot * DD + (tid % D) * DP + tid / D] = Ops::from(hpre);
             if (e_thread) sE0[slot * NE0 + tid] = df_make(a.mu - epre);
             else if (q_thread) sEq[tid - NE0] = df_make(a.mu - epre);
             if (k + 1 < kend) prefetch(k + 1);
@@ -561,7 +525,7 @@ __global__ void __launch_bounds__(TT<DP, MODE>::NT, 1) k_lat_tc(TcKArgs g) {
             bool ok = multiply(true, 0);
             if (ok && it > 0) bar_sync(MODE == TC_DERIV ? BAR_DONE : BAR_EMPTY, NT);
             if (ok) drain(false, 0);
-            if (T::NA < T::NP && ok) {
+            if (T::PARTS && ok) {
                 ok = multiply(false, 1);
                 if (ok) drain(false, 1);
             }
@@ -585,7 +549,7 @@ __global__ void __launch_bounds__(TT<DP, MODE>::NT, 1) k_lat_tc(TcKArgs g) {
                     bar_sync(BAR_EMPTY, NT);
                     drain(true, 0);
                 }
-                if (T::NA < T::NP && ok) {
+                if (T::PARTS && ok) {
                     ok = multiply(false, 1);
                     if (ok) drain(true, 1);
                 }
@@ -610,7 +574,22 @@ __global__ void __launch_bounds__(TT<DP, MODE>::NT, 1) k_lat_tc(TcKArgs g) {
         const int fc = min(f, a.nf2 - 1);
         const dfl wr = df_make(wfreq(fc)), w2f = df_mul(wr, wr);
         const pdf *zs = g.zs + (size_t)fc * DD + c;
-        pdf *tS = sS + (size_t)fl * DD, *tR = sR + (size_t)fl * DD;
+        pdf *tS = sS + (size_t)fl * T::TILE, *tR = sR + (size_t)fl * T::TILE;
+        // entry (r, c), or (c, r) with tr, of A + iB from the dofs at t; dg: the diagonal entry of this lane's column.  In the
+        // lanes of the padding (c >= D) it is some finite number: their columns only ever change themselves
+        auto diagonal = [&](const pdf *t) {
+            const int i = npair + (min(c, D - 1) >> 1);
+            const pdf A = t[i], B = t[T::RS + i];
+            return c & 1 ? pdf{p2(A.h.y, B.h.y), p2(A.l.y, B.l.y)} : pdf{p2(A.h.x, B.h.x), p2(A.l.x, B.l.x)};
+        };
+        auto entry = [&](const pdf *t, const pdf &dg, int r, bool tr) {
+            if (r >= D) return Ops::zero();
+            const int i = r < c ? c * (c - 1) / 2 + r : r * (r - 1) / 2 + min(c, r);
+            const pdf A = t[i], B = t[T::RS + i];
+            const float s = (r < c) != tr ? 1.f : -1.f;
+            const pdf x = pdf_add({p2(A.h.x, s * A.h.y), p2(A.l.x, s * A.l.y)}, {p2(-s * B.h.y, B.h.x), p2(-s * B.l.y, B.l.x)});
+            return r == c ? dg : x;
+        };
         const pdf *zs0 = T::G0I ? g.zs0 + (size_t)fc * DD + c : nullptr;
         pdf accG[MODE == TC_BLOCK ? DP : 1], accG0[T::G0I ? DP : 1];
 #pragma unroll
@@ -621,6 +600,7 @@ __global__ void __launch_bounds__(TT<DP, MODE>::NT, 1) k_lat_tc(TcKArgs g) {
         bool sing = false, ok = true;
         for (int k = kbeg, it = 0; k < kend; k++, it++) {
             pdf col[DP], R[MODE == TC_BLOCK ? 1 : DP], col0[T::G0I ? DP : 1];
+            const pdf *hk = sH + (it % 3) * DD + c;
 #pragma unroll
             for (int r = 0; r < DP; r++) col[r] = zs[r * DP];
             bar_sync(BAR_FULL, NT);
@@ -628,17 +608,27 @@ __global__ void __launch_bounds__(TT<DP, MODE>::NT, 1) k_lat_tc(TcKArgs g) {
                 ok = false;
                 break;
             }
-            if (T::G0I) {
+            {
+                const pdf dg = diagonal(tS);
 #pragma unroll
-                for (int r = 0; r < DP; r++) col0[T::G0I ? r : 0] = Ops::sub(zs0[r * DP], tS[r * DP + c]);
+                for (int r = 0; r < DP; r++) {
+                    const pdf x = entry(tS, dg, r, false);
+                    if (T::G0I) col0[T::G0I ? r : 0] = Ops::sub(zs0[r * DP], x);
+                    col[r] = Ops::sub(col[r], x);
+                }
             }
+            if (MODE != TC_BLOCK) {  // I + R, TRACE: transposed
+                const pdf dg = Ops::add(Ops::one(), diagonal(tR));
 #pragma unroll
-            for (int r = 0; r < DP; r++) col[r] = Ops::sub(col[r], tS[r * DP + c]);
-            if (MODE != TC_BLOCK) {
-#pragma unroll
-                for (int r = 0; r < DP; r++) R[MODE == TC_BLOCK ? 0 : r] = tR[r * DP + c];
+                for (int r = 0; r < DP; r++) R[MODE == TC_BLOCK ? 0 : r] = entry(tR, dg, r, MODE == TC_TRACE);
             }
             bar_arrive(BAR_EMPTY, NT);
+#pragma unroll
+            for (int r = 0; r < DP; r++) {  // H_PP, in its own slot: the tiles are free before this
+                const pdf h = hk[r * DP];
+                col[r] = Ops::sub(col[r], h);
+                if (T::G0I) col0[T::G0I ? r : 0] = Ops::sub(col0[T::G0I ? r : 0], h);
+            }
             sing |= group_gj_inverse<Ops, DP>(col, c, base) && fvalid && c < D;
             if (MODE == TC_BLOCK) {
 #pragma unroll
@@ -697,9 +687,10 @@ __global__ void __launch_bounds__(TT<DP, MODE>::NT, 1) k_lat_tc(TcKArgs g) {
                 }
                 d = Ops::zero();
                 if (c < D) {
+                    const pdf dg = diagonal(tS);
 #pragma unroll
                     for (int r = 0; r < DP; r++)
-                        if (r < D) d = re_dot(col[r], tS[r * DP + c], d);  // G(r, c) T(c, r)
+                        if (r < D) d = re_dot(col[r], entry(tS, dg, r, true), d);  // G(r, c) T(c, r)
                 }
                 const dfl gt = re_val(d);
                 t2 = df_sub(t2, df_add(gt, gt));
@@ -760,11 +751,10 @@ constexpr int G0T = 256, G0K = 2;
 template <int DP>
 struct T0 {
     using T = TT<DP, TC_BLOCK>;
-    static constexpr int NG = T::NP / 16, NGH = (NG + 1) / 2;  // column groups, per warp of a TMEM quarter's two
+    static constexpr int NGH = (T::NA / 16 + 1) / 2;           // column groups per warp: two warps share a TMEM quarter
     static constexpr int O_A = 0;
     static constexpr int O_B = O_A + G0K * T::A_EL * 2;
-    static constexpr int O_TOP = O_B + G0K * T::B_EL * 2;      // [BLK][LDH] floats: the shared levels' sums
-    static constexpr int O_E = O_TOP + (BLK * T::LDH * 4 + 15) / 16 * 16;  // [2][G0K][KP] dfl: mu - e0_j
+    static constexpr int O_E = O_B + G0K * T::B_EL * 2;        // [2][G0K][KP] dfl: mu - e0_j
     static constexpr int O_ROW = O_E + 2 * G0K * KP * 8;
     static constexpr int O_BAR = O_ROW + BLK * 4;              // barB[G0K], barM, TMEM slot, error flag
     static constexpr int SMEM = O_BAR + 48;
@@ -786,7 +776,6 @@ __global__ void __launch_bounds__(G0T, 1) k_g0_tc(G0Args g) {
     typedef OpsP Ops;
     extern __shared__ __align__(1024) unsigned char sm[];
     __nv_bfloat16 *sA = reinterpret_cast<__nv_bfloat16 *>(sm + S::O_A), *sB = reinterpret_cast<__nv_bfloat16 *>(sm + S::O_B);
-    float *sTop = reinterpret_cast<float *>(sm + S::O_TOP);
     dfl *sE = reinterpret_cast<dfl *>(sm + S::O_E);
     float *rowsc = reinterpret_cast<float *>(sm + S::O_ROW);
     uint64_t *barB = reinterpret_cast<uint64_t *>(sm + S::O_BAR), *barM = barB + G0K;
@@ -827,7 +816,7 @@ __global__ void __launch_bounds__(G0T, 1) k_g0_tc(G0Args g) {
 #pragma unroll
         for (int j = 0; j < 8; j++) acc[q][j] = Ops::zero();
     const int quarter = warp & 3, half = warp >> 2;
-    const bool low = quarter < 2;  // lanes 0 .. 63: the frequencies; 64 .. 127: the shared levels
+    const int first = quarter < 2 ? 0 : T::LO, last = min(D * D, quarter < 2 ? T::LO : T::NP);  // this quarter's columns
     const uint32_t la = tbase + ((uint32_t)(quarter * 32) << 16);
     const int row = (quarter & 1) * 32 + lane;
     bool ok = true;
@@ -871,13 +860,12 @@ __global__ void __launch_bounds__(G0T, 1) k_g0_tc(G0Args g) {
         __syncthreads();
         if (tid == 0) {
             tc::fence_after_sync();
-            int started = 0;
             bool there = true;
             for (int kk = 0; kk < cnt && there; kk++) {
                 there = tc::mbar_wait(barB + kk, gi, WAIT_LIMIT);
-                if (there)
-                    issue_mmas<T, T::NP>(tbase, tc::smem_u32(sA + (size_t)kk * T::A_EL),
-                                         tc::smem_u32(sB + (size_t)kk * T::B_EL), started);
+                const uint32_t a0 = tc::smem_u32(sA + (size_t)kk * T::A_EL), b0 = tc::smem_u32(sB + (size_t)kk * T::B_EL);
+                if (there && kk == 0) issue_mmas<T, T::NA, true>(tbase, a0, b0);
+                else if (there) issue_mmas<T, T::NA, false>(tbase, a0, b0);
             }
             tc::mma_commit(barM);
             if (!there) *err = 1;
@@ -889,52 +877,43 @@ __global__ void __launch_bounds__(G0T, 1) k_g0_tc(G0Args g) {
         if (!ok) break;
         tc::fence_after_sync();
         if (i0 + G0K < nk) copy_b(i0 + G0K);  // the MMAs are done with B
-        if (!low)
-            for (int qg = half; qg * 16 < D * D; qg += 2) {
-                float v[16];
-                __syncwarp();
-                tmem_ld16_tied(la + (uint32_t)(qg * 16), v);
+        const float rs = rowsc[row];
 #pragma unroll
-                for (int j = 0; j < 16; j++) sTop[(size_t)row * T::LDH + qg * 16 + j] = v[j];
-            }
-        __syncthreads();
-        if (low) {
-            const float rs = rowsc[row];
+        for (int q = 0; q < S::NGH; q++) {
+            const int c0 = first + (2 * q + half) * 16;
+            if (c0 >= last) break;
+            uint32_t v[4][16];
+            float top[16];
+            __syncwarp();
+            tmem_ld16_tied(la + (uint32_t)(c0 - first + 4 * T::NA), top);
+            tmem_ld16x4(la + (uint32_t)(c0 - first), (uint32_t)T::NA, v);
 #pragma unroll
-            for (int q = 0; q < S::NGH; q++) {
-                const int qg = 2 * q + half;
-                if (qg * 16 >= D * D) break;
-                uint32_t v[4][16];
-                __syncwarp();
-                tmem_ld16x4(la + (uint32_t)(qg * 16), (uint32_t)T::NP, v);
-#pragma unroll
-                for (int j = 0; j < 8; j++) {
-                    const pdf x = drained<true>(v, j, sTop + (size_t)row * T::LDH + qg * 16);
-                    acc[q][j] = Ops::add(acc[q][j], {p2_mul(x.h, p2(rs)), p2_mul(x.l, p2(rs))});
-                }
+            for (int j = 0; j < 8; j++) {
+                const pdf x = drained<true>(v, j, top);
+                acc[q][j] = Ops::add(acc[q][j], {p2_mul(x.h, p2(rs)), p2_mul(x.l, p2(rs))});
             }
         }
         tc::fence_before_sync();
         __syncthreads();  // the next group's MMAs overwrite the accumulators, its builds the images and scales
         tc::fence_after_sync();
     }
-    if (low) {
+    {
         // A and B of this lane pair's frequency -> the complex entries
         const int npair = D * (D - 1) / 2, f = f0 + (row >> 1);
         const bool odd = lane & 1, put = ok && f < g.nf2;
         double2 *o = g.pblk0 + ((size_t)chunk * g.nf2 + min(f, g.nf2 - 1)) * D * D;
 #pragma unroll
         for (int q = 0; q < S::NGH; q++) {
-            const int qg = 2 * q + half;
-            if (qg * 16 >= D * D) break;
+            const int c0 = first + (2 * q + half) * 16;
+            if (c0 >= last) break;
 #pragma unroll
             for (int j = 0; j < 8; j++) {
-                const int p = qg * 16 + 2 * j;
-                if (p >= D * D) break;
+                const int p = c0 + 2 * j;
+                if (p >= last) break;
                 const pdf own = acc[q][j], oth = shfl_xor1(own);
                 if (p < 2 * npair) {
                     int a, c;
-                    pair_of(p >> 1, D, a, c);
+                    pair_of(p >> 1, a, c);
                     const pdf x = combine(own, oth, odd);
                     if (put) o[odd ? c + a * D : a + c * D] = Ops::to(x);
                 } else {
@@ -945,7 +924,8 @@ __global__ void __launch_bounds__(G0T, 1) k_g0_tc(G0Args g) {
                 }
             }
         }
-    } else if (!ok && tid == 64) {
+    }
+    if (!ok && tid == 64) {
         // copies still in flight land before the CTA's shared memory goes away
         for (int kk = 0; kk < G0K; kk++)
             for (int ph = 0; ph < 2; ph++) tc::mbar_wait(barB + kk, ph, WAIT_LIMIT);
