@@ -23,7 +23,7 @@
 #include "gloc.cuh"
 #include "schur.cuh"
 #include "smallmat.cuh"
-#include "smallmat_df.cuh"
+#include "eig.cuh"
 #include "adjoint.cuh"
 #include "density.cuh"
 #include "lat_tc.h"
@@ -120,195 +120,119 @@ __global__ void k_sigall(int Nf, int D, int nh, int mask, double beta, const dou
     sig[t] = v;
 }
 
-// static eigen-decomposition of H(k) + S_inf on the correlated block (src/GreenFtn.cpp:197-215): outputs
-// eps[k][n], UP[k][l][a] = U(a,l) for a < D (correlated rows of the eigenvectors); and the per-k data of the
-// Schur form: H_QQ = V diag(e) V^H, b_l = H_PQ V(:,l) (Q = orbitals D..n-1).
-// One block per k, in shared memory (smallmat.cuh's block_heig): the static eigen-decomposition of H(k) + m0
-// (same output as k_static_eig) and the Schur data (same output as k_schur_prep).  Shared-memory layout:
-// three n x n complex matrices, then eigenvalues [64], order [64], rotations [33], reduction scratch [128].
-constexpr int EIG_THREADS = 128, EIG_NMAX = 64;
-inline size_t eig_blk_smem(int n) {
-    return (size_t)3 * n * n * sizeof(double2) + EIG_NMAX * sizeof(double) + EIG_NMAX * sizeof(int) +
-           (EIG_NMAX / 2 + 1) * sizeof(DgRot) + EIG_THREADS * sizeof(double);
-}
-struct EigSmem {
-    double2 *A0, *A, *U;
-    double *w;
-    int *ord;
-    DgRot *rot;
-    double *red;
-};
-__device__ inline EigSmem eig_smem(double2 *sm, int n) {
-    EigSmem e;
-    const size_t nn = (size_t)n * n;
-    e.A0 = sm;
-    e.A = sm + nn;
-    e.U = sm + 2 * nn;
-    e.w = (double *)(sm + 3 * nn);
-    e.ord = (int *)(e.w + EIG_NMAX);
-    e.rot = (DgRot *)(e.ord + EIG_NMAX);
-    e.red = (double *)(e.rot + EIG_NMAX / 2 + 1);
-    return e;
-}
+// Static eigen-decomposition of H(k) + S_inf on the correlated block (src/GreenFtn.cpp:197-215): eps[k][n], UP[k][l][a] =
+// U(a, l) for a < D (correlated rows of the eigenvectors), and all of U with Uf; and the per-k data of the Schur form:
+// H_QQ = V diag(e) V^H, b_l = H_PQ V(:,l) (Q = orbitals D..n-1).  T threads per k point (group_heig, eig.cuh), four k points
+// per CTA when that is a warp.
+template <int T>
+constexpr int EIG_PER_CTA = T == 32 ? 4 : 1;
 
-__global__ void __launch_bounds__(EIG_THREADS) k_static_eig_blk(int n, int D, int nh, int mask,
-                                                                const double2 *__restrict__ H,
-                                                                const double2 *__restrict__ m0, double *eps,
-                                                                double2 *UP, double2 *Uf, int *status) {
+template <class Ops, int T>
+__global__ void __launch_bounds__(T * EIG_PER_CTA<T>) k_static_eig(int nk, int n, int D, int nh, int mask,
+                                                                   const double2 *__restrict__ H,
+                                                                   const double2 *__restrict__ m0, double *eps, double2 *UP,
+                                                                   double2 *Uf, int *status) {
     extern __shared__ double2 esm[];
-    const int k = blockIdx.x;
+    const int tid = threadIdx.x % T, grp = threadIdx.x / T, k = blockIdx.x * EIG_PER_CTA<T> + grp;
+    if (k >= nk) return;  // whole groups only
     const size_t nn = (size_t)n * n;
-    EigSmem e = eig_smem(esm, n);
+    const EigMem<Ops> e(reinterpret_cast<unsigned char *>(esm) + grp * eig_bytes<Ops>(n), n);
     const double2 *Hk = H + (size_t)k * nn;
-    for (int q = threadIdx.x; q < (int)nn; q += blockDim.x) {
+    for (int q = tid; q < (int)nn; q += T) {
         const int a = q % n, b = q / n;
         double2 v = Hk[q];
         if (a < D && b < D && (!mask || a / nh == b / nh)) v = cadd(v, m0[a + b * D]);
-        e.A0[q] = v;
+        if (a == b) v.y = 0.0;
+        e.a[q] = Ops::from(v);
     }
-    __syncthreads();
-    const int st = block_heig(n, e.A0, e.A, e.U, e.w, e.ord, e.rot, e.red);
-    for (int l = threadIdx.x; l < n; l += blockDim.x) eps[(size_t)k * n + l] = e.w[l];
-    for (int q = threadIdx.x; q < n * D; q += blockDim.x) {
+    const int st = group_heig<Ops, T>(n, e, std::is_same<Ops, OpsD>::value ? 1e-28 : 1e-24, tid);
+    for (int l = tid; l < n; l += T) eps[(size_t)k * n + l] = e.w[e.order[l]];
+    for (int q = tid; q < n * D; q += T) {
         const int l = q / D, a = q % D;
-        UP[((size_t)k * n + l) * D + a] = DG_AT(e.U, n, a, l);
+        UP[((size_t)k * n + l) * D + a] = Ops::to(e.u[a + e.order[l] * n]);
     }
     if (Uf)
-        for (int q = threadIdx.x; q < (int)nn; q += blockDim.x) Uf[(size_t)k * nn + q] = e.U[q];
-    if (st && threadIdx.x == 0) dg_flag(status, DG_NONCONV);
+        for (int q = tid; q < (int)nn; q += T) Uf[(size_t)k * nn + q] = Ops::to(e.u[q % n + e.order[q / n] * n]);
+    if (st && tid == 0) dg_flag(status, DG_NONCONV);
 }
 
-__global__ void __launch_bounds__(EIG_THREADS) k_schur_prep_blk(int n, int D, const double2 *__restrict__ H,
-                                                                double *epsQ, double2 *B, double2 *Vq, int *status) {
+template <class Ops, int T>
+__global__ void __launch_bounds__(T * EIG_PER_CTA<T>) k_schur_prep(int nk, int n, int D, const double2 *__restrict__ H,
+                                                                   double *epsQ, double2 *B, double2 *Vq, int *status) {
     extern __shared__ double2 esm[];
-    const int k = blockIdx.x, m = n - D;
-    EigSmem e = eig_smem(esm, m);
-    const double2 *Hk = H + (size_t)k * n * n;
-    for (int q = threadIdx.x; q < m * m; q += blockDim.x) {
-        const int i = q % m, j = q / m;
-        e.A0[q] = Hk[(D + i) + (size_t)(D + j) * n];
-    }
-    __syncthreads();
-    const int st = block_heig(m, e.A0, e.A, e.U, e.w, e.ord, e.rot, e.red);
-    for (int l = threadIdx.x; l < m; l += blockDim.x) epsQ[(size_t)k * m + l] = e.w[l];
-    for (int q = threadIdx.x; q < m * D; q += blockDim.x) {
-        const int l = q / D, a = q % D;
-        double2 s = cmk(0, 0);
-        for (int j = 0; j < m; j++) s = cfma(Hk[a + (size_t)(D + j) * n], DG_AT(e.U, m, j, l), s);
-        B[((size_t)k * m + l) * D + a] = s;
-    }
-    if (Vq)
-        for (int q = threadIdx.x; q < m * m; q += blockDim.x) Vq[(size_t)k * m * m + q] = e.U[q];
-    if (st && threadIdx.x == 0) dg_flag(status, DG_NONCONV);
-}
-
-// The same two decompositions with one warp per k point, four k points per CTA: for the matrix sizes up to 32 a
-// block-wide Jacobi spends most of its time in block barriers with idle threads.  Ops = OpsD: warp_heig in FP64;
-// OpsF (the DMFTGPU_MIXED passes): warp_heig_df, every step in double-float on the FP32 pipe.  Per-warp shared
-// region: three n x n complex matrices (16-byte elements either way), eigenvalues [64], order [64], rotations [33].
-constexpr int EIG_WPB = 4;
-template <class Ops>
-__device__ __forceinline__ int warp_heig_ops(int n, const typename Ops::C *A0, typename Ops::C *a,
-                                             typename Ops::C *u, double *w, int *order, DgRot *rot) {
-    if constexpr (std::is_same<Ops, OpsF>::value) return warp_heig_df(n, A0, a, u, w, order, rot, 1e-24f);
-    else return warp_heig(n, A0, a, u, w, order, rot);
-}
-__host__ __device__ inline size_t warp_eig_bytes(int n) {
-    const size_t b = (size_t)3 * n * n * sizeof(double2) + EIG_NMAX * sizeof(double) + EIG_NMAX * sizeof(int) + 16 +
-                     (EIG_NMAX / 2 + 1) * sizeof(DgRot);
-    return (b + 15) & ~(size_t)15;
-}
-__device__ inline EigSmem warp_eig_smem(double2 *sm, int n) {
-    char *base = reinterpret_cast<char *>(sm) + (threadIdx.x >> 5) * warp_eig_bytes(n);
-    EigSmem e;
-    const size_t nn = (size_t)n * n;
-    e.A0 = reinterpret_cast<double2 *>(base);
-    e.A = e.A0 + nn;
-    e.U = e.A + nn;
-    e.w = (double *)(e.U + nn);
-    e.ord = (int *)(e.w + EIG_NMAX);
-    e.rot = (DgRot *)(((size_t)(e.ord + EIG_NMAX) + 15) & ~(size_t)15);
-    e.red = nullptr;
-    return e;
-}
-
-template <class Ops>
-__global__ void __launch_bounds__(32 * EIG_WPB) k_static_eig_warp(int nk, int n, int D, int nh, int mask,
-                                                                  const double2 *__restrict__ H,
-                                                                  const double2 *__restrict__ m0, double *eps,
-                                                                  double2 *UP, double2 *Uf, int *status) {
-    extern __shared__ double2 esm[];
-    const int lane = threadIdx.x & 31, k = blockIdx.x * EIG_WPB + (threadIdx.x >> 5);
-    if (k >= nk) return;  // whole warps only
-    const size_t nn = (size_t)n * n;
-    EigSmem e = warp_eig_smem(esm, n);
+    const int tid = threadIdx.x % T, grp = threadIdx.x / T, k = blockIdx.x * EIG_PER_CTA<T> + grp, m = n - D;
+    if (k >= nk) return;  // whole groups only
     typedef typename Ops::C C;
-    C *A0 = reinterpret_cast<C *>(e.A0), *A = reinterpret_cast<C *>(e.A), *U = reinterpret_cast<C *>(e.U);
-    const double2 *Hk = H + (size_t)k * nn;
-    for (int q = lane; q < (int)nn; q += 32) {
-        const int a = q % n, b = q / n;
-        double2 v = Hk[q];
-        if (a < D && b < D && (!mask || a / nh == b / nh)) v = cadd(v, m0[a + b * D]);
-        A0[q] = Ops::from(v);
-    }
-    __syncwarp();
-    const int st = warp_heig_ops<Ops>(n, A0, A, U, e.w, e.ord, e.rot);
-    for (int l = lane; l < n; l += 32) eps[(size_t)k * n + l] = e.w[l];
-    for (int q = lane; q < n * D; q += 32) {
-        const int l = q / D, a = q % D;
-        UP[((size_t)k * n + l) * D + a] = Ops::to(DG_AT(U, n, a, l));
-    }
-    if (Uf)
-        for (int q = lane; q < (int)nn; q += 32) Uf[(size_t)k * nn + q] = Ops::to(U[q]);
-    if (st && lane == 0) dg_flag(status, DG_NONCONV);
-}
-
-template <class Ops>
-__global__ void __launch_bounds__(32 * EIG_WPB) k_schur_prep_warp(int nk, int n, int D, const double2 *__restrict__ H,
-                                                                  double *epsQ, double2 *B, double2 *Vq, int *status) {
-    extern __shared__ double2 esm[];
-    const int lane = threadIdx.x & 31, k = blockIdx.x * EIG_WPB + (threadIdx.x >> 5), m = n - D;
-    if (k >= nk) return;  // whole warps only
-    EigSmem e = warp_eig_smem(esm, m);
-    typedef typename Ops::C C;
-    C *A0 = reinterpret_cast<C *>(e.A0), *A = reinterpret_cast<C *>(e.A), *U = reinterpret_cast<C *>(e.U);
+    const EigMem<Ops> e(reinterpret_cast<unsigned char *>(esm) + grp * eig_bytes<Ops>(m), m);
     const double2 *Hk = H + (size_t)k * n * n;
-    for (int q = lane; q < m * m; q += 32) {
+    for (int q = tid; q < m * m; q += T) {
         const int i = q % m, j = q / m;
-        A0[q] = Ops::from(Hk[(D + i) + (size_t)(D + j) * n]);
+        double2 v = Hk[(D + i) + (size_t)(D + j) * n];
+        if (i == j) v.y = 0.0;
+        e.a[q] = Ops::from(v);
     }
-    __syncwarp();
-    const int st = warp_heig_ops<Ops>(m, A0, A, U, e.w, e.ord, e.rot);
-    for (int l = lane; l < m; l += 32) epsQ[(size_t)k * m + l] = e.w[l];
+    const int st = group_heig<Ops, T>(m, e, std::is_same<Ops, OpsD>::value ? 1e-28 : 1e-24, tid);
+    for (int l = tid; l < m; l += T) epsQ[(size_t)k * m + l] = e.w[e.order[l]];
     // b_l = H_PQ V(:, l): in the arithmetic of the decomposition, stored in FP64
-    for (int q = lane; q < m * D; q += 32) {
+    for (int q = tid; q < m * D; q += T) {
         const int l = q / D, a = q % D;
+        const C *v = e.u + e.order[l] * m;
         C s = Ops::zero();
-        for (int j = 0; j < m; j++) s = Ops::fma(Ops::from(Hk[a + (size_t)(D + j) * n]), DG_AT(U, m, j, l), s);
+        for (int j = 0; j < m; j++) s = Ops::fma(Ops::from(Hk[a + (size_t)(D + j) * n]), v[j], s);
         B[((size_t)k * m + l) * D + a] = Ops::to(s);
     }
     if (Vq)
-        for (int q = lane; q < m * m; q += 32) Vq[(size_t)k * m * m + q] = Ops::to(U[q]);
-    if (st && lane == 0) dg_flag(status, DG_NONCONV);
+        for (int q = tid; q < m * m; q += T) Vq[(size_t)k * m * m + q] = Ops::to(e.u[q % m + e.order[q / m] * m]);
+    if (st && tid == 0) dg_flag(status, DG_NONCONV);
 }
 
-// the Schur data of every k point (H_QQ = V diag(e) V^H, b_l = H_PQ V(:, l)), by warps for m <= 32
+// Threads per matrix: four warps shorten the chain of rounds, one has no block barriers and no idle lanes in small matrices.
+// Time of a G_loc pass over 32 frequencies, us, double-float, 32 / 128 threads at 2, 150, 1,000, 4,000 k points:
+//   n = 8:  256 / 262, 296 / 350, 374 / 418, 733 / 906        n = 16: 426 / 341, 427 / 417, 676 / 717, 1,699 / 1,952
+//   n = 20: 603 / 408, 635 / 517, 1,228 / 1,019, 2,826 / 2,913   n = 28: 1,303 / 656, 1,366 / 1,213, 2,467 / 2,157, 7,883 / 6,950
+// FP64 has its crossing in the same places, within 5 % of each other on both sides of it.
+bool eig_one_warp(dmftgpu_ctx *ctx, int nk, int n) {
+    int nsm = 152;
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, ctx->device);
+    return n <= 8 || (n <= 16 && nk > 2 * nsm);
+}
+
+template <class Ops, int T>
+int launch_static_eig_t(dmftgpu_ctx *ctx, cudaStream_t s, int nk, int n, int D, int nh, int mask, const double2 *H,
+                        const double2 *m0, double *eps, double2 *UP, double2 *Uf) {
+    const size_t sm = EIG_PER_CTA<T> * eig_bytes<Ops>(n);
+    DG_CUDA(cudaFuncSetAttribute(k_static_eig<Ops, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    k_static_eig<Ops, T><<<dg_ceil_div(nk, EIG_PER_CTA<T>), T * EIG_PER_CTA<T>, sm, s>>>(nk, n, D, nh, mask, H, m0, eps, UP, Uf,
+                                                                                         ctx->d_status);
+    DG_LAUNCH(ctx, "k_static_eig");
+    return DMFTGPU_OK;
+}
+template <class Ops>
+int launch_static_eig(dmftgpu_ctx *ctx, cudaStream_t s, int nk, int n, int D, int nh, int mask, const double2 *H,
+                      const double2 *m0, double *eps, double2 *UP, double2 *Uf) {
+    if (eig_one_warp(ctx, nk, n)) return launch_static_eig_t<Ops, 32>(ctx, s, nk, n, D, nh, mask, H, m0, eps, UP, Uf);
+    return launch_static_eig_t<Ops, 128>(ctx, s, nk, n, D, nh, mask, H, m0, eps, UP, Uf);
+}
+template <class Ops, int T>
+int launch_schur_prep_t(dmftgpu_ctx *ctx, cudaStream_t s, int nk, int n, int D, const double2 *H, double *epsQ, double2 *B,
+                        double2 *Vq) {
+    const size_t sm = EIG_PER_CTA<T> * eig_bytes<Ops>(n - D);
+    DG_CUDA(cudaFuncSetAttribute(k_schur_prep<Ops, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    k_schur_prep<Ops, T><<<dg_ceil_div(nk, EIG_PER_CTA<T>), T * EIG_PER_CTA<T>, sm, s>>>(nk, n, D, H, epsQ, B, Vq, ctx->d_status);
+    DG_LAUNCH(ctx, "k_schur_prep");
+    return DMFTGPU_OK;
+}
+template <class Ops>
+int launch_schur_prep_ops(dmftgpu_ctx *ctx, cudaStream_t s, int nk, int n, int D, const double2 *H, double *epsQ, double2 *B,
+                          double2 *Vq) {
+    if (eig_one_warp(ctx, nk, n - D)) return launch_schur_prep_t<Ops, 32>(ctx, s, nk, n, D, H, epsQ, B, Vq);
+    return launch_schur_prep_t<Ops, 128>(ctx, s, nk, n, D, H, epsQ, B, Vq);
+}
+// the Schur data of every k point; df: in double-float (up to 32 ligands, FP64 beyond)
 int launch_schur_prep(dmftgpu_ctx *ctx, cudaStream_t s, int nk, int n, int D, const double2 *H, double *epsQ,
                       double2 *B, double2 *Vq, bool df = false) {
-    const int m = n - D;
-    if (m <= 32) {
-        const size_t sm = EIG_WPB * warp_eig_bytes(m);
-        auto kern = df ? k_schur_prep_warp<OpsF> : k_schur_prep_warp<OpsD>;
-        DG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-        kern<<<dg_ceil_div(nk, EIG_WPB), 32 * EIG_WPB, sm, s>>>(nk, n, D, H, epsQ, B, Vq, ctx->d_status);
-        DG_LAUNCH(ctx, "k_schur_prep_warp");
-    } else {
-        const size_t sm = eig_blk_smem(m);
-        DG_CUDA(cudaFuncSetAttribute(k_schur_prep_blk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-        k_schur_prep_blk<<<nk, EIG_THREADS, sm, s>>>(n, D, H, epsQ, B, Vq, ctx->d_status);
-        DG_LAUNCH(ctx, "k_schur_prep_blk");
-    }
-    return DMFTGPU_OK;
+    if (df && n - D <= 32) return launch_schur_prep_ops<OpsP>(ctx, s, nk, n, D, H, epsQ, B, Vq);
+    return launch_schur_prep_ops<OpsD>(ctx, s, nk, n, D, H, epsQ, B, Vq);
 }
 
 // Fermi parts: occ_k = P U f U^H P (with the +-100 cut-offs of src/GreenFtn.cpp:314-316) for NumMatrix,
@@ -608,26 +532,13 @@ int prepare(dmftgpu_ctx *ctx, const dmftgpu_lattice *L, const double2 *dH, const
     long long tot = 2LL * Nf * D * D;
     k_sigall<<<dg_ceil_div(tot, 256), 256, 0, s>>>(Nf, D, P.nh, mask, P.beta, dS, P.mom, P.sig, P.m0);
     DG_LAUNCH(ctx, "k_sigall");
-    // the Schur data (eigen-decomposition of H_QQ) is needed first, by k_schur, on the main stream; the
-    // static eigen-decomposition of H + m0 feeds only the Fermi terms, so it runs on the side stream
-    // (FP64-pipe work) while the lattice kernel (FP32 pipe in the mixed form) proceeds
-    if (m > 0) DG_TRY(launch_schur_prep(ctx, s, nk, n, D, P.H, P.epsQ, P.B, P.Vq, df));
+    // the Schur data (eigen-decomposition of H_QQ) is needed first, on the main stream; the static eigen-decomposition of
+    // H + m0 feeds the Fermi terms, Tr G0 and GwHF: it runs beside it, and beside the lattice kernel, on the side stream
     DG_CUDA(cudaEventRecord(ctx->ev_fork, s));
     DG_CUDA(cudaStreamWaitEvent(ctx->side, ctx->ev_fork, 0));
-    cudaStream_t es = df ? s : ctx->side;
-    if (n <= 32) {
-        const size_t sm = EIG_WPB * warp_eig_bytes(n);
-        auto kern = df ? k_static_eig_warp<OpsF> : k_static_eig_warp<OpsD>;
-        DG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-        kern<<<dg_ceil_div(nk, EIG_WPB), 32 * EIG_WPB, sm, es>>>(nk, n, D, P.nh, mask, P.H, P.m0, P.eps, P.UP, P.Uf,
-                                                                 ctx->d_status);
-        DG_LAUNCH(ctx, "k_static_eig_warp");
-    } else {
-        const size_t sm = eig_blk_smem(n);
-        DG_CUDA(cudaFuncSetAttribute(k_static_eig_blk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-        k_static_eig_blk<<<nk, EIG_THREADS, sm, es>>>(n, D, P.nh, mask, P.H, P.m0, P.eps, P.UP, P.Uf, ctx->d_status);
-        DG_LAUNCH(ctx, "k_static_eig_blk");
-    }
+    if (m > 0) DG_TRY(launch_schur_prep(ctx, s, nk, n, D, P.H, P.epsQ, P.B, P.Vq, df));
+    if (df && n <= 32) DG_TRY(launch_static_eig<OpsP>(ctx, ctx->side, nk, n, D, P.nh, mask, P.H, P.m0, P.eps, P.UP, P.Uf));
+    else DG_TRY(launch_static_eig<OpsD>(ctx, ctx->side, nk, n, D, P.nh, mask, P.H, P.m0, P.eps, P.UP, P.Uf));
     DG_CUDA(cudaEventRecord(ctx->ev_join, ctx->side));
     P.static_ready = ctx->ev_join;
     return DMFTGPU_OK;

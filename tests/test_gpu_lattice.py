@@ -390,3 +390,19 @@ def test_retarded_gloc_real_axis(ctx, orc, case, mixed):
     tol = 1e-9 if mixed else 1e-10
     assert rel_err(g, g_o) < tol
     assert rel_err(tr, tr_o) < tol
+
+
+@pytest.mark.parametrize("n,D,nk", [(2, 1, 3), (3, 1, 2), (8, 2, 3), (9, 1, 2), (9, 1, 306), (16, 3, 306), (17, 1, 2), (18, 2, 306),
+                                    (19, 2, 5), (31, 8, 2), (32, 10, 3), (33, 1, 2), (63, 2, 1), (64, 3, 2)])
+def test_eigensolver_sizes(ctx, orc, n, D, nk):
+    """Both decompositions (H + m0: n, H_QQ: n - D) at the edges of their thread groups: odd and even sizes around 8, 16, 32
+    and 64, few k points and more than two per SM; with two equal ligand levels and one that nothing couples to.  FP64
+    to 1e-11 and the mixed form to the mixed tolerance, as the other passes are held."""
+    H, S, lat = _random_lattice(n, D, (nk, 1, 1), 24, [n, D, nk])
+    if n - D >= 3:
+        H[:, n - 1, :] = H[:, :, n - 1] = 0
+        H[:, n - 1, n - 1] = H[:, n - 2, n - 2]
+    want = orc.greenftn_w(H, S, 0.2, 15.0, 1, D)
+    for mixed, tol in ((False, 1e-11), (True, TOL_MIXED)):
+        for g, w in zip(ctx.GreenFtn_w(lat, H, S, 0.2, mixed=mixed), want):
+            assert rel_err(g, w) < tol
