@@ -1077,20 +1077,23 @@ int launch_trace(dmftgpu_ctx *ctx, const LatTcArgs &a, bool *ready, double *tr, 
 }  // namespace
 
 // Which pass comes here rather than to the lane groups of k_schur: k_schur's time grows with the poles (S, R and T are m
-// rank-one updates each), this one's hardly does.  512 k points x 1,024 frequencies, eigensolver included, ms k_schur / here:
-//              m = 0         m = 3         m = 5 .. 6    m = 20
-//   N(mu)      D = 4  0.45 / 1.77   0.87 / 1.92   1.28 / 2.05   (m = 10: 1.96 / 2.33)
-//              D = 6  1.14 / 2.40   2.02 / 2.61
-//              D = 8  1.79 / 3.38   2.98 / 3.62
-//   dN/dmu     D = 6  2.53 / 4.40                 5.94 / 4.73   15.5 / 6.89
-//              D = 7  4.20 / 5.49                 7.65 / 5.76
-//   G_loc      D = 6  2.08 / 2.81                 3.04 / 3.12    6.87 / 5.27
-//              D = 7  2.73 / 4.31                 4.22 / 4.65
-// The lines below are where these cross; at D = 4 they do only past 16 poles.
+// rank-one updates each), this one's hardly does.  512 k points x 768 frequencies, eigensolver included, ms k_schur / here:
+//              m = 0        m = 2        m = 4        m = 6
+//   G_loc   D = 6   1.63 / 1.93  1.84 / 1.97  2.05 / 1.99  2.25 / 2.03
+//           D = 8   2.38 / 2.66  2.88 / 2.70  3.33 / 2.75  3.81 / 2.81
+//           D = 10  4.75 / 4.36  5.71 / 4.47  6.64 / 4.60  7.62 / 4.66
+//   N(mu)   D = 6   0.92 / 1.53  1.33 / 1.62  1.74 / 1.68
+//           D = 10  2.61 / 3.99  3.48 / 4.07  4.28 / 4.13
+//   dN/dmu  D = 6   1.98 / 2.46  2.82 / 2.54
+//           D = 10  6.46 / 7.24  10.1 / 7.30
+// The lines below are where these cross.  At D = 4 N(mu) takes k_schur 0.45 (m = 0) and 1.96 (m = 10) and 1.77 and 2.33
+// here at 1,024 frequencies: they cross only past 16 poles.
 static bool covered(int n, int D, int least) { return D >= 5 && D <= 10 && n - D >= least && n - D <= KP && n <= NE0; }
-bool dg_lat_tc_supported(int n, int D) { return covered(n, D, 6); }
-bool dg_lat_tc_deriv_supported(int n, int D) { return covered(n, D, 4); }
-bool dg_lat_tc_block_supported(int n, int D) { return covered(n, D, 8) && (D <= 6 || n <= KP); }
+bool dg_lat_tc_supported(int n, int D) { return covered(n, D, 4); }
+bool dg_lat_tc_deriv_supported(int n, int D) { return covered(n, D, 2); }
+bool dg_lat_tc_block_supported(int n, int D) {
+    return covered(n, D, D <= 6 ? 4 : (D <= 8 ? 2 : 0)) && (D <= 6 || n <= KP);
+}
 
 int dg_lat_tc_trace(dmftgpu_ctx *ctx, const LatTcArgs &a, bool *ready, double *tr, double *dtr) {
     if (!(dtr ? dg_lat_tc_deriv_supported(a.n, a.D) : dg_lat_tc_supported(a.n, a.D))) return dg_fail(ctx, DMFTGPU_BADARG, "lat_tc: unsupported sizes");

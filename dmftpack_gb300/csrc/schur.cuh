@@ -569,12 +569,15 @@ __global__ void __launch_bounds__(128, tpi_shared<Ops, D> ? 3 : 1) k_schur_tpi(S
 // and only real parts are summed.  2 x 2 blocks take the closed form Tr[adj(M) (I + R)] / det M, so the whole point of
 // a ligand-free two-orbital model is one complex determinant.  In FP64 the kernel is bound by the FP64 pipe (0.63e12
 // FMA/s), where a division costs as much as ten products: the real fractions of a point (the block's trace and the
-// x_j / (x_j^2 + w^2) of Tr G0) are therefore added over a common denominator, four at a time.  A pass over 64 x 64 k
-// and 4096 points of the two-orbital model takes 1.3 ms (lane groups: 4.1 ms), in double-float 0.37 ms (0.89 ms).
+// x_j / (x_j^2 + w^2) of Tr G0) are therefore added over a common denominator, eight at a time and across k points.  Where
+// no frequency of the CTA has an off-diagonal Sigma, the 2 x 2 block without ligands takes H_01 H_10 from the staged data.
+// A pass over 64 x 64 k and 4096 points of the two-orbital model takes 1.04 ms (1.27 with a division per point and the
+// general determinant, 42 FP64 instructions; lane groups: 4.1), in double-float 0.37 ms (0.89).
 __host__ __device__ inline size_t trace_tpi_stage(int kc, int D, int m, int n) {
     return schur_tpi_stage(kc, D, m) + ((size_t)kc * n * 8 + 15) / 16 * 16;
 }
-// running sum of real fractions: FP64 keeps one numerator and denominator for four terms, double-float (whose
+// running sum of real fractions: FP64 keeps one numerator and denominator for eight terms (products of eight |det|^2 or
+// x^2 + w^2 stay far inside the range: flushed before that where they would not), double-float (whose
 // reciprocal costs less than the products) divides each
 template <class Ops>
 struct FracSum;
@@ -590,12 +593,14 @@ struct FracSum<OpsD> {
             num = ::fma(num, d, n * den);
             den *= d;
         }
-        if (++cnt == 4) flush();
+        // 2^-498 < den < 2^498, by its exponent: a comparison would be another FP64 instruction
+        if (++cnt == 8 || (((unsigned)__double2hiint(den) >> 20) & 0x7ff) - 525u > 996u) flush();
     }
     __device__ __forceinline__ void flush() {
         if (cnt) sum += num / den;
         cnt = 0;
     }
+    __device__ __forceinline__ void end_point(double &) {}
     __device__ __forceinline__ double value() {
         flush();
         return sum;
@@ -605,7 +610,11 @@ template <>
 struct FracSum<OpsP> {
     dfl sum = {0.f, 0.f};
     __device__ __forceinline__ void add(dfl n, dfl d) { sum = df_fma(n, df_rcp(d), sum); }
-    __device__ __forceinline__ double value() { return df_val(sum); }
+    __device__ __forceinline__ void end_point(double &acc) {
+        acc += df_val(sum);
+        sum = {0.f, 0.f};
+    }
+    __device__ __forceinline__ double value() { return 0.0; }
 };
 
 template <class Ops, int D, bool DERIV>
@@ -637,10 +646,20 @@ __global__ void __launch_bounds__(128) k_trace_tpi(SchurArgs g) {
         }
     double acc1 = 0.0, acc2 = 0.0;
     bool sing = false;
+    FracSum<Ops> fr;
+    constexpr bool CAN_DIAG = D == 2 && !DERIV && std::is_same<Ops, OpsD>::value;
+    bool diag = false;
+    if constexpr (CAN_DIAG) diag = m == 0 && __syncthreads_and(Ops::mag2(zs[0][1]) == 0 && Ops::mag2(zs[1][0]) == 0);
     for (int k0 = kbeg; k0 < kend; k0 += g.kc) {
         const int nkc = min(g.kc, kend - k0);
         __syncthreads();
         tpi_stage<Ops, D>(g, k0, nkc, sPo, sPd, sE, sH, false);
+        if constexpr (CAN_DIAG) {
+            if (diag) {  // H_01 H_10 in the place of -H_10
+                __syncthreads();
+                for (int t = threadIdx.x; t < nkc; t += blockDim.x) sH[t * DD + 1] = Ops::mul(sH[t * DD + 1], sH[t * DD + 2]);
+            }
+        }
         for (int t = threadIdx.x; t < nkc * n; t += blockDim.x) sE0[t] = Ops::rfrom(g.mu - g.eps0[(size_t)k0 * n + t]);
         __syncthreads();
         for (int kk = 0; kk < nkc; kk++) {
@@ -696,6 +715,16 @@ __global__ void __launch_bounds__(128) k_trace_tpi(SchurArgs g) {
                 const R Ar = Ops::cre(Qr[t][q]), Br = Ops::cim(Qr[t][q]), Ai = Ops::cre(Qi[t][q]), Bi = Ops::cim(Qi[t][q]);
                 return a < b ? Ops::mk(Ops::rsub(Ar, Bi), Ops::radd(Ai, Br)) : Ops::mk(Ops::radd(Ar, Bi), Ops::rsub(Br, Ai));
             };
+            if constexpr (CAN_DIAG) {
+                if (diag) {
+                    const C p = Ops::add(hp[0], zs[0][0]), q = Ops::add(hp[3], zs[1][1]);
+                    const C det = Ops::sub(Ops::mul(p, q), hp[1]), num = Ops::add(p, q);
+                    sing |= !(Ops::mag2(det) > 0);
+                    fr.add(Ops::rdotc(num, det), Ops::rdotc(det, det));
+                    for (int j = 0; j < n; j++) fr.add(Ops::rneg(e0[j]), Ops::rfma(e0[j], e0[j], w2));
+                    continue;
+                }
+            }
             C M[D][D];
 #pragma unroll
             for (int a = 0; a < D; a++)
@@ -713,7 +742,6 @@ __global__ void __launch_bounds__(128) k_trace_tpi(SchurArgs g) {
                 C v = m > 0 ? entry(1, a, b) : Ops::zero();
                 return a == b ? Ops::add(v, Ops::one()) : v;
             };
-            FracSum<Ops> fr;
             if constexpr (D == 2 && !DERIV) {
                 C det = Ops::fms(M[0][1], M[1][0], Ops::mul(M[0][0], M[1][1]));
                 C num;
@@ -769,9 +797,10 @@ __global__ void __launch_bounds__(128) k_trace_tpi(SchurArgs g) {
                     acc2 += Ops::re(Ops::mul(r, r));
                 }
             }
-            acc1 += fr.value();
+            fr.end_point(acc1);
         }
     }
+    acc1 += fr.value();
     if (sing && fvalid) dg_flag(g.status, DG_SINGULAR);
     if (fvalid) g.ptr[(size_t)chunk * g.nf2 + f] = cmk(acc1, acc2);
 }

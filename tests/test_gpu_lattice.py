@@ -305,10 +305,11 @@ def test_nele_tensor_cores_match_oracle(ctx, orc, n, D, nf):
 
 @pytest.mark.parametrize("n,D,nk,nf", [(4, 4, 1, 24), (5, 5, 2, 33), (9, 6, 3, 40), (7, 7, 5, 31), (22, 8, 6, 32),
                                        (32, 9, 9, 24), (10, 10, 4, 65), (28, 10, 17, 47), (32, 10, 26, 24), (9, 5, 3, 33),
-                                       (13, 5, 2, 40), (14, 6, 18, 24), (38, 6, 9, 31), (12, 8, 3, 24), (15, 7, 3, 33)])
+                                       (13, 5, 2, 40), (14, 6, 18, 24), (38, 6, 9, 31), (12, 8, 3, 24), (15, 7, 3, 33), (7, 5, 3, 24),
+                                       (8, 5, 2, 25), (9, 7, 4, 33), (9, 8, 2, 24), (9, 9, 3, 24)])
 def test_tensor_core_block_and_derivative_passes(ctx, orc, n, D, nk, nf):
     """G_loc, GwHF and NumMatrix, and dN/dmu, of the mixed form at 4 <= D <= 10: no ligands up to the 32 poles a k point
-    may have, the counts from which each pass is on the tensor cores (4, 6, 8), k counts around the points GwHF's sums
+    may have, the counts from which each pass is on the tensor cores (0, 2, 4), k counts around the points GwHF's sums
     share and the chunks, frequency counts that leave partial tiles of 32.  Against the FP64 oracle (the mixed tolerance)
     and the GPU's FP64 pass (1e-11: the slices leave less than 2^-41, inversions of matrices of condition < 1e2)."""
     H, S, lat = _random_lattice(n, D, (nk, 1, 1), nf, [n, D, nk])
@@ -406,3 +407,23 @@ def test_eigensolver_sizes(ctx, orc, n, D, nk):
     for mixed, tol in ((False, 1e-11), (True, TOL_MIXED)):
         for g, w in zip(ctx.GreenFtn_w(lat, H, S, 0.2, mixed=mixed), want):
             assert rel_err(g, w) < tol
+
+
+@pytest.mark.parametrize("dense", ["none", "one frequency", "all"])
+@pytest.mark.parametrize("nk,nf,scale", [(1, 24, 1.0), (7, 65, 1.0), (37, 129, 1.0), (5, 24, 1e20)])
+def test_nele_two_orbitals_without_ligands(ctx, orc, nk, nf, scale, dense):
+    """N(mu) of the 2 x 2 block: the determinant with and without off-diagonal self-energies (in one frequency of a CTA's
+    only, too), fractions that run over k points and, with energies of 1e20, past the range of their common denominator.
+    FP64 1e-11, double-float 1e-9, as for the other N(mu) passes (double-float: FP32's range, so not at 1e20)."""
+    H, S, lat = _random_lattice(2, 2, (nk, 1, 1), nf, [nk, nf])
+    if dense != "none":
+        f = slice(None) if dense == "all" else slice(nf // 2, nf // 2 + 1)
+        S[f, 0, 1] += 0.1 - 0.2j
+        S[f, 1, 0] += 0.1 - 0.2j
+    for mu in (-0.4, 0.3):
+        N = orc.nele(H, S, mu, 15.0, 1, 2)
+        N = N[0] if isinstance(N, tuple) else N
+        big = lib.Lattice(2, nk, nf, 15.0 / scale, 1, 2)
+        assert abs(ctx.GiwToNele(big, H * scale, S * scale, mu * scale) - N) <= 1e-11 * max(1, abs(N))
+        if scale == 1.0:
+            assert abs(ctx.GiwToNele(lat, H, S, mu, mixed=True) - N) <= 1e-9 * max(1, abs(N))
