@@ -635,7 +635,8 @@ int run_schur(dmftgpu_ctx *ctx, const Prepared &P, int mode, double mu, int wgri
     const size_t smem = smem_of(kc);
     if (smem > 200 * 1024) return dg_fail(ctx, DMFTGPU_BADARG, "lattice: correlated block too large");
     DG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    // k chunks: enough CTAs for `cps` per SM (8 unless tuned), at least 8 k points per chunk (below that a CTA's setup
+    // k chunks: enough CTAs for `cps` per SM (unless tuned 8, and 24 where three are resident: with 8 the last two of an SM
+    // run without a third; t2g + p, 13,824 k: 24.4 -> 23.7 ms), at least 8 k points per chunk (below that a CTA's setup
     // and the partial sums cost more than the idle SMs; with 64 a 484-k, 800-point pass ran 56 CTAs on 152 SMs)
     const int fblocks = dg_ceil_div(nf2, NG);
     int nsm = 152;
@@ -649,7 +650,7 @@ int run_schur(dmftgpu_ctx *ctx, const Prepared &P, int mode, double mu, int wgri
     const std::string key = std::string(tpi ? "schur_tpi/" : "schur/") + std::to_string(in->DP) + "/" + std::to_string(mode) + "/" +
                             std::to_string((int)mixed) + "/" + std::to_string(P.nk) + "/" + std::to_string(nf2);
     int kch_max;
-    const int nchunk_max = chunks(16, &kch_max);
+    const int cps0 = tpi && !trace && mixed && P.D == 3 ? 24 : 8, nchunk_max = chunks(std::max(cps0, 16), &kch_max);
     double2 *pblk = nullptr, *pblk0 = nullptr, *ptr = nullptr;
     if (mode & dg::S_BLOCK) {
         pblk = (double2 *)dg_buf(ctx, "schur.pblk", (size_t)nchunk_max * nf2 * DD * sizeof(double2));
@@ -661,7 +662,7 @@ int run_schur(dmftgpu_ctx *ctx, const Prepared &P, int mode, double mu, int wgri
         if (!ptr) return DMFTGPU_NOMEM;
     }
     int kchunk;
-    int nchunk = chunks(8, &kchunk);
+    int nchunk = chunks(cps0, &kchunk);
     dg::SchurArgs g;
     g.H = P.H;
     g.B = P.B;

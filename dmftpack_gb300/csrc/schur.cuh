@@ -571,7 +571,7 @@ __global__ void __launch_bounds__(128, tpi_shared<Ops, D> ? 3 : 1) k_schur_tpi(S
 // FMA/s), where a division costs as much as ten products: the real fractions of a point (the block's trace and the
 // x_j / (x_j^2 + w^2) of Tr G0) are therefore added over a common denominator, eight at a time and across k points.  Where
 // no frequency of the CTA has an off-diagonal Sigma, the 2 x 2 block without ligands takes H_01 H_10 from the staged data.
-// A pass over 64 x 64 k and 4096 points of the two-orbital model takes 1.04 ms (1.27 with a division per point and the
+// A pass over 64 x 64 k and 4096 points of the two-orbital model takes 1.06 ms (1.27 with a division per point and the
 // general determinant, 42 FP64 instructions; lane groups: 4.1), in double-float 0.37 ms (0.89).
 __host__ __device__ inline size_t trace_tpi_stage(int kc, int D, int m, int n) {
     return schur_tpi_stage(kc, D, m) + ((size_t)kc * n * 8 + 15) / 16 * 16;
