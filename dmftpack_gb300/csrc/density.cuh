@@ -18,7 +18,13 @@
 // Mapping: one CTA per k point (and frequency split); a lane group of W lanes owns one frequency at a time, lane c
 // holds column c of S and inverts it with gj_inverse (schur.cuh); the group's products and accumulators live in its
 // own shared-memory tiles, reduced over groups in a fixed order at the end.  FP64 (Ops = OpsD) or double-float on
-// the FP32 pipe (OpsF, DMFTGPU_MIXED), with 16-byte complex elements either way.
+// the FP32 pipe (DMFTGPU_MIXED), with 16-byte complex elements either way: packed (OpsP), but scalar (OpsF) beyond 16
+// orbitals, whose columns leave the packed form too few registers (D = 20, n = 28, 216 k x 512 points: 11.0 and 12.8 ms).
+//
+// What bounds it is the double-float arithmetic of whole warps: with shared memory for some 16 groups per SM, the CTAs
+// are chosen for the most groups in whole warps.  (Chosen for the most warps they were single 16-lane groups, half a
+// warp each: 216 k x 2,048 points of the d + p model took 39.3 ms, in whole warps 21.3, packed 17.3.)  Sums shared by a warp's
+// groups leave room for half as many warps again and were slower, 20.5.
 #pragma once
 #include "schur.cuh"
 
@@ -195,6 +201,8 @@ DG_DENS_DECL(12)
 DG_DENS_DECL(16)
 DG_DENS_DECL(20)
 #define DG_DENS_INST(DP, W) \
-    DensKernel dens_kernel_##DP(bool mixed) { return mixed ? k_dens_sum<OpsF, DP, W> : k_dens_sum<OpsD, DP, W>; }
+    DensKernel dens_kernel_##DP(bool mixed) {                                                                  \
+        return mixed ? k_dens_sum<std::conditional<(DP > 16), OpsF, OpsP>::type, DP, W> : k_dens_sum<OpsD, DP, W>; \
+    }
 
 }  // namespace dg

@@ -1025,16 +1025,16 @@ int run_density(dmftgpu_ctx *ctx, const Prepared &P, double mu, double2 *dens, b
     DensKernel kern = si ? pick_dens(si->DP, mixed) : nullptr;
     if (!kern) return dg_fail(ctx, DMFTGPU_BADARG, "density: unsupported correlated block");
     const int DP = si->DP, W = si->W;
-    // groups per CTA: the most resident warps per SM within 227 KB of shared memory per CTA
+    // groups per CTA: the most resident ones per SM within 227 KB of shared memory per CTA, whole warps before half ones
     const size_t smem_cap = 227 * 1024, sm_per_sm = 228 * 1024;
     int ng = 0, best = -1;
     for (int g = 1; g * W <= 128; g++) {
         const size_t sm = dg::dens_smem(DP, D, m, n, g);
         if (sm > smem_cap) break;
-        const int ctas = std::min((int)(sm_per_sm / (sm + 1024)), 2048 / (g * W));
-        const int warps = ctas * ((g * W + 31) / 32);
-        if (warps >= best) {
-            best = warps;
+        const int ctas = std::min((int)(sm_per_sm / (sm + 1024)), 2048 / std::max(g * W, 32));
+        const int groups = ctas * g * ((g * W) % 32 ? 1 : 2);
+        if (groups >= best) {
+            best = groups;
             ng = g;
         }
     }
