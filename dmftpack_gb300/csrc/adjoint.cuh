@@ -23,13 +23,17 @@
 // 56 orbitals, D = 20, 125 k x 512 frequencies: 61.8 -> 23.9 ms (JVP) and 72.6 -> 23.9 (VJP),
 // the eigensolvers of the preparation (3.5 ms) included; 10 + 18 orbitals 9.4 -> 4.6 and 10.8 -> 4.7, 4 + 12 2.4 -> 0.9 and 2.7 -> 1.0.
 // CTA = F frequencies x one chunk of k points; per-chunk sums are reduced in fixed order.
+//
+// The forward passes in FP64 run in the same way from some 5 orbitals on (run_schur): AD_BLOCK, G_loc and GwHF (the inverse of M and of
+// z - m0 - H_PP - S in its second tile), and AD_TRACE, N(mu) (Re[Tr G - Tr G0] of k_schur's TRACE form, the second tile
+// I + R).  343 k x 400 frequencies of 10 + 18 orbitals: G_loc 17.3 -> 12.5 ms, N(mu) 18.0 -> 11.7 against the columns of k_schur.
 #pragma once
 #include "internal.h"
-#include "linalg.cuh"
+#include "schur.cuh"
 
 namespace dg {
 
-enum { AD_VJP = 1, AD_JVP = 2 };
+enum { AD_VJP = 1, AD_JVP = 2, AD_BLOCK = 3, AD_TRACE = 4 };
 constexpr int AD_EL = 13;        // matrix elements per lane at most
 constexpr int AD_THREADS = 256;  // at most; two CTAs per SM
 
@@ -37,23 +41,27 @@ struct AdArgs {
     const double2 *H, *B;  // [nk][n][n]; [nk][m][D] b_l(a)
     const double *epsQ;    // [nk][m]
     const double2 *sig;    // [nf][D][D] Sigma(iw_n), n < nf
+    const double2 *m0;     // BLOCK: [D][D] the static moment
+    const double *eps0;    // TRACE: [nk][n] eigenvalues of H + m0
+    int wgrid;             // TRACE: the N(mu) frequency grid
     const double2 *gin;    // VJP: Gbar [nf][D][D]; JVP: Sigma_dot [nf][D][D]
     double mu_dot;         // JVP
     int n, m, nk, nf, D, kchunk, F;
     double beta, mu;
     double2 *pout;         // [nchunk][nf][D][D] per-chunk sums (Sigma_bar or G_loc_dot, before the 1/N_k)
     double *pmu;           // [nchunk][nf] VJP: per-chunk Re Tr[(G S' G)^H Gbar]
+    double2 *pout0;        // BLOCK: the sums of G0_PP; TRACE: [nchunk][nf] (Re[Tr G - Tr G0], 0)
     int *status;
 };
 
 // shared memory of one frequency, in double2: two tiles, the weights (w_l, w_l^2), and the inversion's row, column and
-// pivot buffers, which lie over the second tile (VJP) or over the weights (JVP), both free then
+// pivot buffers, which lie over the second tile (VJP) or over the weights (else), both free then
 __host__ __device__ inline int ad_bufs(int D) { return 2 * D + (D + 3) / 4; }
 __host__ __device__ inline int ad_tile1(int D, int mode) {
     return mode == AD_VJP && ad_bufs(D) > D * D ? ad_bufs(D) : D * D;
 }
 __host__ __device__ inline int ad_weights(int D, int m, int mode) {
-    return mode == AD_JVP && ad_bufs(D) > 2 * m ? ad_bufs(D) : 2 * m;
+    return mode != AD_VJP && ad_bufs(D) > 2 * m ? ad_bufs(D) : 2 * m;
 }
 inline size_t ad_smem(int F, int D, int m, int mode) {
     return (size_t)F * (D * D + ad_tile1(D, mode) + ad_weights(D, m, mode)) * 16 + (size_t)(D * (D + 1) / 2) * 4;
@@ -152,7 +160,8 @@ struct PairSum {
 template <int LW, int MODE>
 __global__ void __launch_bounds__(AD_THREADS, 2) k_gloc_ad(AdArgs g) {
     typedef double2 C;
-    constexpr int SUB = MODE == AD_JVP ? 4 : 8;
+    constexpr bool TWO = MODE == AD_JVP || MODE == AD_TRACE;  // S and S' at once
+    constexpr int SUB = TWO ? 4 : 8;
     extern __shared__ double2 sm[];
     const int D = g.D, DD = D * D, m = g.m, F = g.F, npair = D * (D + 1) / 2;
     const int t1 = ad_tile1(D, MODE), ws = ad_weights(D, m, MODE);
@@ -169,9 +178,16 @@ __global__ void __launch_bounds__(AD_THREADS, 2) k_gloc_ad(AdArgs g) {
         while ((c + 1) * (c + 2) / 2 <= t) c++;
         sPair[t] = make_ushort2((unsigned short)(t - c * (c + 1) / 2), (unsigned short)c);
     }
-    C acc[AD_EL];
+    auto wfreq = [&](int ff) {
+        return MODE == AD_TRACE && g.wgrid ? (DG_PI / g.beta + ff * ((2 * DG_PI) / g.beta)) : (DG_PI * (2. * ff + 1.) / g.beta);
+    };
+    constexpr int NACC = MODE == AD_TRACE ? 1 : AD_EL;
+    C acc[NACC], acc0[MODE == AD_BLOCK ? AD_EL : 1];
 #pragma unroll
-    for (int i = 0; i < AD_EL; i++) acc[i] = cmk(0, 0);
+    for (int i = 0; i < NACC; i++) acc[i] = cmk(0, 0);
+#pragma unroll
+    for (int i = 0; i < (MODE == AD_BLOCK ? AD_EL : 1); i++) acc0[i] = cmk(0, 0);
+    FracSum<OpsD> fr;
     double accmu = 0.0;
     bool sing = false;
     const int nsub = (F + SUB - 1) / SUB;
@@ -180,22 +196,32 @@ __global__ void __launch_bounds__(AD_THREADS, 2) k_gloc_ad(AdArgs g) {
         __syncthreads();
         for (int t = threadIdx.x; t < F * m; t += blockDim.x) {
             const int fl = t / m, l = t - fl * m;
-            const double w = DG_PI * (2. * min(f0 + fl, g.nf - 1) + 1.) / g.beta;
+            const double w = wfreq(min(f0 + fl, g.nf - 1));
             const C wl = crcp(cmk(g.mu - g.epsQ[(size_t)k * m + l], w));
             sW[(size_t)fl * ws + 2 * l] = wl;
-            sW[(size_t)fl * ws + 2 * l + 1] = cmul(wl, wl);
+            if (MODE != AD_BLOCK) sW[(size_t)fl * ws + 2 * l + 1] = cmul(wl, wl);
+        }
+        if (MODE == AD_TRACE) {  // - Tr G0
+            const double w = wfreq(f), w2 = w * w;
+            for (int j = lane; j < g.n; j += LW) {
+                const double x = g.mu - g.eps0[(size_t)k * g.n + j];
+                fr.add(-x, fma(x, x, w2));
+            }
         }
         __syncthreads();
-        // M = z - H_PP - Sigma - S into the first tile; JVP: Sigma_dot - mu_dot S' into the second
+        if (MODE == AD_TRACE)
+            for (int l = lane; l < m; l += LW) accmu += sW[(size_t)grp * ws + 2 * l].x;
+        // M = z - H_PP - Sigma - S into the first tile; into the second JVP: Sigma_dot - mu_dot S', BLOCK: M with m0 in the place of
+        // Sigma, TRACE: S', transposed
         for (int t = threadIdx.x; t < npair * nsub; t += blockDim.x) {
             const int s = t / npair;
             const ushort2 pr = sPair[t - s * npair];
             const int a = pr.x, c = pr.y;
-            PairSum x[SUB], y[MODE == AD_JVP ? SUB : 1];
+            PairSum x[SUB], y[TWO ? SUB : 1];
 #pragma unroll
             for (int i = 0; i < SUB; i++) {
                 x[i] = {0, 0, 0, 0};
-                if (MODE == AD_JVP) y[i] = {0, 0, 0, 0};
+                if (TWO) y[i] = {0, 0, 0, 0};
             }
             for (int l = 0; l < m; l++) {
                 const C pq = cmulc(Bk[l * D + a], Bk[l * D + c]);
@@ -203,7 +229,7 @@ __global__ void __launch_bounds__(AD_THREADS, 2) k_gloc_ad(AdArgs g) {
                 for (int i = 0; i < SUB; i++) {
                     const C *w = sW + (size_t)min(s * SUB + i, F - 1) * ws + 2 * l;
                     x[i].add(w[0], pq.x, pq.y);
-                    if (MODE == AD_JVP) y[i].add(w[1], pq.x, pq.y);
+                    if (TWO) y[i].add(w[1], pq.x, pq.y);
                 }
             }
             const C h = Hk[a + c * g.n], ht = Hk[c + a * g.n];
@@ -213,10 +239,26 @@ __global__ void __launch_bounds__(AD_THREADS, 2) k_gloc_ad(AdArgs g) {
                 if (fl >= F) break;
                 const int ff = min(f0 + fl, g.nf - 1);
                 const C *sg = g.sig + (size_t)ff * DD;
-                C d = cneg(cadd(cadd(h, sg[a + c * D]), x[i].ac())), e = cneg(cadd(cadd(ht, sg[c + a * D]), x[i].ca()));
-                if (a == c) d = e = cadd(d, cmk(g.mu, DG_PI * (2. * ff + 1.) / g.beta));
-                T0[(size_t)fl * DD + a + c * D] = d;
-                T0[(size_t)fl * DD + c + a * D] = e;
+                C hs = cneg(cadd(h, x[i].ac())), hst = cneg(cadd(ht, x[i].ca()));
+                if (a == c) hs = hst = cadd(hs, cmk(g.mu, wfreq(ff)));
+                T0[(size_t)fl * DD + a + c * D] = csub(hs, sg[a + c * D]);
+                T0[(size_t)fl * DD + c + a * D] = csub(hst, sg[c + a * D]);
+                if (MODE == AD_BLOCK) {
+                    // m0 as it is below 8 orbitals, from 8 on its lower triangle, as the static spectrum reads it
+                    C mt = g.m0[c + a * D], mu_ = g.m0[a + c * D];
+                    if (D >= 8) {
+                        if (a == c) mt.y = 0.0;
+                        mu_ = cconj(mt);
+                    }
+                    T1[(size_t)fl * DD + a + c * D] = csub(hs, mu_);
+                    T1[(size_t)fl * DD + c + a * D] = csub(hst, mt);
+                }
+                if (MODE == AD_TRACE) {
+                    const double one = a == c ? 1.0 : 0.0;
+                    const C u = y[i].ac(), v = y[i].ca();
+                    T1[(size_t)fl * DD + c + a * D] = cmk(one + u.x, u.y);
+                    T1[(size_t)fl * DD + a + c * D] = cmk(one + v.x, v.y);
+                }
                 if (MODE == AD_JVP) {
                     const C *sd = g.gin + (size_t)ff * DD;
                     const double one = a == c ? 1.0 : 0.0;
@@ -228,7 +270,19 @@ __global__ void __launch_bounds__(AD_THREADS, 2) k_gloc_ad(AdArgs g) {
         }
         __syncthreads();
         sing |= tile_inverse<LW>(A, D, buf, buf + D, reinterpret_cast<int *>(buf + 2 * D), lane) && fvalid;
-        if (MODE == AD_JVP) {
+        if (MODE == AD_BLOCK) {
+            sing |= tile_inverse<LW>(V, D, buf, buf + D, reinterpret_cast<int *>(buf + 2 * D), lane) && fvalid;
+#pragma unroll
+            for (int i = 0; i < AD_EL; i++) {
+                const int e = lane + i * LW;
+                if (e < DD) {
+                    acc[MODE == AD_BLOCK ? i : 0] = cadd(acc[MODE == AD_BLOCK ? i : 0], A[e]);
+                    acc0[MODE == AD_BLOCK ? i : 0] = cadd(acc0[MODE == AD_BLOCK ? i : 0], V[e]);
+                }
+            }
+        } else if (MODE == AD_TRACE) {
+            for (int e = lane; e < DD; e += LW) accmu = fma(A[e].x, V[e].x, fma(-A[e].y, V[e].y, accmu));  // G(r,c) S'(c,r)
+        } else if constexpr (MODE == AD_JVP) {
             // elements e = r + D c: X G, then G (X G)
             C v[AD_EL];
 #pragma unroll
@@ -257,7 +311,7 @@ __global__ void __launch_bounds__(AD_THREADS, 2) k_gloc_ad(AdArgs g) {
                     acc[i] = cadd(acc[i], x);
                 }
             }
-        } else {
+        } else if constexpr (MODE == AD_VJP) {
             // elements e = c + D r, so that lanes read along columns of G: Gbar G^H, then Z = G^H (Gbar G^H), transposed
             const C *gb = g.gin + (size_t)f * DD;
 #pragma unroll 1
@@ -315,16 +369,24 @@ __global__ void __launch_bounds__(AD_THREADS, 2) k_gloc_ad(AdArgs g) {
         }
     }
     if (sing) dg_flag(g.status, DG_SINGULAR);
-    if (MODE == AD_VJP) {
+    if (MODE == AD_VJP || MODE == AD_TRACE) {
+        if (MODE == AD_TRACE) accmu += fr.value();
 #pragma unroll
         for (int o = LW / 2; o > 0; o >>= 1) accmu += __shfl_xor_sync(0xffffffffu, accmu, o, LW);
     }
     if (!fvalid) return;
+    if (MODE == AD_TRACE) {
+        if (lane == 0) g.pout0[(size_t)chunk * g.nf + f] = cmk(accmu, 0.0);
+        return;
+    }
     C *o = g.pout + ((size_t)chunk * g.nf + f) * DD;
 #pragma unroll
-    for (int i = 0; i < AD_EL; i++) {
+    for (int i = 0; i < NACC; i++) {
         const int e = lane + i * LW;
-        if (e < DD) o[MODE == AD_JVP ? e : e / D + (e % D) * D] = acc[i];
+        if (e < DD) {
+            o[MODE != AD_VJP ? e : e / D + (e % D) * D] = acc[i];
+            if (MODE == AD_BLOCK) g.pout0[((size_t)chunk * g.nf + f) * DD + e] = acc0[MODE == AD_BLOCK ? i : 0];
+        }
     }
     if (MODE == AD_VJP && lane == 0) g.pmu[(size_t)chunk * g.nf + f] = accmu;
 }

@@ -2,13 +2,18 @@
 #include "adjoint.cuh"
 
 namespace dg {
+template <int LW>
+static AdKernel pick(int mode) {
+    switch (mode) {
+        case AD_VJP: return k_gloc_ad<LW, AD_VJP>;
+        case AD_JVP: return k_gloc_ad<LW, AD_JVP>;
+        case AD_BLOCK: return k_gloc_ad<LW, AD_BLOCK>;
+        default: return k_gloc_ad<LW, AD_TRACE>;
+    }
+}
 AdKernel ad_kernel(int D, int mode, int *lanes) {
-    const int lw = D <= 7 ? 4 : (D <= 10 ? 8 : (D <= 14 ? 16 : 32));
-    *lanes = lw;
+    *lanes = D <= 7 ? 4 : (D <= 10 ? 8 : (D <= 14 ? 16 : 32));
     if (D > 20) return nullptr;
-    if (lw == 4) return mode == AD_VJP ? k_gloc_ad<4, AD_VJP> : k_gloc_ad<4, AD_JVP>;
-    if (lw == 8) return mode == AD_VJP ? k_gloc_ad<8, AD_VJP> : k_gloc_ad<8, AD_JVP>;
-    if (lw == 16) return mode == AD_VJP ? k_gloc_ad<16, AD_VJP> : k_gloc_ad<16, AD_JVP>;
-    return mode == AD_VJP ? k_gloc_ad<32, AD_VJP> : k_gloc_ad<32, AD_JVP>;
+    return *lanes == 4 ? pick<4>(mode) : (*lanes == 8 ? pick<8>(mode) : (*lanes == 16 ? pick<16>(mode) : pick<32>(mode)));
 }
 }  // namespace dg

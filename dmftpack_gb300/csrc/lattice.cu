@@ -611,9 +611,94 @@ __global__ void k_schur_reduce(int nchunk, int nf2, int DD, int mode, const doub
     }
 }
 
+// the shape of a k_gloc_ad launch over nf frequencies
+struct AdShape {
+    int F, fblocks, kchunk, nchunk;
+    size_t smem;
+};
+AdShape ad_shape(dmftgpu_ctx *ctx, const Prepared &P, int mode, int lanes, int nf) {
+    AdShape s;
+    const int m = P.n - P.D, step = std::max(1, 32 / lanes);
+    // frequencies per CTA: whole warps, no more than there are, two CTAs per SM (228 KB, 1 KB of it taken per CTA)
+    s.F = std::min(dg::AD_THREADS / lanes, dg_ceil_div(nf, step) * step);
+    while (s.F > step && dg::ad_smem(s.F, P.D, m, mode) > 113 * 1024) s.F -= step;
+    s.smem = dg::ad_smem(s.F, P.D, m, mode);
+    s.fblocks = dg_ceil_div(nf, s.F);
+    // k points per CTA: the fewest rounds of CTAs x (their k points and a little for their start), at most eight rounds
+    int nsm = 152;
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, ctx->device);
+    const int slots = 2 * nsm;
+    s.kchunk = P.nk;
+    double best = 1e300;
+    for (int r = 1; r <= 8; r++) {
+        const int nc = (int)std::max(1LL, std::min((long long)P.nk, (long long)r * slots / s.fblocks)), kch = dg_ceil_div(P.nk, nc);
+        const double cost = dg_ceil_div((long long)s.fblocks * dg_ceil_div(P.nk, kch), slots) * (kch + 0.3);
+        if (cost < best) {
+            best = cost;
+            s.kchunk = kch;
+        }
+    }
+    s.nchunk = dg_ceil_div(P.nk, s.kchunk);
+    return s;
+}
+
+// the FP64 G_loc / GwHF and N(mu) passes by k_gloc_ad (see there); the caller has checked the mode and the size
+int run_tiles(dmftgpu_ctx *ctx, const Prepared &P, bool trace, double mu, int wgrid, double2 *blk, double2 *blk0, double *tr) {
+    const int mode = trace ? dg::AD_TRACE : dg::AD_BLOCK, nf2 = 2 * P.Nf, DD = P.D * P.D;
+    int lanes = 0;
+    dg::AdKernel kern = dg::ad_kernel(P.D, mode, &lanes);
+    const AdShape sh = ad_shape(ctx, P, mode, lanes, nf2);
+    DG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh.smem));
+    dg::AdArgs g = {};
+    if (trace) {
+        g.pout0 = (double2 *)dg_buf(ctx, "schur.ptr", (size_t)sh.nchunk * nf2 * sizeof(double2));
+        if (!g.pout0) return DMFTGPU_NOMEM;
+        DG_CUDA(cudaStreamWaitEvent(ctx->stream, P.static_ready, 0));
+    } else {
+        g.pout = (double2 *)dg_buf(ctx, "schur.pblk", (size_t)sh.nchunk * nf2 * DD * sizeof(double2));
+        g.pout0 = (double2 *)dg_buf(ctx, "schur.pblk0", (size_t)sh.nchunk * nf2 * DD * sizeof(double2));
+        if (!g.pout || !g.pout0) return DMFTGPU_NOMEM;
+    }
+    g.H = P.H;
+    g.B = P.B;
+    g.epsQ = P.epsQ;
+    g.sig = P.sig;
+    g.m0 = P.m0;
+    g.eps0 = P.eps;
+    g.wgrid = wgrid;
+    g.n = P.n;
+    g.m = P.n - P.D;
+    g.nk = P.nk;
+    g.nf = nf2;
+    g.D = P.D;
+    g.kchunk = sh.kchunk;
+    g.F = sh.F;
+    g.beta = P.beta;
+    g.mu = mu;
+    g.status = ctx->d_status;
+    {
+        DgTimer tm(ctx, "k_gloc_ad");
+        kern<<<dim3(sh.fblocks, sh.nchunk), sh.F * lanes, sh.smem, ctx->stream>>>(g);
+    }
+    DG_LAUNCH(ctx, "k_gloc_ad");
+    const long long nred = trace ? nf2 : (long long)nf2 * DD;
+    k_schur_reduce<<<dg_ceil_div(nred, 256), 256, 0, ctx->stream>>>(sh.nchunk, nf2, DD, trace ? dg::S_TRACE : dg::S_BLOCK, g.pout,
+                                                                    g.pout0, g.pout0, blk, blk0, tr, nullptr);
+    DG_LAUNCH(ctx, "k_schur_reduce");
+    return DMFTGPU_OK;
+}
+
 // the Schur-form pass (default); mode: dg::S_BLOCK (GreenFtn_w) or S_TRACE[|S_DERIV] (N(mu))
 int run_schur(dmftgpu_ctx *ctx, const Prepared &P, int mode, double mu, int wgrid, double2 *blk, double2 *blk0,
               double *tr, double *dtr, bool mixed) {
+    // FP64 passes by k_gloc_ad's tiles, except where k_schur's lanes are all columns and the poles few.  343 k x 400 points, ms,
+    // k_schur / tiles: G_loc D = 4, no poles 0.94 / 1.02, 12 poles 2.10 / 2.21; D = 5 2.86 / 1.59; D = 8 3.90 / 4.06, 16 poles
+    // 12.7 / 9.88; D = 10, 18 poles 17.3 / 12.5; D = 20, 8 poles 101 / 50.5; N(mu) D = 4 0.61 / 0.66, 12 poles 2.93 / 2.13;
+    // D = 10, 18 poles 18.0 / 11.7
+    const int poles = P.n - P.D;
+    const bool tiles = (mode & dg::S_TRACE) ? P.D >= 5 || (P.D == 4 && poles >= 4) : P.D >= 5 && (P.D != 8 || poles > 0);
+    if (!mixed && !(mode & (dg::S_REAL | dg::S_DERIV)) && tiles)
+        return run_tiles(ctx, P, (mode & dg::S_TRACE) != 0, mu, wgrid, blk, blk0, tr);
     const SInst *in = pick_schur(P.D);
     // Matsubara passes of correlated blocks up to 3 x 3: one thread per frequency (k_schur_tpi, k_trace_tpi), which beats
     // the lane groups at every width they cover (their groups idle at D = 3 and spend their issue slots on exchanges).
@@ -845,28 +930,10 @@ int run_ad(dmftgpu_ctx *ctx, const Prepared &P, int mode, double mu, const doubl
     int lanes = 0;
     dg::AdKernel kern = dg::ad_kernel(P.D, mode, &lanes);
     if (!kern) return dg_fail(ctx, DMFTGPU_BADARG, "derivatives: correlated block larger than 20");
-    const int m = P.n - P.D, nf = P.Nf, DD = P.D * P.D, step = std::max(1, 32 / lanes);
-    // frequencies per CTA: whole warps, no more than there are, two CTAs per SM (228 KB, 1 KB of it taken per CTA)
-    int F = std::min(dg::AD_THREADS / lanes, dg_ceil_div(nf, step) * step);
-    while (F > step && dg::ad_smem(F, P.D, m, mode) > 113 * 1024) F -= step;
-    const size_t smem = dg::ad_smem(F, P.D, m, mode);
-    DG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    // k points per CTA: the fewest rounds of CTAs x (their k points and a little for their start), at most eight rounds
-    int nsm = 152;
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, ctx->device);
-    const int fblocks = dg_ceil_div(nf, F), slots = 2 * nsm;
-    int kchunk = P.nk;
-    double best = 1e300;
-    for (int kch = P.nk; kch >= 1; kch--) {
-        const long long ctas = (long long)fblocks * dg_ceil_div(P.nk, kch), rounds = (ctas + slots - 1) / slots;
-        if (rounds > 8 && kch < P.nk) break;
-        const double cost = rounds * (kch + 0.3);
-        if (cost < best) {
-            best = cost;
-            kchunk = kch;
-        }
-    }
-    const int nchunk = dg_ceil_div(P.nk, kchunk);
+    const int m = P.n - P.D, nf = P.Nf, DD = P.D * P.D;
+    const AdShape sh = ad_shape(ctx, P, mode, lanes, nf);
+    DG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh.smem));
+    const int nchunk = sh.nchunk;
     double2 *pout = (double2 *)dg_buf(ctx, "ad.pout", (size_t)nchunk * nf * DD * sizeof(double2));
     double *pmu = (double *)dg_buf(ctx, "ad.pmu", (size_t)nchunk * nf * sizeof(double));
     if (!pout || !pmu) return DMFTGPU_NOMEM;
@@ -882,8 +949,8 @@ int run_ad(dmftgpu_ctx *ctx, const Prepared &P, int mode, double mu, const doubl
     g.nk = P.nk;
     g.nf = nf;
     g.D = P.D;
-    g.kchunk = kchunk;
-    g.F = F;
+    g.kchunk = sh.kchunk;
+    g.F = sh.F;
     g.beta = P.beta;
     g.mu = mu;
     g.pout = pout;
@@ -891,7 +958,7 @@ int run_ad(dmftgpu_ctx *ctx, const Prepared &P, int mode, double mu, const doubl
     g.status = ctx->d_status;
     {
         DgTimer tm(ctx, "k_gloc_ad");
-        kern<<<dim3(fblocks, nchunk), F * lanes, smem, ctx->stream>>>(g);
+        kern<<<dim3(sh.fblocks, nchunk), sh.F * lanes, sh.smem, ctx->stream>>>(g);
     }
     DG_LAUNCH(ctx, "k_gloc_ad");
     const long long len = (long long)nf * DD;

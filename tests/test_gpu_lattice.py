@@ -427,3 +427,17 @@ def test_nele_two_orbitals_without_ligands(ctx, orc, nk, nf, scale, dense):
         assert abs(ctx.GiwToNele(big, H * scale, S * scale, mu * scale) - N) <= 1e-11 * max(1, abs(N))
         if scale == 1.0:
             assert abs(ctx.GiwToNele(lat, H, S, mu, mixed=True) - N) <= 1e-9 * max(1, abs(N))
+
+
+@pytest.mark.parametrize("n,D,nk,nf", [(4, 4, 3, 33), (8, 4, 2, 65), (5, 5, 3, 24), (18, 7, 5, 33), (8, 8, 2, 31), (9, 8, 7, 32),
+                                       (28, 10, 3, 40), (11, 11, 2, 24), (20, 14, 3, 25), (17, 15, 2, 33), (64, 20, 2, 24)])
+def test_fp64_passes_by_tiles(ctx, orc, n, D, nk, nf):
+    """G_loc, GwHF, NumMatrix and N(mu) in FP64 at the edges of the lane groups (7, 10, 14, 20 orbitals) and of the rule that
+    chooses them, with no poles and the most, frequency counts that leave partial CTAs; 1e-11 as for the other FP64 passes."""
+    H, S, lat = _random_lattice(n, D, (nk, 1, 1), nf, [n, D, nk, nf])
+    for mu in (-0.4, 0.3):
+        for g, w in zip(ctx.GreenFtn_w(lat, H, S, mu), orc.greenftn_w(H, S, mu, 15.0, 1, D)):
+            assert rel_err(g, w) < 1e-11
+        N = orc.nele(H, S, mu, 15.0, 1, D)
+        N = N[0] if isinstance(N, tuple) else N
+        assert abs(ctx.GiwToNele(lat, H, S, mu) - N) <= 1e-11 * max(1, abs(N))
