@@ -783,7 +783,7 @@ def run_ours(args, rank, world, local_rank):
     try:
         with open(os.path.join(os.path.dirname(os.path.abspath(__file__)), "profiles", "traffic.json")) as fh:
             measured = json.load(fh)
-        tname = ("k_schur_tpi<%s, %d>" % ("OpsF" if mixed else "OpsD", wl.D)) if (not explicit and wl.D <= 3) else None
+        tname = ("k_schur_tpi<%s, %d>" % ("OpsP" if mixed else "OpsD", wl.D)) if (not explicit and wl.D <= 3) else None
         rec = measured.get(tname) if tname else None
         if rec and rec["workload"] == {"n": wl.n, "D": wl.D, "nk": wl.nk, "nfreq": wl.nfreq,
                                        "precision": args.precision}:
