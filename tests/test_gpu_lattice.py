@@ -441,3 +441,20 @@ def test_fp64_passes_by_tiles(ctx, orc, n, D, nk, nf):
         N = orc.nele(H, S, mu, 15.0, 1, D)
         N = N[0] if isinstance(N, tuple) else N
         assert abs(ctx.GiwToNele(lat, H, S, mu) - N) <= 1e-11 * max(1, abs(N))
+
+
+@pytest.mark.parametrize("n,nk,nf", [(2, 5, 33), (2, 130, 24), (5, 7, 64)])
+def test_two_orbital_closed_forms(ctx, orc, n, nk, nf):
+    """G_loc, GwHF, NumMatrix, N(mu) and dN/dmu of 2 x 2 blocks with a dense self-energy whose determinant has its larger
+    product off the diagonal (the pivot's place), with and without ligands; the bounds of the other sizes."""
+    H, S, lat = _random_lattice(n, 2, (nk, 1, 1), nf, [n, nk])
+    H[:, 0, 1] += 3.0
+    H[:, 1, 0] += 3.0
+    for mu in (-0.4, 0.3):
+        want = orc.greenftn_w(H, S, mu, 15.0, 1, 2)
+        N, dN = orc.nele(H, S, mu, 15.0, 1, 2, deriv=True)
+        for mixed, tol in ((False, 1e-11), (True, TOL_MIXED)):
+            for g, w in zip(ctx.GreenFtn_w(lat, H, S, mu, mixed=mixed), want):
+                assert rel_err(g, w) < tol
+            g, dg = ctx.GiwToNele(lat, H, S, mu, deriv=True, mixed=mixed)
+            assert abs(g - N) <= tol * max(1, abs(N)) and abs(dg - dN) <= 10 * tol * max(1, abs(dN))
