@@ -1098,21 +1098,26 @@ int launch_trace(dmftgpu_ctx *ctx, const LatTcArgs &a, bool *ready, double *tr, 
 //           D = 10  6.46 / 7.24  10.1 / 7.30
 // The lines below are where these cross.  At D = 4 N(mu) takes k_schur 0.45 (m = 0) and 1.96 (m = 10) and 1.77 and 2.33
 // here at 1,024 frequencies: they cross only past 16 poles.
-static bool covered(int n, int D, int least) { return D >= 5 && D <= 10 && n - D >= least && n - D <= KP && n <= NE0; }
-bool dg_lat_tc_supported(int n, int D) { return covered(n, D, 4); }
-bool dg_lat_tc_deriv_supported(int n, int D) { return covered(n, D, 2); }
-bool dg_lat_tc_block_supported(int n, int D) {
-    return covered(n, D, D <= 6 ? 4 : (D <= 8 ? 2 : 0)) && (D <= 6 || n <= KP);
+// And the images, 43 KB per k point at D = 10 (G_loc: two), stay within 64 GB; k_schur needs none.
+static bool covered(int n, int D, int nk, int least, int images) {
+    const size_t image = (size_t)NSB * KSTEPS * np_of((D + 1) / 2 * 2) * 16 * 2;
+    return D >= 5 && D <= 10 && n - D >= least && n - D <= KP && n <= NE0 && image * images * nk <= (size_t)64 << 30;
+}
+bool dg_lat_tc_supported(int n, int D, int nk) { return covered(n, D, nk, 4, 1); }
+bool dg_lat_tc_deriv_supported(int n, int D, int nk) { return covered(n, D, nk, 2, 1); }
+bool dg_lat_tc_block_supported(int n, int D, int nk) {
+    return covered(n, D, nk, D <= 6 ? 4 : (D <= 8 ? 2 : 0), 2) && (D <= 6 || n <= KP);
 }
 
 int dg_lat_tc_trace(dmftgpu_ctx *ctx, const LatTcArgs &a, bool *ready, double *tr, double *dtr) {
-    if (!(dtr ? dg_lat_tc_deriv_supported(a.n, a.D) : dg_lat_tc_supported(a.n, a.D))) return dg_fail(ctx, DMFTGPU_BADARG, "lat_tc: unsupported sizes");
+    if (!(dtr ? dg_lat_tc_deriv_supported(a.n, a.D, a.nk) : dg_lat_tc_supported(a.n, a.D, a.nk)))
+        return dg_fail(ctx, DMFTGPU_BADARG, "lat_tc: unsupported sizes");
     if (a.D <= 6) return launch_trace<6>(ctx, a, ready, tr, dtr);
     if (a.D <= 8) return launch_trace<8>(ctx, a, ready, tr, dtr);
     return launch_trace<10>(ctx, a, ready, tr, dtr);
 }
 int dg_lat_tc_block(dmftgpu_ctx *ctx, const LatTcArgs &a, double2 *blk, double2 *blk0) {
-    if (!dg_lat_tc_block_supported(a.n, a.D)) return dg_fail(ctx, DMFTGPU_BADARG, "lat_tc: unsupported sizes");
+    if (!dg_lat_tc_block_supported(a.n, a.D, a.nk)) return dg_fail(ctx, DMFTGPU_BADARG, "lat_tc: unsupported sizes");
     if (a.D <= 6) return launch_block<6>(ctx, a, blk, blk0);
     if (a.D <= 8) return launch_block<8>(ctx, a, blk, blk0);
     return launch_block<10>(ctx, a, blk, blk0);
