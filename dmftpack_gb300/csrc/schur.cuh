@@ -588,6 +588,29 @@ __global__ void __launch_bounds__(128, tpi_shared<Ops, D> ? 3 : 1) k_schur_tpi(S
 __host__ __device__ inline size_t trace_tpi_stage(int kc, int D, int m, int n) {
     return schur_tpi_stage(kc, D, m) + ((size_t)kc * n * 8 + 15) / 16 * 16;
 }
+// k sum of real numbers in FP64.  The double-float terms of one point are added up before they go into it: two conversions
+// and two additions for each held the FP64 pipe, and five terms a point with the derivative made that pass 2.8 times the
+// plain one
+template <class Ops>
+struct KSum;
+template <>
+struct KSum<OpsD> {
+    double sum = 0.0;
+    __device__ __forceinline__ void add(double x) { sum += x; }
+    __device__ __forceinline__ void end_point() {}
+    __device__ __forceinline__ double value() { return sum; }
+};
+template <>
+struct KSum<OpsP> {
+    double sum = 0.0;
+    dfl part = {0.f, 0.f};
+    __device__ __forceinline__ void add(dfl x) { part = df_add(part, x); }
+    __device__ __forceinline__ void end_point() {
+        sum += df_val(part);
+        part = {0.f, 0.f};
+    }
+    __device__ __forceinline__ double value() { return sum; }
+};
 // running sum of real fractions: FP64 keeps one numerator and denominator for eight terms (products of eight |det|^2 or
 // x^2 + w^2 stay far inside the range: flushed before that where they would not), double-float (whose
 // reciprocal costs less than the products) divides each
@@ -612,7 +635,7 @@ struct FracSum<OpsD> {
         if (cnt) sum += num / den;
         cnt = 0;
     }
-    __device__ __forceinline__ void end_point(double &) {}
+    __device__ __forceinline__ void end_point(KSum<OpsD> &) {}
     __device__ __forceinline__ double value() {
         flush();
         return sum;
@@ -622,8 +645,8 @@ template <>
 struct FracSum<OpsP> {
     dfl sum = {0.f, 0.f};
     __device__ __forceinline__ void add(dfl n, dfl d) { sum = df_fma(n, df_rcp(d), sum); }
-    __device__ __forceinline__ void end_point(double &acc) {
-        acc += df_val(sum);
+    __device__ __forceinline__ void end_point(KSum<OpsP> &acc) {
+        acc.add(sum);
         sum = {0.f, 0.f};
     }
     __device__ __forceinline__ double value() { return 0.0; }
@@ -656,7 +679,7 @@ __global__ void __launch_bounds__(128) k_trace_tpi(SchurArgs g) {
             const C sg = Ops::from(g.sig[(size_t)f * DD + a + b * D]);
             zs[a][b] = a == b ? Ops::sub(Ops::from(cmk(g.mu, w)), sg) : Ops::neg(sg);
         }
-    double acc1 = 0.0, acc2 = 0.0;
+    KSum<Ops> acc1, acc2;
     bool sing = false;
     FracSum<Ops> fr;
     constexpr bool CAN_DIAG = D == 2 && !DERIV && std::is_same<Ops, OpsD>::value;
@@ -782,8 +805,8 @@ __global__ void __launch_bounds__(128) k_trace_tpi(SchurArgs g) {
                     Ops::balance(scale, det);
                     sing |= !(Ops::mag2(det) > 0);
                     const C ip = Ops::pscale(Ops::rcp(det), Ops::cre(scale));
-                    acc1 += Ops::re(Ops::mul(sum, ip));
-                    acc2 -= Ops::re(Ops::mul(Ops::mul(sq, ip), ip));
+                    acc1.add(Ops::cre(Ops::mul(sum, ip)));
+                    acc2.add(Ops::rneg(Ops::cre(Ops::mul(Ops::mul(sq, ip), ip))));
                 } else {
                     sing |= thread_inverse<Ops, D>(M);
                     C t = Ops::zero(), t2 = Ops::zero(), X[D][D];
@@ -802,32 +825,36 @@ __global__ void __launch_bounds__(128) k_trace_tpi(SchurArgs g) {
                             if (a == b) t = Ops::add(t, X[a][b]);
                             if (DERIV && m > 0) t2 = Ops::fma(Ops::add(M[a][b], M[a][b]), entry(2, b, a), t2);
                         }
-                    acc1 += Ops::re(t);
+                    acc1.add(Ops::cre(t));
                     if (DERIV) {
 #pragma unroll
                         for (int a = 0; a < D; a++)
 #pragma unroll
                             for (int b = 0; b < D; b++) t2 = Ops::fma(X[a][b], X[b][a], t2);
-                        acc2 -= Ops::re(Ops::add(t2, sw2));
+                        acc2.add(Ops::rneg(Ops::cre(Ops::add(t2, sw2))));
                     }
                 }
             }
-            if (m > 0) acc1 += Ops::re(sw);
+            if (m > 0) acc1.add(Ops::cre(sw));
             // - Tr G0 = - sum_j Re 1/(z - e0_j) (and + sum_j Re 1/(z - e0_j)^2)
             for (int j = 0; j < n; j++) {
                 const R x = e0[j], d = Ops::rfma(x, x, w2);
-                fr.add(Ops::rneg(x), d);
-                if (DERIV) {
-                    const C r = Ops::pscale(Ops::mk(x, Ops::rneg(wr)), Ops::rrcp(d));
-                    acc2 += Ops::re(Ops::mul(r, r));
+                if (DERIV) {  // x / (x^2 + w^2) and (x^2 - w^2) / (x^2 + w^2)^2
+                    const R ri = Ops::rrcp(d), xr = Ops::rmul(x, ri), yr = Ops::rmul(wr, ri);
+                    acc1.add(Ops::rneg(xr));
+                    acc2.add(Ops::rmul(Ops::rsub(xr, yr), Ops::radd(xr, yr)));
+                } else {
+                    fr.add(Ops::rneg(x), d);
                 }
             }
             fr.end_point(acc1);
+            acc1.end_point();
+            if (DERIV) acc2.end_point();
         }
     }
-    acc1 += fr.value();
+    const double s1 = acc1.value() + fr.value(), s2 = acc2.value();
     if (sing && fvalid) dg_flag(g.status, DG_SINGULAR);
-    if (fvalid) g.ptr[(size_t)chunk * g.nf2 + f] = cmk(acc1, acc2);
+    if (fvalid) g.ptr[(size_t)chunk * g.nf2 + f] = cmk(s1, s2);
 }
 
 // shared-memory bytes of one k_schur launch
