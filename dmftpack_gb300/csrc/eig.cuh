@@ -89,6 +89,18 @@ template <class Ops>
 __host__ __device__ constexpr size_t eig_bytes(int n) {
     return ((size_t)2 * n * n * 16 + EIG_NMAX * 12 + EIG_NMAX / 2 * sizeof(JRot<Ops>) + 64 + 15) & ~(size_t)15;
 }
+// The place of value i in ascending order, equal values by their index and NaN after every number (NaN, as it is in an input,
+// fails every plain comparison): over i always a permutation, whatever is in w, for the vectors are addressed through it.
+__host__ __device__ inline int eig_rank(const double *w, int n, int i) {
+    const double wi = w[i];
+    const bool nan = wi != wi;
+    int rank = 0;
+    for (int j = 0; j < n; j++) {
+        const double wj = w[j];
+        rank += nan ? (wj == wj || j < i) : (wj < wi || (wj == wi && j < i));
+    }
+    return rank;
+}
 template <int T>
 __device__ __forceinline__ void eig_sync() {
     if constexpr (T == 32) __syncwarp();
@@ -214,12 +226,7 @@ __device__ int group_heig(int n, const EigMem<Ops> &e, typename Ops::M tol, int 
     }
     for (int i = tid; i < n; i += T) e.w[i] = Ops::re(a[i + i * n]);
     eig_sync<T>();
-    for (int i = tid; i < n; i += T) {
-        const double wi = e.w[i];
-        int rank = 0;
-        for (int j = 0; j < n; j++) rank += e.w[j] < wi || (e.w[j] == wi && j < i);
-        e.order[rank] = i;
-    }
+    for (int i = tid; i < n; i += T) e.order[eig_rank(e.w, n, i)] = i;
     eig_sync<T>();
     return st;
 }
