@@ -26,6 +26,12 @@ int dg_fail(dmftgpu_ctx *ctx, int code, const char *msg) {
     return code;
 }
 
+void dg_drop_graph(dmftgpu_ctx *ctx) {
+    if (ctx->graph) cudaGraphExecDestroy(ctx->graph);
+    ctx->graph = nullptr;
+    ctx->graph_key.clear();
+}
+
 void *dg_buf(dmftgpu_ctx *ctx, const char *name, size_t bytes) {
     if (bytes == 0) bytes = 16;
     auto &b = ctx->bufs[ctx->buf_ns.empty() ? std::string(name) : ctx->buf_ns + name];
@@ -40,6 +46,8 @@ void *dg_buf(dmftgpu_ctx *ctx, const char *name, size_t bytes) {
             cudaFree(b.p);
             b.p = nullptr;
             b.bytes = 0;
+            // a kept batched graph has the addresses of the batch's workspaces (the ones with a namespace) in it
+            if (!ctx->buf_ns.empty()) dg_drop_graph(ctx);
         }
         size_t want = bytes + bytes / 8;
         cudaError_t e = cudaMalloc(&b.p, want);

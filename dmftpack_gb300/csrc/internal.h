@@ -107,6 +107,8 @@ int dg_set_cuda_error(dmftgpu_ctx *ctx, cudaError_t e, const char *what);
 int dg_fail(dmftgpu_ctx *ctx, int code, const char *msg);
 // device workspace `name` of at least `bytes` (contents undefined); nullptr + error text on failure
 void *dg_buf(dmftgpu_ctx *ctx, const char *name, size_t bytes);
+// forget the kept graph of a batched pass: the next DMFTGPU_GRAPH call warms up again
+void dg_drop_graph(dmftgpu_ctx *ctx);
 // checks the last launch, counts it
 int dg_launched(dmftgpu_ctx *ctx, const char *what);
 // zero the status word, read it back (synchronising the stream)

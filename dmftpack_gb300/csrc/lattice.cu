@@ -1362,13 +1362,12 @@ int dmftgpu_greenftn_w_batched(dmftgpu_ctx *ctx, int nprob, const dmftgpu_lattic
             cudaGraph_t graph = nullptr;
             ctx->capturing = false;
             cudaError_t e = cudaStreamEndCapture(origin, &graph);
+            dg_drop_graph(ctx);  // a capture that fails is not tried again before another warm-up call
             if (rc) {
                 if (graph) cudaGraphDestroy(graph);
                 return rc;
             }
             if (e != cudaSuccess) return dg_set_cuda_error(ctx, e, "greenftn_w_batched: capture");
-            if (ctx->graph) cudaGraphExecDestroy(ctx->graph);
-            ctx->graph = nullptr;
             e = cudaGraphInstantiate(&ctx->graph, graph, 0);
             cudaGraphDestroy(graph);
             if (e != cudaSuccess) return dg_set_cuda_error(ctx, e, "greenftn_w_batched: instantiate");

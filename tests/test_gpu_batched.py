@@ -92,3 +92,37 @@ def test_batched_without_gwhf(ctx):
         g, _, n = ctx.GreenFtn_w(p["lat"], p["H"], p["S"], p["mu"])
         assert rel_err(gw[i].transpose(-1, -2).cpu().numpy(), g.cpu().numpy()) < 1e-12
         assert rel_err(nm[i].transpose(-1, -2).cpu().numpy(), n.cpu().numpy()) < 1e-12
+
+
+def test_graph_is_dropped_when_a_larger_batch_moves_its_workspaces(ctx):
+    """A graph holds the addresses of the batch's workspaces.  A larger batch without the graph flag enlarges those of the
+    same names: the graph must not be replayed on the old ones, the smaller batch warms up and captures again."""
+    probs, dev = _problems(ctx, nprob=3)
+    big = []
+    for p in probs:
+        w = p["w"]
+        H = p["H"].repeat(5, 1, 1).contiguous()
+        lat = lib.Lattice(w.n, 5 * w.nk, w.nfreq, w.beta, 1, w.D)
+        big.append(dict(p, lat=lat, H=H, Hcm=H.transpose(-1, -2).contiguous()))
+    import torch
+    out = [[torch.zeros((p["w"].nfreq, p["w"].D, p["w"].D), dtype=torch.complex128, device=dev) for p in probs],
+           [torch.zeros((p["w"].nfreq, p["w"].D, p["w"].D), dtype=torch.complex128, device=dev) for p in probs],
+           [torch.zeros((p["w"].D, p["w"].D), dtype=torch.complex128, device=dev) for p in probs]]
+    args = ([p["lat"] for p in probs], [p["Hcm"] for p in probs], [p["Scm"] for p in probs], [p["mu"] for p in probs], *out)
+    back = lambda ts: [t.transpose(-1, -2).cpu().numpy() for t in ts]
+    c2 = lib.Context(0)
+    try:
+        def launched():
+            n0 = c2.launches()
+            c2.GreenFtn_w_batched(*args, graph=True)
+            return c2.launches() - n0
+        full = launched()
+        assert full > 0 and launched() > 0      # warm-up, capture
+        assert launched() == 0                  # replay
+        _check(ctx, big, _run_batched(c2, big, dev))
+        assert launched() == full               # the graph went with its workspaces: a warm-up call again
+        _check(ctx, probs, [back(t) for t in out])
+        assert launched() > 0 and launched() == 0
+        _check(ctx, probs, [back(t) for t in out])
+    finally:
+        c2.close()
