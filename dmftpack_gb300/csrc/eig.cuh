@@ -1,7 +1,7 @@
 // eig.cuh -- Hermitian eigen-decompositions of the lattice's per-k matrices (n <= 64) in shared memory by groups of T threads
 // (one warp or four per matrix): cyclic Jacobi in round-robin order, n/2 disjoint pairs (p, q) per round, in FP64
 // (Ops = OpsD) or packed double-float on the FP32 pipe (OpsP, the DMFTGPU_MIXED passes).  The lower triangle is read and the
-// diagonal taken real; the rotation is jacobi_rotation's (unitary to rounding, the angle from FP32); it stops when the
+// diagonal taken real; the rotation is jacobi_rotation's (an FP32 angle refined); it stops when the
 // off-diagonal mass is <= tol of the total.
 //
 // A round is two steps: the rotations (one per thread), then A' = J^H A J by the 2 x 2 blocks of pairs i <= j -- rows and
@@ -39,6 +39,15 @@ __device__ __forceinline__ void eig_rotation(JRot<OpsD> &R, double2 apq, double2
     R.s = r.s;
     R.ph = r.ph;
 }
+// jacobi_tan in double-float, r in [0.5, 1.5): the FP32 root and one Newton step
+__host__ __device__ __forceinline__ dfl jacobi_tan(dfl r, dfl d) {
+    const float ax = fabsf(d.h);
+    if (!(ax <= 1e30f)) return {0.f, 0.f};
+    const float slope = ax > 1e9f ? ax : sqrtf(fmaf(d.h, d.h, 4.f * r.h * r.h));
+    const float t = copysignf(fast_div(2.f * r.h, ax + slope), d.h);
+    const dfl g = df_sub(df_mul(df_add(df_mul(r, {t, 0.f}), d), {t, 0.f}), r);
+    return fast_two_sum(t, -g.h * copysignf(fast_div(1.f, slope), d.h));
+}
 __device__ __forceinline__ void eig_rotation(JRot<OpsP> &R, pdf apq, pdf app, pdf aqq) {
     R.on = 0;
     R.c = {1.f, 0.f};
@@ -52,15 +61,10 @@ __device__ __forceinline__ void eig_rotation(JRot<OpsP> &R, pdf apq, pdf app, pd
     const dfl ar = {apq.h.x * sc, apq.l.x * sc}, ai = {apq.h.y * sc, apq.l.y * sc};
     const dfl r2 = df_fma(ai, ai, df_mul(ar, ar));
     const dfl ir = df_rsqrt(r2);
-    const float r = r2.h * ir.h;  // |a_pq| sc
-    const float x = df_sub(OpsP::cre(aqq), OpsP::cre(app)).h * sc, ax = fabsf(x);
-    float t;
-    if (ax > 1e9f) t = __fdividef(r, ax);
-    else t = __fdividef(2.f * r, ax + sqrtf(fmaf(x, x, 4.f * r * r)));
-    if (!(ax < 1e30f)) t = 0.f;
-    if (x < 0.f) t = -t;
-    R.c = df_rsqrt(df_fma({t, 0.f}, {t, 0.f}, {1.f, 0.f}));
-    R.s = df_mul({t, 0.f}, R.c);
+    const dfl r = df_mul(r2, ir);  // |a_pq| sc
+    const dfl d = df_sub(OpsP::cre(aqq), OpsP::cre(app)), t = jacobi_tan(r, {d.h * sc, d.l * sc});
+    R.c = df_rsqrt(df_fma(t, t, {1.f, 0.f}));
+    R.s = df_mul(t, R.c);
     R.ph = OpsP::mk(df_mul(ar, ir), df_mul(ai, ir));
     R.on = 1;
 }

@@ -22,11 +22,31 @@ struct DgRot {
     double2 ph;
 };
 
-// The rotation of the (p, q) plane.  What must hold to rounding is that it is unitary: c^2 + s^2 = 1 and |ph| = 1; the
-// angle only has to be close (each rotation then leaves 1e-6 of a_pq, and the sweeps still end quadratically), so it
-// comes from FP32, and c = (1 + t^2)^-1/2 and ph = a_pq / |a_pq| from one reciprocal-square-root refinement each.  A lone
-// warp's FP64 instruction takes 64 cycles, so the square roots and divisions of the exact angle (seven, ~10 dependent
-// instructions each) were two thirds of a round; this is 24 instructions.
+__host__ __device__ __forceinline__ float fast_div(float a, float b) {
+#ifdef __CUDA_ARCH__
+    return __fdividef(a, b);
+#else
+    return a / b;
+#endif
+}
+// The tangent of the rotation that removes a_pq: the root |t| <= 1 of r t^2 + d t - r = 0 with r = |a_pq| in [1, 3) and d = a_qq -
+// a_pp in the same units.  Found in FP32 and refined by two Newton steps with the residual in FP64 and the slope,
+// +-sqrt(d^2 + 4 r^2), in FP32; each leaves some 1e-7 of the error: 1e-7, 1e-14, rounding.  0 where d is beyond 1e30 r (or not
+// a number).
+__host__ __device__ __forceinline__ double jacobi_tan(double r, double d) {
+    const float x = (float)d, rf = (float)r, ax = fabsf(x);
+    if (!(ax <= 1e30f)) return 0.0;
+    const float slope = ax > 1e9f ? ax : sqrtf(fmaf(x, x, 4.f * rf * rf));
+    const double step = copysignf(fast_div(1.f, slope), x);
+    double t = copysignf(fast_div(2.f * rf, ax + slope), x);
+    t = fma(-step, fma(fma(r, t, d), t, -r), t);
+    return fma(-step, fma(fma(r, t, d), t, -r), t);
+}
+// The rotation of the (p, q) plane: c = (1 + t^2)^-1/2 and ph = a_pq / |a_pq| from one reciprocal-square-root refinement each.  A
+// lone warp's FP64 instruction takes 64 cycles, so the square roots and divisions of the plain formulas (seven, ~10
+// dependent instructions each) were two thirds of a round; this is 32 instructions.  (24 with the angle left at FP32: every
+// rotation then leaves 1e-7 of a_pq, sweeps end up to 1e-14 of the total away in place of rounding, and one in four
+// matrices of 8 x 8 takes another sweep.)
 __device__ __forceinline__ double fast_rsqrt(double x) {  // x in [0.25, 1e30]
     double y;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
@@ -47,15 +67,9 @@ __device__ __forceinline__ DgRot jacobi_rotation(int p, int q, double2 apq, doub
     const double sc = __hiloint2double(0x7fe00000 - ex, 0);
     const double2 z = cscale(apq, sc);
     const double r2 = cabs2(z), inv = fast_rsqrt(r2);
-    const double rr = r2 * inv, d = (aqq - app) * sc;
-    const float x = (float)d, r = (float)rr, ax = fabsf(x);
-    float t;
-    if (ax > 1e9f) t = __fdividef(r, ax);
-    else t = __fdividef(2.f * r, ax + sqrtf(fmaf(x, x, 4.f * r * r)));
-    if (ax > 1e30f) t = 0.f;
-    const double td = x < 0.f ? -(double)t : (double)t;
-    R.c = fast_rsqrt(fma(td, td, 1.0));
-    R.s = td * R.c;
+    const double t = jacobi_tan(r2 * inv, (aqq - app) * sc);
+    R.c = fast_rsqrt(fma(t, t, 1.0));
+    R.s = t * R.c;
     R.ph = cscale(z, inv);
     R.on = 1;
     return R;

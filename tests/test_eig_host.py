@@ -43,3 +43,29 @@ def test_order_of_eigenvalues_is_a_permutation(harness):
         rank = np.array([int(x) for x in r])
         assert sorted(rank) == list(range(len(w)))
         assert np.array_equal(np.array(w)[np.argsort(rank)], np.sort(w), equal_nan=True)
+
+
+@pytest.mark.parametrize("op,lo,bound", [("tan", 1.0, 2.0 ** -50), ("tandf", 0.5, 2.0 ** -44)])
+def test_rotation_angle(harness, op, lo, bound):
+    """The rotation's tangent against r t^2 + d t - r = 0 solved in 60 digits: an eigenvector is as good as its last
+    rotations, so the angle is rounding in its own arithmetic (FP64: two Newton steps end at a residual of some 3 roundings
+    of r over a slope >= 2 r; double-float: one step from 2^-23 leaves 2^-46 and its operations 2^-45)."""
+    from decimal import Decimal as Dc, getcontext
+    getcontext().prec = 60
+    rng = np.random.default_rng(11)
+    cases = []
+    for i in range(600):
+        r = rng.uniform(lo, 1.4 * 2 * lo)
+        d = float(np.exp(rng.uniform(-40, 30)) * rng.choice([-1, 1])) if i % 3 else float(rng.normal() * r)
+        if op == "tandf":
+            r, d = [(float(np.float32(x)), float(np.float32(x - float(np.float32(x))))) for x in (r, d)]
+            cases.append((r[0], r[1], d[0], d[1]))
+        else:
+            cases.append((r, d))
+    cases.append((1.25, 0.0) if op == "tan" else (1.25, 0.0, 0.0, 0.0))
+    out = harness(["%s %s\n" % (op, " ".join(x.hex() for x in c)) for c in cases])
+    for c, o in zip(cases, out):
+        r, d = (Dc(c[0]), Dc(c[1])) if op == "tan" else (Dc(c[0]) + Dc(c[1]), Dc(c[2]) + Dc(c[3]))
+        t = sum((Dc(float.fromhex(x)) for x in o), Dc(0))
+        exact = 2 * r / (abs(d) + (d * d + 4 * r * r).sqrt()) * (1 if d >= 0 else -1)
+        assert abs(t - exact) <= Dc(bound) * abs(exact)
