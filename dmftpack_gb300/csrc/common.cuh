@@ -67,3 +67,18 @@ __device__ __forceinline__ void dg_flag(int *status, int code) {
     } while (0)
 
 static inline int dg_ceil_div(long long a, long long b) { return (int)((a + b - 1) / b); }
+
+// `bytes` of dynamic shared memory for a kernel that shares SMs with kernels of another stream (the static eigen-decomposition
+// runs beside the Schur data and the lattice kernels), with the same carve-out, the largest, for all of them: an SM changes
+// its split between L1 and shared memory only when it is empty, so kernels of different splits wait for one another or run with
+// the blocks that fit the other's.  Left to the driver, the same call took 0.90 or 2.03 ms (G_loc in FP64, 4 + 8 orbitals,
+// 216 k x 512 points), 0.80 or 1.86 (densities, 3 + 8), 6.6 or 11.4 (G_loc, 6 + 36), whichever kernel came first.
+// tight: the smallest carve-out that holds the block, for the tensor-core kernels, whose block fills an SM and which read
+// z - Sigma of their frequencies through L1 (in the largest one G_loc at D = 10, 216 k x 512 points, takes 0.56 ms, not 0.51).
+template <class K>
+inline cudaError_t dg_smem_attr(K kernel, size_t bytes, bool tight = false) {
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e != cudaSuccess) return e;
+    const int sm = 228 * 1024, percent = tight ? (int)((bytes + 1024) * 100 / sm) : (int)cudaSharedmemCarveoutMaxShared;
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, percent);
+}

@@ -1008,7 +1008,7 @@ int launch_lat(dmftgpu_ctx *ctx, const LatTcArgs &a, bool *ready, double *tr, do
         k_tc_zsig<DP><<<zblocks, 256, 0, ctx->stream>>>(a.nf2, a.D, a.wgrid, a.beta, a.mu, a.m0, 0, zs0);
         DG_LAUNCH(ctx, "k_tc_zsig");
     }
-    DG_CUDA(cudaFuncSetAttribute(k_lat_tc<DP, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, T::SMEM));
+    DG_CUDA((dg_smem_attr(k_lat_tc<DP, MODE>, T::SMEM, true)));
     g.a = a;
     g.Bimg = Bimg;
     g.colscale = col;
@@ -1065,7 +1065,7 @@ int launch_block(dmftgpu_ctx *ctx, const LatTcArgs &a, double2 *blk, double2 *bl
         g.pblk0 = p0;
         g.status = ctx->d_status;
         using S = T0<DP>;
-        DG_CUDA(cudaFuncSetAttribute(k_g0_tc<DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::SMEM));
+        DG_CUDA(dg_smem_attr(k_g0_tc<DP>, S::SMEM, true));
         {
             DgTimer tm(ctx, "k_g0_tc");
             k_g0_tc<DP><<<dim3(fblocks0, n0), G0T, S::SMEM, ctx->stream>>>(g);

@@ -201,7 +201,7 @@ template <class Ops, int T>
 int launch_static_eig_t(dmftgpu_ctx *ctx, cudaStream_t s, int nk, int n, int D, int nh, int mask, const double2 *H,
                         const double2 *m0, double *eps, double2 *UP, double2 *Uf) {
     const size_t sm = EIG_PER_CTA<T> * eig_bytes<Ops>(n);
-    DG_CUDA(cudaFuncSetAttribute(k_static_eig<Ops, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    DG_CUDA((dg_smem_attr(k_static_eig<Ops, T>, sm)));
     k_static_eig<Ops, T><<<dg_ceil_div(nk, EIG_PER_CTA<T>), T * EIG_PER_CTA<T>, sm, s>>>(nk, n, D, nh, mask, H, m0, eps, UP, Uf,
                                                                                          ctx->d_status);
     DG_LAUNCH(ctx, "k_static_eig");
@@ -217,7 +217,7 @@ template <class Ops, int T>
 int launch_schur_prep_t(dmftgpu_ctx *ctx, cudaStream_t s, int nk, int n, int D, const double2 *H, double *epsQ, double2 *B,
                         double2 *Vq) {
     const size_t sm = EIG_PER_CTA<T> * eig_bytes<Ops>(n - D);
-    DG_CUDA(cudaFuncSetAttribute(k_schur_prep<Ops, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    DG_CUDA((dg_smem_attr(k_schur_prep<Ops, T>, sm)));
     k_schur_prep<Ops, T><<<dg_ceil_div(nk, EIG_PER_CTA<T>), T * EIG_PER_CTA<T>, sm, s>>>(nk, n, D, H, epsQ, B, Vq, ctx->d_status);
     DG_LAUNCH(ctx, "k_schur_prep");
     return DMFTGPU_OK;
@@ -556,7 +556,7 @@ int run_gloc(dmftgpu_ctx *ctx, const Prepared &P, int mode, double mu, int wgrid
     while (fpb > 1 && smem_for(fpb) > 160 * 1024) fpb--;
     size_t smem = smem_for(fpb);
     if (smem > 200 * 1024) return dg_fail(ctx, DMFTGPU_BADARG, "lattice: correlated block too large");
-    DG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    DG_CUDA(dg_smem_attr(kern, smem));
     GlocArgs g;
     g.H = P.H;
     g.sig = P.sig;
@@ -648,7 +648,7 @@ int run_tiles(dmftgpu_ctx *ctx, const Prepared &P, bool trace, double mu, int wg
     int lanes = 0;
     dg::AdKernel kern = dg::ad_kernel(P.D, mode, &lanes);
     const AdShape sh = ad_shape(ctx, P, mode, lanes, nf2);
-    DG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh.smem));
+    DG_CUDA(dg_smem_attr(kern, sh.smem));
     dg::AdArgs g = {};
     if (trace) {
         g.pout0 = (double2 *)dg_buf(ctx, "schur.ptr", (size_t)sh.nchunk * nf2 * sizeof(double2));
@@ -719,7 +719,7 @@ int run_schur(dmftgpu_ctx *ctx, const Prepared &P, int mode, double mu, int wgri
     while (kc > 1 && smem_of(kc) > cap) kc /= 2;
     const size_t smem = smem_of(kc);
     if (smem > 200 * 1024) return dg_fail(ctx, DMFTGPU_BADARG, "lattice: correlated block too large");
-    DG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    DG_CUDA(dg_smem_attr(kern, smem));
     // k chunks: enough CTAs for `cps` per SM (unless tuned 8, and 24 where three are resident: with 8 the last two of an SM
     // run without a third; t2g + p, 13,824 k: 24.4 -> 23.7 ms), at least 8 k points per chunk (below that a CTA's setup
     // and the partial sums cost more than the idle SMs; with 64 a 484-k, 800-point pass ran 56 CTAs on 152 SMs)
@@ -932,7 +932,7 @@ int run_ad(dmftgpu_ctx *ctx, const Prepared &P, int mode, double mu, const doubl
     if (!kern) return dg_fail(ctx, DMFTGPU_BADARG, "derivatives: correlated block larger than 20");
     const int m = P.n - P.D, nf = P.Nf, DD = P.D * P.D;
     const AdShape sh = ad_shape(ctx, P, mode, lanes, nf);
-    DG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh.smem));
+    DG_CUDA(dg_smem_attr(kern, sh.smem));
     const int nchunk = sh.nchunk;
     double2 *pout = (double2 *)dg_buf(ctx, "ad.pout", (size_t)nchunk * nf * DD * sizeof(double2));
     double *pmu = (double *)dg_buf(ctx, "ad.pmu", (size_t)nchunk * nf * sizeof(double));
@@ -1131,14 +1131,14 @@ int run_density(dmftgpu_ctx *ctx, const Prepared &P, double mu, double2 *dens, b
     g.Y = Y;
     g.R = R;
     g.status = ctx->d_status;
-    DG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    DG_CUDA(dg_smem_attr(kern, smem));
     {
         DgTimer tm(ctx, "k_dens_sum");
         kern<<<dim3(nk, nsplit), ng * W, smem, ctx->stream>>>(g);
     }
     DG_LAUNCH(ctx, "k_dens_sum");
     const size_t fs = 2 * (size_t)n * n * sizeof(double2) + n * sizeof(double);
-    DG_CUDA(cudaFuncSetAttribute(k_dens_finish, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fs));
+    DG_CUDA(dg_smem_attr(k_dens_finish, fs));
     k_dens_finish<<<nk, 128, fs, ctx->stream>>>(nk, n, D, nsplit, P.beta, mu, Y, R, P.Vq, P.Uf, P.eps, P.perm, dens);
     DG_LAUNCH(ctx, "k_dens_finish");
     return DMFTGPU_OK;
