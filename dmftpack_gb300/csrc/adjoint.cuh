@@ -209,8 +209,9 @@ __global__ void __launch_bounds__(AD_THREADS, 2) k_gloc_ad(AdArgs g) {
             }
         }
         __syncthreads();
+        double tk = 0.0;  // this k point's terms of accmu
         if (MODE == AD_TRACE)
-            for (int l = lane; l < m; l += LW) accmu += sW[(size_t)grp * ws + 2 * l].x;
+            for (int l = lane; l < m; l += LW) tk += sW[(size_t)grp * ws + 2 * l].x;
         // M = z - H_PP - Sigma - S into the first tile; into the second JVP: Sigma_dot - mu_dot S', BLOCK: M with m0 in the place of
         // Sigma, TRACE: S', transposed
         for (int t = threadIdx.x; t < npair * nsub; t += blockDim.x) {
@@ -281,7 +282,8 @@ __global__ void __launch_bounds__(AD_THREADS, 2) k_gloc_ad(AdArgs g) {
                 }
             }
         } else if (MODE == AD_TRACE) {
-            for (int e = lane; e < DD; e += LW) accmu = fma(A[e].x, V[e].x, fma(-A[e].y, V[e].y, accmu));  // G(r,c) S'(c,r)
+            for (int e = lane; e < DD; e += LW) tk = fma(A[e].x, V[e].x, fma(-A[e].y, V[e].y, tk));  // G(r,c) S'(c,r)
+            accmu += tk;
         } else if constexpr (MODE == AD_JVP) {
             // elements e = r + D c: X G, then G (X G)
             C v[AD_EL];
@@ -365,7 +367,8 @@ __global__ void __launch_bounds__(AD_THREADS, 2) k_gloc_ad(AdArgs g) {
                 }
             }
             __syncthreads();
-            for (int e = lane; e < DD; e += LW) accmu = fma(A[e].x, V[e].x, fma(A[e].y, V[e].y, accmu));
+            for (int e = lane; e < DD; e += LW) tk = fma(A[e].x, V[e].x, fma(A[e].y, V[e].y, tk));
+            accmu += tk;
         }
     }
     if (sing) dg_flag(g.status, DG_SINGULAR);

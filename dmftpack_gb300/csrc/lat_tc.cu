@@ -942,8 +942,7 @@ __global__ void k_tc_reduce_trace(int nchunk, int nf2, const double2 *__restrict
                                   double *__restrict__ dtr) {
     const int f = blockIdx.x * blockDim.x + threadIdx.x;
     if (f >= nf2) return;
-    double2 s = cmk(0, 0);
-    for (int q = 0; q < nchunk; q++) s = cadd(s, ptr[(size_t)q * nf2 + f]);
+    const double2 s = chunk_sum(nchunk, [&](int q) { return ptr[(size_t)q * nf2 + f]; });
     tr[f] = s.x;
     if (dtr) dtr[f] = s.y;
 }
@@ -951,11 +950,8 @@ __global__ void k_tc_reduce_block(int n1, int n0, long long len, const double2 *
                                   const double2 *__restrict__ p0, double2 *__restrict__ blk, double2 *__restrict__ blk0) {
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= len) return;
-    double2 s = cmk(0, 0), s0 = cmk(0, 0);
-    for (int q = 0; q < n1; q++) s = cadd(s, p1[(size_t)q * len + t]);
-    for (int q = 0; q < n0; q++) s0 = cadd(s0, p0[(size_t)q * len + t]);
-    blk[t] = s;
-    blk0[t] = s0;
+    const double2 *p = blockIdx.y ? p0 : p1;
+    (blockIdx.y ? blk0 : blk)[t] = chunk_sum(blockIdx.y ? n0 : n1, [&](int q) { return p[(size_t)q * len + t]; });
 }
 
 int sm_count(dmftgpu_ctx *ctx) {
@@ -1072,7 +1068,7 @@ int launch_block(dmftgpu_ctx *ctx, const LatTcArgs &a, double2 *blk, double2 *bl
         }
         DG_LAUNCH(ctx, "k_g0_tc");
     }
-    k_tc_reduce_block<<<rblocks, 256, 0, ctx->stream>>>(n1, n0, len, p1, p0, blk, blk0);
+    k_tc_reduce_block<<<dim3(rblocks, 2), 256, 0, ctx->stream>>>(n1, n0, len, p1, p0, blk, blk0);
     DG_LAUNCH(ctx, "k_tc_reduce_block");
     return DMFTGPU_OK;
 }

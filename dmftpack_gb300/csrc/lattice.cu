@@ -587,27 +587,18 @@ int run_gloc(dmftgpu_ctx *ctx, const Prepared &P, int mode, double mu, int wgrid
 }
 
 
-// fixed-order sum of the per-chunk partial sums
+// fixed-order sums of the per-chunk partial sums; grid y: G (and the traces), G0
 __global__ void k_schur_reduce(int nchunk, int nf2, int DD, int mode, const double2 *pblk, const double2 *pblk0,
                                const double2 *ptr, double2 *blk, double2 *blk0, double *tr, double *dtr) {
     long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if ((mode & dg::S_BLOCK) && t < (long long)nf2 * DD) {
-        double2 s = cmk(0, 0), s0 = cmk(0, 0);
-        for (int q = 0; q < nchunk; q++) {
-            s = cadd(s, pblk[(size_t)q * nf2 * DD + t]);
-            s0 = cadd(s0, pblk0[(size_t)q * nf2 * DD + t]);
-        }
-        blk[t] = s;
-        if (blk0) blk0[t] = s0;
+        const double2 *p = blockIdx.y ? pblk0 : pblk;
+        (blockIdx.y ? blk0 : blk)[t] = chunk_sum(nchunk, [&](int q) { return p[(size_t)q * nf2 * DD + t]; });
     }
-    if ((mode & dg::S_TRACE) && t < nf2) {
-        double a = 0, b = 0;
-        for (int q = 0; q < nchunk; q++) {
-            a += ptr[(size_t)q * nf2 + t].x;
-            b += ptr[(size_t)q * nf2 + t].y;
-        }
-        tr[t] = a;
-        if (dtr) dtr[t] = b;
+    if ((mode & dg::S_TRACE) && blockIdx.y == 0 && t < nf2) {
+        const double2 s = chunk_sum(nchunk, [&](int q) { return ptr[(size_t)q * nf2 + t]; });
+        tr[t] = s.x;
+        if (dtr) dtr[t] = s.y;
     }
 }
 
@@ -624,14 +615,16 @@ AdShape ad_shape(dmftgpu_ctx *ctx, const Prepared &P, int mode, int lanes, int n
     while (s.F > step && dg::ad_smem(s.F, P.D, m, mode) > 113 * 1024) s.F -= step;
     s.smem = dg::ad_smem(s.F, P.D, m, mode);
     s.fblocks = dg_ceil_div(nf, s.F);
-    // k points per CTA: the fewest rounds of CTAs x (their k points and a little for their start), at most eight rounds
+    // k points per CTA: the fewest rounds of CTAs x (their k points and a little for their start), at most eight rounds; of 64 k at
+    // most where four rounds of chunks reach that, for a chunk's running sums lose digits with its length
     int nsm = 152;
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, ctx->device);
-    const int slots = 2 * nsm;
+    const int slots = 2 * nsm, least = std::min(dg_ceil_div(P.nk, 64), std::max(1, 4 * slots / s.fblocks));
     s.kchunk = P.nk;
     double best = 1e300;
     for (int r = 1; r <= 8; r++) {
-        const int nc = (int)std::max(1LL, std::min((long long)P.nk, (long long)r * slots / s.fblocks)), kch = dg_ceil_div(P.nk, nc);
+        const int nc = (int)std::max((long long)least, std::min((long long)P.nk, (long long)r * slots / s.fblocks)),
+                  kch = dg_ceil_div(P.nk, nc);
         const double cost = dg_ceil_div((long long)s.fblocks * dg_ceil_div(P.nk, kch), slots) * (kch + 0.3);
         if (cost < best) {
             best = cost;
@@ -682,7 +675,7 @@ int run_tiles(dmftgpu_ctx *ctx, const Prepared &P, bool trace, double mu, int wg
     }
     DG_LAUNCH(ctx, "k_gloc_ad");
     const long long nred = trace ? nf2 : (long long)nf2 * DD;
-    k_schur_reduce<<<dg_ceil_div(nred, 256), 256, 0, ctx->stream>>>(sh.nchunk, nf2, DD, trace ? dg::S_TRACE : dg::S_BLOCK, g.pout,
+    k_schur_reduce<<<dim3(dg_ceil_div(nred, 256), trace ? 1 : 2), 256, 0, ctx->stream>>>(sh.nchunk, nf2, DD, trace ? dg::S_TRACE : dg::S_BLOCK, g.pout,
                                                                     g.pout0, g.pout0, blk, blk0, tr, nullptr);
     DG_LAUNCH(ctx, "k_schur_reduce");
     return DMFTGPU_OK;
@@ -820,8 +813,8 @@ int run_schur(dmftgpu_ctx *ctx, const Prepared &P, int mode, double mu, int wgri
     }
     DG_LAUNCH(ctx, "k_schur");
     const long long nred = (mode & dg::S_BLOCK) ? std::max((long long)nf2 * DD, (long long)nf2) : nf2;
-    k_schur_reduce<<<dg_ceil_div(nred, 256), 256, 0, ctx->stream>>>(nchunk, nf2, DD, mode, pblk, pblk0, ptr, blk, blk0,
-                                                                     tr, dtr);
+    k_schur_reduce<<<dim3(dg_ceil_div(nred, 256), (mode & dg::S_BLOCK) && blk0 ? 2 : 1), 256, 0, ctx->stream>>>(
+        nchunk, nf2, DD, mode, pblk, pblk0, ptr, blk, blk0, tr, dtr);
     DG_LAUNCH(ctx, "k_schur_reduce");
     return DMFTGPU_OK;
 }
@@ -906,9 +899,7 @@ int check_lat(const dmftgpu_lattice *L) {
 __global__ void k_ad_reduce(int nchunk, long long len, double scale, const double2 *p, double2 *out) {
     long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= len) return;
-    double2 s = cmk(0, 0);
-    for (int q = 0; q < nchunk; q++) s = cadd(s, p[(size_t)q * len + t]);
-    out[t] = cscale(s, scale);
+    out[t] = cscale(chunk_sum(nchunk, [&](int q) { return p[(size_t)q * len + t]; }), scale);
 }
 __global__ void k_ad_mu(int n, double scale, const double *p, double *out) {
     __shared__ double red[256];

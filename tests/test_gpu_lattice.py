@@ -458,3 +458,22 @@ def test_two_orbital_closed_forms(ctx, orc, n, nk, nf):
                 assert rel_err(g, w) < tol
             g, dg = ctx.GiwToNele(lat, H, S, mu, deriv=True, mixed=mixed)
             assert abs(g - N) <= tol * max(1, abs(N)) and abs(dg - dN) <= 10 * tol * max(1, abs(dN))
+
+
+@pytest.mark.parametrize("D", [1, 4, 6])
+def test_k_sum_keeps_its_digits(ctx, D):
+    """20,000 k points and 32 frequencies: the sum is split into some thousand chunks, which one running sum would add up with
+    an error of 12 u (u = 2^-53; u/sqrt(3) per addition, of a partial sum of 0.58 of the total, sqrt(1,216) of them).  The
+    blocks of 64 make it 1.5 u; the bound is three times that.  Diagonal H, so that the sums are of scalars (long double)."""
+    rng = np.random.default_rng(D)
+    nk, nf, beta, mu = 20000, 16, 20.0, 0.2
+    e = rng.normal(size=(nk, D))
+    H = np.zeros((nk, D, D), complex)
+    H[:, range(D), range(D)] = e
+    w = np.pi * (2 * np.arange(nf) + 1) / beta
+    S = (-0.5j / (w + 1.0))[:, None, None] * np.eye(D)
+    G = ctx.GreenFtn_w(lib.Lattice(D, nk, nf, beta, 1, D), H, S, mu)[0]
+    z = (np.longdouble(mu) - e)[:, :, None] + np.clongdouble(1j) * (w + 0.5 / (w + 1.0)).astype(np.longdouble)
+    exact = (1 / z).sum(0) / nk                                        # [D][nf]
+    err = np.array([G[:, a, a] - exact[a] for a in range(D)])
+    assert np.sqrt((abs(err) ** 2).sum() / (abs(exact) ** 2).sum()) < 4.5 * 2.0 ** -53
