@@ -107,7 +107,7 @@ __device__ __forceinline__ bool tile_inverse(double2 *A, int D, double2 *rowb, d
         }
         const double2 piv = A[k + k * D];
         const double den = fma(piv.x, piv.x, piv.y * piv.y);
-        sing |= !(den > 0.0);
+        sing |= (unsigned)__double2hiint(den) - 1u >= 0x7fefffffu;  // zero, infinite or NaN
         const double q = 1.0 / den;
         const double2 ip = cmk(piv.x * q, -piv.y * q);
         for (int c = g; c < D; c += LW) {

@@ -35,3 +35,17 @@ def test_nan_is_refused(ctx, n, D, mixed):
         with pytest.raises(lib.DmftGpuError):
             ctx.GreenFtn_w_vjp(lat, h, s, 0.1, S)
     assert rel_err(ctx.GreenFtn_w(lat, H, S, 0.1, mixed=mixed)[0], good) == 0.0
+
+
+@pytest.mark.parametrize("n,D", [(1, 1), (5, 3), (12, 8), (20, 20)])
+def test_derivatives_refuse_an_infinite_self_energy(ctx, n, D):
+    """An infinite last pivot: |pivot|^2 is not zero, but there is no inverse."""
+    lat, H, S = _problem(n, D)
+    bad = S.copy()
+    bad[3, D - 1, D - 1] = np.inf
+    good = ctx.GreenFtn_w_jvp(lat, H, S, 0.1, S, 0.2)
+    with pytest.raises(lib.DmftGpuError):
+        ctx.GreenFtn_w_jvp(lat, H, bad, 0.1, S, 0.2)
+    with pytest.raises(lib.DmftGpuError):
+        ctx.GreenFtn_w_vjp(lat, H, bad, 0.1, S)
+    assert rel_err(ctx.GreenFtn_w_jvp(lat, H, S, 0.1, S, 0.2), good) == 0.0
