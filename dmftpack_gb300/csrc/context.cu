@@ -32,23 +32,33 @@ void dg_drop_graph(dmftgpu_ctx *ctx) {
     ctx->graph_key.clear();
 }
 
+static void release(dmftgpu_ctx *ctx, dmftgpu_ctx::Buf &b) {
+    if (!b.p) return;
+    cudaStreamSynchronize(ctx->stream);
+    if (ctx->side) cudaStreamSynchronize(ctx->side);
+    cudaFree(b.p);
+    b.p = nullptr;
+    b.bytes = 0;
+    // a kept batched graph has the addresses of the batch's workspaces (the ones with a namespace) in it
+    if (!ctx->buf_ns.empty()) dg_drop_graph(ctx);
+}
+static dmftgpu_ctx::Buf &workspace(dmftgpu_ctx *ctx, const char *name) {
+    return ctx->bufs[ctx->buf_ns.empty() ? std::string(name) : ctx->buf_ns + name];
+}
+
+void dg_release(dmftgpu_ctx *ctx, const char *name) {
+    if (!ctx->capturing) release(ctx, workspace(ctx, name));
+}
+
 void *dg_buf(dmftgpu_ctx *ctx, const char *name, size_t bytes) {
     if (bytes == 0) bytes = 16;
-    auto &b = ctx->bufs[ctx->buf_ns.empty() ? std::string(name) : ctx->buf_ns + name];
+    auto &b = workspace(ctx, name);
     if (b.bytes < bytes && ctx->capturing) {
         dg_fail(ctx, DMFTGPU_BADARG, "workspace growth during graph capture");
         return nullptr;
     }
     if (b.bytes < bytes) {
-        if (b.p) {
-            cudaStreamSynchronize(ctx->stream);
-            if (ctx->side) cudaStreamSynchronize(ctx->side);
-            cudaFree(b.p);
-            b.p = nullptr;
-            b.bytes = 0;
-            // a kept batched graph has the addresses of the batch's workspaces (the ones with a namespace) in it
-            if (!ctx->buf_ns.empty()) dg_drop_graph(ctx);
-        }
+        release(ctx, b);
         size_t want = bytes + bytes / 8;
         cudaError_t e = cudaMalloc(&b.p, want);
         if (e != cudaSuccess) {

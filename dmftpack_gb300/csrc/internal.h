@@ -18,6 +18,9 @@ struct DgPulay {
     std::vector<double> om;
 };
 
+// operand images of the tensor-core lattice passes: the most one call (a batch is one) may hold
+constexpr size_t DG_IMAGE_BYTES = (size_t)64 << 30;
+
 struct dmftgpu_ctx {
     int device = 0;
     cudaStream_t stream = nullptr;
@@ -56,6 +59,7 @@ struct dmftgpu_ctx {
     size_t pinned_bytes = 0;
     std::string hk_phase_key;         // (k mesh, R list) of the phase-slice image in workspace "hk.tc.A"
     bool tensor = true;               // tensor-core contractions allowed in the mixed form (!DMFTGPU_NO_TENSOR)
+    size_t image_left = DG_IMAGE_BYTES; // what the tensor-core lattice passes of this call may still take for operand images
     int nk_krylov = 0;                // Jacobian-vector products of the last Newton-Krylov mixer step (0: none)
     double nk_relres = 0.0;           // its linear solve's relative residual
     double mix_resid = 0.0;           // |SE_out - SelfEnergy_w| / |SelfEnergy_w| of the last DMFT iteration
@@ -67,6 +71,13 @@ struct DgTensorMode {
     bool saved;
     DgTensorMode(dmftgpu_ctx *c, int flags) : ctx(c), saved(c->tensor) { ctx->tensor = !(flags & DMFTGPU_NO_TENSOR); }
     ~DgTensorMode() { ctx->tensor = saved; }
+};
+
+// the operand images of a batch count together: each problem has its own (dg_lat_tc_reserve)
+struct DgImageShare {
+    dmftgpu_ctx *ctx;
+    explicit DgImageShare(dmftgpu_ctx *c) : ctx(c) { ctx->image_left = DG_IMAGE_BYTES; }
+    ~DgImageShare() { ctx->image_left = DG_IMAGE_BYTES; }
 };
 
 // sets ctx->ft_direct and ctx->imp_mixed from a call's flags for the call's duration
@@ -107,6 +118,8 @@ int dg_set_cuda_error(dmftgpu_ctx *ctx, cudaError_t e, const char *what);
 int dg_fail(dmftgpu_ctx *ctx, int code, const char *msg);
 // device workspace `name` of at least `bytes` (contents undefined); nullptr + error text on failure
 void *dg_buf(dmftgpu_ctx *ctx, const char *name, size_t bytes);
+// give the workspace `name` back to the device
+void dg_release(dmftgpu_ctx *ctx, const char *name);
 // forget the kept graph of a batched pass: the next DMFTGPU_GRAPH call warms up again
 void dg_drop_graph(dmftgpu_ctx *ctx);
 // checks the last launch, counts it

@@ -1094,26 +1094,43 @@ int launch_trace(dmftgpu_ctx *ctx, const LatTcArgs &a, bool *ready, double *tr, 
 //           D = 10  6.46 / 7.24  10.1 / 7.30
 // The lines below are where these cross.  At D = 4 N(mu) takes k_schur 0.45 (m = 0) and 1.96 (m = 10) and 1.77 and 2.33
 // here at 1,024 frequencies: they cross only past 16 poles.
-// And the images, 43 KB per k point at D = 10 (G_loc: two), stay within 64 GB; k_schur needs none.
-static bool covered(int n, int D, int nk, int least, int images) {
-    const size_t image = (size_t)NSB * KSTEPS * np_of((D + 1) / 2 * 2) * 16 * 2;
-    return D >= 5 && D <= 10 && n - D >= least && n - D <= KP && n <= NE0 && image * images * nk <= (size_t)64 << 30;
-}
-bool dg_lat_tc_supported(int n, int D, int nk) { return covered(n, D, nk, 4, 1); }
-bool dg_lat_tc_deriv_supported(int n, int D, int nk) { return covered(n, D, nk, 2, 1); }
-bool dg_lat_tc_block_supported(int n, int D, int nk) {
-    return covered(n, D, nk, D <= 6 ? 4 : (D <= 8 ? 2 : 0), 2) && (D <= 6 || n <= KP);
+static bool covered(int n, int D, int least) { return D >= 5 && D <= 10 && n - D >= least && n - D <= KP && n <= NE0; }
+bool dg_lat_tc_supported(int n, int D) { return covered(n, D, 4); }
+bool dg_lat_tc_deriv_supported(int n, int D) { return covered(n, D, 2); }
+bool dg_lat_tc_block_supported(int n, int D) { return covered(n, D, D <= 6 ? 4 : (D <= 8 ? 2 : 0)) && (D <= 6 || n <= KP); }
+
+// The images, 43 KB per k point at D = 10 and two sets of them in G_loc's pass, are what k_schur does without: they stay
+// within 64 GB in a call, and where they cannot be had at all the pass is k_schur's.
+bool dg_lat_tc_reserve(dmftgpu_ctx *ctx, int n, int D, int nk, bool block) {
+    const size_t np = np_of((D + 1) / 2 * 2), img = (size_t)nk * NSB * KSTEPS * np * 16 * 2, col = (size_t)nk * np * 4;
+    const bool two = block && D > 6;  // with the images of U (launch_block)
+    const size_t need = img * (two ? 2 : 1);
+    if (need > ctx->image_left) return false;
+    const struct {
+        const char *name;
+        size_t bytes;
+    } part[] = {{"tc.B", img}, {"tc.col", col}, {"tc.U", img}, {"tc.ucol", col}};
+    const int parts = two ? 4 : 2;
+    for (int i = 0; i < parts; i++)
+        if (!dg_buf(ctx, part[i].name, part[i].bytes)) {
+            cudaGetLastError();
+            ctx->err.clear();
+            for (int j = 0; j < i; j++) dg_release(ctx, part[j].name);
+            return false;
+        }
+    if (!ctx->buf_ns.empty()) ctx->image_left -= need;
+    return true;
 }
 
 int dg_lat_tc_trace(dmftgpu_ctx *ctx, const LatTcArgs &a, bool *ready, double *tr, double *dtr) {
-    if (!(dtr ? dg_lat_tc_deriv_supported(a.n, a.D, a.nk) : dg_lat_tc_supported(a.n, a.D, a.nk)))
+    if (!(dtr ? dg_lat_tc_deriv_supported(a.n, a.D) : dg_lat_tc_supported(a.n, a.D)))
         return dg_fail(ctx, DMFTGPU_BADARG, "lat_tc: unsupported sizes");
     if (a.D <= 6) return launch_trace<6>(ctx, a, ready, tr, dtr);
     if (a.D <= 8) return launch_trace<8>(ctx, a, ready, tr, dtr);
     return launch_trace<10>(ctx, a, ready, tr, dtr);
 }
 int dg_lat_tc_block(dmftgpu_ctx *ctx, const LatTcArgs &a, double2 *blk, double2 *blk0) {
-    if (!dg_lat_tc_block_supported(a.n, a.D, a.nk)) return dg_fail(ctx, DMFTGPU_BADARG, "lat_tc: unsupported sizes");
+    if (!dg_lat_tc_block_supported(a.n, a.D)) return dg_fail(ctx, DMFTGPU_BADARG, "lat_tc: unsupported sizes");
     if (a.D <= 6) return launch_block<6>(ctx, a, blk, blk0);
     if (a.D <= 8) return launch_block<8>(ctx, a, blk, blk0);
     return launch_block<10>(ctx, a, blk, blk0);

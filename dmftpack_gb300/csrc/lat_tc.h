@@ -18,9 +18,12 @@ struct LatTcArgs {
 };
 
 // true when the N(mu) pass, its derivative, the block pass are the faster form for this lattice (see lat_tc.cu)
-bool dg_lat_tc_supported(int n, int D, int nk);
-bool dg_lat_tc_deriv_supported(int n, int D, int nk);
-bool dg_lat_tc_block_supported(int n, int D, int nk);
+bool dg_lat_tc_supported(int n, int D);
+bool dg_lat_tc_deriv_supported(int n, int D);
+bool dg_lat_tc_block_supported(int n, int D);
+// room for the operand images of a supported pass (block: dg_lat_tc_block); false, with nothing held, where the call's share
+// (ctx->image_left) or the device has no room for them: the caller takes run_schur, which has no images
+bool dg_lat_tc_reserve(dmftgpu_ctx *ctx, int n, int D, int nk, bool block);
 // prepare the per-k operand images once (*ready tracks it for the caller's prepared lattice), then run one pass:
 // tr[f] = sum_k Re[Tr G(k, iw_f) - Tr G0(k, iw_f)] for f < nf2, and with dtr its derivative by mu (device)
 int dg_lat_tc_trace(dmftgpu_ctx *ctx, const LatTcArgs &a, bool *ready, double *tr, double *dtr);

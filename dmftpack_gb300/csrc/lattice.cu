@@ -860,7 +860,8 @@ int nele_pass(dmftgpu_ctx *ctx, const Prepared &P, double mu, bool deriv, double
     if (explicit_inv) {
         DG_TRY(run_gloc(ctx, P, deriv ? (M_TRACE | M_DERIV) : M_TRACE, mu, 1, nullptr, nullptr, tr, dtr, mixed));
     } else if (mixed && ctx->tensor && !ctx->capturing &&
-               (deriv ? dg_lat_tc_deriv_supported(P.n, P.D, P.nk) : dg_lat_tc_supported(P.n, P.D, P.nk))) {
+               (deriv ? dg_lat_tc_deriv_supported(P.n, P.D) : dg_lat_tc_supported(P.n, P.D)) &&
+               dg_lat_tc_reserve(ctx, P.n, P.D, P.nk, false)) {
         // the pole sums on the tensor cores (lat_tc.cu)
         DG_CUDA(cudaStreamWaitEvent(ctx->stream, P.static_ready, 0));
         DG_TRY(dg_lat_tc_trace(ctx, lat_tc_args(P, mu, 1), &P.tc_ready, tr, deriv ? dtr : nullptr));
@@ -977,7 +978,8 @@ int greenftn_w_dev(dmftgpu_ctx *ctx, const dmftgpu_lattice *L, const double2 *dH
     if (!blk || !blk0 || !occ || !fs) return DMFTGPU_NOMEM;
     if (flags & DMFTGPU_EXPLICIT)
         DG_TRY(run_gloc(ctx, P, M_BLOCK, mu, 0, blk, blk0, nullptr, nullptr, (flags & DMFTGPU_MIXED) != 0));
-    else if ((flags & DMFTGPU_MIXED) && !(flags & DMFTGPU_NO_TENSOR) && ctx->tensor && dg_lat_tc_block_supported(P.n, D, P.nk)) {
+    else if ((flags & DMFTGPU_MIXED) && !(flags & DMFTGPU_NO_TENSOR) && ctx->tensor && dg_lat_tc_block_supported(P.n, D) &&
+             dg_lat_tc_reserve(ctx, P.n, D, P.nk, true)) {
         // pole sums and GwHF on the tensor cores (lat_tc.cu)
         DG_TRY(dg_lat_tc_block(ctx, lat_tc_args(P, mu, 0), blk, blk0));
     } else DG_TRY(run_schur(ctx, P, dg::S_BLOCK, mu, 0, blk, blk0, nullptr, nullptr, (flags & DMFTGPU_MIXED) != 0));
@@ -1309,6 +1311,7 @@ int dmftgpu_greenftn_w_batched(dmftgpu_ctx *ctx, int nprob, const dmftgpu_lattic
                  (void *)nummat[i]);
         key += b;
     }
+    DgImageShare share(ctx);
     DG_TRY(dg_status_reset(ctx));
     if ((flags & DMFTGPU_GRAPH) && ctx->graph && ctx->graph_key == key) {
         DG_CUDA(cudaGraphLaunch(ctx->graph, ctx->stream));

@@ -477,3 +477,43 @@ def test_k_sum_keeps_its_digits(ctx, D):
     exact = (1 / z).sum(0) / nk                                        # [D][nf]
     err = np.array([G[:, a, a] - exact[a] for a in range(D)])
     assert np.sqrt((abs(err) ** 2).sum() / (abs(exact) ** 2).sum()) < 4.5 * 2.0 ** -53
+
+
+def test_mixed_passes_without_room_for_operand_images(ctx):
+    """24,000 k points whose operand images (2.1 GB for G_loc, 1.0 for N(mu)) do not fit in what is left of the device: the
+    passes run without them, as with tensor=False, and the next call with room takes the tensor cores again."""
+    import torch
+    n, D, nk, nf = 14, 10, 24000, 8
+    g = torch.Generator(device="cuda").manual_seed(5)
+    A = torch.view_as_complex(torch.randn(nk, n, n, 2, dtype=torch.float64, device="cuda", generator=g))
+    H = (A + A.conj().transpose(1, 2)) / 4
+    S = torch.eye(D, dtype=torch.complex128, device="cuda").repeat(nf, 1, 1) * (-0.2j)
+    lat = lib.Lattice(n, nk, nf, 10.0, 1, D)
+    want = [ctx.GiwToNele(lat, H, S, 0.3, mixed=True, tensor=False), ctx.GiwToNele(lat, H, S, 0.3, deriv=True, mixed=True, tensor=False)]
+    full = ctx.GreenFtn_w(lat, H, S, 0.3)[0].cpu()
+    c = lib.Context(0)
+    hog = None
+    try:
+        c.GiwToNele(lat, H, S, 0.3, mixed=True, tensor=False)      # what every pass needs is there
+        c.GreenFtn_w(lat, H, S, 0.3)
+        torch.cuda.empty_cache()
+        free = torch.cuda.mem_get_info()[0]
+        hog = torch.empty(free - (900 << 20), dtype=torch.uint8, device="cuda")
+        got = [c.GiwToNele(lat, H, S, 0.3, mixed=True), c.GiwToNele(lat, H, S, 0.3, deriv=True, mixed=True)]
+        G = c.GreenFtn_w(lat, H, S, 0.3, mixed=True)[0].cpu()
+        assert got == want
+        assert float((G - full).abs().max() / full.abs().max()) < TOL_MIXED
+        n0 = c.launches()
+        c.GreenFtn_w(lat, H, S, 0.3, mixed=True)
+        without = c.launches() - n0
+        del hog
+        hog = None
+        torch.cuda.empty_cache()
+        n0 = c.launches()
+        G = c.GreenFtn_w(lat, H, S, 0.3, mixed=True)[0].cpu()
+        assert c.launches() - n0 != without
+        assert float((G - full).abs().max() / full.abs().max()) < TOL_MIXED
+    finally:
+        del hog
+        torch.cuda.empty_cache()
+        c.close()
