@@ -726,7 +726,7 @@ int run_schur(dmftgpu_ctx *ctx, const Prepared &P, int mode, double mu, int wgri
         return dg_ceil_div(P.nk, kch);
     };
     const std::string key = std::string(tpi ? "schur_tpi/" : "schur/") + std::to_string(in->DP) + "/" + std::to_string(mode) + "/" +
-                            std::to_string((int)mixed) + "/" + std::to_string(P.nk) + "/" + std::to_string(nf2);
+                            std::to_string((int)mixed) + "/" + std::to_string(P.nk) + "/" + std::to_string(nf2) + "/" + std::to_string(m);
     int kch_max;
     const int cps0 = tpi && !trace && mixed && P.D == 3 ? 24 : 8, nchunk_max = chunks(std::max(cps0, 16), &kch_max);
     double2 *pblk = nullptr, *pblk0 = nullptr, *ptr = nullptr;
@@ -769,7 +769,8 @@ int run_schur(dmftgpu_ctx *ctx, const Prepared &P, int mode, double mu, int wgri
     // the TRACE passes read the static eigenvalues (Tr G0), computed on the side stream
     if (!(mode & dg::S_REAL) && (trace || ((mode & dg::S_BLOCK) && in->DP >= 8)))
         DG_CUDA(cudaStreamWaitEvent(ctx->stream, P.static_ready, 0));
-    // autotuning: time 4, 8 and 16 CTAs per SM once per (width, mode, precision, N_k, points) and keep the fastest
+    // autotuning: time the untuned number, 4, 8 and 16 CTAs per SM once per (width, mode, precision, N_k, points, poles) and keep
+    // the fastest
     auto tuned = ctx->tuned.find(key);
     if (tuned != ctx->tuned.end()) {
         nchunk = chunks(tuned->second, &kchunk);
@@ -786,8 +787,10 @@ int run_schur(dmftgpu_ctx *ctx, const Prepared &P, int mode, double mu, int wgri
         DG_CUDA(cudaEventCreate(&ev.a));
         DG_CUDA(cudaEventCreate(&ev.b));
         float best = 1e30f;
-        int best_cps = 8;
-        for (int cps : {4, 8, 16}) {
+        int best_cps = cps0, cand[4];
+        const int ncand = dg::schur_cps_candidates(cps0, cand);
+        for (int i = 0; i < ncand; i++) {
+            const int cps = cand[i];
             int kch;
             const int nc = chunks(cps, &kch);
             g.kchunk = kch;

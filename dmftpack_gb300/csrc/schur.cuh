@@ -857,6 +857,15 @@ __global__ void __launch_bounds__(128) k_trace_tpi(SchurArgs g) {
     if (fvalid) g.ptr[(size_t)chunk * g.nf2 + f] = cmk(s1, s2);
 }
 
+// CTAs per SM that the autotuner times: the untuned launch's own number first, so that it never ends up with a slower one
+inline int schur_cps_candidates(int untuned, int (&c)[4]) {
+    int n = 0;
+    c[n++] = untuned;
+    for (int x : {4, 8, 16})
+        if (x != untuned) c[n++] = x;
+    return n;
+}
+
 // shared-memory bytes of one k_schur launch
 inline size_t schur_smem(int DP, int W, int mode, int kc, int D, int m, int n) {
     const int NG = schur_groups(W);

@@ -44,7 +44,9 @@ enum {
                                    reference does (default: the exact correlated-block Schur form); FP64, or
                                    double-float with DMFTGPU_MIXED */
 #define DMFTGPU_GRAPH 0x20     /* dmftgpu_greenftn_w_batched: replay the batched pass as one CUDA graph */
-#define DMFTGPU_AUTOTUNE 0x40  /* dmftgpu_greenftn_w_batched: tune each Schur kernel's k chunking on first use */
+#define DMFTGPU_AUTOTUNE 0x40  /* dmftgpu_greenftn_w_batched: tune the k chunking of the lane-group and thread-per-frequency
+                                  kernels (k_schur, k_schur_tpi) on first use; the tensor-core and tile passes choose theirs
+                                  by rounds of resident CTAs */
 #define DMFTGPU_NO_TENSOR 0x80 /* with DMFTGPU_MIXED: keep the contractions (H(k), the N(mu) pole sums) on the
                                   CUDA cores instead of the tensor cores */
 #define DMFTGPU_DIRECT_DFT 0x10 /* iw <-> tau transforms by the reference's direct per-point sums (default: the
