@@ -291,10 +291,11 @@ class Context:
         self._check("dmftgpu_moments", st)
         return out.result()
 
-    def GreenFtn_w(self, lat, H_k, SelfE_w, mu, mixed=False, with_gwhf=True, explicit=False):
+    def GreenFtn_w(self, lat, H_k, SelfE_w, mu, mixed=False, with_gwhf=True, explicit=False, tensor=True):
         """GreenFtn_w: returns (Gw[nfreq,D,D], GwHF[nfreq,D,D] or None, NumMatrix[D,D]).
         explicit=True inverts every (k, iw) matrix in full as the reference does; the default computes the
-        same correlated block through its exact Schur complement."""
+        same correlated block through its exact Schur complement.  In the mixed form the pass over correlated
+        blocks of 5 .. 10 orbitals runs its pole sums on the tensor cores unless tensor=False."""
         dev = _is_torch(H_k)
         h, s = _Arr(H_k, dev), _Arr(SelfE_w, dev)
         D = lat.D
@@ -304,14 +305,15 @@ class Context:
         L = lat._c()
         st = self.lib.dmftgpu_greenftn_w(self.h, C.byref(L), _vp(h.ptr), _vp(s.ptr), float(mu), _vp(gw.ptr),
                                          _vp(g0.ptr) if g0 else None, _vp(nm.ptr),
-                                         self._flags(dev, (MIXED if mixed else 0) | (EXPLICIT if explicit else 0)))
+                                         self._flags(dev, (MIXED if mixed else 0) | (EXPLICIT if explicit else 0)
+                                                     | (0 if tensor else NO_TENSOR)))
         self._check("dmftgpu_greenftn_w", st)
         return gw.result(), (g0.result() if g0 else None), nm.result()
 
     def GreenFtn_w_batched(self, lats, Hk_cm, Sig_cm, mus, gw_cm, gwhf_cm, num_cm, mixed=False, graph=False,
-                           autotune=False):
+                           autotune=False, tensor=True):
         """GreenFtn_w over a batch of problems; every array a CUDA tensor in the library's column-major layout,
-        outputs written in place (gwhf_cm may be None)."""
+        outputs written in place (gwhf_cm may be None); tensor as in GreenFtn_w."""
         import torch  # noqa: F401
         n = len(lats)
         Ls = (_Lat * n)(*[lt._c() for lt in lats])
@@ -319,7 +321,8 @@ class Context:
         st = self.lib.dmftgpu_greenftn_w_batched(
             self.h, n, Ls, ptr(Hk_cm), ptr(Sig_cm), (C.c_double * n)(*[float(m) for m in mus]), ptr(gw_cm),
             ptr(gwhf_cm) if gwhf_cm is not None else None, ptr(num_cm),
-            self._flags(True, (MIXED if mixed else 0) | (GRAPH if graph else 0) | (AUTOTUNE if autotune else 0)))
+            self._flags(True, (MIXED if mixed else 0) | (GRAPH if graph else 0) | (AUTOTUNE if autotune else 0)
+                        | (0 if tensor else NO_TENSOR)))
         self._check("dmftgpu_greenftn_w_batched", st)
 
     def retarded_GreenFtn(self, lat, H_k, SelfE_E, e0, de, eta, mu, mixed=False):

@@ -47,8 +47,8 @@ enum {
 #define DMFTGPU_AUTOTUNE 0x40  /* dmftgpu_greenftn_w_batched: tune the k chunking of the lane-group and thread-per-frequency
                                   kernels (k_schur, k_schur_tpi) on first use; the tensor-core and tile passes choose theirs
                                   by rounds of resident CTAs */
-#define DMFTGPU_NO_TENSOR 0x80 /* with DMFTGPU_MIXED: keep the contractions (H(k), the N(mu) pole sums) on the
-                                  CUDA cores instead of the tensor cores */
+#define DMFTGPU_NO_TENSOR 0x80 /* with DMFTGPU_MIXED: keep the contractions (H(k), and the pole sums of G_loc, GwHF, N(mu) and
+                                  dN/dmu) on the CUDA cores instead of the tensor cores */
 #define DMFTGPU_DIRECT_DFT 0x10 /* iw <-> tau transforms by the reference's direct per-point sums (default: the
                                    same sums by FFT when N_tau is a power of two <= 8192) */
 

@@ -517,3 +517,26 @@ def test_mixed_passes_without_room_for_operand_images(ctx):
         del hog
         torch.cuda.empty_cache()
         c.close()
+
+
+def test_tensor_switch_of_the_lattice_sum(ctx, orc):
+    """tensor=False keeps G_loc and GwHF of a 10-orbital block off the tensor cores, alone and in a batch (fewer launches: no
+    operand images), with the oracle's values either way."""
+    import torch
+    wl = models.dp28(k=2, nfreq=24, ntau=16, beta=20.0)
+    H, lat = _setup(orc, wl)
+    ref = orc.greenftn_w(H, wl.sigma, 0.2, wl.beta, wl.ncl, wl.nh)
+    n, cm = [], lambda x: torch.from_numpy(np.ascontiguousarray(x.transpose(0, 2, 1))).cuda()
+    for tensor in (True, False):
+        n0 = ctx.launches()
+        G, G0, N = ctx.GreenFtn_w(lat, H, wl.sigma, 0.2, mixed=True, tensor=tensor)
+        n.append(ctx.launches() - n0)
+        for x, y in zip((G, G0, N), ref):
+            assert rel_err(x, y) < TOL_MIXED
+        out = [torch.zeros((wl.nfreq, wl.D, wl.D), dtype=torch.complex128, device="cuda") for _ in range(2)]
+        num = torch.zeros((wl.D, wl.D), dtype=torch.complex128, device="cuda")
+        n0 = ctx.launches()
+        ctx.GreenFtn_w_batched([lat], [cm(H)], [cm(wl.sigma)], [0.2], out[:1], out[1:], [num], mixed=True, tensor=tensor)
+        assert ctx.launches() - n0 == n[-1]
+        assert rel_err(out[0].transpose(1, 2).cpu().numpy(), G) == 0.0
+    assert n[1] < n[0]
