@@ -1,6 +1,6 @@
-// lat_tc.cu -- the mixed-precision (DMFTGPU_MIXED) lattice passes of correlated blocks of 5 .. 10 orbitals, with the pole
-// sums on the tensor cores: the N(mu) and dN/dmu passes of the mu search (GiwToNele, src/GreenFtn.cpp:513-635, in the
-// trace form) and the G_loc / GwHF pass (GreenFtn_w, src/GreenFtn.cpp:142-422).
+// lat_tc.cu -- mixed-precision (DMFTGPU_MIXED) lattice passes with the pole sums on the tensor cores: the N(mu) and dN/dmu
+// passes of the mu search (GiwToNele, src/GreenFtn.cpp:513-635, in the trace form) of correlated blocks of 4 .. 10 orbitals
+// and the G_loc / GwHF pass (GreenFtn_w, src/GreenFtn.cpp:142-422) of 5 .. 10.
 //
 // Per (k, iw_f), with w_l = 1/(z - e_l), P_l = b_l b_l^H and M = z - H_PP - Sigma(iw_f) - S (schur.cuh):
 //     S = sum_l w_l P_l,   R = sum_l w_l^2 P_l,   T = sum_l w_l^3 P_l
@@ -22,7 +22,8 @@
 // and the highest levels share one.
 //   N(mu) passes: 5 slices, levels 0, 1, 2 exact, 3 and 4 shared: values below 2^-19 of the row x column scale, so the
 //     accumulator's rounding adds ~2^-44 of it, as much as the slices leave.  Four accumulators x NP columns fit TMEM's
-//     512, and all 128 lanes carry rows.
+//     512, and all 128 lanes carry rows.  (Blocks of 4, whose 16 columns leave room, take six: N(mu) is then as close as
+//     k_schur's, 1e-15, where five leave 1e-14.)
 //   dN/dmu: 6 slices, levels 0 .. 3 exact, 4 and 5 shared (rounding ~2^-52).  Five accumulators of 112 columns (D > 8) do
 //     not fit: the columns are then multiplied and drained in two parts, 64 and NP - 64.
 //   G_loc / GwHF: 6 slices likewise, but only 64 rows are needed (32 frequencies x Re w, Im w): the lower columns
@@ -86,7 +87,7 @@ template <int DP, int MODE>
 struct TT {
     static constexpr bool TWO = MODE == TC_BLOCK;        // two channels (rows 2 f, 2 f + 1), else four (4 f ..)
     static constexpr bool G0I = TWO && DP < 8;           // GwHF by a second inversion (else k_g0_tc)
-    static constexpr int NS = MODE == TC_TRACE ? 5 : 6;  // slices
+    static constexpr int NS = MODE == TC_TRACE && DP > 4 ? 5 : 6;  // slices
     static constexpr int NP = np_of(DP);                 // MMA N: dofs padded to a multiple of 16
     static constexpr int DD = DP * DP;
     static constexpr int GPW = 32 / DP;                  // frequency groups per inversion warp
@@ -1092,12 +1093,17 @@ int launch_trace(dmftgpu_ctx *ctx, const LatTcArgs &a, bool *ready, double *tr, 
 //           D = 10  2.61 / 3.99  3.48 / 4.07  4.28 / 4.13
 //   dN/dmu  D = 6   1.98 / 2.46  2.82 / 2.54
 //           D = 10  6.46 / 7.24  10.1 / 7.30
-// The lines below are where these cross.  At D = 4 N(mu) takes k_schur 0.45 (m = 0) and 1.96 (m = 10) and 1.77 and 2.33
-// here at 1,024 frequencies: they cross only past 16 poles.
-static bool covered(int n, int D, int least) { return D >= 5 && D <= 10 && n - D >= least && n - D <= KP && n <= NE0; }
-bool dg_lat_tc_supported(int n, int D) { return covered(n, D, 4); }
-bool dg_lat_tc_deriv_supported(int n, int D) { return covered(n, D, 2); }
-bool dg_lat_tc_block_supported(int n, int D) { return covered(n, D, D <= 6 ? 4 : (D <= 8 ? 2 : 0)) && (D <= 6 || n <= KP); }
+// The lines below are where these cross.  At D = 4 (512 k x 4,096 frequencies)
+//              m = 8        m = 12       m = 16       m = 20       m = 28
+//   N(mu)                   3.30 / 3.14  4.12 / 3.24  5.11 / 3.40  8.02 / 3.99
+//   dN/dmu     4.74 / 4.59  6.52 / 4.76  8.15 / 4.86  9.93 / 5.05  14.0 / 5.64
+// G_loc of four orbitals stays with k_schur (without poles 1.34 / 1.84).
+static bool covered(int n, int D, int least) { return D <= 10 && n - D >= least && n - D <= KP && n <= NE0; }
+bool dg_lat_tc_supported(int n, int D) { return D >= 4 && covered(n, D, D == 4 ? 12 : 4); }
+bool dg_lat_tc_deriv_supported(int n, int D) { return D >= 4 && covered(n, D, D == 4 ? 8 : 2); }
+bool dg_lat_tc_block_supported(int n, int D) {
+    return D >= 5 && covered(n, D, D <= 6 ? 4 : (D <= 8 ? 2 : 0)) && (D <= 6 || n <= KP);
+}
 
 // The images, 43 KB per k point at D = 10 and two sets of them in G_loc's pass, are what k_schur does without: they stay
 // within 64 GB in a call, and where they cannot be had at all the pass is k_schur's.
@@ -1125,6 +1131,7 @@ bool dg_lat_tc_reserve(dmftgpu_ctx *ctx, int n, int D, int nk, bool block) {
 int dg_lat_tc_trace(dmftgpu_ctx *ctx, const LatTcArgs &a, bool *ready, double *tr, double *dtr) {
     if (!(dtr ? dg_lat_tc_deriv_supported(a.n, a.D) : dg_lat_tc_supported(a.n, a.D)))
         return dg_fail(ctx, DMFTGPU_BADARG, "lat_tc: unsupported sizes");
+    if (a.D == 4) return launch_trace<4>(ctx, a, ready, tr, dtr);
     if (a.D <= 6) return launch_trace<6>(ctx, a, ready, tr, dtr);
     if (a.D <= 8) return launch_trace<8>(ctx, a, ready, tr, dtr);
     return launch_trace<10>(ctx, a, ready, tr, dtr);

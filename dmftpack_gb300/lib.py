@@ -479,7 +479,7 @@ class Context:
         return out
 
     def GiwToNele(self, lat, H_k, SelfE_w, mu, deriv=False, mixed=False, explicit=False, tensor=True):
-        """N(mu) (and dN/dmu with deriv).  In the mixed form the pass over correlated blocks of 5 .. 10 orbitals
+        """N(mu) (and dN/dmu with deriv).  In the mixed form the pass over correlated blocks of 4 .. 10 orbitals
         runs its pole sums on the tensor cores unless tensor=False."""
         dev = _is_torch(H_k)
         h, s = _Arr(H_k, dev), _Arr(SelfE_w, dev)

@@ -540,3 +540,19 @@ def test_tensor_switch_of_the_lattice_sum(ctx, orc):
         assert ctx.launches() - n0 == n[-1]
         assert rel_err(out[0].transpose(1, 2).cpu().numpy(), G) == 0.0
     assert n[1] < n[0]
+
+
+@pytest.mark.parametrize("n,nk,nf", [(15, 5, 33), (16, 1, 24), (16, 7, 31), (11, 4, 40), (12, 3, 25), (36, 9, 48), (32, 20, 64),
+                                     (37, 2, 24)])
+def test_nele_of_four_orbitals_with_many_ligands(ctx, n, nk, nf):
+    """N(mu) and dN/dmu of 4 x 4 blocks below, at and above the pole counts (12, 8; 32 the most) from which their pole sums are on
+    the tensor cores, partial tiles of 32 frequencies and single k points among them: the mixed form against FP64 within
+    the slices' 2^-41 of sums over matrices of condition < 1e2, and against its form on the CUDA cores."""
+    H, S, lat = _random_lattice(n, 4, (nk, 1, 1), nf, [n, 4, nk])
+    for mu in (-0.4, 0.3):
+        N, dN = ctx.GiwToNele(lat, H, S, mu, deriv=True)
+        for tensor in (True, False):
+            g = ctx.GiwToNele(lat, H, S, mu, mixed=True, tensor=tensor)
+            assert abs(g - N) <= 1e-11 * max(1, abs(N))
+            g, dg = ctx.GiwToNele(lat, H, S, mu, deriv=True, mixed=True, tensor=tensor)
+            assert abs(g - N) <= 1e-11 * max(1, abs(N)) and abs(dg - dN) <= 1e-10 * max(1, abs(dN))
