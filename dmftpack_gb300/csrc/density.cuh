@@ -161,31 +161,40 @@ __global__ void __launch_bounds__(128) k_dens_sum(DensArgs g) {
     }
     if (sing) dg_flag(g.status, DG_SINGULAR);
     __syncthreads();
-    // fixed-order sum over the groups into this split's partial Y and R
+    // fixed-order sums over the groups into this split's partial Y and R.  Small matrices leave most threads without an element:
+    // P of them then share one, the groups dealt over them and their sums added as a tree (2 orbitals, 128 groups: one
+    // thread's FP64 conversions and additions of 128 terms took 100 us, a third of the call)
+    auto over_groups = [&](int count, auto term, auto put) {
+        int P = 1;
+        while (blockDim.x % 32 == 0 && 2 * P <= 32 && 2 * P <= NG && 2 * P * count <= (int)blockDim.x) P *= 2;
+        const int per = blockDim.x / P, part = threadIdx.x % P;
+        for (int q0 = 0; q0 < count; q0 += per) {
+            const int q = q0 + threadIdx.x / P;
+            double2 v = cmk(0, 0);
+            if (q < count)
+                for (int gg = part; gg < NG; gg += P) v = cadd(v, term(q, gbase + gg * PG));
+            for (int o = P / 2; o > 0; o >>= 1)
+                v = cadd(v, cmk(__shfl_xor_sync(0xffffffffu, v.x, o), __shfl_xor_sync(0xffffffffu, v.y, o)));
+            if (q < count && part == 0) put(q, v);
+        }
+    };
     double2 *Yo = g.Y + ((size_t)split * g.nk + k) * n * n;
-    for (int q = threadIdx.x; q < n * n; q += blockDim.x) {
-        const int i = q % n, j = q / n;
-        double2 v = cmk(0, 0);
-        for (int gg = 0; gg < NG; gg++) {
-            const C *gb = gbase + gg * PG;
+    over_groups(
+        n * n,
+        [&](int q, const C *gb) {
+            const int i = q % n, j = q / n;
             const C *gG = gb + m, *gX = gG + DP * DP + (size_t)m * D, *gY = gX + (size_t)D * m, *gw = gY + (size_t)m * m;
-            if (i < D && j < D) v = cadd(v, Ops::to(gG[i + j * DP]));
-            else if (i < D) v = cadd(v, Ops::to(gX[i + (size_t)(j - D) * D]));
-            else if (j >= D) {
-                v = cadd(v, Ops::to(gY[(i - D) + (size_t)(j - D) * m]));
-                if (i == j) v = cadd(v, Ops::to(gw[i - D]));
-            }
-        }
-        Yo[q] = v;
-    }
-    for (int j = threadIdx.x; j < n; j += blockDim.x) {
-        double r = 0;
-        for (int gg = 0; gg < NG; gg++) {
-            const C *gb = gbase + gg * PG;
-            r += Ops::re((gb + m + DP * DP + 2 * (size_t)m * D + (size_t)m * m + m)[j]);
-        }
-        g.R[((size_t)split * g.nk + k) * n + j] = r;
-    }
+            if (i < D && j < D) return Ops::to(gG[i + j * DP]);
+            if (i < D) return Ops::to(gX[i + (size_t)(j - D) * D]);
+            if (j < D) return cmk(0, 0);
+            const double2 y = Ops::to(gY[(i - D) + (size_t)(j - D) * m]);
+            return i == j ? cadd(y, Ops::to(gw[i - D])) : y;
+        },
+        [&](int q, double2 v) { Yo[q] = v; });
+    double *Ro = g.R + ((size_t)split * g.nk + k) * n;
+    over_groups(
+        n, [&](int j, const C *gb) { return cmk(Ops::re((gb + m + DP * DP + 2 * (size_t)m * D + (size_t)m * m + m)[j]), 0.0); },
+        [&](int j, double2 v) { Ro[j] = v.x; });
 }
 
 typedef void (*DensKernel)(DensArgs);
