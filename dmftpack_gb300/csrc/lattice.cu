@@ -1127,14 +1127,14 @@ int run_density(dmftgpu_ctx *ctx, const Prepared &P, double mu, double2 *dens, b
     g.Y = Y;
     g.R = R;
     g.status = ctx->d_status;
-    DG_CUDA(dg_smem_attr(kern, smem));
+    DG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));  // alone on the SMs
     {
         DgTimer tm(ctx, "k_dens_sum");
         kern<<<dim3(nk, nsplit), ng * W, smem, ctx->stream>>>(g);
     }
     DG_LAUNCH(ctx, "k_dens_sum");
     const size_t fs = 2 * (size_t)n * n * sizeof(double2) + n * sizeof(double);
-    DG_CUDA(dg_smem_attr(k_dens_finish, fs));
+    DG_CUDA(cudaFuncSetAttribute(k_dens_finish, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fs));
     k_dens_finish<<<nk, 128, fs, ctx->stream>>>(nk, n, D, nsplit, P.beta, mu, Y, R, P.Vq, P.Uf, P.eps, P.perm, dens);
     DG_LAUNCH(ctx, "k_dens_finish");
     return DMFTGPU_OK;
