@@ -147,11 +147,11 @@ __device__ __forceinline__ uint32_t bf16x2(float lo, float hi) {
     const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<const uint32_t *>(&v);
 }
-// the power of two that takes |x| <= mx to [0, 1]
+// the power of two that takes |x| <= mx to [0, 1]; at least 2^-125, for its reciprocal is taken (rows of w^3 at energies of 1e12)
 __device__ __forceinline__ float scale_of(float mx) {
     int ex = 0;
     frexpf(mx, &ex);
-    return mx > 0.f ? ldexpf(1.f, ex) : 1.f;
+    return mx > 0.f ? ldexpf(1.f, max(ex, -125)) : 1.f;
 }
 
 // per k: the B operand image (dofs of the poles b_l b_l^H, sliced per dof column) and the column scales (unit: 1 for every

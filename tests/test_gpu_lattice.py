@@ -556,3 +556,14 @@ def test_nele_of_four_orbitals_with_many_ligands(ctx, n, nk, nf):
             assert abs(g - N) <= 1e-11 * max(1, abs(N))
             g, dg = ctx.GiwToNele(lat, H, S, mu, deriv=True, mixed=True, tensor=tensor)
             assert abs(g - N) <= 1e-11 * max(1, abs(N)) and abs(dg - dN) <= 1e-10 * max(1, abs(dN))
+
+
+@pytest.mark.parametrize("n,D", [(16, 4), (10, 6), (14, 10)])
+def test_units_of_energy(ctx, n, D):
+    """All energies times 2^40 and beta by 2^-40: the same numbers in other units, dN/dmu smaller by 2^40.  The pole sums' rows of
+    w^3 are 1e-36 and less then, their low halves beyond FP32: digits go (2^-20 of dN/dmu are left), the number does not."""
+    H, S, lat = _random_lattice(n, D, (5, 1, 1), 40, [n, D])
+    N, dN = ctx.GiwToNele(lat, H, S, 0.3, deriv=True, mixed=True)
+    big = lib.Lattice(n, lat.nk, lat.nfreq, lat.beta / 2.0 ** 40, 1, D)
+    M, dM = ctx.GiwToNele(big, H * 2.0 ** 40, S * 2.0 ** 40, 0.3 * 2.0 ** 40, deriv=True, mixed=True)
+    assert abs(M - N) <= 1e-11 * abs(N) and abs(dM * 2.0 ** 40 - dN) <= 2.0 ** -20 * abs(dN)
