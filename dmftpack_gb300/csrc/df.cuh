@@ -207,6 +207,8 @@ struct OpsD {
     static DG_HD C pscale(C a, R r) { return cmk(a.x * r, a.y * r); }
     static DG_HD R rdotc(C a, C b) { return ::fma(a.x, b.x, a.y * b.y); }  // Re(a conj b)
     static DG_HD void balance(C &, C &) {}
+    // a d - b c from rounded products: equal products cancel to an exact zero, the sign of a singular matrix
+    static DG_HD C det2(C a, C b, C c, C d) { return csub(cmul(a, d), cmul(b, c)); }
     static DG_HD C times_i(C a) { return cmk(-a.y, a.x); }
 };
 
@@ -389,6 +391,7 @@ struct OpsP {
     static __device__ __forceinline__ C pnorm(C a) { return pdf_fast_two_sum(a.h, a.l); }
     static __device__ __forceinline__ C pscale(C a, R r) { return pdf_mul(a, pdf_both(r)); }
     static __device__ __forceinline__ C times_i(C a) { return pdf_i(a); }
+    static __device__ __forceinline__ C det2(C a, C b, C c, C d) { return fms(b, c, mul(a, d)); }
     // num and den by the power of two that takes |den| to about 1, so that |den|^2 stays in the FP32 range
     static __device__ __forceinline__ void balance(C &num, C &den) {
         const float mx = fmaxf(fabsf(den.h.x), fabsf(den.h.y));

@@ -326,14 +326,14 @@ __global__ void __launch_bounds__(128) k_schur(SchurArgs g) {
 // swaps are predicated moves between compile-time indices (no local memory), undone as column swaps at the end.
 // Each step stores the pivot's reciprocal in place and updates only the other columns: row j becomes
 // a_jc / a_jj, row r becomes a_rc - a_rj a_jc for c != j, and column j becomes -a_rj / a_jj (no products with the
-// known 1 and 0 entries).  A 2 x 2 matrix takes adj(M) / det M, one reciprocal and 24 fewer FP64 instructions of 60 (the
+// known 1 and 0 entries).  A 2 x 2 matrix takes adj(M) / det M, one reciprocal and 22 fewer FP64 instructions of 60 (the
 // determinant scaled by a power of two in double-float, whose range is FP32's).
 template <class Ops, int N>
 DG_HD bool thread_inverse(typename Ops::C (&a)[N][N]) {
     typedef typename Ops::C C;
     typedef typename Ops::M M;
     if constexpr (N == 2) {
-        C det = Ops::fms(a[0][1], a[1][0], Ops::mul(a[0][0], a[1][1])), scale = Ops::one();
+        C det = Ops::det2(a[0][0], a[0][1], a[1][0], a[1][1]), scale = Ops::one();
         Ops::balance(scale, det);
         const bool zero = !(Ops::mag2(det) > M(0));
         const C ip = Ops::pscale(Ops::rcp(det), Ops::cre(scale)), in = Ops::neg(ip), d0 = a[0][0];
@@ -778,7 +778,7 @@ __global__ void __launch_bounds__(128) k_trace_tpi(SchurArgs g) {
                 return a == b ? Ops::add(v, Ops::one()) : v;
             };
             if constexpr (D == 2 && !DERIV) {
-                C det = Ops::fms(M[0][1], M[1][0], Ops::mul(M[0][0], M[1][1]));
+                C det = Ops::det2(M[0][0], M[0][1], M[1][0], M[1][1]);
                 C num;
                 if (m > 0) {
                     num = Ops::fma(M[0][0], IR(1, 1), Ops::mul(M[1][1], IR(0, 0)));

@@ -3,6 +3,7 @@ import os
 import shutil
 import subprocess
 
+import numpy as np
 import pytest
 
 from conftest import ROOT
@@ -31,3 +32,25 @@ def harness(tmp_path_factory):
 def test_autotuner_times_the_untuned_launch(harness, untuned):
     c = [int(x) for x in harness(["cps %d\n" % untuned])[0]]
     assert c[0] == untuned and len(set(c)) == len(c) and {4, 8, 16} <= set(c)
+
+
+def _line(op, M):
+    return "%s %s\n" % (op, " ".join("%s %s" % (float(z.real).hex(), float(z.imag).hex()) for z in np.ravel(M)))
+
+
+def test_two_by_two_inverse(harness):
+    """The closed form of the 2 x 2 inverse: singular matrices whose products are equal (rows alike, zero rows, powers of two)
+    are flagged, also where the products round; z - H - Sigma is inverted to a few roundings times its condition."""
+    rng = np.random.default_rng(4)
+    sing = [np.zeros((2, 2)), np.array([[1.0, 0], [0, 0]]), np.array([[0, 0], [0.3, 2j]])]
+    for c in rng.normal(size=40):
+        sing += [np.full((2, 2), c), np.array([[c, 2 * c], [c, 2 * c]]), np.array([[c, -c], [4 * c, -4 * c]]) * 1j]
+    assert all(r[0] == "1" for r in harness([_line("inv2d", M) for M in sing]))
+    good = []
+    for _ in range(300):
+        H = rng.normal(size=(2, 2)) + 1j * rng.normal(size=(2, 2))
+        good.append((rng.normal() + 1j * np.exp(rng.uniform(-4, 4))) * np.eye(2) - (H + H.conj().T) / 2)
+    for M, r in zip(good, harness([_line("inv2d", M) for M in good])):
+        v = np.array([float.fromhex(x) for x in r[1:]])
+        X, exact = (v[0::2] + 1j * v[1::2]).reshape(2, 2), np.linalg.inv(M)
+        assert r[0] == "0" and np.abs(X - exact).max() <= 16 * 2.0 ** -53 * np.linalg.cond(M) * np.abs(exact).max()
