@@ -18,6 +18,7 @@
 // registers side by side costs two moves, so a pdf is kept as (re.h, im.h, re.l, im.l) in registers and in memory.
 #pragma once
 #include <cmath>
+#include <cstring>
 
 #include "common.cuh"
 
@@ -52,6 +53,24 @@ DG_HD float f_fma(float a, float b, float c) {
     return __fmaf_rn(a, b, c);
 #else
     return std::fma(a, b, c);
+#endif
+}
+DG_HD int bits_of(float a) {
+#ifdef __CUDA_ARCH__
+    return __float_as_int(a);
+#else
+    int i;
+    std::memcpy(&i, &a, sizeof i);
+    return i;
+#endif
+}
+DG_HD float float_of(int i) {
+#ifdef __CUDA_ARCH__
+    return __int_as_float(i);
+#else
+    float a;
+    std::memcpy(&a, &i, sizeof a);
+    return a;
 #endif
 }
 // 1/a to within an ulp: on the device the approximate reciprocal and one Newton step (the correctly rounded division
@@ -268,11 +287,12 @@ struct OpsF {
     }
 };
 
-// ---- packed pairs (device only) ----
-__device__ __forceinline__ float2 p2(float x, float y) { return make_float2(x, y); }
-__device__ __forceinline__ float2 p2(float x) { return make_float2(x, x); }
-#define DG_P2_OP(NAME, INSN)                                                                               \
-    __device__ __forceinline__ float2 NAME(float2 a, float2 b) {                                           \
+// ---- packed pairs; on the host the same operations one after the other (OpsP::shfl: device only) ----
+DG_HD float2 p2(float x, float y) { return make_float2(x, y); }
+DG_HD float2 p2(float x) { return make_float2(x, x); }
+#ifdef __CUDA_ARCH__
+#define DG_P2_OP(NAME, INSN, SCALAR)                                                                       \
+    DG_HD float2 NAME(float2 a, float2 b) {                                                                \
         float2 d;                                                                                          \
         asm("{\n\t.reg .b64 a, b, d;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\t" INSN              \
             " d, a, b;\n\tmov.b64 {%0, %1}, d;\n\t}"                                                       \
@@ -280,39 +300,47 @@ __device__ __forceinline__ float2 p2(float x) { return make_float2(x, x); }
             : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));                                                     \
         return d;                                                                                          \
     }
-DG_P2_OP(p2_add, "add.rn.f32x2")
-DG_P2_OP(p2_sub, "sub.rn.f32x2")
-DG_P2_OP(p2_mul, "mul.rn.f32x2")
+#else
+#define DG_P2_OP(NAME, INSN, SCALAR) \
+    DG_HD float2 NAME(float2 a, float2 b) { return p2(SCALAR(a.x, b.x), SCALAR(a.y, b.y)); }
+#endif
+DG_P2_OP(p2_add, "add.rn.f32x2", f_add)
+DG_P2_OP(p2_sub, "sub.rn.f32x2", f_sub)
+DG_P2_OP(p2_mul, "mul.rn.f32x2", f_mul)
 #undef DG_P2_OP
-__device__ __forceinline__ float2 p2_fma(float2 a, float2 b, float2 c) {
+DG_HD float2 p2_fma(float2 a, float2 b, float2 c) {
+#ifdef __CUDA_ARCH__
     float2 d;
     asm("{\n\t.reg .b64 a, b, c, d;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tmov.b64 c, {%6, %7};\n\t"
         "fma.rn.f32x2 d, a, b, c;\n\tmov.b64 {%0, %1}, d;\n\t}"
         : "=f"(d.x), "=f"(d.y)
         : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
     return d;
+#else
+    return p2(f_fma(a.x, b.x, c.x), f_fma(a.y, b.y, c.y));
+#endif
 }
-__device__ __forceinline__ float2 p2_neg(float2 a) { return p2(-a.x, -a.y); }
+DG_HD float2 p2_neg(float2 a) { return p2(-a.x, -a.y); }
 
 // two double-float numbers side by side: the parts of a complex number, or two real sums
 struct __align__(16) pdf {
     float2 h, l;
 };
-__device__ __forceinline__ pdf pdf_fast_two_sum(float2 a, float2 b) {
+DG_HD pdf pdf_fast_two_sum(float2 a, float2 b) {
     const float2 s = p2_add(a, b);
     return {s, p2_sub(b, p2_sub(s, a))};
 }
-__device__ __forceinline__ pdf pdf_two_sum(float2 a, float2 b) {
+DG_HD pdf pdf_two_sum(float2 a, float2 b) {
     const float2 s = p2_add(a, b), bb = p2_sub(s, a);
     return {s, p2_add(p2_sub(a, p2_sub(s, bb)), p2_sub(b, bb))};
 }
-__device__ __forceinline__ pdf pdf_neg(pdf a) { return {p2_neg(a.h), p2_neg(a.l)}; }
-__device__ __forceinline__ pdf pdf_add(pdf a, pdf b) {
+DG_HD pdf pdf_neg(pdf a) { return {p2_neg(a.h), p2_neg(a.l)}; }
+DG_HD pdf pdf_add(pdf a, pdf b) {
     const pdf s = pdf_two_sum(a.h, b.h);
     return pdf_fast_two_sum(s.h, p2_add(s.l, p2_add(a.l, b.l)));
 }
 // df_prod on both halves
-__device__ __forceinline__ float2 pdf_prod(pdf a, pdf b, float2 &e) {
+DG_HD float2 pdf_prod(pdf a, pdf b, float2 &e) {
     const float2 p = p2_mul(a.h, b.h);
     e = p2_fma(a.h, b.h, p2_neg(p));
     e = p2_fma(a.h, b.l, e);
@@ -320,86 +348,86 @@ __device__ __forceinline__ float2 pdf_prod(pdf a, pdf b, float2 &e) {
     return p;
 }
 // df_mul, df_dot2 (a1 b1 + a2 b2), df_fma2 (acc + a1 b1 + a2 b2) and df_fma_lazy on both halves
-__device__ __forceinline__ pdf pdf_mul(pdf a, pdf b) {
+DG_HD pdf pdf_mul(pdf a, pdf b) {
     float2 e;
     const float2 p = pdf_prod(a, b, e);
     return pdf_fast_two_sum(p, e);
 }
-__device__ __forceinline__ pdf pdf_dot2(pdf a1, pdf b1, pdf a2, pdf b2) {
+DG_HD pdf pdf_dot2(pdf a1, pdf b1, pdf a2, pdf b2) {
     float2 e1, e2;
     const float2 x1 = pdf_prod(a1, b1, e1), x2 = pdf_prod(a2, b2, e2);
     const pdf s = pdf_two_sum(x1, x2);
     return pdf_fast_two_sum(s.h, p2_add(s.l, p2_add(e1, e2)));
 }
-__device__ __forceinline__ pdf pdf_fma2(pdf a1, pdf b1, pdf a2, pdf b2, pdf acc) {
+DG_HD pdf pdf_fma2(pdf a1, pdf b1, pdf a2, pdf b2, pdf acc) {
     float2 e1, e2;
     const float2 x1 = pdf_prod(a1, b1, e1), x2 = pdf_prod(a2, b2, e2);
     const pdf s1 = pdf_two_sum(acc.h, x1);
     const pdf s2 = pdf_two_sum(s1.h, x2);
     return pdf_fast_two_sum(s2.h, p2_add(p2_add(s1.l, s2.l), p2_add(acc.l, p2_add(e1, e2))));
 }
-__device__ __forceinline__ pdf pdf_fma_lazy(pdf a, pdf b, pdf acc) {
+DG_HD pdf pdf_fma_lazy(pdf a, pdf b, pdf acc) {
     float2 e;
     const float2 x = pdf_prod(a, b, e);
     const pdf s = pdf_two_sum(acc.h, x);
     return {s.h, p2_add(p2_add(acc.l, e), s.l)};
 }
-__device__ __forceinline__ pdf pdf_both(dfl a) { return {p2(a.h), p2(a.l)}; }
+DG_HD pdf pdf_both(dfl a) { return {p2(a.h), p2(a.l)}; }
 // real part twice, imaginary part twice, and i z = (-im, re)
-__device__ __forceinline__ pdf pdf_re(pdf z) { return {p2(z.h.x), p2(z.l.x)}; }
-__device__ __forceinline__ pdf pdf_im(pdf z) { return {p2(z.h.y), p2(z.l.y)}; }
-__device__ __forceinline__ pdf pdf_i(pdf z) { return {p2(-z.h.y, z.h.x), p2(-z.l.y, z.l.x)}; }
+DG_HD pdf pdf_re(pdf z) { return {p2(z.h.x), p2(z.l.x)}; }
+DG_HD pdf pdf_im(pdf z) { return {p2(z.h.y), p2(z.l.y)}; }
+DG_HD pdf pdf_i(pdf z) { return {p2(-z.h.y, z.h.x), p2(-z.l.y, z.l.x)}; }
 
 struct OpsP {
     typedef pdf C;
     typedef float M;
-    static __device__ __forceinline__ C zero() { return {p2(0.f), p2(0.f)}; }
-    static __device__ __forceinline__ C one() { return {p2(1.f, 0.f), p2(0.f)}; }
-    static __device__ __forceinline__ C from(double2 z) { return mk(df_make(z.x), df_make(z.y)); }
-    static __device__ __forceinline__ double2 to(C z) { return make_double2(df_val(cre(z)), df_val(cim(z))); }
-    static __device__ __forceinline__ C add(C a, C b) { return pdf_add(a, b); }
-    static __device__ __forceinline__ C sub(C a, C b) { return pdf_add(a, pdf_neg(b)); }
-    static __device__ __forceinline__ C neg(C a) { return pdf_neg(a); }
-    static __device__ __forceinline__ C conj(C a) { return {p2(a.h.x, -a.h.y), p2(a.l.x, -a.l.y)}; }
-    static __device__ __forceinline__ C mul(C a, C b) { return pdf_dot2(pdf_re(a), b, pdf_im(a), pdf_i(b)); }
-    static __device__ __forceinline__ C mulc(C a, C b) {  // a conj(b) = b.re a + b.im (-i a)
+    static DG_HD C zero() { return {p2(0.f), p2(0.f)}; }
+    static DG_HD C one() { return {p2(1.f, 0.f), p2(0.f)}; }
+    static DG_HD C from(double2 z) { return mk(df_make(z.x), df_make(z.y)); }
+    static DG_HD double2 to(C z) { return make_double2(df_val(cre(z)), df_val(cim(z))); }
+    static DG_HD C add(C a, C b) { return pdf_add(a, b); }
+    static DG_HD C sub(C a, C b) { return pdf_add(a, pdf_neg(b)); }
+    static DG_HD C neg(C a) { return pdf_neg(a); }
+    static DG_HD C conj(C a) { return {p2(a.h.x, -a.h.y), p2(a.l.x, -a.l.y)}; }
+    static DG_HD C mul(C a, C b) { return pdf_dot2(pdf_re(a), b, pdf_im(a), pdf_i(b)); }
+    static DG_HD C mulc(C a, C b) {  // a conj(b) = b.re a + b.im (-i a)
         return pdf_dot2(a, pdf_re(b), pdf_neg(pdf_i(a)), pdf_im(b));
     }
-    static __device__ __forceinline__ C fma(C a, C b, C acc) { return pdf_fma2(pdf_re(a), b, pdf_im(a), pdf_i(b), acc); }
-    static __device__ __forceinline__ C fms(C a, C b, C acc) {
+    static DG_HD C fma(C a, C b, C acc) { return pdf_fma2(pdf_re(a), b, pdf_im(a), pdf_i(b), acc); }
+    static DG_HD C fms(C a, C b, C acc) {
         return pdf_fma2(pdf_re(a), pdf_neg(b), pdf_im(a), pdf_neg(pdf_i(b)), acc);
     }
-    static __device__ __forceinline__ C rcp(C a) {  // conj(a)/|a|^2
+    static DG_HD C rcp(C a) {  // conj(a)/|a|^2
         return pdf_mul(conj(a), pdf_both(df_rcp(rdotc(a, a))));
     }
-    static __device__ __forceinline__ double re(C a) { return df_val(cre(a)); }
-    static __device__ __forceinline__ double im(C a) { return df_val(cim(a)); }
-    static __device__ __forceinline__ float mag2(C a) { return f_fma(a.h.x, a.h.x, f_mul(a.h.y, a.h.y)); }
+    static DG_HD double re(C a) { return df_val(cre(a)); }
+    static DG_HD double im(C a) { return df_val(cim(a)); }
+    static DG_HD float mag2(C a) { return f_fma(a.h.x, a.h.x, f_mul(a.h.y, a.h.y)); }
     typedef dfl R;
-    static __device__ __forceinline__ R rfrom(double x) { return df_make(x); }
-    static __device__ __forceinline__ R rfma(R a, R b, R acc) { return df_fma(a, b, acc); }
-    static __device__ __forceinline__ R rmul(R a, R b) { return df_mul(a, b); }
-    static __device__ __forceinline__ R radd(R a, R b) { return df_add(a, b); }
-    static __device__ __forceinline__ R rsub(R a, R b) { return df_sub(a, b); }
-    static __device__ __forceinline__ R rneg(R a) { return df_neg(a); }
-    static __device__ __forceinline__ R rrcp(R a) { return df_rcp(a); }
-    static __device__ __forceinline__ C mk(R re, R im) { return {p2(re.h, im.h), p2(re.l, im.l)}; }
-    static __device__ __forceinline__ R cre(C a) { return {a.h.x, a.l.x}; }
-    static __device__ __forceinline__ R cim(C a) { return {a.h.y, a.l.y}; }
+    static DG_HD R rfrom(double x) { return df_make(x); }
+    static DG_HD R rfma(R a, R b, R acc) { return df_fma(a, b, acc); }
+    static DG_HD R rmul(R a, R b) { return df_mul(a, b); }
+    static DG_HD R radd(R a, R b) { return df_add(a, b); }
+    static DG_HD R rsub(R a, R b) { return df_sub(a, b); }
+    static DG_HD R rneg(R a) { return df_neg(a); }
+    static DG_HD R rrcp(R a) { return df_rcp(a); }
+    static DG_HD C mk(R re, R im) { return {p2(re.h, im.h), p2(re.l, im.l)}; }
+    static DG_HD R cre(C a) { return {a.h.x, a.l.x}; }
+    static DG_HD R cim(C a) { return {a.h.y, a.l.y}; }
     // two lazy real sums with a common second factor: acc + (wx, wy) p
-    static __device__ __forceinline__ C pacc(C w, R p, C acc) { return pdf_fma_lazy(w, pdf_both(p), acc); }
-    static __device__ __forceinline__ C pnorm(C a) { return pdf_fast_two_sum(a.h, a.l); }
-    static __device__ __forceinline__ C pscale(C a, R r) { return pdf_mul(a, pdf_both(r)); }
-    static __device__ __forceinline__ C times_i(C a) { return pdf_i(a); }
-    static __device__ __forceinline__ C det2(C a, C b, C c, C d) { return fms(b, c, mul(a, d)); }
+    static DG_HD C pacc(C w, R p, C acc) { return pdf_fma_lazy(w, pdf_both(p), acc); }
+    static DG_HD C pnorm(C a) { return pdf_fast_two_sum(a.h, a.l); }
+    static DG_HD C pscale(C a, R r) { return pdf_mul(a, pdf_both(r)); }
+    static DG_HD C times_i(C a) { return pdf_i(a); }
+    static DG_HD C det2(C a, C b, C c, C d) { return fms(b, c, mul(a, d)); }
     // num and den by the power of two that takes |den| to about 1, so that |den|^2 stays in the FP32 range
-    static __device__ __forceinline__ void balance(C &num, C &den) {
+    static DG_HD void balance(C &num, C &den) {
         const float mx = fmaxf(fabsf(den.h.x), fabsf(den.h.y));
-        const float2 sc = p2(__int_as_float((254 << 23) - (__float_as_int(mx) & 0x7f800000)));
+        const float2 sc = p2(float_of((254 << 23) - (bits_of(mx) & 0x7f800000)));
         num = {p2_mul(num.h, sc), p2_mul(num.l, sc)};
         den = {p2_mul(den.h, sc), p2_mul(den.l, sc)};
     }
-    static __device__ __forceinline__ R rdotc(C a, C b) {  // Re(a conj b)
+    static DG_HD R rdotc(C a, C b) {  // Re(a conj b)
         float2 e;
         const float2 p = pdf_prod(a, b, e);
         const dfl s = two_sum(p.x, p.y);

@@ -19,8 +19,12 @@ DG_HD dfl df_div(dfl a, dfl b) {
 
 // a^-1/2, a > 0: the approximate root refined in FP32, then one double-float step on its residual e = 1 - a y^2,
 // y (1 + e/2 + 3/8 e^2)
-__device__ __forceinline__ dfl df_rsqrt(dfl a) {
+DG_HD dfl df_rsqrt(dfl a) {
+#ifdef __CUDA_ARCH__
     float y = rsqrtf(a.h);
+#else
+    float y = 1.f / sqrtf(a.h);
+#endif
     y = fmaf(0.5f * y, fmaf(-a.h * y, y, 1.f), y);
     const dfl y2 = df_mul({y, 0.f}, {y, 0.f});
     const dfl e = df_sub({1.f, 0.f}, df_mul(a, y2));

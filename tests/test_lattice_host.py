@@ -54,3 +54,47 @@ def test_two_by_two_inverse(harness):
         v = np.array([float.fromhex(x) for x in r[1:]])
         X, exact = (v[0::2] + 1j * v[1::2]).reshape(2, 2), np.linalg.inv(M)
         assert r[0] == "0" and np.abs(X - exact).max() <= 16 * 2.0 ** -53 * np.linalg.cond(M) * np.abs(exact).max()
+
+
+def _split(x):
+    h = float(np.float32(x))
+    return h, float(np.float32(x - h))
+
+
+def test_packed_arithmetic_has_the_scalar_bits(harness):
+    """OpsP, which the lattice and eigensolver kernels compute in, against OpsF, whose operations are held to exact rational
+    arithmetic: the same bits."""
+    rng = np.random.default_rng(9)
+    lines = []
+    for _ in range(500):
+        d = [_split(float(x)) for x in np.exp(rng.uniform(-8, 8, 6)) * rng.choice([-1, 1], 6)]
+        lines.append("pack %s\n" % " ".join(x.hex() for hl in d for x in hl))
+    assert all(r == ["0"] * 6 for r in harness(lines))
+
+
+@pytest.mark.parametrize("n", [2, 3])
+def test_packed_inverse(harness, n):
+    """The 2 x 2 closed form and the 3 x 3 elimination of the thread-per-frequency kernels in packed double-float: z - H - Sigma
+    over the energies a determinant in FP32's range allows, and rows in other orders; within 2^-44 of the entries' scale
+    times the condition, as the scalar form is held to."""
+    rng = np.random.default_rng(n)
+    mats = []
+    for t in range(300):
+        H = rng.normal(size=(n, n)) + 1j * rng.normal(size=(n, n))
+        M = (0.3 + 1j * np.exp(rng.uniform(-3, 2))) * np.eye(n) - (H + H.conj().T) / 2
+        M = M[rng.permutation(n)] * 10.0 ** rng.integers(-8, 9)
+        mats.append(np.array([complex(sum(_split(z.real)), sum(_split(z.imag))) for z in M.ravel()]).reshape(n, n))
+    for M, r in zip(mats, harness([_line("inv%dp" % n, M) for M in mats])):
+        v = np.array([float.fromhex(x) for x in r[1:]])
+        X, exact = (v[0::2] + 1j * v[1::2]).reshape(n, n), np.linalg.inv(M)
+        assert r[0] == "0" and np.abs(X - exact).max() <= 2.0 ** -44 * np.linalg.cond(M) * np.abs(exact).max()
+
+
+def test_reciprocal_root(harness):
+    from decimal import Decimal as Dc, getcontext
+    getcontext().prec = 50
+    rng = np.random.default_rng(6)
+    xs = [_split(float(x)) for x in np.exp(rng.uniform(-20, 20, 300))]
+    for x, r in zip(xs, harness(["rsqrt %s %s\n" % (a.hex(), b.hex()) for a, b in xs])):
+        exact = 1 / (Dc(x[0]) + Dc(x[1])).sqrt()
+        assert abs(Dc(float.fromhex(r[0])) + Dc(float.fromhex(r[1])) - exact) <= Dc(2.0 ** -44) * exact
