@@ -1,5 +1,5 @@
 // adjoint.cuh -- reverse- and forward-mode derivatives of the lattice sum G_loc(iw) = (1/N_k) sum_k G_PP(k, iw)
-// with respect to the self-energy and the chemical potential, k_gloc_ad<DP, W, MODE>.
+// with respect to the self-energy and the chemical potential, k_gloc_ad<LW, MODE> (LW lanes per matrix).
 //
 // With G = (z - H - Sigma)^-1 on the full orbital space and Sigma acting on the correlated block P:
 //   dG_PP = G_PP dSigma G_PP                      (dSigma lives on P, so only the P block of G enters)

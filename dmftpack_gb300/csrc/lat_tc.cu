@@ -242,7 +242,8 @@ __device__ __forceinline__ dfl re_val(pdf acc) {
     return df_sub({acc.h.x, acc.l.x}, {acc.h.y, acc.l.y});
 }
 
-// 16 columns of the four accumulators (levels 2, 3, 4, >= 5) of this thread's TMEM lane, one wait for all
+// 16 columns of the first four accumulators (levels 0, 1, 2 and, with five slices, 3 and up) of this thread's TMEM lane, one wait
+// for all
 __device__ __forceinline__ void tmem_ld16x4(uint32_t addr, uint32_t stride, uint32_t (&v)[4][16]) {
 #pragma unroll
     for (int i = 0; i < 4; i++)

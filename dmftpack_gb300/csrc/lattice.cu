@@ -458,12 +458,11 @@ int prepare_real(dmftgpu_ctx *ctx, const dmftgpu_lattice *L, const double2 *dH, 
     return DMFTGPU_OK;
 }
 
-// df (the DMFTGPU_MIXED passes): the per-k eigendecompositions (n <= 32) in double-float on the FP32 pipe, and the
-// static one on the main stream after the Schur data instead of on the side stream (the mixed lattice kernels fill
-// the SMs; an eigendecomposition beside them slows them by more than it takes alone).
+// df (the DMFTGPU_MIXED passes): the per-k eigendecompositions (n <= 32) in double-float on the FP32 pipe.  In both
+// precisions the static one runs on the side stream: whoever reads eps, UP or Uf waits for static_ready first.
 // derivs (dmftgpu_gloc_vjp / _jvp): only the Schur data and Sigma(iw_n), n < N_freq, enter the derivatives of G_loc;
-// the tail moments, the 2 N_freq table and the static spectrum (10.5 ms of a 5^3 k call of the 56-orbital model, in
-// front of a 60-70 ms derivative kernel) are left out.
+// the tail moments, the 2 N_freq table and the static spectrum (10.5 ms of a 5^3 k call of the 56-orbital model when they
+// were dropped, whose derivative kernel takes some 20) are left out.
 int prepare(dmftgpu_ctx *ctx, const dmftgpu_lattice *L, const double2 *dH, const double2 *dS, int mask, Prepared &P,
             bool vectors = false, bool df = false, bool derivs = false) {
     P.n = L->n;

@@ -116,16 +116,6 @@ __host__ __device__ inline int thread_gj_inverse(int n, double2 *a, int *perm) {
     return st;
 }
 
-// C = A * B   (all n x n, distinct buffers)
-__host__ __device__ inline void thread_matmul(int n, const double2 *A, const double2 *B, double2 *C) {
-    for (int j = 0; j < n; j++)
-        for (int i = 0; i < n; i++) {
-            double2 s = cmk(0, 0);
-            for (int k = 0; k < n; k++) s = cfma(DG_AT(A, n, i, k), DG_AT(B, n, k, j), s);
-            DG_AT(C, n, i, j) = s;
-        }
-}
-
 // Hermitian eigen-decomposition from the lower triangle of A0 (A0 untouched).  a, u: n x n scratch;
 // w: n eigenvalues ascending; if u == nullptr only eigenvalues are produced (a still needed).
 // Cyclic Jacobi: the rotation G = [[c, s], [-s conj(u), c conj(u)]] zeroes the (p,q) element of G^H A G.

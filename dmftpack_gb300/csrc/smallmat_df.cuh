@@ -1,4 +1,5 @@
-// smallmat_df.cuh -- square roots and a division in double-float, for the rotations of the double-float eigensolver (eig.cuh).
+// smallmat_df.cuh -- the reciprocal square root in double-float, for the rotations of the double-float eigensolver (eig.cuh), and
+// the square root and division its host tests are written against.
 #pragma once
 #include "df.cuh"
 
