@@ -41,7 +41,8 @@
 // in registers).
 // On the d + p model (n = 28, D = 10, 1,000 k x 2,048 frequencies; 512 k for the search for mu) G_loc took 66.8 ms end to
 // end by k_schur, 30.2 with the complex entries formed and H_PP added in the drain and the shared levels of G_loc in a
-// fifth sum passed through shared memory, and takes 25.7; the search 119.8 (derivatives by k_schur), 69.6, and 60.8.
+// fifth sum passed through shared memory, and 25.7 without; the search 119.8 (derivatives by k_schur), 69.6, and 60.8.  They
+// take 20.8 and 56.7 now, by the eigensolver, the k chunks and the carve-out.
 // The producers were the longer chain then (38,000 cycles per k of which 19,000 the drain, 7,000 the MMAs issued by a
 // rolled loop); now it is the inversions: 36,000 cycles per k and CTA, of which the FP32 pipe is busy 24,000.  Without the
 // producers' work the pass takes as long; searching the next pivot and forming its reciprocal beside the update, or

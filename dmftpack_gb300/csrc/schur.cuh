@@ -455,8 +455,8 @@ __device__ __forceinline__ void tpi_stage(const SchurArgs &g, int k0, int nkc, t
 // Bound by the packed double-float arithmetic and its latency: at D = 3 the k sums of G and G0 and Sigma - m0 (27
 // complex numbers) would take the kernel to 250 registers and two CTAs per SM, so they live in shared memory
 // (`tpi_shared`), one column per thread, and three CTAs fit:
-// the headline pass (24^3 k, 8192 points) takes 25.5 ms against 26.2 ms with all of it in registers and 31.2 ms with
-// scalar double-float instructions.
+// the headline kernel (24^3 k, 8192 points) takes 22.2 ms; when the forms were compared, in fewer and longer k chunks, 25.5 ms
+// against 26.2 with all of it in registers and 31.2 with scalar double-float instructions.
 template <class Ops, int D>
 constexpr bool tpi_shared = std::is_same<Ops, OpsP>::value && D == 3;
 template <class Ops, int D>
