@@ -55,29 +55,39 @@ __device__ __forceinline__ void atomic_add_c(double2 *p, double2 v) {
     atomicAdd(&p->y, v.y);
 }
 
-// Sum of at(0) + .. + at(n - 1) in a fixed order: eight running sums over 64 terms, added as a tree, then the next 64.  As many
-// additions as one running sum, whose rounding errors grow with the root of n when the terms are alike (k chunks of a lattice
-// sum: G_loc in FP64 at 1,200 k in 150 chunks 3.5e-16 off by one running sum, 1.6e-16 in 19 longer chunks).
+// Sum of at(0) + .. + at(n - 1) in a fixed order: up to 16 terms one after the other, else eight running sums over 64 terms,
+// added as a tree, then the next 64.  n - 1 additions like one running sum, whose rounding errors grow with the root of n when
+// the terms are alike (k chunks of a lattice sum: G_loc in FP64 at 1,200 k in 150 chunks 3.5e-16 off by one running sum,
+// 1.6e-16 in 19 longer chunks).
 template <class F>
 __device__ __forceinline__ double2 chunk_sum(int n, F at) {
-    double2 total = cmk(0, 0);
+    double2 total = at(0);
+    if (n <= 16) {
+#pragma unroll 4
+        for (int q = 1; q < n; q++) total = cadd(total, at(q));
+        return total;
+    }
     for (int q0 = 0; q0 < n; q0 += 64) {
-        double2 a[8];
-#pragma unroll
-        for (int j = 0; j < 8; j++) a[j] = cmk(0, 0);
         const int end = min(n, q0 + 64);
+        double2 s;
         int q = q0;
-        for (; q + 8 <= end; q += 8)
+        if (end - q0 >= 8) {
+            double2 a[8];
 #pragma unroll
-            for (int j = 0; j < 8; j++) a[j] = cadd(a[j], at(q + j));
+            for (int j = 0; j < 8; j++) a[j] = at(q0 + j);
+            for (q = q0 + 8; q + 8 <= end; q += 8)
 #pragma unroll
-        for (int j = 0; j < 7; j++)
-            if (q + j < end) a[j] = cadd(a[j], at(q + j));
+                for (int j = 0; j < 8; j++) a[j] = cadd(a[j], at(q + j));
 #pragma unroll
-        for (int h = 4; h > 0; h >>= 1)
+            for (int h = 4; h > 0; h >>= 1)
 #pragma unroll
-            for (int j = 0; j < h; j++) a[j] = cadd(a[j], a[j + h]);
-        total = cadd(total, a[0]);
+                for (int j = 0; j < h; j++) a[j] = cadd(a[j], a[j + h]);
+            s = a[0];
+        } else {
+            s = at(q++);
+        }
+        for (; q < end; q++) s = cadd(s, at(q));
+        total = q0 ? cadd(total, s) : s;
     }
     return total;
 }
